@@ -52,7 +52,7 @@ def listed():
         dict(name="sampled_z3_s23", kind="sampled", graph="kron", n=1 << 23, z=3, nbfs=128, W=32, H=0,
              bader_c=0, nchecks=1),
         # the mesh configuration: 2048^2 grid, dependency-weighted sampling with
-        # Bader's stop: about 4000 narrow levels each way
+        # Bader's stop: hundreds of narrow levels each way
         dict(name="sampled_z4_grid2048", kind="sampled", graph="grid", n=2048 * 2048, z=4, nbfs=2048, W=64, H=0,
              bader_c=1, nchecks=8),
         # many pivots on a mesh (road-network-like): wide pass, many levels
