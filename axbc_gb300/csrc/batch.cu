@@ -45,41 +45,6 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
     return (unsigned long long)lo | ((unsigned long long)hi << 32);
 }
 
-// A warp stages the masks of a 32-position chunk in shared memory as K
-// arrays of 32 words, one per 32-bit half (sg + 32 h), so that a half's
-// consumer holds 32-bit words only.
-template <int K> __device__ __forceinline__ typename MaskOf<K>::T staged_mask(const uint32_t *sg, int i)
-{
-    typedef typename MaskOf<K>::T M;
-    if (K == 1) return (M)sg[i];
-    return (M)((unsigned long long)sg[i] | ((unsigned long long)sg[32 + i] << 32));
-}
-
-// Stage the chunk's positions that have a parent (act: their lanes),
-// compacted to slots 0..nh-1 in position order, and zero masks in slots
-// nh..31, so that the consumer walks ceil(nh / 8) groups of 8 instead of every
-// group holding a hit.  Returns nh.
-template <int K, class M>
-__device__ __forceinline__ int stage_compact(uint32_t *su, uint32_t *sg, uint32_t *sk, unsigned act, uint32_t v,
-                                             M fm, uint32_t k)
-{
-    const unsigned lane = lane_id();
-    const int nh = __popc(act);
-    if (fm) {
-        const int pos = __popc(act & ((1u << lane) - 1u));
-        su[pos] = v;
-        sg[pos] = (uint32_t)fm;
-        if (K == 2) sg[32 + pos] = (uint32_t)((unsigned long long)fm >> 32);
-        if (sk) sk[pos] = k;
-    }
-    if ((int)lane >= nh) {
-        su[lane] = 0;
-        sg[lane] = 0;
-        if (K == 2) sg[32 + lane] = 0;
-    }
-    return nh;
-}
-
 // eight staged words of group g (16-byte shared loads)
 __device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
 {
@@ -91,7 +56,7 @@ __device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
 // resident blocks per SM the kernels are compiled for (their register
 // budgets); the backward runs 32 pivots at a time at either width
 #ifndef AXBC_PULL_MIN_BLOCKS
-#define AXBC_PULL_MIN_BLOCKS 6
+#define AXBC_PULL_MIN_BLOCKS 7
 #endif
 #ifndef AXBC_BWD_MIN_BLOCKS
 #define AXBC_BWD_MIN_BLOCKS 8
@@ -114,7 +79,7 @@ struct LevelLists {
     uint32_t *start;  // per level: offset into pool
     uint32_t *count;  // per level: vertices appended
     uint32_t *cap;    // per level: capacity
-    uint32_t *heavy;  // per level: listed vertices with more than AXBC_SPAN neighbours
+    uint32_t *heavy;  // per level: listed vertices with more than AXBC_BIG neighbours
 };
 
 
@@ -216,7 +181,7 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         const uint32_t firsts = __ballot_sync(FULL_MASK, first);
         if (first) ll.pool[nroots + __popc(firsts & ((1u << l) - 1u))] = rt;
         nroots += __popc(firsts);
-        heavy_roots += __popc(__ballot_sync(FULL_MASK, first && col[rt + 1] - col[rt] > AXBC_SPAN));
+        heavy_roots += __popc(__ballot_sync(FULL_MASK, first && col[rt + 1] - col[rt] > AXBC_BIG));
     }
     for (int o = 16; o; o >>= 1) {
         fd += __shfl_xor_sync(FULL_MASK, fd, o);
@@ -247,7 +212,7 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
 // items of heavy vertices (largest first), the remaining units cover four
 // light tasks each (light tasks: degree-ordered groups of <= 32 vertices with
 // about one span of adjacency).
-#define LIGHT_PER_UNIT 4
+#define LIGHT_PER_UNIT 1
 
 __device__ __forceinline__ uint32_t grab_unit(uint32_t *ctr)
 {
@@ -289,6 +254,21 @@ __device__ __forceinline__ uint32_t list_unit(uint32_t lcnt)
 {
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     return max(1u, min(32u, lcnt / nwarps));
+}
+
+// Items per work unit of the forward kernels: at least `least`, and as many as
+// leave every resident warp about four units (at most 32, one per lane).
+__device__ __forceinline__ uint32_t unit_of(uint64_t items, uint32_t least)
+{
+    const uint64_t nwarps = gridDim.x * (blockDim.x / 32);
+    return (uint32_t)max((uint64_t)least, min((uint64_t)32, items / (4 * nwarps)));
+}
+// A warp's first unit is its own number; further ones come from the counter,
+// which nobody touches when there are no more units than warps.
+__device__ __forceinline__ uint64_t next_unit(uint32_t *ctr, uint64_t nu)
+{
+    const uint64_t nwarps = gridDim.x * (blockDim.x / 32);
+    return nu <= nwarps ? nu : nwarps + grab_unit(ctr);
 }
 
 // the stored list of level L, or nullptr when the level overflowed its capacity
@@ -435,221 +415,237 @@ __device__ __forceinline__ void fwd_push_body(const Adj &a, const typename MaskO
     const unsigned lane = lane_id();
     uint32_t lcnt = 0;
     const uint32_t *lst = level_list(ll, L - 1, lcnt);  // the frontier, when stored
-    // heavy span items only when a heavy vertex is in the frontier
-    const uint64_t nhi = lst && ll.heavy[L - 1] == 0 ? 0 : a.n_heavy_items;
-    const uint32_t ent = list_unit(lcnt);
-    const uint64_t nu = lst ? nhi + (lcnt + ent - 1) / ent : n_units(a);
-    if (warp_global() >= nu) return;  // fewer units than warps: no contention
-    for (;;) {
-        const uint32_t t = grab_unit(ctr);
-        if (t >= nu) break;
-        if (t < nhi) {
-            const uint32_t v = a.hitem_v[t];
-            const M f = fprev[v];
-            if (lane == 0) wc.add(WC_BYTES, 4 * K);
-            if (!f) continue;
-            const uint32_t b0 = a.col[v] + a.hitem_k[t] * AXBC_SPAN;
-            push_span<K>(a, v, f, b0, min(a.col[v + 1], b0 + AXBC_SPAN), seen, fcur, msigma, ll, L, wc);
+    // parts of big vertices only when one is in the frontier
+    const uint64_t np = lst && ll.heavy[L - 1] == 0 ? 0 : a.n_part;
+    const uint64_t nl = lst ? lcnt : a.n_linked - a.n_big;
+    const uint32_t gp = unit_of(np, 1), ent = unit_of(nl, 1);
+    const uint64_t up = (np + gp - 1) / gp, nu = up + (nl + ent - 1) / ent;
+    for (uint64_t t = warp_global(); t < nu; t = next_unit(ctr, nu)) {
+        if (t < up) {
+            // a unit of parts: one lane looks each part's frontier mask up
+            const uint64_t i = lane * up + t;  // a hub's parts fall into different units
+            uint2 pt = make_uint2(0, 0);
+            M f_l = 0;
+            if (lane < gp && i < np) {
+                pt = a.part[i];
+                f_l = fprev[pt.x];
+                wc.add(WC_BYTES, 4 * K);
+            }
+            for (unsigned act = __ballot_sync(FULL_MASK, f_l != 0); act; act &= act - 1) {
+                const int j = __ffs(act) - 1;
+                const uint32_t v = __shfl_sync(FULL_MASK, pt.x, j);
+                const uint32_t b0 = a.col[v] + __shfl_sync(FULL_MASK, pt.y, j) * a.part_len;
+                push_span<K>(a, v, __shfl_sync(FULL_MASK, f_l, j), b0, min(a.col[v + 1], b0 + a.part_len), seen, fcur,
+                             msigma, ll, L, wc);
+            }
             continue;
         }
-        if (lst) {
-            const uint32_t i = (uint32_t)(t - nhi) * ent + lane;
-            uint32_t v_l = 0;
-            M f_l = 0;
-            if (lane < ent && i < lcnt) {
-                v_l = lst[i];
-                if (a.col[v_l + 1] - a.col[v_l] <= AXBC_SPAN) f_l = fprev[v_l];
-                wc.add(WC_BYTES, 4 + 4 * K);  // list entry, level mask
-            }
-            push_light32<K>(a, v_l, f_l, seen, fcur, msigma, ll, L, wc);
-            continue;
+        const uint64_t i = (t - up) * ent + lane;
+        uint32_t v_l = 0;
+        M f_l = 0;
+        if (lane < ent && i < nl) {
+            v_l = lst ? lst[i] : a.order[a.n_big + i];
+            if (a.col[v_l + 1] - a.col[v_l] <= AXBC_BIG) f_l = fprev[v_l];
+            wc.add(WC_BYTES, lst ? 4 + 4 * K : 4 * K);  // list entry, level mask
         }
-        const uint64_t l0 = (uint64_t)(t - nhi) * LIGHT_PER_UNIT;
-        for (uint64_t lt = l0; lt < l0 + LIGHT_PER_UNIT && lt < a.n_ltask; lt++) {
-            const uint32_t beg = a.ltask[lt], cnt = a.ltask[lt + 1] - beg;
-            uint32_t v_l = 0;
-            M f_l = 0;
-            if (lane < cnt) {
-                v_l = a.order[beg + lane];
-                f_l = fprev[v_l];
-                wc.add(WC_BYTES, 4 * K);  // level mask
-            }
-            push_light32<K>(a, v_l, f_l, seen, fcur, msigma, ll, L, wc);
-        }
+        push_light32<K>(a, v_l, f_l, seen, fcur, msigma, ll, L, wc);
     }
 }
 
-// Forward level L, pull into vertex u for the pivots `ns` that have not seen
-// it: sum sigma_s over every in-neighbour at depth L-1 from pivot s (u32 sums:
-// any order gives the same bits).  The positions of a 32-wide chunk that have
-// a parent are staged in shared memory, compacted; each group of 8 issues its
-// gathers (8 per half) before any is consumed.
+// Forward level L, pull: every vertex u that some pivots (`ns`) have not seen
+// sums sigma_s over its in-neighbours at depth L-1 from pivot s (u32 sums: any
+// order gives the same bits).  Bound by instruction issue, not by memory, so
+// the gathers are laid out for few instructions: a lane owns four neighbouring
+// pivots (one 16-byte load per parent row), 8 K lanes -- a subgroup -- cover a
+// row, and the warp's 4 / K subgroups gather that many parents at once.  The
+// positions with a parent are staged in shared memory as (parent, mask) pairs,
+// one array per 32-pivot half, compacted.
+template <int K> struct PullShape {
+    static constexpr int SUB = 8 * K;       // lanes that cover one row
+    static constexpr int NSUB = 32 / SUB;   // rows gathered at once
+    // staged pairs of one warp: slot i of half h at 37 h + i + i / 8, so that
+    // the subgroups' simultaneous reads fall into different banks
+    static constexpr int STAGE = K == 1 ? 36 : 74;
+};
+__device__ __forceinline__ int stage_at(int i) { return i + (i >> 3); }
+
+template <int K>
+__device__ __forceinline__ void stage_pair(uint2 *st, int slot, uint32_t v, typename MaskOf<K>::T m)
+{
+    st[stage_at(slot)] = make_uint2(v, (uint32_t)m);
+    if (K == 2) st[37 + stage_at(slot)] = make_uint2(v, (uint32_t)((unsigned long long)m >> 32));
+}
+
+// Add the rows staged in slots first, first + stride, ... (cnt of them, the
+// slots after them hold empty masks) into the lane's four sums; fo collects
+// the lane's found pivots.  st_h: the stage of the lane's half.
+template <int K>
+__device__ __forceinline__ void pull_rows(const uint2 *st_h, int first, int stride, int cnt,
+                                          const uint32_t *__restrict__ msig_l, unsigned sh, uint32_t acc[4],
+                                          uint32_t &fo)
+{
+#pragma unroll 1
+    for (int i = 0; i < cnt; i += 2) {
+        const int s0 = first + i * stride, s1 = s0 + stride;
+        const uint2 e0 = st_h[stage_at(s0)], e1 = st_h[stage_at(s1)];
+        const uint32_t n0 = (e0.y >> sh) & 15u, n1 = (e1.y >> sh) & 15u;
+        uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+        if (n0) x0 = *reinterpret_cast<const uint4 *>(msig_l + row_base<K>(e0.x));
+        if (n1) x1 = *reinterpret_cast<const uint4 *>(msig_l + row_base<K>(e1.x));
+        if (n0 & 1u) acc[0] += x0.x;
+        if (n0 & 2u) acc[1] += x0.y;
+        if (n0 & 4u) acc[2] += x0.z;
+        if (n0 & 8u) acc[3] += x0.w;
+        if (n1 & 1u) acc[0] += x1.x;
+        if (n1 & 2u) acc[1] += x1.y;
+        if (n1 & 4u) acc[2] += x1.z;
+        if (n1 & 8u) acc[3] += x1.w;
+        fo |= n0 | n1;
+    }
+}
+
+// One part [b0, b1) of a big vertex's in-adjacency: all subgroups share it,
+// slot i of a chunk's staged pairs going to subgroup i mod NSUB.  Adjacency
+// entries load two chunks ahead and level masks one ahead.
 template <int K, class WC>
-__device__ __forceinline__ typename MaskOf<K>::T pull_span(const Adj &rv, typename MaskOf<K>::T ns, uint32_t b0,
-                                                           uint32_t b1,
-                                                           const typename MaskOf<K>::T *__restrict__ fprev,
-                                                           const uint32_t *__restrict__ msigma, uint32_t *su,
-                                                           uint32_t *sg, uint32_t acc[K], WC &wc)
+__device__ __forceinline__ void pull_part(const Adj &rv, uint32_t u, typename MaskOf<K>::T ns, uint32_t b0,
+                                          uint32_t b1, const typename MaskOf<K>::T *__restrict__ fprev,
+                                          typename MaskOf<K>::T *fcur, uint32_t *msigma, uint2 *st,
+                                          const LevelLists &ll, int L, WC &wc)
 {
     typedef typename MaskOf<K>::T M;
+    typedef PullShape<K> S;
     const unsigned lane = lane_id();
-    M found = 0;
-#pragma unroll
-    for (int h = 0; h < K; h++) acc[h] = 0;
-    // the next chunk's adjacency entries load while this chunk is consumed
-    uint32_t vn = b0 + lane < b1 ? rv.row[b0 + lane] : 0u;
-    for (uint32_t base = b0; base < b1; base += 32) {
-        const uint32_t e = base + lane;
-        const uint32_t v = vn;
-        vn = e + 32 < b1 ? rv.row[e + 32] : 0u;
-        const M fm = e < b1 ? fprev[v] & ns : (M)0;
+    const int sl = lane & (S::SUB - 1), g = lane / S::SUB;
+    const unsigned sh = 4 * (sl & 7);
+    const uint2 *st_h = st + (K == 2 && sl >= 8 ? 37 : 0);
+    uint32_t acc[4] = {0, 0, 0, 0}, fo = 0;
+    uint32_t e = b0 + lane;
+    uint32_t v = e < b1 ? rv.row[e] : 0u, vn = e + 32 < b1 ? rv.row[e + 32] : 0u;
+    M fm = e < b1 ? fprev[v] & ns : (M)0;
+    for (; e - lane < b1; e += 32) {
         if (e < b1) {
             wc.add(WC_ENTRIES, 1);
             wc.add(WC_GATHERS, __popcll((unsigned long long)fm));
             wc.add(WC_BYTES, 4 + 4 * K + 4 * __popcll((unsigned long long)fm));  // entry, mask, parents' counts
         }
         const unsigned act = __ballot_sync(FULL_MASK, fm != 0);
-        if (!act) continue;
-        found |= warp_or(fm);
-        const int nh = stage_compact<K>(su, sg, (uint32_t *)nullptr, act, v, fm, 0u);
-        __syncwarp();
-#pragma unroll 1
-        for (int g = 0; 8 * g < nh; g++) {
-            uint32_t u[8];
-            load8u(su, g, u);
-#pragma unroll
-            for (int h = 0; h < K; h++) {
-                uint32_t m[8], x[8];
-                load8u(sg + 32 * h, g, m);
-#pragma unroll
-                for (int q = 0; q < 8; q++)
-                    x[q] = ((m[q] >> lane) & 1u) ? msigma[row_base<K>(u[q]) + 32 * h + lane] : 0u;
-#pragma unroll
-                for (int q = 0; q < 8; q++) acc[h] += x[q];
-            }
+        const int nh = __popc(act);
+        if (nh) {
+            if (fm) stage_pair<K>(st, __popc(act & ((1u << lane) - 1u)), v, fm);
+            if ((int)lane >= nh) stage_pair<K>(st, lane, 0u, (M)0);
         }
+        v = vn;
+        vn = e + 64 < b1 ? rv.row[e + 64] : 0u;
+        fm = e + 32 < b1 ? fprev[v] & ns : (M)0;
+        if (!nh) continue;
+        __syncwarp();
+        pull_rows<K>(st_h, g, S::NSUB, (nh + S::NSUB - 1) / S::NSUB, msigma + 4 * sl, sh, acc, fo);
         __syncwarp();
     }
-    return found;
+#pragma unroll
+    for (int o = S::SUB; o < 32; o <<= 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[q] += __shfl_xor_sync(FULL_MASK, acc[q], o);
+        fo |= __shfl_xor_sync(FULL_MASK, fo, o);
+    }
+    // the other parts of u add into the same row; subgroup g adds pivots g,
+    // g + NSUB, ... of each lane's four
+    uint32_t *r = msigma + row_base<K>(u) + 4 * sl;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if ((q & (S::NSUB - 1)) == g && ((fo >> q) & 1u)) {
+            atomicAdd(r + q, acc[q]);
+            wc.add(WC_PAIRS, 1);
+            wc.add(WC_BYTES, 4);
+        }
+    M nm = (M)__reduce_or_sync(FULL_MASK, sl < 8 ? fo << sh : 0u);
+    if (K == 2) nm |= (M)((unsigned long long)__reduce_or_sync(FULL_MASK, sl < 8 ? 0u : fo << sh) << 32);
+    bool first = false;
+    if (lane == 0 && nm) {
+        first = atomicOr(&fcur[u], nm) == 0;
+        wc.add(WC_BYTES, first ? 4 + 4 * K : 4 * K);  // level mask, list entry
+    }
+    list_append(ll, L, first, u);
 }
 
-// Pull into up to 32 light vertices at once, one per lane (pivots ns_l; 0:
-// none), edge-parallel over the concatenation of their in-adjacency lists:
-// lane e finds its vertex by a binary search over the inclusive degree prefix
-// held across the lanes.  Positions arrive grouped by vertex (compaction keeps
-// their order), so one running sum per lane (pivot) is written out whenever
-// the vertex changes.  Returns the discovered mask of the lane's own vertex.
+// Up to 32 vertices of at most AXBC_BIG in-neighbours, one per lane (pivots
+// ns_l; 0: none).  Each subgroup takes one of them at a time: its lanes read
+// 8 K positions per step and then gather the rows of those with a parent.
 template <int K, class WC>
-__device__ __forceinline__ typename MaskOf<K>::T pull_light32(const Adj &rv, uint32_t u_l,
-                                                              typename MaskOf<K>::T ns_l,
-                                                              const typename MaskOf<K>::T *__restrict__ fprev,
-                                                              uint32_t *msigma, uint32_t *su,
-                                                              uint32_t *sg, uint32_t *sk, WC &wc)
+__device__ __forceinline__ void pull_small(const Adj &rv, uint32_t u_l, typename MaskOf<K>::T ns_l,
+                                           const typename MaskOf<K>::T *__restrict__ fprev,
+                                           typename MaskOf<K>::T *fcur, uint32_t *msigma, uint2 *st,
+                                           const LevelLists &ll, int L, WC &wc)
 {
     typedef typename MaskOf<K>::T M;
+    typedef PullShape<K> S;
     const unsigned lane = lane_id();
-    uint32_t b = 0, d = 0;
+    const int sl = lane & (S::SUB - 1), g = lane / S::SUB;
+    const unsigned sh = 4 * (sl & 7);
+    const uint2 *st_h = st + (K == 2 && sl >= 8 ? 37 : 0);
+    uint32_t b_l = 0, d_l = 0;
     if (ns_l) {
-        b = rv.col[u_l];
-        d = rv.col[u_l + 1] - b;
+        b_l = rv.col[u_l];
+        d_l = rv.col[u_l + 1] - b_l;
         wc.add(WC_BYTES, 8);  // adjacency bounds
     }
-    uint32_t inc = d;
+    for (unsigned act = __ballot_sync(FULL_MASK, d_l != 0); act;) {
+        // the next NSUB vertices, one per subgroup
+        int j = -1;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(FULL_MASK, inc, o);
-        if ((int)lane >= o) inc += t;
-    }
-    const uint32_t total = __shfl_sync(FULL_MASK, inc, 31);
-    const uint32_t shift = b - (inc - d);  // position of concatenated index e: shift_k + e
-    M mine = 0, fo = 0;
-    uint32_t acc[K];
-#pragma unroll
-    for (int h = 0; h < K; h++) acc[h] = 0;
-    int cur = -1;
-    // the finished running sums of vertex `cur` go to its row
-    auto flush = [&]() {
-        const uint32_t uc = __shfl_sync(FULL_MASK, u_l, cur);
-#pragma unroll
-        for (int h = 0; h < K; h++)
-            if (pbit(fo, h)) msigma[row_base<K>(uc) + 32 * h + lane] = acc[h];
-        if ((int)lane == cur) mine = fo;
-    };
-    for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t e = base + lane;
-        uint32_t k = 0;
-#pragma unroll
-        for (int step = 16; step; step >>= 1)
-            if (__shfl_sync(FULL_MASK, inc, k + step - 1) <= e) k += step;
-        const uint32_t pk = __shfl_sync(FULL_MASK, shift, k) + e;
-        const M nk = __shfl_sync(FULL_MASK, ns_l, k);
-        uint32_t v = 0;
-        M fm = 0;
-        if (e < total) {
-            v = rv.row[pk];
-            fm = fprev[v] & nk;
-            wc.add(WC_ENTRIES, 1);
-            wc.add(WC_GATHERS, __popcll((unsigned long long)fm));
-            wc.add(WC_BYTES, 4 + 4 * K + 4 * __popcll((unsigned long long)fm));  // entry, mask, parents' counts
+        for (int q = 0; q < S::NSUB; q++) {
+            if (q == g && act) j = __ffs(act) - 1;
+            act &= act - 1;
         }
-        const unsigned act = __ballot_sync(FULL_MASK, fm != 0);
-        if (!act) continue;
-        const int nh = stage_compact<K>(su, sg, sk, act, v, fm, k);
-        __syncwarp();
-#pragma unroll 1
-        for (int g = 0; 8 * g < nh; g++) {
-            uint32_t u4[8];
-            load8u(su, g, u4);
-            uint32_t x[K][8];
-            M mor = 0;
-#pragma unroll
-            for (int h = 0; h < K; h++) {
-                uint32_t m4[8], mh = 0;
-                load8u(sg + 32 * h, g, m4);
-#pragma unroll
-                for (int q = 0; q < 8; q++) {
-                    x[h][q] = ((m4[q] >> lane) & 1u) ? msigma[row_base<K>(u4[q]) + 32 * h + lane] : 0u;
-                    mh |= m4[q];
-                }
-                mor |= (M)((unsigned long long)mh << (32 * h));
+        const uint32_t u = __shfl_sync(FULL_MASK, u_l, j & 31), b = __shfl_sync(FULL_MASK, b_l, j & 31);
+        const M ns = __shfl_sync(FULL_MASK, ns_l, j & 31);
+        const uint32_t dj = __shfl_sync(FULL_MASK, d_l, j & 31);
+        const uint32_t d = j < 0 ? 0u : dj;
+        const uint32_t dmax = __reduce_max_sync(FULL_MASK, d);
+        uint32_t acc[4] = {0, 0, 0, 0}, fo = 0;
+        uint32_t vn = (uint32_t)sl < d ? rv.row[b + sl] : 0u;
+        for (uint32_t s = 0; s < dmax; s += S::SUB) {
+            const uint32_t e = s + sl, v = vn;
+            vn = e + S::SUB < d ? rv.row[b + e + S::SUB] : 0u;
+            M fm = 0;
+            if (e < d) {
+                fm = fprev[v] & ns;
+                wc.add(WC_ENTRIES, 1);
+                wc.add(WC_GATHERS, __popcll((unsigned long long)fm));
+                wc.add(WC_BYTES, 4 + 4 * K + 4 * __popcll((unsigned long long)fm));  // entry, mask, parents' counts
             }
-            const int k0 = (int)sk[8 * g], k7 = (int)sk[min(8 * g + 7, nh - 1)];
-            if (k0 == k7) {
-                // all eight positions belong to one vertex (k is nondecreasing)
-                if (k0 != cur) {
-                    if (cur >= 0) flush();
-                    cur = k0;
-#pragma unroll
-                    for (int h = 0; h < K; h++) acc[h] = 0;
-                    fo = 0;
-                }
-#pragma unroll
-                for (int h = 0; h < K; h++)
-                    acc[h] += ((x[h][0] + x[h][1]) + (x[h][2] + x[h][3])) + ((x[h][4] + x[h][5]) + (x[h][6] + x[h][7]));
-                fo |= mor;
-                continue;
-            }
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const M mq = staged_mask<K>(sg, 8 * g + q);
-                if (!mq) continue;
-                const int kq = (int)sk[8 * g + q];
-                if (kq != cur) {
-                    if (cur >= 0) flush();
-                    cur = kq;
-#pragma unroll
-                    for (int h = 0; h < K; h++) acc[h] = 0;
-                    fo = 0;
-                }
-#pragma unroll
-                for (int h = 0; h < K; h++) acc[h] += x[h][q];
-                fo |= mq;
-            }
+            const unsigned hit = __ballot_sync(FULL_MASK, fm != 0);
+            if (!hit) continue;
+            const unsigned mine = (hit >> (S::SUB * g)) & ((1u << S::SUB) - 1u);
+            const int nh = __popc(mine);
+            if (fm) stage_pair<K>(st, S::SUB * g + __popc(mine & ((1u << sl) - 1u)), v, fm);
+            if (sl >= nh) stage_pair<K>(st, S::SUB * g + sl, 0u, (M)0);
+            const int most = (int)__reduce_max_sync(FULL_MASK, (unsigned)nh);
+            __syncwarp();
+            pull_rows<K>(st_h, S::SUB * g, 1, most, msigma + 4 * sl, sh, acc, fo);
+            __syncwarp();
         }
-        __syncwarp();
+        // this vertex has no other part: plain stores
+        if (!__any_sync(FULL_MASK, fo != 0)) continue;
+        uint32_t *r = msigma + row_base<K>(u) + 4 * sl;
+        if (fo & 1u) r[0] = acc[0];
+        if (fo & 2u) r[1] = acc[1];
+        if (fo & 4u) r[2] = acc[2];
+        if (fo & 8u) r[3] = acc[3];
+        uint32_t w = fo << sh;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(FULL_MASK, w, o);
+        M nm = (M)w;
+        if (K == 2) nm |= (M)((unsigned long long)__shfl_xor_sync(FULL_MASK, w, 8) << 32);  // read at sl == 0
+        const bool isnew = sl == 0 && nm != 0;
+        if (isnew) {
+            fcur[u] = nm;
+            wc.add(WC_PAIRS, __popcll((unsigned long long)nm));
+            wc.add(WC_BYTES, 4 + 4 * K + 4 * __popcll((unsigned long long)nm));  // mask, list, counts
+        }
+        list_append(ll, L, isnew, u);
     }
-    if (cur >= 0) flush();
-    return mine;
 }
 
 template <int K, class WC>
@@ -657,56 +653,41 @@ __device__ __forceinline__ void fwd_pull_body(const Adj &rv, typename MaskOf<K>:
                                               const typename MaskOf<K>::T *__restrict__ fprev,
                                               typename MaskOf<K>::T *fcur,
                                               const typename MaskOf<K>::T *__restrict__ seen, uint32_t *msigma,
-                                              uint32_t *ctr, uint32_t *su, uint32_t *sg,
-                                              uint32_t *sk, const LevelLists &ll, int L, WC &wc)
+                                              uint32_t *ctr, uint2 *st, const LevelLists &ll, int L, WC &wc)
 {
     typedef typename MaskOf<K>::T M;
     const unsigned lane = lane_id();
-    const uint64_t nhi = rv.n_heavy_items, nu = n_units(rv);
-    if (warp_global() >= nu) return;  // fewer units than warps: no contention
-    for (;;) {
-        const uint32_t t = grab_unit(ctr);
-        if (t >= nu) break;
-        if (t < nhi) {
-            const uint32_t u = rv.hitem_v[t];
-            const M ns = srcmask & ~seen[u];
-            if (lane == 0) wc.add(WC_BYTES, 4 * K);  // seen mask
-            if (!ns) continue;
-            const uint32_t b0 = rv.col[u] + rv.hitem_k[t] * AXBC_SPAN;
-            uint32_t acc[K];
-            const M nm = pull_span<K>(rv, ns, b0, min(rv.col[u + 1], b0 + AXBC_SPAN), fprev, msigma, su, sg,
-                                      acc, wc);
-#pragma unroll
-            for (int h = 0; h < K; h++)
-                if (pbit(nm, h)) {
-                    atomicAdd(&msigma[row_base<K>(u) + 32 * h + lane], acc[h]);
-                    wc.add(WC_PAIRS, 1);
-                    wc.add(WC_BYTES, 4);
-                }
-            bool first = false;
-            if (lane == 0 && nm) first = atomicOr(&fcur[u], nm) == 0;
-            if (lane == 0 && nm) wc.add(WC_BYTES, first ? 4 + 4 * K : 4 * K);  // level mask, list entry
-            list_append(ll, L, first, u);
-            continue;
-        }
-        const uint64_t l0 = (uint64_t)(t - nhi) * LIGHT_PER_UNIT;
-        for (uint64_t lt = l0; lt < l0 + LIGHT_PER_UNIT && lt < rv.n_ltask; lt++) {
-            const uint32_t beg = rv.ltask[lt], cnt = rv.ltask[lt + 1] - beg;
-            uint32_t u_l = 0;
-            M ns_l = 0;
-            if (lane < cnt) {
-                u_l = rv.order[beg + lane];
-                ns_l = srcmask & ~seen[u_l];
+    const uint64_t np = rv.n_part, nl = rv.n_linked - rv.n_big;
+    const uint32_t gp = unit_of(np, 1), gl = unit_of(nl, PullShape<K>::NSUB);
+    const uint64_t up = (np + gp - 1) / gp, nu = up + (nl + gl - 1) / gl;
+    for (uint64_t t = warp_global(); t < nu; t = next_unit(ctr, nu)) {
+        uint2 pt = make_uint2(0, 0);
+        M ns_l = 0;
+        if (t < up) {
+            // a unit of parts: one lane looks each part's unseen pivots up
+            const uint64_t i = lane * up + t;  // a hub's parts fall into different units
+            if (lane < gp && i < np) {
+                pt = rv.part[i];
+                ns_l = srcmask & ~seen[pt.x];
                 wc.add(WC_BYTES, 4 * K);  // seen mask
             }
-            const M mine = pull_light32<K>(rv, u_l, ns_l, fprev, msigma, su, sg, sk, wc);
-            if (mine) {
-                fcur[u_l] = mine;
-                wc.add(WC_PAIRS, __popcll((unsigned long long)mine));
-                wc.add(WC_BYTES, 4 + 4 * K + 4 * __popcll((unsigned long long)mine));  // mask, list, counts
+            for (unsigned act = __ballot_sync(FULL_MASK, ns_l != 0); act; act &= act - 1) {
+                const int j = __ffs(act) - 1;
+                const uint32_t u = __shfl_sync(FULL_MASK, pt.x, j);
+                const uint32_t b0 = rv.col[u] + __shfl_sync(FULL_MASK, pt.y, j) * rv.part_len;
+                pull_part<K>(rv, u, __shfl_sync(FULL_MASK, ns_l, j), b0, min(rv.col[u + 1], b0 + rv.part_len), fprev,
+                             fcur, msigma, st, ll, L, wc);
             }
-            list_append(ll, L, mine != 0, u_l);
+            continue;
         }
+        const uint64_t i = (t - up) * gl + lane;
+        uint32_t u_l = 0;
+        if (lane < gl && i < nl) {
+            u_l = rv.order[rv.n_big + i];
+            ns_l = srcmask & ~seen[u_l];
+            wc.add(WC_BYTES, 4 * K);  // seen mask
+        }
+        pull_small<K>(rv, u_l, ns_l, fprev, fcur, msigma, st, ll, L, wc);
     }
 }
 
@@ -739,16 +720,12 @@ __global__ void __launch_bounds__(BATCH_TPB, PULL_BLOCKS(K)) k_fwd_pull_step(Adj
                                                              LevelLists ll, unsigned long long *wc)
 {
     typedef typename MaskOf<K>::T M;
-    __shared__ __align__(16) uint32_t s_u[BATCH_TPB];
-    __shared__ __align__(16) uint32_t s_g[BATCH_TPB * K];
-    __shared__ uint32_t s_k[BATCH_TPB];
+    __shared__ uint2 s_st[BATCH_TPB / 32][PullShape<K>::STAGE];
     if (!bi->alive || bi->push_next) return;
     const int L = bi->cur + 1;
-    const unsigned w0 = threadIdx.x & ~31u;
     WorkCount<CNT> cnt;
     fwd_pull_body<K>(rv, (M)bi->srcmask, reinterpret_cast<const M *>(tab[L - 1]), reinterpret_cast<M *>(tab[L]),
-                     reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L, s_u + w0, s_g + w0 * K, s_k + w0,
-                     ll, L, cnt);
+                     reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L, s_st[threadIdx.x >> 5], ll, L, cnt);
     cnt.flush(wc);
 }
 
@@ -796,7 +773,7 @@ __device__ __forceinline__ void stats_body(uint64_t n, BatchInfo *bi, int L, typ
 #pragma unroll
     for (int h = 0; h < K; h++) cnt[h] = te[h] = rs[h] = 0;
     unsigned long long fdeg = 0, udec = 0, tsum = 0;
-    uint32_t hv = 0;  // heavy vertices of the level (their span items are scanned)
+    uint32_t hv = 0;  // big vertices of the level (their parts or span items are scanned)
     bool any = false;
     for (uint64_t t = tid / 32; t < nblk; t += nw) {
         const uint64_t i = t * 32 + lane;
@@ -805,7 +782,7 @@ __device__ __forceinline__ void stats_body(uint64_t n, BatchInfo *bi, int L, typ
         if (i < items) {
             const uint64_t u = lst ? lst[i] : i;
             stats_vertex<M>(u, srcmask, fcur, seen, col, rcol, reach, nm, d, r, fdeg, udec, any);
-            if (nm && d > AXBC_SPAN) hv++;
+            if (nm && d > AXBC_BIG) hv++;
             tsum += (unsigned long long)d * __popcll((unsigned long long)nm);
         }
         unsigned act = __ballot_sync(FULL_MASK, nm != 0);
@@ -1316,8 +1293,8 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
 {
     typedef typename MaskOf<K>::T M;
     __shared__ __align__(16) uint32_t s_u[BATCH_TPB];
-    __shared__ __align__(16) uint32_t s_g[BATCH_TPB * K];
-    __shared__ uint32_t s_k[BATCH_TPB];
+    __shared__ __align__(16) uint32_t s_g[BATCH_TPB];
+    __shared__ uint2 s_st[BATCH_TPB / 32][PullShape<K>::STAGE];
     const unsigned w0 = threadIdx.x & ~31u;
     M *seen = reinterpret_cast<M *>(seen_);
     WorkCount<false> none;
@@ -1334,8 +1311,8 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
         if (vload_i(&bi->push_next))
             fwd_push_body<K>(a, fprev, fcur, seen, msigma, ctrs + 2 * L, ll, L, none);
         else
-            fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, s_u + w0, s_g + w0 * K,
-                             s_k + w0, ll, L, none);
+            fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, s_st[threadIdx.x >> 5], ll, L,
+                             none);
         if (!grid_barrier(gs, budget, 1, NoLead{})) return;
         stats_body<K>(n, bi, L, srcmask, fcur, seen, a.col, rv.col, reach, ll);
         if (!grid_barrier(gs, budget, 2, adv)) return;

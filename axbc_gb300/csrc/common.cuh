@@ -19,6 +19,8 @@
 #define AXBC_CHUNK 32
 #define AXBC_SPAN 1024
 #define AXBC_SAMPLE_BLOCK 1024
+// Vertices with more than AXBC_BIG neighbours are split over several warps.
+#define AXBC_BIG 128
 #define AXBC_W 32     // lanes of a warp, pivots per mask word
 #define AXBC_WMAX 64  // pivots of one multi-source pass (two mask words per vertex)
 #define FULL_MASK 0xffffffffu
@@ -76,6 +78,13 @@ struct Adj {
     uint32_t *order = nullptr;        // n
     uint32_t *ltask = nullptr;        // n_ltask + 1 offsets into order
     uint64_t n_ltask = 0;
+    // the forward kernels' split of the same order: order[0..n_big) have more
+    // than AXBC_BIG neighbours and are walked in parts of part_len positions
+    // (part[i]: vertex, part number), order[n_big..n_linked) at least one
+    uint32_t n_big = 0, n_linked = 0;
+    uint2 *part = nullptr;            // n_part
+    uint64_t n_part = 0;
+    uint32_t part_len = 0;
     bool owns = true;
 };
 

@@ -137,6 +137,10 @@ static void task_tables(const uint32_t *col, uint64_t n, std::vector<uint32_t> &
     ltask.push_back((uint32_t)n);
 }
 
+// Positions per part of a big vertex: short parts spread a small graph over the
+// whole chip, long ones amortise a part's atomics once every warp has many.
+static uint32_t part_len_of(uint64_t m) { return m >= (1ull << 25) ? 512 : 128; }
+
 // heavy-vertex span items and light-vertex tasks of an adjacency whose col
 // (host copy: col) is on the device
 static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, uint32_t *maxdeg)
@@ -163,6 +167,20 @@ static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, u
     TRY(axbc_dalloc((void **)&a.ltask, ltask.size() * 4, acct));
     CU(cudaMemcpy(a.order, order.data(), n * 4, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(a.ltask, ltask.data(), ltask.size() * 4, cudaMemcpyHostToDevice));
+    // parts of the big vertices
+    auto deg = [&](uint64_t i) { return col[order[i] + 1] - col[order[i]]; };
+    a.part_len = part_len_of(a.m);
+    std::vector<uint2> part;
+    uint64_t i = 0;
+    for (; i < n && deg(i) > AXBC_BIG; i++)
+        for (uint32_t k = 0; k * a.part_len < deg(i); k++) part.push_back(make_uint2(order[i], k));
+    a.n_big = (uint32_t)i;
+    a.n_linked = (uint32_t)(std::partition_point(order.begin() + i, order.end(),
+                                                 [&](uint32_t v) { return col[v + 1] > col[v]; }) -
+                            order.begin());
+    a.n_part = part.size();
+    TRY(axbc_dalloc((void **)&a.part, part.size() * sizeof(uint2), acct));
+    if (!part.empty()) CU(cudaMemcpy(a.part, part.data(), part.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     return AXBC_OK;
 }
 
@@ -286,6 +304,7 @@ static void free_adj(Adj &a)
     axbc_dfree(a.hitem_k);
     axbc_dfree(a.order);
     axbc_dfree(a.ltask);
+    axbc_dfree(a.part);
     a = Adj();
 }
 
