@@ -45,14 +45,6 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
     return (unsigned long long)lo | ((unsigned long long)hi << 32);
 }
 
-// eight staged words of group g (16-byte shared loads)
-__device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
-{
-    const uint4 *p = reinterpret_cast<const uint4 *>(su) + 2 * g;
-    const uint4 a = p[0], b = p[1];
-    u[0] = a.x, u[1] = a.y, u[2] = a.z, u[3] = a.w, u[4] = b.x, u[5] = b.y, u[6] = b.z, u[7] = b.w;
-}
-
 // resident blocks per SM the kernels are compiled for (their register
 // budgets); the backward runs 32 pivots at a time at either width
 #ifndef AXBC_PULL_MIN_BLOCKS
@@ -60,6 +52,12 @@ __device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
 #endif
 #ifndef AXBC_BWD_MIN_BLOCKS
 #define AXBC_BWD_MIN_BLOCKS 8
+#endif
+#ifndef AXBC_BWD_TILE_BLOCKS
+#define AXBC_BWD_TILE_BLOCKS 5
+#endif
+#ifndef AXBC_BWD_WIDE_MIN
+#define AXBC_BWD_WIDE_MIN (1u << 22)
 #endif
 #ifndef AXBC_PUSH_MIN_BLOCKS2
 #define AXBC_PUSH_MIN_BLOCKS2 5
@@ -139,7 +137,6 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         bi->alive = 1;
         bi->lend = 0;
         bi->dmax = -1;
-        bi->bd = -1;
         bi->push_factor = push_factor;
         bi->lvl_te = 0;
         bi->any_new = 0;
@@ -208,12 +205,7 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
 }
 
 // ---------------------------------------------------------- task scheduling
-// Work units handed out by an atomic counter: units [0, nhi) are the span
-// items of heavy vertices (largest first), the remaining units cover four
-// light tasks each (light tasks: degree-ordered groups of <= 32 vertices with
-// about one span of adjacency).
-#define LIGHT_PER_UNIT 1
-
+// Work units are handed out by an atomic counter.
 __device__ __forceinline__ uint32_t grab_unit(uint32_t *ctr)
 {
     uint32_t t = 0;
@@ -221,17 +213,9 @@ __device__ __forceinline__ uint32_t grab_unit(uint32_t *ctr)
     return __shfl_sync(FULL_MASK, t, 0);
 }
 
-// A level with fewer work units than the grid has warps lets only as many
-// warps as units reach the counter: ~10^4 warps contending for one address
-// would cost tens of microseconds on a small level.
 __device__ __forceinline__ uint32_t warp_global()
 {
     return (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-}
-
-__host__ __device__ __forceinline__ uint64_t n_units(const Adj &a)
-{
-    return a.n_heavy_items + (a.n_ltask + LIGHT_PER_UNIT - 1) / LIGHT_PER_UNIT;
 }
 
 __device__ __forceinline__ void list_append(const LevelLists &ll, int L, bool isnew, uint32_t v)
@@ -247,16 +231,7 @@ __device__ __forceinline__ void list_append(const LevelLists &ll, int L, bool is
     if (isnew && idx < ll.cap[L]) ll.pool[ll.start[L] + idx] = v;
 }
 
-// List entries per work unit: 32, or fewer when the list is too short to give
-// every resident warp a unit (a short list of high-degree vertices would
-// otherwise sit on a few warps).
-__device__ __forceinline__ uint32_t list_unit(uint32_t lcnt)
-{
-    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-    return max(1u, min(32u, lcnt / nwarps));
-}
-
-// Items per work unit of the forward kernels: at least `least`, and as many as
+// Items per work unit: at least `least`, and as many as
 // leave every resident warp about four units (at most 32, one per lane).
 __device__ __forceinline__ uint32_t unit_of(uint64_t items, uint32_t least)
 {
@@ -457,7 +432,9 @@ __device__ __forceinline__ void fwd_push_body(const Adj &a, const typename MaskO
 // order gives the same bits).  Bound by instruction issue, not by memory, so
 // the gathers are laid out for few instructions: a lane owns four neighbouring
 // pivots (one 16-byte load per parent row), 8 K lanes -- a subgroup -- cover a
-// row, and the warp's 4 / K subgroups gather that many parents at once.  The
+// row, and the warp's 4 / K subgroups gather that many parents at once.  One
+// row per instruction took 18.8 ms of three scale-23 passes, this 13.6 ms;
+// 573 M against 411 M warp instructions on a scale-20 level of 64 pivots.  The
 // positions with a parent are staged in shared memory as (parent, mask) pairs,
 // one array per 32-pivot half, compacted.
 template <int K> struct PullShape {
@@ -891,7 +868,6 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
             bi->alive = 0;
             bi->lend = L;
             bi->dmax = L - 1;
-            bi->bd = L - 1;
             bi->depth0mask = d0;
         }
         bi->push_next = push;
@@ -925,12 +901,406 @@ template <int K> __device__ __forceinline__ uint32_t half_of(typename MaskOf<K>:
     return (uint32_t)((unsigned long long)m >> (32 * hh));
 }
 
+// Layout of the dependency sums: a lane owns four neighbouring pivots (one
+// 16-byte load per successor row) and eight lanes cover the half's 32; the
+// warp's four groups of eight lanes work on the four 8-position subtrees of a
+// chunk's canonical tree (or on four tiny vertices) at once, so that 16 rows
+// are in flight per load round at one quarter of the load, address and
+// test instructions of one row per instruction.  Folding the four subtrees
+// leaves the lane with the sum of one pivot, own_pivot().
+__device__ __forceinline__ int own_slot() { return 2 * ((lane_id() >> 3) & 1) + (lane_id() >> 4); }
+__device__ __forceinline__ int own_pivot() { return 4 * (lane_id() & 7) + own_slot(); }
+__device__ __forceinline__ float own_of(const float s[4])
+{
+    const unsigned lane = lane_id();
+    const float a = lane & 16 ? s[1] : s[0], b = lane & 16 ? s[3] : s[2];
+    return lane & 8 ? b : a;
+}
+
+// Terms of four staged successors as a tree (pairs differing in the lowest
+// position bit first).  q[u][s] = (delta_s[u] + 1) / sigma_s[u] was stored when
+// u's dependency was final, so a term is q * sigma_s[v], bit for bit the
+// reference's ((delta + 1) / sigma[r]) * sigma[c].  mq_l points at the lane's
+// columns of row 0.
+template <int K>
+__device__ __forceinline__ void quad_sum(const uint2 *st, const float *__restrict__ mq_l, unsigned sh,
+                                         const float sv[4], float out[4])
+{
+    float4 x[4];
+    uint32_t nb[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const uint2 e = st[j];
+        nb[j] = (e.y >> sh) & 15u;
+        x[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (nb[j]) x[j] = *reinterpret_cast<const float4 *>(mq_l + row_base<K>(e.x));
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float t[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float xq = q == 0 ? x[j].x : q == 1 ? x[j].y : q == 2 ? x[j].z : x[j].w;
+            t[j] = (nb[j] >> q) & 1u ? __fmul_rn(xq, sv[q]) : 0.0f;
+        }
+        out[q] = __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
+    }
+}
+
+// The 8-position subtree sums of the lane's group for its four pivots, of the
+// chunk whose lanes hold successors u with pivots gm (pm: lanes with any).  A
+// quad of positions without successors in any group sums to +0 and is skipped.
+template <int K>
+__device__ __forceinline__ void group_sums(uint2 *st, uint32_t u, uint32_t gm, unsigned pm,
+                                           const float *__restrict__ mq_l, const float sv[4], float s[4])
+{
+    const unsigned lane = lane_id(), g9 = 9 * (lane >> 3), sh = 4 * (lane & 7);
+    st[g9 + (lane & 7)] = make_uint2(u, gm);
+    __syncwarp();
+    unsigned pj = pm | pm >> 16;
+    pj |= pj >> 8;
+    float b[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    s[0] = s[1] = s[2] = s[3] = 0.0f;
+    if (pj & 0x0fu) quad_sum<K>(st + g9, mq_l, sh, sv, s);
+    if (pj & 0xf0u) quad_sum<K>(st + g9 + 4, mq_l, sh, sv, b);
+#pragma unroll
+    for (int q = 0; q < 4; q++) s[q] = __fadd_rn(s[q], b[q]);
+    __syncwarp();
+}
+
+// The top two levels of the chunk's tree: groups g and g ^ 1, then the two
+// halves, each lane keeping fewer pivots of more positions.
+__device__ __forceinline__ float fold_groups(const float s[4])
+{
+    const unsigned lane = lane_id();
+    const bool h1 = (lane & 8) != 0, h2 = (lane & 16) != 0;
+    const float r0 = __fadd_rn(h1 ? s[2] : s[0], __shfl_xor_sync(FULL_MASK, h1 ? s[0] : s[2], 8));
+    const float r1 = __fadd_rn(h1 ? s[3] : s[1], __shfl_xor_sync(FULL_MASK, h1 ? s[1] : s[3], 8));
+    return __fadd_rn(h2 ? r1 : r0, __shfl_xor_sync(FULL_MASK, h2 ? r0 : r1, 16));
+}
+
+// path counts of v for the lane's four pivots (of those in f)
+template <int K>
+__device__ __forceinline__ void load_sv(const uint32_t *__restrict__ msigma, uint32_t v, uint32_t f, float sv[4])
+{
+    const unsigned l = lane_id() & 7;
+    uint4 x = make_uint4(0, 0, 0, 0);
+    if ((f >> (4 * l)) & 15u) x = *reinterpret_cast<const uint4 *>(msigma + row_base<K>(v) + 4 * l);
+    sv[0] = __uint2float_rn(x.x);
+    sv[1] = __uint2float_rn(x.y);
+    sv[2] = __uint2float_rn(x.z);
+    sv[3] = __uint2float_rn(x.w);
+}
+
+// delta and q of vertex v for one pivot; sv: its path count
+template <int K>
+__device__ __forceinline__ void write_dep(float *mdelta, float *mq, uint32_t v, int pivot, float delta, float sv)
+{
+    mdelta[row_base<K>(v) + pivot] = delta;
+    mq[row_base<K>(v) + pivot] = __fdiv_rn(__fadd_rn(delta, 1.0f), sv);
+}
+
+// work counts of one lane's adjacency entry
+template <class WC> __device__ __forceinline__ void count_entry(WC &wc, bool valid, uint32_t gm)
+{
+    if (!valid) return;
+    wc.add(WC_ENTRIES, 1);
+    wc.add(WC_GATHERS, __popc(gm));
+    wc.add(WC_BYTES, 8 + 4 * __popc(gm));  // adjacency entry, level mask word, successors' q
+}
+
+// Backward depth d for the half's pivots: arrays of one pass half.
+struct BwdHalf {
+    uint32_t dmask;   // the half's pivots that are processed at this depth
+    int no_succ;      // the deepest depth: nothing lies below, delta = reach
+    const uint32_t *fd, *fnext;
+    const uint32_t *msigma;
+    float *mdelta, *mq, *mpartial;
+    uint32_t *harrive;
+    const uint32_t *reach;
+};
+
+// Positions [b0, b1) of a vertex by one warp: chunk sums left to right, own
+// pivot per lane.  Adjacency entries load two chunks ahead and level masks one.
+template <int K, class WC>
+__device__ __forceinline__ float bwd_span(const Adj &a, const BwdHalf &B, uint32_t f, const float sv[4], uint32_t b0,
+                                          uint32_t b1, uint2 *st, WC &wc)
+{
+    const unsigned lane = lane_id();
+    float P = 0.0f;
+    if (!B.no_succ) {
+        const float *mq_l = B.mq + 4 * (lane & 7);
+        uint32_t e = b0 + lane;
+        uint32_t u = e < b1 ? a.row[e] : 0u, un = e + 32 < b1 ? a.row[e + 32] : 0u;
+        uint32_t gm = e < b1 ? B.fnext[(uint64_t)u * K] & f : 0u;
+        for (; e - lane < b1; e += 32) {
+            count_entry(wc, e < b1, gm);
+            const uint32_t uc = u, gc = gm;
+            u = un;
+            un = e + 64 < b1 ? a.row[e + 64] : 0u;
+            gm = e + 32 < b1 ? B.fnext[(uint64_t)u * K] & f : 0u;
+            const unsigned pm = __ballot_sync(FULL_MASK, gc != 0);
+            if (!pm) continue;
+            float s[4];
+            group_sums<K>(st, uc, gc, pm, mq_l, sv, s);
+            P = __fadd_rn(P, fold_groups(s));
+        }
+    }
+    return P;
+}
+
+// Vertices of at most AXBC_BIG neighbours, one per lane (pivots f_l; 0: none):
+// those of at most 8 four at a time, one group of lanes each, the others one
+// by one.
+template <int K, class WC>
+__device__ __forceinline__ void bwd_small(const Adj &a, const BwdHalf &B, uint32_t v_l, uint32_t f_l, uint2 *st,
+                                          WC &wc)
+{
+    const unsigned lane = lane_id();
+    const int l = lane & 7, g = lane >> 3;
+    if (!__ballot_sync(FULL_MASK, f_l != 0)) return;
+    uint32_t b_l = 0, d_l = 0;
+    if (f_l) {
+        b_l = a.col[v_l];
+        d_l = a.col[v_l + 1] - b_l;
+        if (d_l > AXBC_BIG) f_l = 0;  // in a tile
+    }
+    if (f_l) {
+        // adjacency bounds and reach; per pivot its path count read, its
+        // dependency and q written
+        wc.add(WC_BYTES, (B.no_succ ? 4 : 12) + 12 * __popc(f_l));
+        wc.add(WC_PAIRS, __popc(f_l));
+    }
+    for (unsigned act = __ballot_sync(FULL_MASK, f_l != 0 && d_l > 8); act; act &= act - 1) {
+        const int j = __ffs(act) - 1;
+        const uint32_t v = __shfl_sync(FULL_MASK, v_l, j), f = __shfl_sync(FULL_MASK, f_l, j);
+        const uint32_t b0 = __shfl_sync(FULL_MASK, b_l, j);
+        float sv[4];
+        load_sv<K>(B.msigma, v, f, sv);
+        const float P = bwd_span<K>(a, B, f, sv, b0, b0 + __shfl_sync(FULL_MASK, d_l, j), st, wc);
+        if ((f >> own_pivot()) & 1u)
+            write_dep<K>(B.mdelta, B.mq, v, own_pivot(), __fadd_rn(__uint2float_rn(B.reach[v]), P), own_of(sv));
+    }
+    for (unsigned act = __ballot_sync(FULL_MASK, f_l != 0 && d_l <= 8); act;) {
+        int j = -1;
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (q == g && act) j = __ffs(act) - 1;
+            act &= act - 1;
+        }
+        const uint32_t v = __shfl_sync(FULL_MASK, v_l, j & 31), fj = __shfl_sync(FULL_MASK, f_l, j & 31);
+        const uint32_t b0 = __shfl_sync(FULL_MASK, b_l, j & 31), dj = __shfl_sync(FULL_MASK, d_l, j & 31);
+        const uint32_t f = j < 0 ? 0u : fj, d = j < 0 || B.no_succ ? 0u : dj;
+        const uint32_t u = (uint32_t)l < d ? a.row[b0 + l] : 0u;
+        float sv[4], s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        load_sv<K>(B.msigma, v, f, sv);
+        const uint32_t gm = (uint32_t)l < d ? B.fnext[(uint64_t)u * K] & f : 0u;
+        count_entry(wc, (uint32_t)l < d, gm);
+        const unsigned pm = __ballot_sync(FULL_MASK, gm != 0);
+        if (pm) group_sums<K>(st, u, gm, pm, B.mq + 4 * l, sv, s);
+        if (f) {
+            const float rf = __uint2float_rn(B.reach[v]);
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if ((f >> (4 * l + q)) & 1u) write_dep<K>(B.mdelta, B.mq, v, 4 * l + q, __fadd_rn(rf, s[q]), sv[q]);
+        }
+    }
+}
+
+// The span sums of a heavy vertex added in span order: delta and q of the
+// lane's pivot `own`.  Out of line: once per heavy vertex, and inlined it would
+// cost the traversal loops registers.
+template <int K>
+__device__ __noinline__ void bwd_combine(const float *part, uint32_t spans, const uint32_t *reach,
+                                         const uint32_t *msigma, float *mdelta, float *mq, uint32_t v, bool mine,
+                                         int own)
+{
+    float acc = __uint2float_rn(reach[v]);
+    for (uint32_t i = 0; i < spans; i += 8) {
+        float x[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = i + q < spans ? __ldcg(part + (uint64_t)(i + q) * (AXBC_W * K)) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            if (i + q < spans) acc = __fadd_rn(acc, x[q]);
+    }
+    if (mine) write_dep<K>(mdelta, mq, v, own, acc, __uint2float_rn(msigma[row_base<K>(v) + own]));
+}
+
+// The span sum P of a heavy vertex is written (own: the lane's pivot); the warp
+// that writes the vertex's last one adds them up.
+template <int K>
+__device__ __forceinline__ void bwd_span_done(const Adj &a, const BwdHalf &B, uint32_t v, uint32_t f, uint32_t hx,
+                                              uint64_t row, uint32_t k, int own, float P)
+{
+    const unsigned lane = lane_id();
+    B.mpartial[row * (AXBC_W * K) + lane] = P;
+    __threadfence();
+    __syncwarp();
+    const uint32_t spans = (a.col[v + 1] - a.col[v] + AXBC_SPAN - 1) / AXBC_SPAN;
+    uint32_t last = 0;
+    if (lane == 0) {
+        last = atomicAdd(&B.harrive[hx], 1u) == spans - 1;
+        if (last) B.harrive[hx] = 0;
+    }
+    if (!__shfl_sync(FULL_MASK, last, 0)) return;
+    __threadfence();
+    bwd_combine<K>(B.mpartial + (row - k) * (AXBC_W * K) + lane, spans, B.reach, B.msigma, B.mdelta, B.mq, v,
+                   (f >> own) & 1u, own);
+}
+
+// A tile of big vertices by one block: its chunks go round the warps (up to
+// four each, their adjacency entries and then their masks loaded together),
+// the chunk sums meet in shared memory and are added left to right.  A span of
+// 1024 positions on one warp took 42 us, longer than a whole depth of a
+// scale-14 graph should.
+template <int K, class WC>
+__device__ __forceinline__ void bwd_tile(const Adj &a, const BwdHalf &B, uint64_t t, uint2 tl, uint2 *st,
+                                         float (*csum)[32], WC &wc)
+{
+    constexpr int NW = BATCH_TPB / 32;
+    const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+    const bool span = (tl.y & BWD_SPAN_TILE) != 0;
+    const uint32_t k = span ? tl.y & ~BWD_SPAN_TILE : 0u, cnt = span ? 1u : tl.y;
+    uint32_t v_l = 0, f_l = 0, b_l = 0, e_l = 0, c_l = 0;
+    if (lane < cnt) {
+        v_l = a.order[tl.x + lane];
+        f_l = B.fd[(uint64_t)v_l * K] & B.dmask;
+    }
+    if (f_l) {
+        b_l = a.col[v_l] + k * AXBC_SPAN;
+        e_l = min(a.col[v_l + 1], b_l + AXBC_SPAN);
+        if (!B.no_succ) c_l = (e_l - b_l + AXBC_CHUNK - 1) / AXBC_CHUNK;
+        if (wid == 0) {
+            wc.add(WC_BYTES, span ? 4 + 8 * __popc(f_l) : (B.no_succ ? 4 : 12) + 12 * __popc(f_l));
+            if (!span) wc.add(WC_PAIRS, __popc(f_l));
+        }
+    }
+    uint32_t inc = c_l;  // chunks up to and including this vertex's
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(FULL_MASK, inc, o);
+        if ((int)lane >= o) inc += x;
+    }
+    const uint32_t S = __shfl_sync(FULL_MASK, inc, 7);
+    const float *mq_l = B.mq + 4 * (lane & 7);
+    uint32_t u[BWD_TILE_CHUNKS / NW], gm[BWD_TILE_CHUNKS / NW];
+#pragma unroll
+    for (int i = 0; i < BWD_TILE_CHUNKS / NW; i++) {
+        const uint32_t s = wid + NW * i;
+        u[i] = 0xffffffffu;
+        if (s < S) {
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            const uint32_t e = __shfl_sync(FULL_MASK, b_l + AXBC_CHUNK * (s - (inc - c_l)), j) + lane;
+            if (e < __shfl_sync(FULL_MASK, e_l, j)) u[i] = a.row[e];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < BWD_TILE_CHUNKS / NW; i++) {
+        const uint32_t s = wid + NW * i;
+        gm[i] = 0;
+        if (s < S) {
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            const uint32_t f = __shfl_sync(FULL_MASK, f_l, j);
+            if (u[i] != 0xffffffffu) gm[i] = B.fnext[(uint64_t)u[i] * K] & f;
+            count_entry(wc, u[i] != 0xffffffffu, gm[i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < BWD_TILE_CHUNKS / NW; i++) {
+        const uint32_t s = wid + NW * i;
+        if (s >= S) break;
+        const unsigned pm = __ballot_sync(FULL_MASK, gm[i] != 0);
+        float r = 0.0f;
+        if (pm) {
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            float sv[4], q[4];
+            load_sv<K>(B.msigma, __shfl_sync(FULL_MASK, v_l, j), __shfl_sync(FULL_MASK, f_l, j), sv);
+            group_sums<K>(st, u[i], gm[i], pm, mq_l, sv, q);
+            r = fold_groups(q);
+        }
+        csum[s][lane] = r;
+    }
+    __syncthreads();
+    for (uint32_t j = wid; j < cnt; j += NW) {
+        const uint32_t f = __shfl_sync(FULL_MASK, f_l, j);
+        if (!f) continue;
+        const uint32_t v = __shfl_sync(FULL_MASK, v_l, j), s1 = __shfl_sync(FULL_MASK, inc, j);
+        float P = 0.0f;
+        for (uint32_t s = s1 - __shfl_sync(FULL_MASK, c_l, j); s < s1; s++) P = __fadd_rn(P, csum[s][lane]);
+        if (span) {
+            bwd_span_done<K>(a, B, v, f, tl.x, t, k, own_pivot(), P);
+        } else if ((f >> own_pivot()) & 1u) {
+            const float sv = __uint2float_rn(B.msigma[row_base<K>(v) + own_pivot()]);
+            write_dep<K>(B.mdelta, B.mq, v, own_pivot(), __fadd_rn(__uint2float_rn(B.reach[v]), P), sv);
+        }
+    }
+}
+
+template <int K, class WC>
+__device__ __forceinline__ void bwd_body(const Adj &a, const BwdHalf &B, uint32_t *ctr, uint2 *st,
+                                         float (*csum)[BWD_TILE_CHUNKS][32], const uint32_t *lst, uint32_t lcnt,
+                                         uint32_t lheavy, int symmetric, WC &wc)
+{
+    const unsigned lane = lane_id();
+    // tiles only when a big vertex is at this depth; every warp of a block
+    // looks up the same 32 tiles and walks those with a vertex at this depth
+    if (!(lst && lheavy == 0)) {
+        int buf = 0;
+        for (uint64_t base = blockIdx.x; base < a.n_tile; base += 32ull * gridDim.x) {
+            const uint64_t t_l = base + (uint64_t)lane * gridDim.x;
+            uint2 tl = make_uint2(0, 0);
+            uint32_t any = 0;
+            if (t_l < a.n_tile) {
+                tl = a.tile[t_l];
+                const uint32_t cnt = tl.y & BWD_SPAN_TILE ? 1u : tl.y;
+                for (uint32_t j = 0; j < cnt; j++) any |= B.fd[(uint64_t)a.order[tl.x + j] * K];
+                if (threadIdx.x < 32) wc.add(WC_BYTES, 4 * cnt);  // level mask words
+            }
+            for (unsigned act = __ballot_sync(FULL_MASK, (any & B.dmask) != 0); act; act &= act - 1, buf ^= 1) {
+                const int j = __ffs(act) - 1;
+                bwd_tile<K>(a, B, base + (uint64_t)j * gridDim.x,
+                            make_uint2(__shfl_sync(FULL_MASK, tl.x, j), __shfl_sync(FULL_MASK, tl.y, j)), st,
+                            csum[buf], wc);
+            }
+        }
+    }
+    // the others by warps, from the level's list or by a scan; a directed
+    // graph's vertices without out-neighbours are at some depth too
+    const uint64_t nl = lst ? lcnt : (symmetric ? a.n_linked : a.n) - a.n_big;
+    const uint32_t ent = unit_of(nl, 1);
+    const uint64_t nu = (nl + ent - 1) / ent;
+    for (uint64_t t = warp_global(); t < nu; t = next_unit(ctr, nu)) {
+        const uint64_t i = t * ent + lane;
+        uint32_t v_l = 0, f_l = 0;
+        if (lane < ent && i < nl) {
+            v_l = lst ? lst[i] : a.order[a.n_big + i];
+            f_l = B.fd[(uint64_t)v_l * K] & B.dmask;
+            wc.add(WC_BYTES, lst ? 8 : 4);  // list entry, level mask word
+        }
+        bwd_small<K>(a, B, v_l, f_l, st, wc);
+    }
+}
+
+// The same depth on a graph large enough to keep every warp busy: lane =
+// pivot, a warp takes a span of a heavy vertex (its span sums are combined by
+// k_bwd_combine_step) or a group of about one span of the others.  At full
+// occupancy (32 registers) this form does more per second than the tiles; see
+// bwd_wide() for the line between them.
+// eight staged words of group g (16-byte shared loads)
+__device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
+{
+    const uint4 *p = reinterpret_cast<const uint4 *>(su) + 2 * g;
+    const uint4 a = p[0], b = p[1];
+    u[0] = a.x, u[1] = a.y, u[2] = a.z, u[3] = a.w, u[4] = b.x, u[5] = b.y, u[6] = b.z, u[7] = b.w;
+}
+
 // Sum of the 8 staged successor terms of group g as a balanced tree (pairs
 // differing in the lowest position bit first).  mq_l points at the lane's
 // column of row 0.
 template <int K>
-__device__ __forceinline__ float tree8(const uint32_t *su, const uint32_t *sg, int g,
-                                       const float *__restrict__ mq_l, float sv)
+__device__ __forceinline__ float tree8(const uint32_t *su, const uint32_t *sg, int g, const float *__restrict__ mq_l,
+                                       float sv)
 {
     uint32_t u[8], m[8];
     load8u(su, g, u);
@@ -940,12 +1310,49 @@ __device__ __forceinline__ float tree8(const uint32_t *su, const uint32_t *sg, i
 #pragma unroll
     for (int jj = 0; jj < 8; jj++) {
         const bool hit = (m[jj] >> lane) & 1u;
-        const float q = hit ? mq_l[(uint64_t)u[jj] * (AXBC_W * K)] : 0.0f;
+        const float q = hit ? mq_l[row_base<K>(u[jj])] : 0.0f;
         t[jj] = hit ? __fmul_rn(q, sv) : 0.0f;
     }
     const float a = __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
     const float b = __fadd_rn(__fadd_rn(t[4], t[5]), __fadd_rn(t[6], t[7]));
     return __fadd_rn(a, b);
+}
+
+// the same for a subtree whose successors all lie in one half of it (quad: the
+// half's number in the chunk): the other half sums to +0
+template <int K>
+__device__ __forceinline__ float tree4(const uint32_t *su, const uint32_t *sg, int quad, const float *__restrict__ mq_l, float sv)
+{
+    const uint4 u4 = reinterpret_cast<const uint4 *>(su)[quad], m4 = reinterpret_cast<const uint4 *>(sg)[quad];
+    const uint32_t u[4] = {u4.x, u4.y, u4.z, u4.w}, m[4] = {m4.x, m4.y, m4.z, m4.w};
+    const unsigned lane = lane_id();
+    float t[4];
+#pragma unroll
+    for (int jj = 0; jj < 4; jj++) {
+        const bool hit = (m[jj] >> lane) & 1u;
+        const float q = hit ? mq_l[row_base<K>(u[jj])] : 0.0f;
+        t[jj] = hit ? __fmul_rn(q, sv) : 0.0f;
+    }
+    return __fadd_rn(__fadd_rn(t[0], t[1]), __fadd_rn(t[2], t[3]));
+}
+template <int K>
+__device__ __forceinline__ float subtree(const uint32_t *su, const uint32_t *sg, int g, unsigned pm, const float *__restrict__ mq_l,
+                                         float sv)
+{
+    const unsigned h = (pm >> (8 * g)) & 0xffu;
+    if (!h) return 0.0f;
+    if (!(h & 0xf0u)) return tree4<K>(su, sg, 2 * g, mq_l, sv);
+    if (!(h & 0x0fu)) return tree4<K>(su, sg, 2 * g + 1, mq_l, sv);
+    return tree8<K>(su, sg, g, mq_l, sv);
+}
+
+// List entries per work unit: 32, or fewer when the list is too short to give
+// every resident warp a unit (a short list of high-degree vertices would
+// otherwise sit on a few warps).
+__device__ __forceinline__ uint32_t list_unit(uint32_t lcnt)
+{
+    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+    return max(1u, min(32u, lcnt / nwarps));
 }
 
 // Canonical dependency sum of vertex v over adjacency positions [b0,b1) for
@@ -979,11 +1386,8 @@ __device__ __forceinline__ float dep_span_from(const Adj &a, uint32_t f, float s
         su[lane] = u;
         sg[lane] = gm;
         __syncwarp();
-        float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, g3 = 0.0f;
-        if (pm & 0x000000ffu) g0 = tree8<K>(su, sg, 0, mq_l, sv);
-        if (pm & 0x0000ff00u) g1 = tree8<K>(su, sg, 1, mq_l, sv);
-        if (pm & 0x00ff0000u) g2 = tree8<K>(su, sg, 2, mq_l, sv);
-        if (pm & 0xff000000u) g3 = tree8<K>(su, sg, 3, mq_l, sv);
+        const float g0 = subtree<K>(su, sg, 0, pm, mq_l, sv), g1 = subtree<K>(su, sg, 1, pm, mq_l, sv);
+        const float g2 = subtree<K>(su, sg, 2, pm, mq_l, sv), g3 = subtree<K>(su, sg, 3, pm, mq_l, sv);
         P = __fadd_rn(P, __fadd_rn(__fadd_rn(g0, g1), __fadd_rn(g2, g3)));
         __syncwarp();
     }
@@ -1001,7 +1405,7 @@ __device__ __forceinline__ float dep_span(const Adj &a, uint32_t f, float sv, ui
 
 // delta and q of vertex v for the half's pivots in f
 template <int K>
-__device__ __forceinline__ void write_dep(float *mdelta, float *mq, uint32_t v, uint32_t f, float delta,
+__device__ __forceinline__ void write_lane(float *mdelta, float *mq, uint32_t v, uint32_t f, float delta,
                                           uint32_t sig)
 {
     const unsigned lane = lane_id();
@@ -1014,7 +1418,7 @@ __device__ __forceinline__ void write_dep(float *mdelta, float *mq, uint32_t v, 
 // Backward depth d for the half's pivots in dmask.  With no_succ (the deepest
 // depth) nothing lies below, so delta = reach.
 template <int K, class WC>
-__device__ __forceinline__ void bwd_vertices(const Adj &a, uint32_t v_l, uint32_t f_l, int no_succ,
+__device__ __forceinline__ void wide_vertices(const Adj &a, uint32_t v_l, uint32_t f_l, int no_succ,
                                              const uint32_t *__restrict__ fnext,
                                              const uint32_t *__restrict__ msigma, float *mdelta,
                                              float *mq, const uint32_t *__restrict__ reach,
@@ -1053,14 +1457,14 @@ __device__ __forceinline__ void bwd_vertices(const Adj &a, uint32_t v_l, uint32_
         const uint32_t sig = ((f >> lane) & 1u) ? msigma[row_base<K>(v) + lane] : 0u;
         float P = 0.0f;
         if (!no_succ) P = dep_span_from<K>(a, f, __uint2float_rn(sig), cb0, cb1, cu, fnext, mq, su, sg, wc);
-        write_dep<K>(mdelta, mq, v, f, __fadd_rn(__uint2float_rn(reach[v]), P), sig);
+        write_lane<K>(mdelta, mq, v, f, __fadd_rn(__uint2float_rn(reach[v]), P), sig);
         if (jn < 0) break;
         j = jn;
     }
 }
 
 template <int K, class WC>
-__device__ __forceinline__ void bwd_body(const Adj &a, uint32_t dmask, int no_succ,
+__device__ __forceinline__ void bwd_body_wide(const Adj &a, uint32_t dmask, int no_succ,
                                          const uint32_t *__restrict__ fd, const uint32_t *__restrict__ fnext,
                                          const uint32_t *__restrict__ msigma, float *mdelta,
                                          float *mq, float *mpartial,
@@ -1072,7 +1476,7 @@ __device__ __forceinline__ void bwd_body(const Adj &a, uint32_t dmask, int no_su
     // heavy span items only when a heavy vertex is at this depth
     const uint64_t nhi = lst && lheavy == 0 ? 0 : a.n_heavy_items;
     const uint32_t ent = list_unit(lcnt);
-    const uint64_t nu = lst ? nhi + (lcnt + ent - 1) / ent : n_units(a);
+    const uint64_t nu = nhi + (lst ? (lcnt + ent - 1) / ent : a.n_ltask);
     if (warp_global() >= nu) return;  // fewer units than warps: no contention
     for (;;) {
         const uint32_t t = grab_unit(ctr);
@@ -1101,52 +1505,18 @@ __device__ __forceinline__ void bwd_body(const Adj &a, uint32_t dmask, int no_su
                 if (a.col[v_l + 1] - a.col[v_l] <= AXBC_SPAN) f_l = fd[(uint64_t)v_l * K] & dmask;
                 wc.add(WC_BYTES, 8);  // list entry, level mask word
             }
-            bwd_vertices<K>(a, v_l, f_l, no_succ, fnext, msigma, mdelta, mq, reach, su, sg, wc);
+            wide_vertices<K>(a, v_l, f_l, no_succ, fnext, msigma, mdelta, mq, reach, su, sg, wc);
             continue;
         }
-        const uint64_t l0 = (uint64_t)(t - nhi) * LIGHT_PER_UNIT;
-        for (uint64_t lt = l0; lt < l0 + LIGHT_PER_UNIT && lt < a.n_ltask; lt++) {
-            const uint32_t beg = a.ltask[lt], cnt = a.ltask[lt + 1] - beg;
-            uint32_t v_l = 0, f_l = 0;
-            if (lane < cnt) {
-                v_l = a.order[beg + lane];
-                f_l = fd[(uint64_t)v_l * K] & dmask;
-                wc.add(WC_BYTES, 4);  // level mask word
-            }
-            bwd_vertices<K>(a, v_l, f_l, no_succ, fnext, msigma, mdelta, mq, reach, su, sg, wc);
+        const uint32_t beg = a.ltask[t - nhi], cnt = a.ltask[t - nhi + 1] - beg;
+        uint32_t v_l = 0, f_l = 0;
+        if (lane < cnt) {
+            v_l = a.order[beg + lane];
+            f_l = fd[(uint64_t)v_l * K] & dmask;
+            wc.add(WC_BYTES, 4);  // level mask word
         }
+        wide_vertices<K>(a, v_l, f_l, no_succ, fnext, msigma, mdelta, mq, reach, su, sg, wc);
     }
-}
-
-// One backward depth, device-driven: d = bi->bd (a no-op once below 0).  The
-// grid's y index is the half: the blocks of half 1 of a 64-pivot pass start as
-// those of half 0 run out of work, each half with its own work counter.  CNT:
-// the counting build (work counts into wc[KP_BWD]).
-template <int K, bool CNT>
-__global__ void __launch_bounds__(BATCH_TPB, AXBC_BWD_MIN_BLOCKS) k_bwd_step(Adj a, const BatchInfo *__restrict__ bi,
-                                                        uint32_t *const *__restrict__ tab,
-                                                        const uint32_t *__restrict__ msigma,
-                                                        float *mdelta, float *mq, float *mpartial,
-                                                        const uint32_t *__restrict__ reach,
-                                                        uint32_t *ctrs, LevelLists ll,
-                                                        unsigned long long *wc)
-{
-    typedef typename MaskOf<K>::T M;
-    __shared__ __align__(16) uint32_t s_u[BATCH_TPB];
-    __shared__ __align__(16) uint32_t s_g[BATCH_TPB];
-    const int d = bi->bd;
-    if (d < 0) return;
-    const int hh = K == 1 ? 0 : blockIdx.y;
-    const uint32_t dmask = half_of<K>((M)(d >= 1 ? bi->srcmask : bi->depth0mask), hh);
-    if (!dmask) return;
-    uint32_t *su = s_u + (threadIdx.x & ~31u), *sg = s_g + (threadIdx.x & ~31u);
-    uint32_t lcnt = 0;
-    const uint32_t *lst = level_list(ll, d, lcnt);
-    WorkCount<CNT> cnt;
-    bwd_body<K>(a, dmask, d == bi->dmax, tab[d] + hh, tab[d + 1] + hh, msigma + 32 * hh, mdelta + 32 * hh,
-                mq + 32 * hh, mpartial + 32 * hh, reach, ctrs + 2 * AXBC_MAX_LEVELS * hh + 2 * d + 1, su, sg, lst,
-                lcnt, ll.heavy[d], cnt);
-    cnt.flush(wc);
 }
 
 template <int K>
@@ -1165,20 +1535,78 @@ __device__ __forceinline__ void combine_body(const Adj &a, uint32_t dmask, const
         for (uint32_t k = a.heavy_first[i]; k < a.heavy_first[i + 1]; k++)
             acc = __fadd_rn(acc, mpartial[(uint64_t)k * (AXBC_W * K) + lane]);
         const uint32_t sig = ((f >> lane) & 1u) ? msigma[row_base<K>(v) + lane] : 0u;
-        write_dep<K>(mdelta, mq, v, f, acc, sig);
+        write_lane<K>(mdelta, mq, v, f, acc, sig);
     }
 }
 
 template <int K>
-__global__ void k_bwd_combine_step(Adj a, const BatchInfo *__restrict__ bi,
-                                   uint32_t *const *__restrict__ tab,
-                                   const uint32_t *__restrict__ msigma, float *mdelta, float *mq,
-                                   const float *__restrict__ mpartial,
-                                   const uint32_t *__restrict__ reach, LevelLists ll)
+__device__ __forceinline__ BwdHalf bwd_half(const BatchInfo *bi, uint32_t *const *tab, int d, int hh,
+                                            const uint32_t *msigma, float *mdelta, float *mq, float *mpartial,
+                                            uint32_t *harrive, uint32_t n_heavy, const uint32_t *reach)
 {
     typedef typename MaskOf<K>::T M;
-    const int d = bi->bd;
-    if (d < 0) return;
+    return BwdHalf{half_of<K>((M)(d >= 1 ? bi->srcmask : bi->depth0mask), hh), d == bi->dmax, tab[d] + hh,
+                   tab[d + 1] + hh, msigma + 32 * hh, mdelta + 32 * hh, mq + 32 * hh, mpartial + 32 * hh,
+                   harrive + (uint64_t)n_heavy * hh, reach};
+}
+
+// Backward depth d.  The grid's y index is the half: the blocks of half 1 of a
+// 64-pivot pass start as those of half 0 run out of work, each half with its
+// own work counter.  CNT: the counting build (work counts into wc[KP_BWD]).
+template <int K, bool CNT>
+__global__ void __launch_bounds__(BATCH_TPB, AXBC_BWD_TILE_BLOCKS) k_bwd_tile_step(Adj a, const BatchInfo *__restrict__ bi,
+                                                        uint32_t *const *__restrict__ tab,
+                                                        const uint32_t *__restrict__ msigma,
+                                                        float *mdelta, float *mq, float *mpartial, uint32_t *harrive,
+                                                        const uint32_t *__restrict__ reach,
+                                                        uint32_t *ctrs, LevelLists ll, int d, int symmetric,
+                                                        unsigned long long *wc)
+{
+    __shared__ uint2 s_st[BATCH_TPB / 32][36];
+    __shared__ float s_csum[2][BWD_TILE_CHUNKS][32];
+    const int hh = K == 1 ? 0 : blockIdx.y;
+    const BwdHalf B = bwd_half<K>(bi, tab, d, hh, msigma, mdelta, mq, mpartial, harrive, a.n_heavy, reach);
+    if (!B.dmask) return;
+    uint32_t lcnt = 0;
+    const uint32_t *lst = level_list(ll, d, lcnt);
+    WorkCount<CNT> cnt;
+    bwd_body<K>(a, B, ctrs + 2 * AXBC_MAX_LEVELS * hh + 2 * d + 1, s_st[threadIdx.x >> 5], s_csum, lst, lcnt,
+                ll.heavy[d], symmetric, cnt);
+    cnt.flush(wc);
+}
+
+template <int K, bool CNT>
+__global__ void __launch_bounds__(BATCH_TPB, AXBC_BWD_MIN_BLOCKS) k_bwd_step(Adj a, const BatchInfo *__restrict__ bi,
+                                                        uint32_t *const *__restrict__ tab,
+                                                        const uint32_t *__restrict__ msigma,
+                                                        float *mdelta, float *mq, float *mpartial,
+                                                        const uint32_t *__restrict__ reach,
+                                                        uint32_t *ctrs, LevelLists ll, int d,
+                                                        unsigned long long *wc)
+{
+    typedef typename MaskOf<K>::T M;
+    __shared__ __align__(16) uint32_t s_u[BATCH_TPB];
+    __shared__ __align__(16) uint32_t s_g[BATCH_TPB];
+    const int hh = K == 1 ? 0 : blockIdx.y;
+    const uint32_t dmask = half_of<K>((M)(d >= 1 ? bi->srcmask : bi->depth0mask), hh);
+    if (!dmask) return;
+    uint32_t *su = s_u + (threadIdx.x & ~31u), *sg = s_g + (threadIdx.x & ~31u);
+    uint32_t lcnt = 0;
+    const uint32_t *lst = level_list(ll, d, lcnt);
+    WorkCount<CNT> cnt;
+    bwd_body_wide<K>(a, dmask, d == bi->dmax, tab[d] + hh, tab[d + 1] + hh, msigma + 32 * hh, mdelta + 32 * hh,
+                     mq + 32 * hh, mpartial + 32 * hh, reach, ctrs + 2 * AXBC_MAX_LEVELS * hh + 2 * d + 1, su, sg, lst,
+                     lcnt, ll.heavy[d], cnt);
+    cnt.flush(wc);
+}
+
+template <int K>
+__global__ void k_bwd_combine_step(Adj a, const BatchInfo *__restrict__ bi, uint32_t *const *__restrict__ tab,
+                                   const uint32_t *__restrict__ msigma, float *mdelta, float *mq,
+                                   const float *__restrict__ mpartial, const uint32_t *__restrict__ reach,
+                                   LevelLists ll, int d)
+{
+    typedef typename MaskOf<K>::T M;
     uint32_t lcnt;
     if (level_list(ll, d, lcnt) && ll.heavy[d] == 0) return;  // no heavy vertex at this depth
     const int hh = K == 1 ? 0 : blockIdx.y;
@@ -1188,10 +1616,6 @@ __global__ void k_bwd_combine_step(Adj a, const BatchInfo *__restrict__ bi,
                     reach);
 }
 
-__global__ void k_bwd_advance(BatchInfo *bi)
-{
-    if (bi->bd >= 0) bi->bd--;
-}
 // ------------------------------------------------ persistent level loop
 // On graphs of many narrow levels (grids, roads) a level's work is a few
 // microseconds and the four launches per forward level and three per
@@ -1199,7 +1623,7 @@ __global__ void k_bwd_advance(BatchInfo *bi)
 // forward level, then every backward depth -- in one cooperative launch whose
 // blocks are all resident, with the step kernels' device bodies separated by a
 // grid barrier: two barriers per forward level (expansion | statistics and
-// level close) and one or two per backward depth.
+// level close) and one per backward depth.
 
 // Wait budget of one barrier in SM clock cycles (about 4 s at 2 GHz): a wait
 // that runs out records its site and every block returns; the host reports
@@ -1271,13 +1695,6 @@ template <int K> struct AdvanceLead {
         level_advance_warp<K>(bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max);
     }
 };
-struct BwdLead {
-    BatchInfo *bi;
-    __device__ void operator()() const
-    {
-        if (lane_id() == 0 && bi->bd >= 0) bi->bd--;
-    }
-};
 
 // The arrays the loop writes are passed without const/__restrict__, so that
 // no load of them goes through the read-only cache: they change between
@@ -1287,15 +1704,14 @@ struct BwdLead {
 template <int K>
 __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
     Adj a, Adj rv, BatchInfo *bi, uint32_t **tab, uint32_t *seen_, uint32_t *msigma, float *mdelta,
-    float *mq, float *mpartial, const uint32_t *reach, uint32_t *ctrs, LevelLists ll,
-    unsigned long long *level_te, unsigned long long *level_cnt, int32_t *level_mode,
+    float *mq, float *mpartial, uint32_t *harrive, const uint32_t *reach, uint32_t *ctrs, LevelLists ll,
+    int symmetric, unsigned long long *level_te, unsigned long long *level_cnt, int32_t *level_mode,
     uint32_t pool_cap, uint32_t list_max, uint64_t n, int lmax, GridSync *gs, long long budget)
 {
     typedef typename MaskOf<K>::T M;
-    __shared__ __align__(16) uint32_t s_u[BATCH_TPB];
-    __shared__ __align__(16) uint32_t s_g[BATCH_TPB];
     __shared__ uint2 s_st[BATCH_TPB / 32][PullShape<K>::STAGE];
-    const unsigned w0 = threadIdx.x & ~31u;
+    __shared__ float s_csum[2][BWD_TILE_CHUNKS][32];
+    uint2 *st = s_st[threadIdx.x >> 5];
     M *seen = reinterpret_cast<M *>(seen_);
     WorkCount<false> none;
     const AdvanceLead<K> adv{bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max};
@@ -1311,40 +1727,28 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
         if (vload_i(&bi->push_next))
             fwd_push_body<K>(a, fprev, fcur, seen, msigma, ctrs + 2 * L, ll, L, none);
         else
-            fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, s_st[threadIdx.x >> 5], ll, L,
-                             none);
+            fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, st, ll, L, none);
         if (!grid_barrier(gs, budget, 1, NoLead{})) return;
         stats_body<K>(n, bi, L, srcmask, fcur, seen, a.col, rv.col, reach, ll);
         if (!grid_barrier(gs, budget, 2, adv)) return;
     }
-    const BwdLead down{bi};
-    for (;;) {
-        const int d = vload_i(&bi->bd);
-        if (d < 0) break;
-        const M dmask = (M)(d >= 1 ? bi->srcmask : bi->depth0mask);
-        if (dmask) {
-            uint32_t lcnt = 0;
-            const uint32_t *lst = level_list(ll, d, lcnt);
-            const uint32_t lheavy = ll.heavy[d];
-            // the halves touch disjoint columns and have their own work
-            // counters: one phase takes both
-        #pragma unroll 1
-    for (int hh = 0; hh < K; hh++)
-                if (half_of<K>(dmask, hh))
-                    bwd_body<K>(a, half_of<K>(dmask, hh), d == bi->dmax, tab[d] + hh, tab[d + 1] + hh,
-                                msigma + 32 * hh, mdelta + 32 * hh, mq + 32 * hh, mpartial + 32 * hh, reach,
-                                ctrs + 2 * AXBC_MAX_LEVELS * hh + 2 * d + 1, s_u + w0, s_g + w0, lst, lcnt, lheavy,
-                                none);
-            if (a.n_heavy && !(lst && lheavy == 0)) {
-                if (!grid_barrier(gs, budget, 3, NoLead{})) return;
-            #pragma unroll 1
-    for (int hh = 0; hh < K; hh++)
-                    if (half_of<K>(dmask, hh))
-                        combine_body<K>(a, half_of<K>(dmask, hh), tab[d] + hh, msigma + 32 * hh, mdelta + 32 * hh,
-                                        mq + 32 * hh, mpartial + 32 * hh, reach);
-            }
+    const uint32_t n_heavy = a.n_heavy;
+    for (int d = vload_i(&bi->dmax); d >= 0; d--) {
+        if (!(d >= 1 ? bi->srcmask : bi->depth0mask)) break;
+        uint32_t lcnt = 0;
+        const uint32_t *lst = level_list(ll, d, lcnt);
+        const uint32_t lheavy = ll.heavy[d];
+        // the halves touch disjoint columns and have their own work counters:
+        // one phase takes both
+#pragma unroll 1
+        for (int hh = 0; hh < K; hh++) {
+            const BwdHalf B = bwd_half<K>(bi, tab, d, hh, msigma, mdelta, mq, mpartial, harrive, n_heavy, reach);
+            if (B.dmask)
+                bwd_body<K>(a, B, ctrs + 2 * AXBC_MAX_LEVELS * hh + 2 * d + 1, st, s_csum, lst, lcnt, lheavy,
+                            symmetric, none);
+            __syncthreads();  // the chunk sums of the next half
         }
-        if (!grid_barrier(gs, budget, 4, down)) return;
+        if (d > 0 && !grid_barrier(gs, budget, 3, NoLead{})) return;
     }
 }
 
@@ -1726,6 +2130,10 @@ int axbc_ensure_batch(axbc_ctx *c)
     ALLOC_MISSING(c->mq, n * AXBC_WMAX * 4, &c->bytes);
     ALLOC_MISSING(c->task_ctr, 64, &c->bytes);
     ALLOC_MISSING(c->mpartial, (c->g->bfwd.n_heavy_items + 1) * AXBC_WMAX * 4, &c->bytes);
+    if (!c->harrive) {
+        TRY(axbc_dalloc((void **)&c->harrive, (uint64_t)(c->g->bfwd.n_heavy + 1) * 2 * 4, &c->bytes));
+        CU(cudaMemset(c->harrive, 0, (uint64_t)(c->g->bfwd.n_heavy + 1) * 2 * 4));
+    }
     ALLOC_MISSING(c->bi, sizeof(BatchInfo), &c->bytes);
     if (!c->bi_host) CU(cudaMallocHost((void **)&c->bi_host, sizeof(BatchInfo)));
     CU(cudaMemset(c->bi, 0, sizeof(BatchInfo)));
@@ -1738,6 +2146,13 @@ int axbc_ensure_batch(axbc_ctx *c)
 // mask words per vertex for a pass of nsrc pivots
 static int width_k(int nsrc) { return nsrc > AXBC_W ? 2 : 1; }
 
+// Backward by warps (true) or with the big vertices in block tiles: tiles while
+// the pass's adjacency work is too small to keep every warp busy.  Measured
+// (us a pass of 32 / 64 pivots, warps against tiles): 0.43 M adjacency entries
+// 382 : 123 and 429 : 157, 1.8 M 334 : 196 and 372 : 339, 3.7 M 377 : 246 and
+// 451 : 469, 7.6 M 417 : 432 and 694 : 866, 31 M (64 pivots) 1590 : 2590.
+static bool bwd_wide(const axbc_graph *g, int K) { return g->m * (uint64_t)K >= AXBC_BWD_WIDE_MIN; }
+
 // dynamic kernels: as many blocks as stay resident; work comes from counters
 template <int K> static int occupancy(axbc_ctx *c)
 {
@@ -1745,7 +2160,8 @@ template <int K> static int occupancy(axbc_ctx *c)
     if (!c->dyn_blocks_per_sm[i]) {
         int a = 0, b = 0, d = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fwd_push_step<K, false>, BATCH_TPB, 0));
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_bwd_step<K, false>, BATCH_TPB, 0));
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &b, bwd_wide(c->g, K) ? (const void *)k_bwd_step<K, false> : (const void *)k_bwd_tile_step<K, false>, BATCH_TPB, 0));
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_fwd_pull_step<K, false>, BATCH_TPB, 0));
         c->dyn_blocks_per_sm[i] = std::max(1, a);
         c->pull_blocks_per_sm[i] = std::max(1, d);
@@ -1755,9 +2171,8 @@ template <int K> static int occupancy(axbc_ctx *c)
 }
 template <int K> static int push_grid(axbc_ctx *c) { return axbc_grid_for(c, BATCH_TPB, c->dyn_blocks_per_sm[K - 1]); }
 template <int K> static int pull_grid(axbc_ctx *c) { return axbc_grid_for(c, BATCH_TPB, c->pull_blocks_per_sm[K - 1]); }
-template <int K> static int bwd_grid(axbc_ctx *c) { return axbc_grid_for(c, BATCH_TPB, c->bwd_blocks_per_sm[K - 1]); }
 
-// the kernels of one forward level / one backward depth, in stream order
+// the kernels of one forward level, in stream order; one backward depth
 template <int K> static void fwd_step_kernels(axbc_ctx *c, int sgrid)
 {
     axbc_graph *g = c->g;
@@ -1772,50 +2187,56 @@ template <int K> static void fwd_step_kernels(axbc_ctx *c, int sgrid)
                                                 c->lpool_cap, list_max_of(c));
 }
 
-template <int K> static void bwd_step_kernels(axbc_ctx *c)
+template <int K> static void bwd_step_kernel(axbc_ctx *c, int d, unsigned long long *wc)
 {
     axbc_graph *g = c->g;
-    k_bwd_step<K, false><<<dim3(bwd_grid<K>(c), K), BATCH_TPB, 0, c->stream>>>(g->bfwd, c->bi, c->fmtab, c->msigma,
-                                                                     c->mdelta, c->mq, c->mpartial, g->breach,
-                                                                     c->ctrs, lists_of(c), nullptr);
-    if (g->bfwd.n_heavy)
-        k_bwd_combine_step<K><<<dim3((g->bfwd.n_heavy + 7) / 8, K), 256, 0, c->stream>>>(
-            g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, lists_of(c));
-    k_bwd_advance<<<1, 1, 0, c->stream>>>(c->bi);
+    const dim3 grid(axbc_grid_for(c, BATCH_TPB, c->bwd_blocks_per_sm[K - 1]), K);
+    cudaStream_t s = c->stream;
+    if (!bwd_wide(g, K)) {
+        (wc ? k_bwd_tile_step<K, true> : k_bwd_tile_step<K, false>)<<<grid, BATCH_TPB, 0, s>>>(
+            g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, c->harrive, g->breach, c->ctrs,
+            lists_of(c), d, g->symmetric, wc);
+        return;
+    }
+    (wc ? k_bwd_step<K, true> : k_bwd_step<K, false>)<<<grid, BATCH_TPB, 0, s>>>(
+        g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, c->ctrs, lists_of(c), d, wc);
+}
+
+template <int K> static void combine_step_kernel(axbc_ctx *c, int d)
+{
+    axbc_graph *g = c->g;
+    k_bwd_combine_step<K><<<dim3((g->bfwd.n_heavy + 7) / 8, K), 256, 0, c->stream>>>(
+        g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, lists_of(c), d);
 }
 
 static void drop_captures(axbc_ctx *c)
 {
     for (int i = 0; i < 2; i++) {
         if (c->fwd_step_exec[i]) cudaGraphExecDestroy(c->fwd_step_exec[i]);
-        if (c->bwd_step_exec[i]) cudaGraphExecDestroy(c->bwd_step_exec[i]);
-        c->fwd_step_exec[i] = c->bwd_step_exec[i] = nullptr;
+        c->fwd_step_exec[i] = nullptr;
     }
 }
 
-// Capture one forward step and one backward step of width K as CUDA graphs;
-// every argument is fixed for the context (levels come from device state).
+// Capture one forward step of width K as a CUDA graph; every argument is fixed
+// for the context (levels come from device state).
 template <int K> static int capture_steps(axbc_ctx *c, int sgrid)
 {
     const int i = K - 1;
-    if (c->fwd_step_exec[i] && c->bwd_step_exec[i]) return AXBC_OK;
-    for (int which = 0; which < 2; which++) {
-        cudaGraph_t gr = nullptr;
-        CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        if (which == 0) fwd_step_kernels<K>(c, sgrid);
-        else bwd_step_kernels<K>(c);
-        cudaError_t e = cudaStreamEndCapture(c->stream, &gr);
-        if (e != cudaSuccess) return axbc_cuda_fail(e, "capture level step", __FILE__, __LINE__);
-        e = cudaGraphInstantiate(which == 0 ? &c->fwd_step_exec[i] : &c->bwd_step_exec[i], gr, 0);
-        cudaGraphDestroy(gr);
-        if (e != cudaSuccess) return axbc_cuda_fail(e, "instantiate level step", __FILE__, __LINE__);
-    }
+    if (c->fwd_step_exec[i]) return AXBC_OK;
+    cudaGraph_t gr = nullptr;
+    CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    fwd_step_kernels<K>(c, sgrid);
+    cudaError_t e = cudaStreamEndCapture(c->stream, &gr);
+    if (e != cudaSuccess) return axbc_cuda_fail(e, "capture level step", __FILE__, __LINE__);
+    e = cudaGraphInstantiate(&c->fwd_step_exec[i], gr, 0);
+    cudaGraphDestroy(gr);
+    if (e != cudaSuccess) return axbc_cuda_fail(e, "instantiate level step", __FILE__, __LINE__);
     return AXBC_OK;
 }
 
 // Forward levels and backward depths as launches of the step kernels: CUDA
-// graph replays of one level step, in blocks (profiling and counting: each
-// kernel launched on its own).  *L_out: the first level that discovered
+// graph replays of one forward level, in blocks (profiling and counting: each
+// kernel launched on its own), then one launch per depth.  *L_out: the first level that discovered
 // nothing.
 template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, int *L_out)
 {
@@ -1826,7 +2247,7 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
     unsigned long long *wc = c->count_on ? c->wcount : nullptr;
     const LevelLists ll = lists_of(c);
     const uint32_t lmax = list_max_of(c);
-    const size_t ctl_off = offsetof(BatchInfo, cur);
+    const size_t ctl_off = offsetof(BatchInfo, depth0mask);
     const size_t ctl_len = offsetof(BatchInfo, push_factor) - ctl_off;
     const size_t prof_first = c->prof.size();
     // forward steps launched before the first look at `alive`: one more than
@@ -1896,11 +2317,10 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
         lte.resize(L + 1);
         lcnt.resize(L + 1);
         lmode.resize(L + 1);
-        // one wait for the three per-level arrays and the depth-0 mask
+        // one wait for the three per-level arrays
         CU(cudaMemcpyAsync(lte.data(), c->d_level_te, (L + 1) * 8, cudaMemcpyDeviceToHost, s));
         CU(cudaMemcpyAsync(lcnt.data(), c->d_level_cnt, (L + 1) * 8, cudaMemcpyDeviceToHost, s));
         CU(cudaMemcpyAsync(lmode.data(), c->d_level_mode, (L + 1) * 4, cudaMemcpyDeviceToHost, s));
-        CU(cudaMemcpyAsync(&c->bi_host->depth0mask, &c->bi->depth0mask, 8, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         const double W = nsrc;
         for (size_t i = prof_first; i < c->prof.size(); i++) {
@@ -1917,15 +2337,16 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
     }
 
     // backward: depths Dmax .. 0 (depth 0 only for pivots whose BFS ended at level 2)
-    unsigned long long depth0 = 0;
+    const unsigned long long depth0 = c->bi_host->depth0mask;
     if (Dmax >= 0) {
-        for (int d = Dmax; d >= 0; d--) {
+        for (int d = Dmax; d >= (depth0 ? 0 : 1); d--) {
+            const bool combine = bwd_wide(g, K) && g->bfwd.n_heavy > 0;
             if (!prof) {
-                CU(cudaGraphLaunch(c->bwd_step_exec[K - 1], s));
-                c->launches += g->bfwd.n_heavy ? 3 : 2;
+                bwd_step_kernel<K>(c, d, nullptr);
+                if (combine) combine_step_kernel<K>(c, d);
+                c->launches += combine ? 2 : 1;
                 continue;
             }
-            if (d == Dmax && c->prof_on) depth0 = c->bi_host->depth0mask;
             const double W = nsrc;
             double bytes = 0.0;
             if (c->prof_on) {
@@ -1940,22 +2361,12 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
             {
                 ProfScope ps(c, KP_BWD, bytes);
                 if (c->prof_on) c->prof.back().tag = d;
-                if (wc)
-                    k_bwd_step<K, true><<<dim3(bwd_grid<K>(c), K), BATCH_TPB, 0, s>>>(
-                        g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, c->ctrs, ll,
-                        wc + KP_BWD * WC_NFIELDS);
-                else
-                    k_bwd_step<K, false><<<dim3(bwd_grid<K>(c), K), BATCH_TPB, 0, s>>>(
-                        g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, c->ctrs, ll,
-                        nullptr);
+                bwd_step_kernel<K>(c, d, wc ? wc + KP_BWD * WC_NFIELDS : nullptr);
             }
-            if (g->bfwd.n_heavy) {
+            if (combine) {
                 ProfScope ps(c, KP_BWD_COMBINE, 0);
-                k_bwd_combine_step<K><<<dim3((g->bfwd.n_heavy + 7) / 8, K), 256, 0, s>>>(
-                    g->bfwd, c->bi, c->fmtab, c->msigma, c->mdelta, c->mq, c->mpartial, g->breach, ll);
+                combine_step_kernel<K>(c, d);
             }
-            k_bwd_advance<<<1, 1, 0, s>>>(c->bi);
-            c->launches++;
         }
         CU_LAUNCH("backward levels");
     }
@@ -2011,8 +2422,8 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
         int lmax = levels;
         void *args[] = {(void *)&g->bfwd, (void *)&g->brev, (void *)&c->bi, (void *)&c->fmtab,
                         (void *)&c->seen, (void *)&c->msigma, (void *)&c->mdelta, (void *)&c->mq,
-                        (void *)&c->mpartial, (void *)&g->breach, (void *)&c->ctrs, (void *)&ll,
-                        (void *)&c->d_level_te, (void *)&c->d_level_cnt, (void *)&c->d_level_mode,
+                        (void *)&c->mpartial, (void *)&c->harrive, (void *)&g->breach, (void *)&c->ctrs,
+                        (void *)&ll, (void *)&g->symmetric, (void *)&c->d_level_te, (void *)&c->d_level_cnt, (void *)&c->d_level_mode,
                         (void *)&pool_cap, (void *)&lmax_list, (void *)&n, (void *)&lmax,
                         (void *)&c->gsync, (void *)&budget};
         {
@@ -2033,7 +2444,7 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
         }
         levels *= 2;
     }
-    const size_t ctl_off = offsetof(BatchInfo, cur);
+    const size_t ctl_off = offsetof(BatchInfo, depth0mask);
     const size_t ctl_len = offsetof(BatchInfo, push_factor) - ctl_off;
     CU(cudaMemcpyAsync((char *)c->bi_host + ctl_off, (char *)c->bi + ctl_off, ctl_len, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));

@@ -21,6 +21,9 @@
 #define AXBC_SAMPLE_BLOCK 1024
 // Vertices with more than AXBC_BIG neighbours are split over several warps.
 #define AXBC_BIG 128
+// A backward tile holds at most this many 32-position chunks.
+#define BWD_TILE_CHUNKS 32
+#define BWD_SPAN_TILE 0x80000000u
 #define AXBC_W 32     // lanes of a warp, pivots per mask word
 #define AXBC_WMAX 64  // pivots of one multi-source pass (two mask words per vertex)
 #define FULL_MASK 0xffffffffu
@@ -85,6 +88,11 @@ struct Adj {
     uint2 *part = nullptr;            // n_part
     uint64_t n_part = 0;
     uint32_t part_len = 0;
+    // the backward kernel's tiles of the big vertices: (index into order,
+    // number of vertices), or (index, BWD_SPAN_TILE | span) for a span of a
+    // heavy vertex; the heavy tiles come first, a vertex's spans in order
+    uint2 *tile = nullptr;            // n_tile
+    uint32_t n_tile = 0;
     bool owns = true;
 };
 
@@ -143,7 +151,6 @@ struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     uint32_t pad0;
     unsigned long long applymask;   // sources whose update is applied (Bader replay)
     unsigned long long srcmask;
-    unsigned long long depth0mask;  // sources whose BFS ended at level 2
     uint32_t root[AXBC_WMAX];
     double p[AXBC_WMAX];
     // per-source totals accumulated by the level-stats kernel
@@ -161,11 +168,11 @@ struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     int32_t H;
     // device-driven level loop: the step kernels read their level and
     // direction here, the advance kernels move them on
+    unsigned long long depth0mask;  // sources whose BFS ended at level 2
     int32_t cur;        // last completed forward level
     int32_t alive;      // 1 while the last completed level discovered vertices
     int32_t lend;       // first level that discovered nothing (once alive == 0)
     int32_t dmax;       // deepest depth = lend - 1
-    int32_t bd;         // next backward depth (counts down to -1)
     int32_t push_next;  // 1: the next forward level pushes from the frontier
     double push_factor;
     unsigned long long push_min;  // frontier degree sums below this always push
@@ -259,7 +266,8 @@ struct axbc_ctx {
     float *mdelta = nullptr;        // n*32
     float *mq = nullptr;            // n*32: (delta + 1) / sigma, per pivot
     uint32_t *task_ctr = nullptr;   // work counters of the dynamic kernels
-    float *mpartial = nullptr;      // heavy items * 32
+    float *mpartial = nullptr;      // span sums of the heavy vertices, 64 per span
+    uint32_t *harrive = nullptr;    // per half and heavy vertex: span sums written (0 between depths)
     BatchInfo *bi = nullptr;
     BatchInfo *bi_host = nullptr;  // pinned
     uint32_t **fmtab = nullptr;               // device copy of the fmask pointers
@@ -272,9 +280,8 @@ struct axbc_ctx {
     uint32_t lpool_cap = 0;
     bool pool_short = false;  // the last batch ran out of list space
     int prev_lend = 0;        // levels of the last batch whose masks need clearing
-    // captured forward / backward level steps, per width (index K - 1)
+    // captured forward level step, per width (index K - 1)
     cudaGraphExec_t fwd_step_exec[2] = {nullptr, nullptr};
-    cudaGraphExec_t bwd_step_exec[2] = {nullptr, nullptr};
     int last_batch_levels = 0;
     int last_batch_nsrc = 0;
     int last_batch_k = 1;  // mask words per vertex of the last batch (1: <= 32 pivots, 2: <= 64)

@@ -181,6 +181,25 @@ static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, u
     a.n_part = part.size();
     TRY(axbc_dalloc((void **)&a.part, part.size() * sizeof(uint2), acct));
     if (!part.empty()) CU(cudaMemcpy(a.part, part.data(), part.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    // tiles of the big vertices: single spans, then groups of vertices
+    std::vector<uint2> tile;
+    for (uint32_t j = 0; j < a.n_big;) {
+        if (deg(j) > AXBC_SPAN) {
+            for (uint32_t k = 0; k * AXBC_SPAN < deg(j); k++) tile.push_back(make_uint2(j, BWD_SPAN_TILE | k));
+            j++;
+            continue;
+        }
+        uint32_t cnt = 0, chunks = 0;
+        for (; j + cnt < a.n_big; cnt++) {
+            chunks += (deg(j + cnt) + AXBC_CHUNK - 1) / AXBC_CHUNK;
+            if (chunks > BWD_TILE_CHUNKS) break;
+        }
+        tile.push_back(make_uint2(j, cnt));
+        j += cnt;
+    }
+    a.n_tile = (uint32_t)tile.size();
+    TRY(axbc_dalloc((void **)&a.tile, tile.size() * sizeof(uint2), acct));
+    if (!tile.empty()) CU(cudaMemcpy(a.tile, tile.data(), tile.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     return AXBC_OK;
 }
 
@@ -305,6 +324,7 @@ static void free_adj(Adj &a)
     axbc_dfree(a.order);
     axbc_dfree(a.ltask);
     axbc_dfree(a.part);
+    axbc_dfree(a.tile);
     a = Adj();
 }
 
