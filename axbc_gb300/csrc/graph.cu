@@ -942,100 +942,6 @@ int axbc_build_deg_dist(axbc_graph *g, cudaStream_t s)
     return AXBC_OK;
 }
 
-// |adj(w) ∩ adj(i)| without i, by binary search of the shorter list's entries
-// in the longer one (adjacency lists are sorted and duplicate-free)
-__device__ __forceinline__ uint32_t isect_count(const uint32_t *a, uint32_t da, const uint32_t *b,
-                                                uint32_t db, uint32_t skip)
-{
-    if (da > db) {
-        const uint32_t *t = a;
-        a = b;
-        b = t;
-        uint32_t td = da;
-        da = db;
-        db = td;
-    }
-    uint32_t c = 0;
-    for (uint32_t k = 0; k < da; k++) {
-        uint32_t x = a[k];
-        if (x == skip) continue;
-        uint32_t lo = 0, hi = db;
-        while (lo < hi) {
-            uint32_t mid = (lo + hi) >> 1;
-            if (b[mid] < x) lo = mid + 1;
-            else hi = mid;
-        }
-        c += (lo < db && b[lo] == x);
-    }
-    return c;
-}
-
-// lcc_func (src/axbc2d.c:1847-1935): counter(i) = sum over neighbours w of
-// |adj(w) \ {i} ∩ adj(i)|, uint32.  Lanes take neighbours; vertices with more
-// than SPAN neighbours are split over their span items.
-__global__ void k_lcc_count(Adj a, uint32_t *__restrict__ counter)
-{
-    const unsigned lane = lane_id();
-    const uint64_t ntask = a.n + a.n_heavy_items;
-    const uint64_t nw = (uint64_t)gridDim.x * blockDim.x / 32;
-    for (uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; t < ntask; t += nw) {
-        uint32_t i, b0, b1;
-        if (t < a.n) {
-            i = (uint32_t)t;
-            uint32_t d = a.col[i + 1] - a.col[i];
-            if (d < 2 || d > AXBC_SPAN) continue;
-            b0 = a.col[i];
-            b1 = a.col[i + 1];
-        } else {
-            i = a.hitem_v[t - a.n];
-            uint32_t k = a.hitem_k[t - a.n];
-            b0 = a.col[i] + k * AXBC_SPAN;
-            b1 = min(a.col[i + 1], b0 + AXBC_SPAN);
-        }
-        const uint32_t *ai = a.row + a.col[i];
-        const uint32_t di = a.col[i + 1] - a.col[i];
-        uint32_t c = 0;
-        for (uint32_t e = b0 + lane; e < b1; e += 32) {
-            uint32_t w = a.row[e];
-            c += isect_count(a.row + a.col[w], a.col[w + 1] - a.col[w], ai, di, i);
-        }
-        c = __reduce_add_sync(FULL_MASK, c);
-        if (lane == 0 && c) atomicAdd(&counter[i], c);
-    }
-}
-
-__global__ void k_lcc_final(const uint32_t *__restrict__ col, const uint32_t *__restrict__ counter,
-                            float *__restrict__ out, uint64_t n)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t d = col[i + 1] - col[i];
-        out[i] = (d < 2) ? 0.0f
-                         : __fdiv_rn(__uint2float_rn(counter[i]), __uint2float_rn(d * (d - 1u)));
-    }
-}
-
-int axbc_build_lcc(axbc_graph *g, cudaStream_t s)
-{
-    if (g->have_lcc) return AXBC_OK;
-    const uint64_t n = g->n;
-    DBuf cnt;
-    TRY(cnt.alloc(n * 4));
-    ALLOC_MISSING(g->lcc, n * 4, &g->bytes);
-    ALLOC_MISSING(g->lcc_local, n * 8, &g->bytes);
-    ALLOC_MISSING(g->lcc_csum, ((n + AXBC_SAMPLE_BLOCK - 1) / AXBC_SAMPLE_BLOCK) * 8, &g->bytes);
-    CU(cudaMemsetAsync(cnt.p, 0, n * 4, s));
-    k_lcc_count<<<4096, 256, 0, s>>>(g->fwd, cnt.as<uint32_t>());
-    k_lcc_final<<<1024, 256, 0, s>>>(g->fwd.col, cnt.as<uint32_t>(), g->lcc, n);
-    CU_LAUNCH("lcc");
-    TRY(axbc_hprefix_launch(g->lcc, n, g->lcc_local, g->lcc_csum, s));
-    const uint64_t nb = (n + AXBC_SAMPLE_BLOCK - 1) / AXBC_SAMPLE_BLOCK;
-    CU(cudaMemcpyAsync(&g->S_lcc, g->lcc_csum + nb - 1, 8, cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
-    g->have_lcc = true;
-    return AXBC_OK;
-}
-
 extern "C" int axbc_graph_degree2(axbc_graph *g, uint32_t *out_host)
 {
     CHECK_ARG(g && out_host, "axbc_graph_degree2: null argument");

@@ -46,3 +46,30 @@ def test_degree_edges(axbc, orc, undirected, k, factor):
         _, lvl, sigma, delta, _ = orc.bc_pivot(g, int(piv[s]), p[s])
         gs, gl, gd = ctx.batch_source(s)
         assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl) and np.array_equal(gd, delta), s
+
+
+@pytest.mark.parametrize("n", [3, 65, 66, 67, 129, 2048, 2049, 2051])
+def test_clustering_of_complete_graphs(axbc, n):
+    # a vertex's higher neighbours number up to n - 1: every table size, and
+    # more members than a block's table holds.  A fan of leaves around vertex 0
+    # makes the graph's largest degree exceed 64, so that ranks exist
+    u, v = np.triu_indices(n, 1)
+    leaves = 80
+    e = np.concatenate([np.stack([u, v], 1), np.stack([np.zeros(leaves, int), n + np.arange(leaves)], 1)])
+    lcc = axbc.Graph.from_edges(e.astype(np.uint64), n + leaves).lcc()
+    d = np.float32(n - 1 + leaves)
+    want = np.concatenate([[np.float32((n - 1) * (n - 2)) / (d * (d - 1))], np.ones(n - 1), np.zeros(leaves)])
+    assert np.array_equal(lcc, want.astype(np.float32))
+
+
+@pytest.mark.parametrize("H", [0, 1])
+def test_clustering_of_a_power_law_graph(axbc, orc, H):
+    e = axbc.kron_edges(12, 16)
+    g = orc.pipeline(e.astype(np.uint64), 1 << 12, True, H)
+    assert np.array_equal(axbc.Graph.from_csc(g.col, g.row, g.reach).lcc(), orc.lcc(g))
+    # a self-loop or a repeated entry takes the general count
+    col, row = g.col.copy(), g.row.copy()
+    v = int(np.flatnonzero(g.deg > 2)[5])
+    row[col[v]] = row[col[v] + 1]
+    h = orc.CSC(col, row)
+    assert np.array_equal(axbc.Graph.from_csc(col, row).lcc(), orc.lcc(h))
