@@ -213,7 +213,6 @@ extern "C" int axbc_ctx_destroy(axbc_ctx *c)
     axbc_dfree(c->bc);
     axbc_dfree(c->delta_last);
     axbc_dfree(c->wcount);
-    axbc_dfree(c->gsync);
     axbc_dfree(c->lvl);
     axbc_dfree(c->sigma);
     axbc_dfree(c->delta);
@@ -226,7 +225,6 @@ extern "C" int axbc_ctx_destroy(axbc_ctx *c)
     axbc_dfree(c->msigma);
     axbc_dfree(c->mdelta);
     axbc_dfree(c->mq);
-    axbc_dfree(c->task_ctr);
     axbc_dfree(c->fmtab);
     axbc_dfree(c->ctrs);
     axbc_dfree(c->d_level_te);
@@ -253,6 +251,8 @@ extern "C" int axbc_ctx_destroy(axbc_ctx *c)
     axbc_dfree(c->dyn_local2);
     axbc_dfree(c->dyn_csum2);
     axbc_dfree(c->wtmp);
+    axbc_dfree(c->hist_v);
+    axbc_dfree(c->hist_p);
     prof_clear(c);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
     if (c->rb_ev) cudaEventDestroy(c->rb_ev);

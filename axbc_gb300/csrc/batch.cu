@@ -47,8 +47,8 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
 
 // resident blocks per SM the kernels are compiled for (their register
 // budgets); the backward runs 32 pivots at a time at either width
-#ifndef AXBC_PULL_MIN_BLOCKS
-#define AXBC_PULL_MIN_BLOCKS 7
+#ifndef AXBC_FWD_MIN_BLOCKS
+#define AXBC_FWD_MIN_BLOCKS 7
 #endif
 #ifndef AXBC_BWD_MIN_BLOCKS
 #define AXBC_BWD_MIN_BLOCKS 8
@@ -59,14 +59,10 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
 #ifndef AXBC_BWD_WIDE_MIN
 #define AXBC_BWD_WIDE_MIN (1u << 22)
 #endif
-#ifndef AXBC_PUSH_MIN_BLOCKS2
-#define AXBC_PUSH_MIN_BLOCKS2 5
+#ifndef AXBC_FWD_MIN_BLOCKS2
+#define AXBC_FWD_MIN_BLOCKS2 4
 #endif
-#ifndef AXBC_PULL_MIN_BLOCKS2
-#define AXBC_PULL_MIN_BLOCKS2 4
-#endif
-#define PUSH_BLOCKS(K) ((K) == 1 ? 8 : AXBC_PUSH_MIN_BLOCKS2)
-#define PULL_BLOCKS(K) ((K) == 1 ? AXBC_PULL_MIN_BLOCKS : AXBC_PULL_MIN_BLOCKS2)
+#define FWD_BLOCKS(K) ((K) == 1 ? AXBC_FWD_MIN_BLOCKS : AXBC_FWD_MIN_BLOCKS2)
 
 // Per-level vertex lists: the vertices whose level-L mask is nonzero, appended
 // by the forward kernels that set the mask.  A level whose list would exceed
@@ -77,48 +73,68 @@ struct LevelLists {
     uint32_t *start;  // per level: offset into pool
     uint32_t *count;  // per level: vertices appended
     uint32_t *cap;    // per level: capacity
-    uint32_t *heavy;  // per level: listed vertices with more than AXBC_BIG neighbours
+    uint32_t *heavy;  // per level: listed vertices with more than Adj::big neighbours
 };
 
 
-// Clear the level masks first..last of the previous batch (levels 0 and 1
-// are cleared with memsets): a level whose list was stored has nonzero
-// entries only at its listed vertices; an overflowed level is cleared whole.
-// The grid walks the levels in order, all blocks sharing each level.
-template <int K>
-__global__ void k_clean_levels(uint32_t *const *__restrict__ tab, const uint32_t *__restrict__ pool,
-                               const uint32_t *__restrict__ lstart,
-                               const uint32_t *__restrict__ lcount,
-                               const uint32_t *__restrict__ lcap, uint64_t n, int first, int last)
+// What a pass starts from.
+struct PassStart {
+    BatchInfo *bi;
+    uint32_t **tab;
+    uint32_t *seen, *msigma, *ctrs;
+    LevelLists ll;
+    unsigned long long *level_te, *level_cnt;
+    const uint32_t *col, *rcol, *reach, *to_view;
+    float *bc;
+    uint64_t n;
+    unsigned long long m, push_min;
+    double push_factor;
+    uint32_t pool_cap, list_max, big;
+    int nsrc, H;
+    int prev_k, prev_last;  // mask words of the previous pass, last level it may have touched
+};
+
+// zero `bytes` (a multiple of 4) from the 16-byte aligned p, all threads of the grid
+__device__ __forceinline__ void grid_zero(void *p, uint64_t bytes, uint64_t tid, uint64_t nt)
 {
-    typedef typename MaskOf<K>::T M;
-    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
-    for (int L = first; L <= last; L++) {
-        M *f = reinterpret_cast<M *>(tab[L]);
-        const uint32_t cnt = lcount[L];
-        if (cnt <= lcap[L]) {
-            const uint32_t *lst = pool + lstart[L];
+    uint4 *q = reinterpret_cast<uint4 *>(p);
+    for (uint64_t i = tid; i < bytes / 16; i += nt) q[i] = make_uint4(0, 0, 0, 0);
+    uint32_t *t = reinterpret_cast<uint32_t *>(q + bytes / 16);
+    if (tid < bytes % 16 / 4) t[tid] = 0;
+}
+
+// Level masks 2..last of the previous pass, width PK: a level whose list was
+// stored has nonzero entries only at its listed vertices; an overflowed level
+// is cleared whole.
+template <int PK>
+__device__ __forceinline__ void clean_levels(const PassStart &P, uint64_t tid, uint64_t nt)
+{
+    typedef typename MaskOf<PK>::T M;
+    for (int L = 2; L <= P.prev_last; L++) {
+        M *f = reinterpret_cast<M *>(P.tab[L]);
+        const uint32_t cnt = P.ll.count[L];
+        if (cnt <= P.ll.cap[L]) {
+            const uint32_t *lst = P.ll.pool + P.ll.start[L];
             for (uint64_t i = tid; i < cnt; i += nt) f[lst[i]] = 0;
         } else {
-            for (uint64_t i = tid; i < n; i += nt) f[i] = 0;
+            for (uint64_t i = tid; i < P.n; i += nt) f[i] = 0;
         }
     }
 }
 
-// roots: depth 0, sigma 1 (set_mlp_cuda, src/cuda_kernels.cu:862-876); one
-// warp, lane l setting up pivots l + 32 h
+// Roots: depth 0, sigma 1 (set_mlp_cuda, src/cuda_kernels.cu:862-876); one
+// warp, lane l setting up pivots l + 32 h.
 template <int K>
-__global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t *fmask0_, uint32_t *seen_,
-                             uint32_t *msigma, const uint32_t *__restrict__ col,
-                             const uint32_t *__restrict__ rcol, unsigned long long m,
-                             double push_factor, unsigned long long push_min,
-                             unsigned long long *level_te,
-                             unsigned long long *level_cnt, LevelLists ll, uint32_t pool_cap,
-                             uint32_t list_max, const uint32_t *__restrict__ to_view)
+__device__ __forceinline__ void pass_roots(const PassStart &P)
 {
     typedef typename MaskOf<K>::T M;
-    M *fmask0 = reinterpret_cast<M *>(fmask0_), *seen = reinterpret_cast<M *>(seen_);
+    BatchInfo *bi = P.bi;
+    const LevelLists &ll = P.ll;
+    M *fmask0 = reinterpret_cast<M *>(P.tab[0]), *seen = reinterpret_cast<M *>(P.seen);
+    uint32_t *msigma = P.msigma;
+    const uint32_t *to_view = P.to_view, *col = P.col, *rcol = P.rcol;
+    const int nsrc = P.nsrc, H = P.H;
+    const uint32_t pool_cap = P.pool_cap, list_max = P.list_max;
     const int l = threadIdx.x;
     // the roots arrive as vertex ids; the pass runs in the graph's view
     if (to_view) {
@@ -137,10 +153,11 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         bi->alive = 1;
         bi->lend = 0;
         bi->dmax = -1;
-        bi->push_factor = push_factor;
+        bi->push_factor = P.push_factor;
         bi->lvl_te = 0;
         bi->any_new = 0;
         bi->pool_short = 0;
+        bi->gs = GridSync{0, 0, 0, 0};
     }
     unsigned long long fd = 0, rd = 0;
     uint32_t nroots = 0, heavy_roots = 0;
@@ -150,9 +167,11 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         const int s = l + 32 * h;
         bi->Ls[s] = 0;
         bi->lvl_new[s] = 0;
-        bi->lane_bc[s] = bc;
+        bi->lane_bc[s] = P.bc;
+        bi->root_reach[s] = 0;
         if (s < nsrc) {
             const uint32_t v = bi->root[s];
+            bi->root_reach[s] = P.reach[v];
             atomicOr(&fmask0[v], lane_mask<M>(s));
             atomicOr(&seen[v], lane_mask<M>(s));
             msigma[row_base<K>(v) + s] = 1;
@@ -178,7 +197,7 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         const uint32_t firsts = __ballot_sync(FULL_MASK, first);
         if (first) ll.pool[nroots + __popc(firsts & ((1u << l) - 1u))] = rt;
         nroots += __popc(firsts);
-        heavy_roots += __popc(__ballot_sync(FULL_MASK, first && col[rt + 1] - col[rt] > AXBC_BIG));
+        heavy_roots += __popc(__ballot_sync(FULL_MASK, first && col[rt + 1] - col[rt] > P.big));
     }
     for (int o = 16; o; o >>= 1) {
         fd += __shfl_xor_sync(FULL_MASK, fd, o);
@@ -188,20 +207,60 @@ __global__ void k_batch_init(BatchInfo *bi, int nsrc, int H, float *bc, uint32_t
         ll.heavy[0] = heavy_roots;
         // a vertex counts as unvisited until every pivot has seen it: with one
         // pivot its root is fully seen at once
-        const unsigned long long unvis = nsrc == 1 ? m - rd : m;
+        const unsigned long long unvis = nsrc == 1 ? P.m - rd : P.m;
         bi->front_deg = 0;
         bi->unvis_deg = unvis;
         bi->unvis_dec = 0;
-        bi->push_min = push_min;
-        bi->push_next = (double)fd * push_factor < (double)unvis || fd < push_min;
-        level_te[0] = fd;
-        level_cnt[0] = nsrc;
+        bi->push_min = P.push_min;
+        bi->push_next = (double)fd * P.push_factor < (double)unvis || fd < P.push_min;
+        P.level_te[0] = fd;
+        P.level_cnt[0] = nsrc;
         ll.start[0] = 0;
         ll.count[0] = nroots;
         ll.cap[0] = nroots;
         ll.start[1] = nroots;
         ll.cap[1] = min(list_max, pool_cap - nroots);
     }
+}
+
+// The last block of a launch to get here (all its threads call); its later
+// loads past L1 see what every block wrote before calling.  The count wraps to
+// zero by itself.
+__device__ __forceinline__ bool last_block(uint32_t *ticket)
+{
+    __shared__ int s_last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    return s_last != 0;
+}
+
+// Everything a pass finds zero, and its roots, in one launch (it took ten: the
+// memsets of five arrays and three tables, the clearing of the level masks and
+// the roots, about 30 us of a 400-us pass at scale 14).  The last block clears
+// the per-level tables, which the others read, and sets the roots.
+template <int K>
+__global__ void __launch_bounds__(256) k_pass_start(PassStart P)
+{
+    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
+    grid_zero(P.seen, P.n * 4 * K, tid, nt);
+    grid_zero(P.tab[0], P.n * 4 * K, tid, nt);
+    grid_zero(P.tab[1], P.n * 4 * K, tid, nt);
+    grid_zero(P.msigma, P.n * AXBC_W * K * 4, tid, nt);
+    if (P.prev_k == 2) clean_levels<2>(P, tid, nt);
+    else clean_levels<1>(P, tid, nt);
+    if (!last_block(&P.bi->ticket[0])) return;
+    const int used = min(P.prev_last + 4, AXBC_MAX_LEVELS);
+    for (int i = threadIdx.x; i < 2 * used; i += blockDim.x)
+        P.ctrs[i] = P.ctrs[2 * AXBC_MAX_LEVELS + i] = 0;
+    for (int i = threadIdx.x; i < used; i += blockDim.x) P.ll.count[i] = P.ll.heavy[i] = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) pass_roots<K>(P);
 }
 
 // ---------------------------------------------------------- task scheduling
@@ -420,10 +479,19 @@ __device__ __forceinline__ void fwd_push_body(const Adj &a, const typename MaskO
         M f_l = 0;
         if (lane < ent && i < nl) {
             v_l = lst ? lst[i] : a.order[a.n_big + i];
-            if (a.col[v_l + 1] - a.col[v_l] <= AXBC_BIG) f_l = fprev[v_l];
+            if (a.col[v_l + 1] - a.col[v_l] <= a.big) f_l = fprev[v_l];
             wc.add(WC_BYTES, lst ? 4 + 4 * K : 4 * K);  // list entry, level mask
         }
-        push_light32<K>(a, v_l, f_l, seen, fcur, msigma, ll, L, wc);
+        // a vertex that fills half a chunk or more by itself: its path counts
+        // load once; the others share chunks
+        const uint32_t b_l = f_l ? a.col[v_l] : 0u, e_l = f_l ? a.col[v_l + 1] : 0u;
+        for (unsigned act = __ballot_sync(FULL_MASK, e_l - b_l >= 16); act; act &= act - 1) {
+            const int j = __ffs(act) - 1;
+            push_span<K>(a, __shfl_sync(FULL_MASK, v_l, j), __shfl_sync(FULL_MASK, f_l, j),
+                         __shfl_sync(FULL_MASK, b_l, j), __shfl_sync(FULL_MASK, e_l, j), seen, fcur, msigma, ll, L, wc);
+        }
+        if (e_l - b_l >= 16) f_l = 0;
+        if (__any_sync(FULL_MASK, f_l != 0)) push_light32<K>(a, v_l, f_l, seen, fcur, msigma, ll, L, wc);
     }
 }
 
@@ -546,7 +614,7 @@ __device__ __forceinline__ void pull_part(const Adj &rv, uint32_t u, typename Ma
     list_append(ll, L, first, u);
 }
 
-// Up to 32 vertices of at most AXBC_BIG in-neighbours, one per lane (pivots
+// Up to 32 vertices of at most rv.big in-neighbours, one per lane (pivots
 // ns_l; 0: none).  Each subgroup takes one of them at a time: its lanes read
 // 8 K positions per step and then gather the rows of those with a parent.
 template <int K, class WC>
@@ -669,28 +737,11 @@ __device__ __forceinline__ void fwd_pull_body(const Adj &rv, typename MaskOf<K>:
 }
 
 // One forward level, device-driven: the level is bi->cur + 1 and the direction
-// bi->push_next (set by the previous k_level_advance).  Both direction kernels
-// are launched every level; the one not chosen returns at once, as both do
-// once a level discovered nothing.  CNT: the counting build (work counts into
+// bi->push_next (set when the previous level was closed); nothing once a level
+// discovered nothing.  CNT: the counting build (work counts into
 // wc[KP_FWD_PUSH / KP_FWD_PULL]).
 template <int K, bool CNT>
-__global__ void __launch_bounds__(BATCH_TPB, PUSH_BLOCKS(K)) k_fwd_push_step(Adj a, const BatchInfo *__restrict__ bi,
-                                                             uint32_t *const *__restrict__ tab,
-                                                             const uint32_t *__restrict__ seen,
-                                                             uint32_t *msigma, uint32_t *ctrs,
-                                                             LevelLists ll, unsigned long long *wc)
-{
-    typedef typename MaskOf<K>::T M;
-    if (!bi->alive || !bi->push_next) return;
-    const int L = bi->cur + 1;
-    WorkCount<CNT> cnt;
-    fwd_push_body<K>(a, reinterpret_cast<const M *>(tab[L - 1]), reinterpret_cast<M *>(tab[L]),
-                     reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L, ll, L, cnt);
-    cnt.flush(wc);
-}
-
-template <int K, bool CNT>
-__global__ void __launch_bounds__(BATCH_TPB, PULL_BLOCKS(K)) k_fwd_pull_step(Adj rv, const BatchInfo *__restrict__ bi,
+__global__ void __launch_bounds__(BATCH_TPB, FWD_BLOCKS(K)) k_fwd_step(Adj a, Adj rv, const BatchInfo *__restrict__ bi,
                                                              uint32_t *const *__restrict__ tab,
                                                              const uint32_t *__restrict__ seen,
                                                              uint32_t *msigma, uint32_t *ctrs,
@@ -698,12 +749,17 @@ __global__ void __launch_bounds__(BATCH_TPB, PULL_BLOCKS(K)) k_fwd_pull_step(Adj
 {
     typedef typename MaskOf<K>::T M;
     __shared__ uint2 s_st[BATCH_TPB / 32][PullShape<K>::STAGE];
-    if (!bi->alive || bi->push_next) return;
-    const int L = bi->cur + 1;
+    if (!bi->alive) return;
+    const int L = bi->cur + 1, push = bi->push_next;
     WorkCount<CNT> cnt;
-    fwd_pull_body<K>(rv, (M)bi->srcmask, reinterpret_cast<const M *>(tab[L - 1]), reinterpret_cast<M *>(tab[L]),
-                     reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L, s_st[threadIdx.x >> 5], ll, L, cnt);
-    cnt.flush(wc);
+    const M *fprev = reinterpret_cast<const M *>(tab[L - 1]);
+    M *fcur = reinterpret_cast<M *>(tab[L]);
+    if (push)
+        fwd_push_body<K>(a, fprev, fcur, reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L, ll, L, cnt);
+    else
+        fwd_pull_body<K>(rv, (M)bi->srcmask, fprev, fcur, reinterpret_cast<const M *>(seen), msigma, ctrs + 2 * L,
+                         s_st[threadIdx.x >> 5], ll, L, cnt);
+    cnt.flush(wc + (push ? KP_FWD_PUSH : KP_FWD_PULL) * WC_NFIELDS);
 }
 
 // After level L = bi->cur + 1: fold the level mask into `seen` and count, per
@@ -730,12 +786,18 @@ __device__ __forceinline__ void stats_vertex(uint64_t u, M srcmask, const M *__r
     if ((sn & srcmask) != srcmask && (sn2 & srcmask) == srcmask) udec += rcol[u + 1] - rcol[u];
 }
 
+// a block's totals: per pivot vertices, degrees and reach, then the level's
+// degree sum, frontier degrees, unvisited decrease, big vertices, and whether any
+template <int K> struct StatsShared {
+    unsigned long long x[3 * 32 * K + 5];
+};
 template <int K>
 __device__ __forceinline__ void stats_body(uint64_t n, BatchInfo *bi, int L, typename MaskOf<K>::T srcmask,
                                            const typename MaskOf<K>::T *__restrict__ fcur,
                                            typename MaskOf<K>::T *seen, const uint32_t *__restrict__ col,
                                            const uint32_t *__restrict__ rcol,
-                                           const uint32_t *__restrict__ reach, const LevelLists &ll)
+                                           const uint32_t *__restrict__ reach, uint32_t big, StatsShared<K> &sh,
+                                           const LevelLists &ll)
 {
     typedef typename MaskOf<K>::T M;
     const unsigned lane = lane_id();
@@ -759,7 +821,7 @@ __device__ __forceinline__ void stats_body(uint64_t n, BatchInfo *bi, int L, typ
         if (i < items) {
             const uint64_t u = lst ? lst[i] : i;
             stats_vertex<M>(u, srcmask, fcur, seen, col, rcol, reach, nm, d, r, fdeg, udec, any);
-            if (nm && d > AXBC_BIG) hv++;
+            if (nm && d > big) hv++;
             tsum += (unsigned long long)d * __popcll((unsigned long long)nm);
         }
         unsigned act = __ballot_sync(FULL_MASK, nm != 0);
@@ -778,50 +840,53 @@ __device__ __forceinline__ void stats_body(uint64_t n, BatchInfo *bi, int L, typ
                 }
         }
     }
+    // the block's totals in shared memory first: ten thousand warps adding to
+    // the same few lines took most of this kernel's time
     {
         uint32_t hsum = hv;
         for (int o = 16; o; o >>= 1) {
             tsum += __shfl_xor_sync(FULL_MASK, tsum, o);
+            fdeg += __shfl_xor_sync(FULL_MASK, fdeg, o);
+            udec += __shfl_xor_sync(FULL_MASK, udec, o);
             hsum += __shfl_xor_sync(FULL_MASK, hsum, o);
         }
-        if (lane == 0 && tsum) atomicAdd(&bi->lvl_te, tsum);
-        if (lane == 0 && hsum) atomicAdd(&ll.heavy[L], hsum);
-    }
+        any = __any_sync(FULL_MASK, any);
+        for (uint32_t i = threadIdx.x; i < 3 * 32 * K + 5; i += blockDim.x) sh.x[i] = 0;
+        __syncthreads();
+        if (any) {
+            if (lane == 0) {
+                atomicAdd(&sh.x[96 * K], tsum);
+                atomicAdd(&sh.x[96 * K + 1], fdeg);
+                atomicAdd(&sh.x[96 * K + 2], udec);
+                atomicAdd(&sh.x[96 * K + 3], (unsigned long long)hsum);
+                sh.x[96 * K + 4] = 1;
+            }
 #pragma unroll
-    for (int h = 0; h < K; h++)
-        if (cnt[h]) {
-            const int s = lane + 32 * h;
-            atomicAdd(&bi->lvl_new[s], cnt[h]);
-            atomicAdd(&bi->nvis[s], cnt[h]);
-            atomicAdd(&bi->te[s], te[h]);
-            atomicAdd(&bi->rsum[s], rs[h]);
+            for (int h = 0; h < K; h++)
+                if (cnt[h]) {
+                    const int s = lane + 32 * h;
+                    atomicAdd(&sh.x[s], cnt[h]);
+                    atomicAdd(&sh.x[32 * K + s], te[h]);
+                    atomicAdd(&sh.x[64 * K + s], rs[h]);
+                }
         }
-    for (int o = 16; o; o >>= 1) {
-        fdeg += __shfl_xor_sync(FULL_MASK, fdeg, o);
-        udec += __shfl_xor_sync(FULL_MASK, udec, o);
+        __syncthreads();
     }
-    any = __any_sync(FULL_MASK, any);
-    if (lane == 0) {
-        if (fdeg) atomicAdd(&bi->front_deg, fdeg);
-        if (udec) atomicAdd(&bi->unvis_dec, udec);
-        if (any) atomicOr(&bi->any_new, 1u);
+    if (!sh.x[96 * K + 4]) return;
+    for (int s = threadIdx.x; s < 32 * K; s += blockDim.x)
+        if (sh.x[s]) {
+            atomicAdd(&bi->lvl_new[s], sh.x[s]);
+            atomicAdd(&bi->nvis[s], sh.x[s]);
+            atomicAdd(&bi->te[s], sh.x[32 * K + s]);
+            atomicAdd(&bi->rsum[s], sh.x[64 * K + s]);
+        }
+    if (threadIdx.x == blockDim.x - 1) {
+        if (sh.x[96 * K]) atomicAdd(&bi->lvl_te, sh.x[96 * K]);
+        if (sh.x[96 * K + 1]) atomicAdd(&bi->front_deg, sh.x[96 * K + 1]);
+        if (sh.x[96 * K + 2]) atomicAdd(&bi->unvis_dec, sh.x[96 * K + 2]);
+        if (sh.x[96 * K + 3]) atomicAdd(&ll.heavy[L], (uint32_t)sh.x[96 * K + 3]);
+        atomicOr(&bi->any_new, 1u);
     }
-}
-
-template <int K>
-__global__ void __launch_bounds__(BATCH_TPB) k_stats_step(uint64_t n, BatchInfo *bi,
-                                                          uint32_t *const *__restrict__ tab,
-                                                          uint32_t *seen,
-                                                          const uint32_t *__restrict__ col,
-                                                          const uint32_t *__restrict__ rcol,
-                                                          const uint32_t *__restrict__ reach,
-                                                          LevelLists ll)
-{
-    typedef typename MaskOf<K>::T M;
-    if (!bi->alive) return;
-    const int L = bi->cur + 1;
-    stats_body<K>(n, bi, L, (M)bi->srcmask, reinterpret_cast<const M *>(tab[L]), reinterpret_cast<M *>(seen),
-                  col, rcol, reach, ll);
 }
 
 // Close forward level L = bi->cur + 1 (one warp, lane l for pivots l + 32 h):
@@ -835,13 +900,13 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
                                                    uint32_t list_max)
 {
     const unsigned l = lane_id();
-    const int L = bi->cur + 1;
+    const int L = __ldcg(&bi->cur) + 1;
     const uint32_t nsrc = bi->nsrc;
     unsigned long long cnt = 0, d0 = 0;
 #pragma unroll
     for (int h = 0; h < K; h++) {
         const uint32_t s = l + 32 * h;
-        const unsigned long long nw = s < nsrc ? bi->lvl_new[s] : 0ull;
+        const unsigned long long nw = s < nsrc ? __ldcg(&bi->lvl_new[s]) : 0ull;
         if (s < nsrc && bi->Ls[s] == 0 && nw == 0) bi->Ls[s] = L;
         cnt += nw;
         const bool two = s < nsrc && bi->Ls[s] == 2;
@@ -850,21 +915,22 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(FULL_MASK, cnt, o);
     __syncwarp();
     if (l == 0) {
-        level_te[L] = bi->lvl_te;
+        const unsigned long long front = __ldcg(&bi->front_deg), unvis = __ldcg(&bi->unvis_deg) - __ldcg(&bi->unvis_dec);
+        const uint32_t listed = __ldcg(&ll.count[L]), cap = __ldcg(&ll.cap[L]);
+        level_te[L] = __ldcg(&bi->lvl_te);
         level_cnt[L] = cnt;
         level_mode[L] = bi->push_next;
-        bi->unvis_deg -= bi->unvis_dec;
+        bi->unvis_deg = unvis;
         bi->unvis_dec = 0;
         // push from a frontier whose degree sum is small against the graph:
         // a pull would scan every vertex some pivot has not seen
-        const bool push = (double)bi->front_deg * bi->push_factor < (double)bi->unvis_deg ||
-                          bi->front_deg < bi->push_min;
+        const bool push = (double)front * bi->push_factor < (double)unvis || front < bi->push_min;
         // where level L+1's list goes and how long it may grow
-        const uint32_t used = ll.start[L] + (ll.count[L] <= ll.cap[L] ? ll.count[L] : 0u);
+        const uint32_t used = __ldcg(&ll.start[L]) + (listed <= cap ? listed : 0u);
         ll.start[L + 1] = used;
         ll.cap[L + 1] = min(list_max, pool_cap - min(pool_cap, used));
         if (pool_cap - min(pool_cap, used) < list_max) bi->pool_short = 1;
-        if (!bi->any_new) {
+        if (!__ldcg(&bi->any_new)) {
             bi->alive = 0;
             bi->lend = L;
             bi->dmax = L - 1;
@@ -880,13 +946,24 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
     for (int h = 0; h < K; h++) bi->lvl_new[l + 32 * h] = 0;
 }
 
+// The level's statistics; the last block to finish closes the level.
 template <int K>
-__global__ void k_level_advance(BatchInfo *bi, unsigned long long *level_te,
-                                unsigned long long *level_cnt, int32_t *level_mode,
-                                LevelLists ll, uint32_t pool_cap, uint32_t list_max)
+__global__ void __launch_bounds__(BATCH_TPB) k_stats_step(uint64_t n, BatchInfo *bi, uint32_t *const *__restrict__ tab,
+                                                          uint32_t *seen, const uint32_t *__restrict__ col,
+                                                          const uint32_t *__restrict__ rcol,
+                                                          const uint32_t *__restrict__ reach, LevelLists ll,
+                                                          unsigned long long *level_te,
+                                                          unsigned long long *level_cnt, int32_t *level_mode,
+                                                          uint32_t pool_cap, uint32_t list_max, uint32_t big)
 {
-    if (!bi->alive) return;
-    level_advance_warp<K>(bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max);
+    typedef typename MaskOf<K>::T M;
+    __shared__ StatsShared<K> sh;
+    if (!__ldcg(&bi->alive)) return;
+    const int L = __ldcg(&bi->cur) + 1;
+    stats_body<K>(n, bi, L, (M)__ldcg(&bi->srcmask), reinterpret_cast<const M *>(tab[L]), reinterpret_cast<M *>(seen),
+                  col, rcol, reach, big, sh, ll);
+    if (last_block(&bi->ticket[1]) && threadIdx.x < 32)
+        level_advance_warp<K>(bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max);
 }
 
 // The backward pass runs one 32-pivot half of a pass at a time (hh = 0, or 0
@@ -1049,7 +1126,7 @@ __device__ __forceinline__ float bwd_span(const Adj &a, const BwdHalf &B, uint32
     return P;
 }
 
-// Vertices of at most AXBC_BIG neighbours, one per lane (pivots f_l; 0: none):
+// Vertices of at most a.big neighbours, one per lane (pivots f_l; 0: none):
 // those of at most 8 four at a time, one group of lanes each, the others one
 // by one.
 template <int K, class WC>
@@ -1063,7 +1140,7 @@ __device__ __forceinline__ void bwd_small(const Adj &a, const BwdHalf &B, uint32
     if (f_l) {
         b_l = a.col[v_l];
         d_l = a.col[v_l + 1] - b_l;
-        if (d_l > AXBC_BIG) f_l = 0;  // in a tile
+        if (d_l > a.big) f_l = 0;  // in a tile
     }
     if (f_l) {
         // adjacency bounds and reach; per pivot its path count read, its
@@ -1178,11 +1255,11 @@ __device__ __forceinline__ void bwd_tile(const Adj &a, const BwdHalf &B, uint64_
     }
     uint32_t inc = c_l;  // chunks up to and including this vertex's
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {
+    for (int o = 1; o < 16; o <<= 1) {
         const uint32_t x = __shfl_up_sync(FULL_MASK, inc, o);
         if ((int)lane >= o) inc += x;
     }
-    const uint32_t S = __shfl_sync(FULL_MASK, inc, 7);
+    const uint32_t S = __shfl_sync(FULL_MASK, inc, 15);  // at most 16 vertices of two chunks
     const float *mq_l = B.mq + 4 * (lane & 7);
     uint32_t u[BWD_TILE_CHUNKS / NW], gm[BWD_TILE_CHUNKS / NW];
 #pragma unroll
@@ -1190,7 +1267,7 @@ __device__ __forceinline__ void bwd_tile(const Adj &a, const BwdHalf &B, uint64_
         const uint32_t s = wid + NW * i;
         u[i] = 0xffffffffu;
         if (s < S) {
-            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 16 && inc <= s));
             const uint32_t e = __shfl_sync(FULL_MASK, b_l + AXBC_CHUNK * (s - (inc - c_l)), j) + lane;
             if (e < __shfl_sync(FULL_MASK, e_l, j)) u[i] = a.row[e];
         }
@@ -1200,7 +1277,7 @@ __device__ __forceinline__ void bwd_tile(const Adj &a, const BwdHalf &B, uint64_
         const uint32_t s = wid + NW * i;
         gm[i] = 0;
         if (s < S) {
-            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 16 && inc <= s));
             const uint32_t f = __shfl_sync(FULL_MASK, f_l, j);
             if (u[i] != 0xffffffffu) gm[i] = B.fnext[(uint64_t)u[i] * K] & f;
             count_entry(wc, u[i] != 0xffffffffu, gm[i]);
@@ -1213,7 +1290,7 @@ __device__ __forceinline__ void bwd_tile(const Adj &a, const BwdHalf &B, uint64_
         const unsigned pm = __ballot_sync(FULL_MASK, gm[i] != 0);
         float r = 0.0f;
         if (pm) {
-            const int j = __popc(__ballot_sync(FULL_MASK, lane < 8 && inc <= s));
+            const int j = __popc(__ballot_sync(FULL_MASK, lane < 16 && inc <= s));
             float sv[4], q[4];
             load_sv<K>(B.msigma, __shfl_sync(FULL_MASK, v_l, j), __shfl_sync(FULL_MASK, f_l, j), sv);
             group_sums<K>(st, u[i], gm[i], pm, mq_l, sv, q);
@@ -1633,28 +1710,40 @@ __global__ void k_bwd_combine_step(Adj a, const BatchInfo *__restrict__ bi, uint
 __device__ __forceinline__ unsigned vload_u(const unsigned *p) { return *(const volatile unsigned *)p; }
 __device__ __forceinline__ int vload_i(const int *p) { return *(const volatile int *)p; }
 
-// All blocks of the cooperative grid meet here.  The last block to arrive runs
-// lead() with its first warp, then releases the others.  Thread 0 of each block
-// fences before arriving and after the wait, as cooperative groups' grid sync
-// does, so the block's later loads see what every block wrote before
-// arriving.  Returns false when this wait, or an earlier one of any block, ran
-// out of its budget.
+// All blocks of the cooperative grid meet here; `epoch` counts the launch's
+// barriers, the same in every block.  Thread 0 of each block fences, adds one to
+// the arrival count and waits: without a lead until the count reaches the
+// barrier's total, with one until the last block to arrive has run lead() with
+// its first warp and says so (gen).  The fences before arriving and after the
+// wait make the block's later loads see what every block wrote before.  A wait
+// polls without sleeping at first (a barrier of 152 blocks took 3.1 us with a
+// sleep in every poll and a generation word to be flipped for each).  Returns
+// false when this wait, or an earlier one of any block, ran out of its budget.
 struct NoLead {
     __device__ void operator()() const {}
 };
+template <class F> struct HasLead {
+    static constexpr bool yes = true;
+};
+template <> struct HasLead<NoLead> {
+    static constexpr bool yes = false;
+};
 template <class F>
-__device__ __forceinline__ bool grid_barrier(GridSync *gs, long long budget, int site, const F &lead)
+__device__ __forceinline__ bool grid_barrier(GridSync *gs, long long budget, int site, unsigned &epoch, const F &lead)
 {
     __shared__ int s_role;  // 1 leader, 0 released, -1 failed
+    const unsigned mine = ++epoch, total = mine * gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned g = vload_u(&gs->gen);
         __threadfence();
-        const unsigned arrived = atomicAdd(&gs->count, 1u);
-        int role = arrived == gridDim.x - 1 ? 1 : 0;
-        if (role == 0) {
+        const unsigned arrived = atomicAdd(&gs->count, 1u) + 1;
+        int role = HasLead<F>::yes && arrived == total ? 1 : 0;
+        if (role == 0 && arrived != total) {
             const long long t0 = clock64();
-            while (vload_u(&gs->gen) == g) {
+            for (unsigned polls = 1;; polls++) {
+                if (HasLead<F>::yes ? (int)(vload_u(&gs->gen) - mine) >= 0 : (int)(vload_u(&gs->count) - total) >= 0)
+                    break;
+                if (polls % 32) continue;
                 if (vload_i(&gs->err)) {
                     role = -1;
                     break;
@@ -1664,7 +1753,7 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs, long long budget, int
                     role = -1;
                     break;
                 }
-                __nanosleep(32);
+                if (polls >= 1024) __nanosleep(64);
             }
         }
         __threadfence();
@@ -1672,13 +1761,12 @@ __device__ __forceinline__ bool grid_barrier(GridSync *gs, long long budget, int
     }
     __syncthreads();
     const int role = s_role;
-    if (role == 1) {
+    if (HasLead<F>::yes && role == 1) {
         if (threadIdx.x < 32) lead();
         __syncthreads();
         if (threadIdx.x == 0) {
-            gs->count = 0;
             __threadfence();
-            atomicAdd(&gs->gen, 1u);
+            atomicExch(&gs->gen, mine);
         }
     }
     return role >= 0;
@@ -1711,9 +1799,11 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
     typedef typename MaskOf<K>::T M;
     __shared__ uint2 s_st[BATCH_TPB / 32][PullShape<K>::STAGE];
     __shared__ float s_csum[2][BWD_TILE_CHUNKS][32];
+    __shared__ StatsShared<K> sh;
     uint2 *st = s_st[threadIdx.x >> 5];
     M *seen = reinterpret_cast<M *>(seen_);
     WorkCount<false> none;
+    unsigned epoch = 0;
     const AdvanceLead<K> adv{bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max};
     for (;;) {
         if (!vload_i(&bi->alive)) break;
@@ -1728,9 +1818,9 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
             fwd_push_body<K>(a, fprev, fcur, seen, msigma, ctrs + 2 * L, ll, L, none);
         else
             fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, st, ll, L, none);
-        if (!grid_barrier(gs, budget, 1, NoLead{})) return;
-        stats_body<K>(n, bi, L, srcmask, fcur, seen, a.col, rv.col, reach, ll);
-        if (!grid_barrier(gs, budget, 2, adv)) return;
+        if (!grid_barrier(gs, budget, 1, epoch, NoLead{})) return;
+        stats_body<K>(n, bi, L, srcmask, fcur, seen, a.col, rv.col, reach, a.big, sh, ll);
+        if (!grid_barrier(gs, budget, 2, epoch, adv)) return;
     }
     const uint32_t n_heavy = a.n_heavy;
     for (int d = vload_i(&bi->dmax); d >= 0; d--) {
@@ -1748,7 +1838,7 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
                             symmetric, none);
             __syncthreads();  // the chunk sums of the next half
         }
-        if (d > 0 && !grid_barrier(gs, budget, 3, NoLead{})) return;
+        if (d > 0 && !grid_barrier(gs, budget, 3, epoch, NoLead{})) return;
     }
 }
 
@@ -1767,8 +1857,9 @@ __global__ void __launch_bounds__(BATCH_TPB) k_barrier_selftest(GridSync *gs, in
 {
     if ((int)blockIdx.x == absent) return;
     const CountLead lead{out};
+    unsigned epoch = 0;
     for (int r = 0; r < rounds; r++)
-        if (!grid_barrier(gs, budget, r + 1, lead)) return;
+        if (!grid_barrier(gs, budget, r + 1, epoch, lead)) return;
 }
 
 // bc update for the applied pivots in lane order (update_bc, src/cuda_kernels.cu:
@@ -2057,7 +2148,12 @@ static int ensure_level_tables(axbc_ctx *c)
 {
     if (c->tables_ready) return AXBC_OK;
     ALLOC_MISSING(c->fmtab, AXBC_MAX_LEVELS * sizeof(uint32_t *), &c->bytes);
-    ALLOC_MISSING(c->ctrs, 2 * AXBC_WMAX / 32 * AXBC_MAX_LEVELS * 4, &c->bytes);
+    // work counters, list lengths: zero here, then cleared by each pass as far
+    // as the one before it went
+    if (!c->ctrs) {
+        TRY(axbc_dalloc((void **)&c->ctrs, 2 * AXBC_WMAX / 32 * AXBC_MAX_LEVELS * 4, &c->bytes));
+        CU(cudaMemsetAsync(c->ctrs, 0, 2 * AXBC_WMAX / 32 * AXBC_MAX_LEVELS * 4, c->stream));
+    }
     ALLOC_MISSING(c->d_level_te, AXBC_MAX_LEVELS * 8, &c->bytes);
     ALLOC_MISSING(c->d_level_cnt, AXBC_MAX_LEVELS * 8, &c->bytes);
     ALLOC_MISSING(c->d_level_mode, AXBC_MAX_LEVELS * 4, &c->bytes);
@@ -2071,9 +2167,15 @@ static int ensure_level_tables(axbc_ctx *c)
         c->lpool_cap = cap;
     }
     ALLOC_MISSING(c->lstart, AXBC_MAX_LEVELS * 4, &c->bytes);
-    ALLOC_MISSING(c->lcount, AXBC_MAX_LEVELS * 4, &c->bytes);
+    if (!c->lcount) {
+        TRY(axbc_dalloc((void **)&c->lcount, AXBC_MAX_LEVELS * 4, &c->bytes));
+        CU(cudaMemsetAsync(c->lcount, 0, AXBC_MAX_LEVELS * 4, c->stream));
+    }
     ALLOC_MISSING(c->lcap, AXBC_MAX_LEVELS * 4, &c->bytes);
-    ALLOC_MISSING(c->lheavy, AXBC_MAX_LEVELS * 4, &c->bytes);
+    if (!c->lheavy) {
+        TRY(axbc_dalloc((void **)&c->lheavy, AXBC_MAX_LEVELS * 4, &c->bytes));
+        CU(cudaMemsetAsync(c->lheavy, 0, AXBC_MAX_LEVELS * 4, c->stream));
+    }
     c->tables_ready = true;
     return AXBC_OK;
 }
@@ -2109,7 +2211,7 @@ int axbc_batch_levels_alloc(axbc_ctx *c, int levels)
         uint32_t *p = nullptr;
         if ((rc = axbc_dalloc((void **)&p, c->g->n * 8, &c->bytes)) != AXBC_OK) break;
         c->fmask.push_back(p);
-        CU(cudaMemset(p, 0, c->g->n * 8));
+        CU(cudaMemsetAsync(p, 0, c->g->n * 8, c->stream));
     }
     if (c->fmask.size() > c->fmtab_synced) {
         CU(cudaMemcpy(c->fmtab + c->fmtab_synced, c->fmask.data() + c->fmtab_synced,
@@ -2128,16 +2230,15 @@ int axbc_ensure_batch(axbc_ctx *c)
     ALLOC_MISSING(c->msigma, n * AXBC_WMAX * 4, &c->bytes);
     ALLOC_MISSING(c->mdelta, n * AXBC_WMAX * 4, &c->bytes);
     ALLOC_MISSING(c->mq, n * AXBC_WMAX * 4, &c->bytes);
-    ALLOC_MISSING(c->task_ctr, 64, &c->bytes);
     ALLOC_MISSING(c->mpartial, (c->g->bfwd.n_heavy_items + 1) * AXBC_WMAX * 4, &c->bytes);
     if (!c->harrive) {
         TRY(axbc_dalloc((void **)&c->harrive, (uint64_t)(c->g->bfwd.n_heavy + 1) * 2 * 4, &c->bytes));
-        CU(cudaMemset(c->harrive, 0, (uint64_t)(c->g->bfwd.n_heavy + 1) * 2 * 4));
+        CU(cudaMemsetAsync(c->harrive, 0, (uint64_t)(c->g->bfwd.n_heavy + 1) * 2 * 4, c->stream));
     }
     ALLOC_MISSING(c->bi, sizeof(BatchInfo), &c->bytes);
     if (!c->bi_host) CU(cudaMallocHost((void **)&c->bi_host, sizeof(BatchInfo)));
-    CU(cudaMemset(c->bi, 0, sizeof(BatchInfo)));
-    CU(cudaMemset(c->seen, 0, n * 8));
+    CU(cudaMemsetAsync(c->bi, 0, sizeof(BatchInfo), c->stream));
+    CU(cudaMemsetAsync(c->seen, 0, n * 8, c->stream));
     TRY(axbc_batch_levels_alloc(c, 10));
     c->batch_ready = true;
     return AXBC_OK;
@@ -2153,44 +2254,59 @@ static int width_k(int nsrc) { return nsrc > AXBC_W ? 2 : 1; }
 // 451 : 469, 7.6 M 417 : 432 and 694 : 866, 31 M (64 pivots) 1590 : 2590.
 static bool bwd_wide(const axbc_graph *g, int K) { return g->m * (uint64_t)K >= AXBC_BWD_WIDE_MIN; }
 
-// dynamic kernels: as many blocks as stay resident; work comes from counters
+// dynamic kernels: as many blocks as stay resident (work comes from counters),
+// or as many as have work
 template <int K> static int occupancy(axbc_ctx *c)
 {
     const int i = K - 1;
-    if (!c->dyn_blocks_per_sm[i]) {
-        int a = 0, b = 0, d = 0;
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fwd_push_step<K, false>, BATCH_TPB, 0));
+    if (!c->fwd_blocks_per_sm[i]) {
+        int a = 0, b = 0;
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_fwd_step<K, false>, BATCH_TPB, 0));
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &b, bwd_wide(c->g, K) ? (const void *)k_bwd_step<K, false> : (const void *)k_bwd_tile_step<K, false>, BATCH_TPB, 0));
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d, k_fwd_pull_step<K, false>, BATCH_TPB, 0));
-        c->dyn_blocks_per_sm[i] = std::max(1, a);
-        c->pull_blocks_per_sm[i] = std::max(1, d);
+            &b, bwd_wide(c->g, K) ? (const void *)k_bwd_step<K, false> : (const void *)k_bwd_tile_step<K, false>,
+            BATCH_TPB, 0));
         c->bwd_blocks_per_sm[i] = std::max(1, b);
+        c->fwd_blocks_per_sm[i] = std::max(1, a);
     }
     return AXBC_OK;
 }
-template <int K> static int push_grid(axbc_ctx *c) { return axbc_grid_for(c, BATCH_TPB, c->dyn_blocks_per_sm[K - 1]); }
-template <int K> static int pull_grid(axbc_ctx *c) { return axbc_grid_for(c, BATCH_TPB, c->pull_blocks_per_sm[K - 1]); }
+static int grid_of(const axbc_ctx *c, int per_sm, uint64_t blocks)
+{
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>(axbc_grid_for(c, BATCH_TPB, per_sm), blocks));
+}
+// warps that could each have a unit of their own
+static uint64_t adj_warps(const Adj &a) { return a.n_part + (a.n_linked - a.n_big); }
+template <int K> static int fwd_grid(const axbc_ctx *c)
+{
+    const uint64_t w = std::max(adj_warps(c->g->bfwd), adj_warps(c->g->brev));
+    return grid_of(c, c->fwd_blocks_per_sm[K - 1], (w + 7) / 8);
+}
+template <int K> static int bwd_grid(const axbc_ctx *c)
+{
+    const Adj &a = c->g->bfwd;
+    return grid_of(c, c->bwd_blocks_per_sm[K - 1],
+                   std::max<uint64_t>(std::max<uint64_t>(a.n_tile, a.n_heavy_items), (c->g->n - a.n_big + 7) / 8));
+}
 
 // the kernels of one forward level, in stream order; one backward depth
-template <int K> static void fwd_step_kernels(axbc_ctx *c, int sgrid)
+template <int K> static void stats_step_kernel(axbc_ctx *c)
 {
     axbc_graph *g = c->g;
-    const LevelLists ll = lists_of(c);
-    k_fwd_push_step<K, false><<<push_grid<K>(c), BATCH_TPB, 0, c->stream>>>(g->bfwd, c->bi, c->fmtab, c->seen,
-                                                                           c->msigma, c->ctrs, ll, nullptr);
-    k_fwd_pull_step<K, false><<<pull_grid<K>(c), BATCH_TPB, 0, c->stream>>>(g->brev, c->bi, c->fmtab, c->seen,
-                                                                           c->msigma, c->ctrs, ll, nullptr);
-    k_stats_step<K><<<sgrid, BATCH_TPB, 0, c->stream>>>(g->n, c->bi, c->fmtab, c->seen, g->bfwd.col, g->brev.col,
-                                                        g->breach, ll);
-    k_level_advance<K><<<1, 32, 0, c->stream>>>(c->bi, c->d_level_te, c->d_level_cnt, c->d_level_mode, ll,
-                                                c->lpool_cap, list_max_of(c));
+    k_stats_step<K><<<grid_of(c, 4, (g->n + BATCH_TPB - 1) / BATCH_TPB), BATCH_TPB, 0, c->stream>>>(
+        g->n, c->bi, c->fmtab, c->seen, g->bfwd.col, g->brev.col, g->breach, lists_of(c), c->d_level_te,
+        c->d_level_cnt, c->d_level_mode, c->lpool_cap, list_max_of(c), g->bfwd.big);
+}
+template <int K> static void fwd_step_kernel(axbc_ctx *c, unsigned long long *wc)
+{
+    axbc_graph *g = c->g;
+    (wc ? k_fwd_step<K, true> : k_fwd_step<K, false>)<<<fwd_grid<K>(c), BATCH_TPB, 0, c->stream>>>(
+        g->bfwd, g->brev, c->bi, c->fmtab, c->seen, c->msigma, c->ctrs, lists_of(c), wc);
 }
 
 template <int K> static void bwd_step_kernel(axbc_ctx *c, int d, unsigned long long *wc)
 {
     axbc_graph *g = c->g;
-    const dim3 grid(axbc_grid_for(c, BATCH_TPB, c->bwd_blocks_per_sm[K - 1]), K);
+    const dim3 grid(bwd_grid<K>(c), K);
     cudaStream_t s = c->stream;
     if (!bwd_wide(g, K)) {
         (wc ? k_bwd_tile_step<K, true> : k_bwd_tile_step<K, false>)<<<grid, BATCH_TPB, 0, s>>>(
@@ -2219,13 +2335,14 @@ static void drop_captures(axbc_ctx *c)
 
 // Capture one forward step of width K as a CUDA graph; every argument is fixed
 // for the context (levels come from device state).
-template <int K> static int capture_steps(axbc_ctx *c, int sgrid)
+template <int K> static int capture_steps(axbc_ctx *c)
 {
     const int i = K - 1;
     if (c->fwd_step_exec[i]) return AXBC_OK;
     cudaGraph_t gr = nullptr;
     CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    fwd_step_kernels<K>(c, sgrid);
+    fwd_step_kernel<K>(c, nullptr);
+    stats_step_kernel<K>(c);
     cudaError_t e = cudaStreamEndCapture(c->stream, &gr);
     if (e != cudaSuccess) return axbc_cuda_fail(e, "capture level step", __FILE__, __LINE__);
     e = cudaGraphInstantiate(&c->fwd_step_exec[i], gr, 0);
@@ -2238,22 +2355,20 @@ template <int K> static int capture_steps(axbc_ctx *c, int sgrid)
 // graph replays of one forward level, in blocks (profiling and counting: each
 // kernel launched on its own), then one launch per depth.  *L_out: the first level that discovered
 // nothing.
-template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, int *L_out)
+template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int *L_out)
 {
     axbc_graph *g = c->g;
     const uint64_t n = g->n;
     cudaStream_t s = c->stream;
     const bool prof = c->prof_on || c->count_on;
     unsigned long long *wc = c->count_on ? c->wcount : nullptr;
-    const LevelLists ll = lists_of(c);
-    const uint32_t lmax = list_max_of(c);
     const size_t ctl_off = offsetof(BatchInfo, depth0mask);
     const size_t ctl_len = offsetof(BatchInfo, push_factor) - ctl_off;
     const size_t prof_first = c->prof.size();
     // forward steps launched before the first look at `alive`: one more than
     // the last batch needed, so a batch like it ends after one host round
-    // trip; later groups double
-    int launched = 0, B = std::max(4, std::min(256, c->last_batch_levels + 1));
+    // trip; then groups of 8, 16, ... 256
+    int launched = 0, B = std::max(4, std::min(4096, c->last_batch_levels + 1)), more = 8;
     if (c->last_batch_levels == 0) B = 8;
     for (;;) {
         TRY(axbc_batch_levels_alloc(c, launched + B + 2));
@@ -2263,49 +2378,32 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
             } else {
                 const int L = launched + i + 1;
                 {
-                    ProfScope ps(c, KP_FWD_PUSH, 0);
-                    if (c->prof_on) c->prof.back().tag = L;
-                    if (wc)
-                        k_fwd_push_step<K, true><<<push_grid<K>(c), BATCH_TPB, 0, s>>>(
-                            g->bfwd, c->bi, c->fmtab, c->seen, c->msigma, c->ctrs, ll, wc + KP_FWD_PUSH * WC_NFIELDS);
-                    else
-                        k_fwd_push_step<K, false><<<push_grid<K>(c), BATCH_TPB, 0, s>>>(
-                            g->bfwd, c->bi, c->fmtab, c->seen, c->msigma, c->ctrs, ll, nullptr);
-                }
-                {
+                    // the direction is known once the level has run
                     ProfScope ps(c, KP_FWD_PULL, 0);
                     if (c->prof_on) c->prof.back().tag = L;
-                    if (wc)
-                        k_fwd_pull_step<K, true><<<pull_grid<K>(c), BATCH_TPB, 0, s>>>(
-                            g->brev, c->bi, c->fmtab, c->seen, c->msigma, c->ctrs, ll, wc + KP_FWD_PULL * WC_NFIELDS);
-                    else
-                        k_fwd_pull_step<K, false><<<pull_grid<K>(c), BATCH_TPB, 0, s>>>(
-                            g->brev, c->bi, c->fmtab, c->seen, c->msigma, c->ctrs, ll, nullptr);
+                    fwd_step_kernel<K>(c, wc);
                 }
                 {
                     ProfScope ps(c, KP_LEVEL_STATS, 0);
                     if (c->prof_on) c->prof.back().tag = L;
-                    k_stats_step<K><<<sgrid, BATCH_TPB, 0, s>>>(n, c->bi, c->fmtab, c->seen, g->bfwd.col,
-                                                                g->brev.col, g->breach, ll);
+                    stats_step_kernel<K>(c);
                 }
-                k_level_advance<K><<<1, 32, 0, s>>>(c->bi, c->d_level_te, c->d_level_cnt, c->d_level_mode, ll,
-                                                    c->lpool_cap, lmax);
-                c->launches++;
             }
         }
         CU_LAUNCH("forward levels");
-        if (!prof) c->launches += 4ull * B;
+        if (!prof) c->launches += 2ull * B;
         launched += B;
         c->prev_lend = std::min(launched, (int)c->fmask.size() - 1);  // masks written so far
         CU(cudaMemcpyAsync((char *)c->bi_host + ctl_off, (char *)c->bi + ctl_off, ctl_len,
                            cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         if (!c->bi_host->alive) break;
-        if (launched + 2 * B + 2 > AXBC_MAX_LEVELS) {
+        B = more;
+        more = std::min(2 * more, 256);
+        if (launched + B + 2 > AXBC_MAX_LEVELS) {
             axbc_set_error("traversal deeper than %d levels", AXBC_MAX_LEVELS - 2);
             return AXBC_ERR_RANGE;
         }
-        B = std::min(2 * B, 256);
     }
     const int L = c->bi_host->lend, Dmax = c->bi_host->dmax;
     *L_out = L;
@@ -2326,10 +2424,9 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
         for (size_t i = prof_first; i < c->prof.size(); i++) {
             ProfRec &r = c->prof[i];
             if (r.tag < 1 || r.tag > L) continue;  // steps past the last level: no work
-            if (r.kind == KP_FWD_PUSH || r.kind == KP_FWD_PULL) {
-                // the byte model goes to the direction that ran; the other launch returned at once
-                const bool ran = (r.kind == KP_FWD_PUSH) == (lmode[r.tag] != 0);
-                r.bytes = ran ? (double)lte[r.tag - 1] * (4.0 / W + 4.0) : 0.0;
+            if (r.kind == KP_FWD_PULL) {
+                if (lmode[r.tag]) r.kind = KP_FWD_PUSH;
+                r.bytes = (double)lte[r.tag - 1] * (4.0 / W + 4.0);
             } else if (r.kind == KP_LEVEL_STATS) {
                 r.bytes = (double)n * 16.0;
             }
@@ -2374,17 +2471,20 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int sgrid, 
 }
 
 // Whether this batch runs as one persistent launch: always or never when the
-// context says so; otherwise for a batch of at most AXBC_PERSIST_AUTO_WIDTH
-// pivots when the last batch was deep, or -- for the first batch -- when no
-// vertex has more than 64 neighbours (meshes and road-like graphs, whose many
-// levels are narrow).  Measured on the 1024^2 grid (wall clock, 32 pivots per
-// run): width 1 41.8 -> 32.8 ms, width 4 32.2 -> 26.0, width 8 34.3 -> 30.2,
-// width 16 42.1 -> 40.2, width 32 even; on shallow graphs the step kernels'
-// fuller grids win.  Counting runs use the step kernels.
+// context says so; otherwise a batch of at most 32 pivots on a graph of less than
+// 2^21 adjacency entries, whose levels are shorter than the launches between
+// them, and a batch of at most AXBC_PERSIST_AUTO_WIDTH pivots when the last
+// batch was deep, or -- for the first batch -- when no vertex has more than 64
+// neighbours (meshes and road-like graphs, whose many levels are narrow).
+// Measured (us a pass, steps : persistent): 0.02 M entries, 1 pivot 170 : 142, 32
+// pivots 219 : 179; 0.43 M 217 : 220 and 347 : 320; 1.8 M 340 : 297 and 486 : 431;
+// 3.7 M 378 : 378 and 612 : 643; 64 pivots 408 : 442 at 0.43 M (two mask words
+// leave the one kernel two blocks per SM).  Counting runs use the step kernels.
 static bool use_persist(axbc_ctx *c, int nsrc)
 {
     if (c->count_on || c->persist_mode < 0) return false;
     if (c->persist_mode > 0) return true;
+    if (nsrc <= AXBC_W && c->g->m < AXBC_PERSIST_AUTO_M) return true;
     if (nsrc > AXBC_PERSIST_AUTO_WIDTH) return false;
     if (c->last_batch_levels > AXBC_PERSIST_AUTO_LEVELS) return true;
     return c->last_batch_levels == 0 && c->g->max_deg <= 64;
@@ -2398,10 +2498,9 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
 {
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
-    ALLOC_MISSING(c->gsync, sizeof(GridSync), &c->bytes);
-    int bps = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_traverse_persist<K>, BATCH_TPB, 0));
-    bps = std::min(bps, std::max(1, c->persist_blocks_per_sm));
+    int &fit = c->persist_fit[K - 1];
+    if (!fit) CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_traverse_persist<K>, BATCH_TPB, 0));
+    const int bps = std::min(fit, std::max(1, c->persist_blocks_per_sm));
     if (bps < 1) {
         axbc_set_error("persistent level loop: no block of it fits on an SM");
         return AXBC_ERR_CUDA;
@@ -2413,25 +2512,29 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
     const uint64_t n = g->n;
     long long budget = AXBC_BAR_BUDGET;
     int levels = std::max(16, c->last_batch_levels + 8);
-    GridSync hs;
-    for (;;) {
+    const size_t ctl_off = offsetof(BatchInfo, depth0mask);
+    const size_t ctl_len = offsetof(BatchInfo, push_factor) - ctl_off;
+    GridSync *gs = &c->bi->gs;
+    const GridSync &hs = c->bi_host->gs;
+    for (bool first = true;; first = false) {
         levels = std::min(levels, AXBC_MAX_LEVELS - 2);
         TRY(axbc_batch_levels_alloc(c, levels));
         c->prev_lend = levels - 1;  // masks the loop may write, cleared before the next batch
-        CU(cudaMemsetAsync(c->gsync, 0, sizeof(GridSync), s));
+        if (!first) CU(cudaMemsetAsync(gs, 0, sizeof(GridSync), s));
         int lmax = levels;
         void *args[] = {(void *)&g->bfwd, (void *)&g->brev, (void *)&c->bi, (void *)&c->fmtab,
                         (void *)&c->seen, (void *)&c->msigma, (void *)&c->mdelta, (void *)&c->mq,
                         (void *)&c->mpartial, (void *)&c->harrive, (void *)&g->breach, (void *)&c->ctrs,
                         (void *)&ll, (void *)&g->symmetric, (void *)&c->d_level_te, (void *)&c->d_level_cnt, (void *)&c->d_level_mode,
                         (void *)&pool_cap, (void *)&lmax_list, (void *)&n, (void *)&lmax,
-                        (void *)&c->gsync, (void *)&budget};
+                        (void *)&gs, (void *)&budget};
         {
             ProfScope ps(c, KP_PERSIST, 0);
             CU(cudaLaunchCooperativeKernel((const void *)k_traverse_persist<K>, grid, BATCH_TPB, args, 0, s));
         }
         CU_LAUNCH("k_traverse_persist");
-        CU(cudaMemcpyAsync(&hs, c->gsync, sizeof(GridSync), cudaMemcpyDeviceToHost, s));
+        // the level state and the barrier's record in one copy
+        CU(cudaMemcpyAsync((char *)c->bi_host + ctl_off, (char *)c->bi + ctl_off, ctl_len, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
         if (hs.err) {
             axbc_set_error("persistent level loop: a grid barrier wait ran out of its budget (site %d)", hs.err);
@@ -2444,10 +2547,6 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
         }
         levels *= 2;
     }
-    const size_t ctl_off = offsetof(BatchInfo, depth0mask);
-    const size_t ctl_len = offsetof(BatchInfo, push_factor) - ctl_off;
-    CU(cudaMemcpyAsync((char *)c->bi_host + ctl_off, (char *)c->bi + ctl_off, ctl_len, cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
     *L_out = c->bi_host->lend;
     return AXBC_OK;
 }
@@ -2461,27 +2560,15 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
     axbc_graph *g = c->g;
     const uint64_t n = g->n;
     cudaStream_t s = c->stream;
-    const int sgrid = axbc_grid_for(c, BATCH_TPB, 8);
     TRY(occupancy<K>(c));
     // per-launch mode: profiling events around each kernel, or the counting builds
     const bool prof = c->prof_on || c->count_on;
     TRY(ensure_level_tables(c));
     TRY(axbc_batch_levels_alloc(c, 10));
-    if (!prof) TRY(capture_steps<K>(c, sgrid));
+    if (!prof) TRY(capture_steps<K>(c));
 
-    // the previous batch's level masks back to zero (in its own width), then a
-    // larger list pool if that batch ran out of list space
-    if (c->prev_lend >= 2) {
-        if (c->last_batch_k == 2)
-            k_clean_levels<2><<<axbc_grid_for(c, 256, 2), 256, 0, s>>>(c->fmtab, c->lpool, c->lstart, c->lcount,
-                                                                     c->lcap, n, 2, c->prev_lend);
-        else
-            k_clean_levels<1><<<axbc_grid_for(c, 256, 2), 256, 0, s>>>(c->fmtab, c->lpool, c->lstart, c->lcount,
-                                                                     c->lcap, n, 2, c->prev_lend);
-        CU_LAUNCH("k_clean_levels");
-        c->launches++;
-    }
-    c->prev_lend = 0;
+    // a larger list pool if the previous batch ran out of list space (its lists,
+    // which say where its masks are set, move along)
     TRY(axbc_batch_settle(c));
     const uint64_t pool_limit = (uint64_t)AXBC_WMAX * n + 64;
     if (c->pool_short && c->lpool_cap < pool_limit) {
@@ -2491,37 +2578,52 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
                                                            0xffffffffull);
         uint32_t *np = nullptr;
         TRY(axbc_dalloc((void **)&np, (uint64_t)ncap * 4, &c->bytes));
+        CU(cudaMemcpyAsync(np, c->lpool, (uint64_t)c->lpool_cap * 4, cudaMemcpyDeviceToDevice, s));
         CU(cudaStreamSynchronize(s));
         axbc_dfree(c->lpool);
         c->lpool = np;
         c->lpool_cap = ncap;
         c->pool_short = false;
         drop_captures(c);
-        if (!prof) TRY(capture_steps<K>(c, sgrid));
+        if (!prof) TRY(capture_steps<K>(c));
     }
-    c->last_batch_k = K;
-    CU(cudaMemsetAsync(c->seen, 0, n * 4 * K, s));
-    CU(cudaMemsetAsync(c->fmask[0], 0, n * 4 * K, s));
-    CU(cudaMemsetAsync(c->fmask[1], 0, n * 4 * K, s));
-    CU(cudaMemsetAsync(c->msigma, 0, n * AXBC_W * K * 4, s));
-    CU(cudaMemsetAsync(c->ctrs, 0, 2 * AXBC_WMAX / 32 * AXBC_MAX_LEVELS * 4, s));
-    CU(cudaMemsetAsync(c->lcount, 0, AXBC_MAX_LEVELS * 4, s));
-    CU(cudaMemsetAsync(c->lheavy, 0, AXBC_MAX_LEVELS * 4, s));
-    const LevelLists ll = lists_of(c);
-    const uint32_t lmax = list_max_of(c);
+    PassStart P;
+    P.bi = c->bi;
+    P.tab = c->fmtab;
+    P.seen = c->seen;
+    P.msigma = c->msigma;
+    P.ctrs = c->ctrs;
+    P.ll = lists_of(c);
+    P.level_te = c->d_level_te;
+    P.level_cnt = c->d_level_cnt;
+    P.col = g->bfwd.col;
+    P.rcol = g->brev.col;
+    P.reach = g->breach;
+    P.to_view = g->to_view;
+    P.bc = c->bc;
+    P.n = n;
+    P.m = g->m;
+    // a factor of 1e30 or more pulls every level
+    P.push_min = c->push_factor_batch >= 1e30 ? 0ull : (unsigned long long)(n / 4);
+    P.push_factor = c->push_factor_batch;
+    P.pool_cap = c->lpool_cap;
+    P.list_max = list_max_of(c);
+    P.big = g->bfwd.big;
+    P.nsrc = nsrc;
+    P.H = H;
+    P.prev_k = c->last_batch_k;
+    P.prev_last = c->prev_lend;
     {
         ProfScope ps(c, KP_LEVEL_STATS, 0);
-        k_batch_init<K><<<1, 32, 0, s>>>(c->bi, nsrc, H, c->bc, c->fmask[0], c->seen, c->msigma, g->bfwd.col,
-                                         g->brev.col, g->m, c->push_factor_batch,
-                                         // a factor of 1e30 or more pulls every level
-                                         c->push_factor_batch >= 1e30 ? 0ull : (unsigned long long)(n / 4),
-                                         c->d_level_te, c->d_level_cnt, ll, c->lpool_cap, lmax, g->to_view);
+        k_pass_start<K><<<grid_of(c, 8, (n * K + 31) / 32), 256, 0, s>>>(P);
     }
-    CU_LAUNCH("k_batch_init");
+    CU_LAUNCH("k_pass_start");
+    c->last_batch_k = K;
+    c->prev_lend = 0;
 
     int L = 0;
     if (use_persist(c, nsrc)) TRY(traverse_persistent<K>(c, &L));
-    else TRY(traverse_stepwise<K>(c, nsrc, sgrid, &L));
+    else TRY(traverse_stepwise<K>(c, nsrc, &L));
     // the per-pivot level counts and the list-pool flag arrive in the
     // background; the next batch (or a caller that reports them) waits for them
     if (!c->rb_ev) CU(cudaEventCreateWithFlags(&c->rb_ev, cudaEventDisableTiming));
@@ -2570,7 +2672,7 @@ static int apply_lanes(axbc_ctx *c, float *const *delta_out, const int *lane_lo,
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_update_m<K>, UPD_TPB(K), 0));
         c->upd_blocks_per_sm[K - 1] = std::max(1, b);
     }
-    const int grid = axbc_grid_for(c, UPD_TPB(K), c->upd_blocks_per_sm[K - 1]);
+    const int grid = grid_of(c, c->upd_blocks_per_sm[K - 1], (g->n + UPD_TPB(K) - 1) / UPD_TPB(K));
     const bool one_seg = nseg == 1 && (!lane_lo || lane_lo[0] == 0) && (!lane_hi || lane_hi[0] >= AXBC_W * K);
     {
         ProfScope ps(c, KP_UPDATE, (double)g->n * c->last_batch_nsrc * 20.0);
@@ -2647,21 +2749,19 @@ extern "C" int axbc_run_batch(axbc_ctx *c, const uint32_t *v0, const double *p, 
         c->bi_host->root[i] = v0[i];
         c->bi_host->p[i] = p[i];
     }
-    CU(cudaMemcpyAsync(&c->bi->root, c->bi_host->root, sizeof(c->bi_host->root),
+    // roots and probabilities lie next to each other
+    static_assert(offsetof(BatchInfo, p) == offsetof(BatchInfo, root) + sizeof(BatchInfo::root), "root, p");
+    CU(cudaMemcpyAsync(&c->bi->root, c->bi_host->root, sizeof(BatchInfo::root) + sizeof(BatchInfo::p),
                        cudaMemcpyHostToDevice, s));
-    CU(cudaMemcpyAsync(&c->bi->p, c->bi_host->p, sizeof(c->bi_host->p), cudaMemcpyHostToDevice, s));
     TRY(axbc_batch_traverse(c, k, H));
     TRY(axbc_batch_apply(c));
+    if (stats) CU(cudaMemcpyAsync(c->bi_host, c->bi, sizeof(BatchInfo), cudaMemcpyDeviceToHost, s));
+    if (stats) CU(cudaStreamSynchronize(s));
     TRY(axbc_batch_settle(c));
     if (stats) {
-        CU(cudaMemcpyAsync(c->bi_host, c->bi, sizeof(BatchInfo), cudaMemcpyDeviceToHost, s));
-        std::vector<uint32_t> rr(k);
-        for (int i = 0; i < k; i++)
-            CU(cudaMemcpyAsync(&rr[i], c->g->reach + v0[i], 4, cudaMemcpyDeviceToHost, s));
-        CU(cudaStreamSynchronize(s));
         for (int i = 0; i < k; i++) {
             stats[i].nvisited = c->bi_host->nvis[i];
-            stats[i].all = (H == 1 ? (uint32_t)c->bi_host->rsum[i] : 0u) + rr[i];
+            stats[i].all = (H == 1 ? (uint32_t)c->bi_host->rsum[i] : 0u) + c->bi_host->root_reach[i];
             stats[i].te = 2 * c->bi_host->te[i];
             stats[i].levels = c->last_Ls[i];
             stats[i].pad = 0;

@@ -19,8 +19,6 @@
 #define AXBC_CHUNK 32
 #define AXBC_SPAN 1024
 #define AXBC_SAMPLE_BLOCK 1024
-// Vertices with more than AXBC_BIG neighbours are split over several warps.
-#define AXBC_BIG 128
 // A backward tile holds at most this many 32-position chunks.
 #define BWD_TILE_CHUNKS 32
 #define BWD_SPAN_TILE 0x80000000u
@@ -82,9 +80,10 @@ struct Adj {
     uint32_t *ltask = nullptr;        // n_ltask + 1 offsets into order
     uint64_t n_ltask = 0;
     // the forward kernels' split of the same order: order[0..n_big) have more
-    // than AXBC_BIG neighbours and are walked in parts of part_len positions
-    // (part[i]: vertex, part number), order[n_big..n_linked) at least one
-    uint32_t n_big = 0, n_linked = 0;
+    // than `big` neighbours (they are split over several warps) and are walked
+    // in parts of part_len positions (part[i]: vertex, part number),
+    // order[n_big..n_linked) have at least one
+    uint32_t big = 0, n_big = 0, n_linked = 0;
     uint2 *part = nullptr;            // n_part
     uint64_t n_part = 0;
     uint32_t part_len = 0;
@@ -146,6 +145,15 @@ struct PivotCounters {  // device, single-source
     unsigned long long visited_rdeg;  // in-degree sum of visited vertices
 };
 
+// Grid barrier of a cooperative launch (batch.cu): arrivals since the launch
+// began, the last barrier whose lead has run, and the failure record of a wait
+// that ran out of its budget.
+struct GridSync {
+    unsigned int count;
+    unsigned int gen;
+    int err;   // nonzero: the site of the barrier whose wait ran out
+    int need;  // the persistent forward loop reached the levels allocated
+};
 struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     uint32_t nsrc;
     uint32_t pad0;
@@ -153,6 +161,7 @@ struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     unsigned long long srcmask;
     uint32_t root[AXBC_WMAX];
     double p[AXBC_WMAX];
+    uint32_t root_reach[AXBC_WMAX];
     // per-source totals accumulated by the level-stats kernel
     unsigned long long nvis[AXBC_WMAX];
     unsigned long long rsum[AXBC_WMAX];
@@ -164,7 +173,7 @@ struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     unsigned long long unvis_dec;   // this level's decrease of unvis_deg
     unsigned long long lvl_te;  // degree sum over the level's new (vertex, pivot) pairs
     uint32_t any_new;
-    uint32_t task_ctr[4];
+    uint32_t ticket[2];  // blocks done: pass reset, level statistics (0 between launches)
     int32_t H;
     // device-driven level loop: the step kernels read their level and
     // direction here, the advance kernels move them on
@@ -174,6 +183,7 @@ struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     int32_t lend;       // first level that discovered nothing (once alive == 0)
     int32_t dmax;       // deepest depth = lend - 1
     int32_t push_next;  // 1: the next forward level pushes from the frontier
+    GridSync gs;        // barrier of the persistent loop
     double push_factor;
     unsigned long long push_min;  // frontier degree sums below this always push
     int32_t Ls[AXBC_WMAX];  // per pivot: first level that discovered nothing
@@ -192,14 +202,6 @@ struct LaneTargets {
 
 struct SamplerState;  // sampler.cu
 
-// Grid barrier of a cooperative launch (batch.cu): arrival count, generation,
-// and the failure record of a wait that ran out of its budget.
-struct GridSync {
-    unsigned int count;
-    unsigned int gen;
-    int err;   // nonzero: the site of the barrier whose wait ran out
-    int need;  // the persistent forward loop reached the levels allocated
-};
 // batches of at most AXBC_PERSIST_AUTO_WIDTH pivots on graphs whose last batch
 // was deeper than AXBC_PERSIST_AUTO_LEVELS run their levels in one persistent
 // launch
@@ -207,6 +209,9 @@ struct GridSync {
 // passes (meshes and road-like graphs keep their own, already local, order)
 #ifndef AXBC_RENUMBER_MIN_DEG
 #define AXBC_RENUMBER_MIN_DEG 64
+#endif
+#ifndef AXBC_PERSIST_AUTO_M
+#define AXBC_PERSIST_AUTO_M (1ull << 21)
 #endif
 #ifndef AXBC_PERSIST_AUTO_LEVELS
 #define AXBC_PERSIST_AUTO_LEVELS 64
@@ -265,7 +270,6 @@ struct axbc_ctx {
     uint32_t *msigma = nullptr;     // n*32
     float *mdelta = nullptr;        // n*32
     float *mq = nullptr;            // n*32: (delta + 1) / sigma, per pivot
-    uint32_t *task_ctr = nullptr;   // work counters of the dynamic kernels
     float *mpartial = nullptr;      // span sums of the heavy vertices, 64 per span
     uint32_t *harrive = nullptr;    // per half and heavy vertex: span sums written (0 between depths)
     BatchInfo *bi = nullptr;
@@ -302,6 +306,9 @@ struct axbc_ctx {
     double *dyn_local2 = nullptr;
     double *dyn_csum2 = nullptr;
     float *wtmp = nullptr;
+    uint32_t *hist_v = nullptr;  // pivots and probabilities of a run, kept between runs
+    double *hist_p = nullptr;
+    uint64_t hist_cap = 0;
     std::vector<uint32_t> run_pivots;
     std::vector<double> run_probs;
     std::vector<uint32_t> run_checks;
@@ -317,7 +324,7 @@ struct axbc_ctx {
     // AXBC_PERSIST_AUTO_LEVELS, 1 always; blocks per SM of its cooperative grid
     int persist_mode = 0;
     int persist_blocks_per_sm = 4;
-    struct GridSync *gsync = nullptr;  // its barrier state (device)
+    int persist_fit[2] = {0, 0};       // blocks of it that fit an SM, per width
     std::vector<cudaEvent_t> ev_pool;
     double level_te_prev = 0;  // degree sum of the previous level's new vertices
     std::vector<double> level_te;
@@ -327,9 +334,8 @@ struct axbc_ctx {
     uint64_t bytes = 0;
     int num_sms = 0;
     // resident blocks per SM, per width (index K - 1)
-    int dyn_blocks_per_sm[2] = {0, 0};   // forward push
+    int fwd_blocks_per_sm[2] = {0, 0};   // forward level
     int upd_blocks_per_sm[2] = {0, 0};   // batched bc update
-    int pull_blocks_per_sm[2] = {0, 0};  // forward pull
     int bwd_blocks_per_sm[2] = {0, 0};   // backward
 };
 

@@ -137,9 +137,14 @@ static void task_tables(const uint32_t *col, uint64_t n, std::vector<uint32_t> &
     ltask.push_back((uint32_t)n);
 }
 
-// Positions per part of a big vertex: short parts spread a small graph over the
-// whole chip, long ones amortise a part's atomics once every warp has many.
-static uint32_t part_len_of(uint64_t m) { return m >= (1ull << 25) ? 512 : 128; }
+// Neighbours above which a vertex is split over warps, and positions per part.
+// Below 2^18 adjacency entries every 32 positions have a warp of the chip to
+// themselves; long parts amortise a part's atomics once every warp has many.
+// Measured (us a pass of one pivot, 32 : 128): 0.02 M entries 170 : 184, 0.13 M
+// 175 : 195, 0.43 M 232 : 217, 1.8 M 405 : 340.
+#define AXBC_SMALL_M (1ull << 18)
+static uint32_t big_of(uint64_t m) { return m < AXBC_SMALL_M ? 32 : 128; }
+static uint32_t part_len_of(uint64_t m) { return m < AXBC_SMALL_M ? 32 : m < (1ull << 25) ? 128 : 512; }
 
 // heavy-vertex span items and light-vertex tasks of an adjacency whose col
 // (host copy: col) is on the device
@@ -169,10 +174,11 @@ static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, u
     CU(cudaMemcpy(a.ltask, ltask.data(), ltask.size() * 4, cudaMemcpyHostToDevice));
     // parts of the big vertices
     auto deg = [&](uint64_t i) { return col[order[i] + 1] - col[order[i]]; };
+    a.big = big_of(a.m);
     a.part_len = part_len_of(a.m);
     std::vector<uint2> part;
     uint64_t i = 0;
-    for (; i < n && deg(i) > AXBC_BIG; i++)
+    for (; i < n && deg(i) > a.big; i++)
         for (uint32_t k = 0; k * a.part_len < deg(i); k++) part.push_back(make_uint2(order[i], k));
     a.n_big = (uint32_t)i;
     a.n_linked = (uint32_t)(std::partition_point(order.begin() + i, order.end(),

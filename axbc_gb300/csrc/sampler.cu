@@ -685,14 +685,37 @@ static void sr_release(SampledRun *r, bool own)
         axbc_dfree(r->dyn_csum);
         axbc_dfree(r->dyn_local2);
         axbc_dfree(r->dyn_csum2);
+        axbc_dfree(r->hist_v);
+        axbc_dfree(r->hist_p);
     }
-    axbc_dfree(r->hist_v);
-    axbc_dfree(r->hist_p);
     r->hist_v = nullptr;
     r->hist_p = nullptr;
 }
 
 void sr_free(SampledRun *r) { sr_release(r, true); }
+
+// the context's own pivot history, kept between runs and grown on demand
+static int ctx_hist(axbc_ctx *c, SampledRun *r)
+{
+    const uint64_t cap = std::min<uint64_t>(r->prm.nbfs, c->g->n) + 1;
+    if (cap > c->hist_cap) {
+        // both new buffers first: a failure keeps the old pair
+        DBuf nv, np;
+        TRY(nv.alloc(cap * 4));
+        TRY(np.alloc(cap * 8));
+        axbc_dfree(c->hist_v);
+        axbc_dfree(c->hist_p);
+        c->hist_v = nv.as<uint32_t>();
+        c->hist_p = np.as<double>();
+        nv.p = np.p = nullptr;
+        c->bytes += 12 * (cap - c->hist_cap);
+        c->hist_cap = cap;
+    }
+    r->hist_v = c->hist_v;
+    r->hist_p = c->hist_p;
+    r->hist_cap = cap;
+    return AXBC_OK;
+}
 
 static int sr_alloc_hist(SampledRun *r, uint64_t n)
 {
@@ -965,9 +988,12 @@ static int sr_round_alone(axbc_ctx *c, SampledRun *r)
             TRY(sr_load(c, r, off, 0, cnt));
             TRY(axbc_batch_traverse(c, cnt, r->prm.H));
             r->batches++;
-            float *tg[AXBC_WMAX];
-            for (int i = 0; i < AXBC_WMAX; i++) tg[i] = r->bc;
-            TRY(axbc_batch_set_targets(c, tg));
+            // the pass's lanes update the context's bc unless told otherwise
+            if (r->bc != c->bc) {
+                float *tg[AXBC_WMAX];
+                for (int i = 0; i < AXBC_WMAX; i++) tg[i] = r->bc;
+                TRY(axbc_batch_set_targets(c, tg));
+            }
         }
         TRY(sr_post(c, r, off, 0, std::max(cnt, 0)));
         if (cnt > 0) {
@@ -1008,7 +1034,7 @@ extern "C" int axbc_run_sampled(axbc_ctx *c, const axbc_run_params *prm, axbc_ru
     r.dyn_csum = c->dyn_csum;
     r.dyn_local2 = c->dyn_local2;
     r.dyn_csum2 = c->dyn_csum2;
-    int st = sr_alloc_hist(&r, c->g->n);
+    int st = ctx_hist(c, &r);
     if (st == AXBC_OK) st = sr_begin(c, &r);
     while (st == AXBC_OK) {
         if ((st = sr_draw(c, &r)) != AXBC_OK) break;

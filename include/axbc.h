@@ -356,12 +356,13 @@ int axbc_ctx_profile_records(axbc_ctx *ctx, int32_t *kinds, int32_t *tags, float
 int axbc_ctx_launches(const axbc_ctx *ctx, uint64_t *launches);
 
 /* ---- persistent level loop ----
- * A batched pass normally launches four kernels per forward level and two or
- * three per backward depth.  On graphs of many narrow levels it can instead
+ * A batched pass normally launches two kernels per forward level and one or
+ * two per backward depth.  On graphs of many narrow levels it can instead
  * run as one cooperative launch (all blocks resident, a bounded grid barrier
  * between phases).  mode 1 always, -1 never, 0 (default) for batches of at
- * most 8 pivots when the context's last batch was deeper than 64 levels or,
- * for its first batch, when no vertex has more than 64 neighbours.
+ * most 32 pivots on graphs of less than 2^21 adjacency entries, and for batches
+ * of at most 8 pivots when the context's last batch was deeper than 64 levels
+ * or, for its first batch, when no vertex has more than 64 neighbours.
  * blocks_per_sm: blocks of the cooperative grid per SM (0 keeps the current
  * setting, default 4).  Results
  * are the same bits either way.  A barrier wait that runs out of its budget
