@@ -201,6 +201,7 @@ struct LaneTargets {
 #define AXBC_MAX_LEVELS (1 << 16)
 
 struct SamplerState;  // sampler.cu
+struct PivotCtl;      // single.cu
 
 // batches of at most AXBC_PERSIST_AUTO_WIDTH pivots on graphs whose last batch
 // was deeper than AXBC_PERSIST_AUTO_LEVELS run their levels in one persistent
@@ -262,6 +263,14 @@ struct axbc_ctx {
     float *partial = nullptr;  // heavy span partials (fwd heavy items)
     PivotCounters *pc = nullptr;
     PivotCounters *pc_host = nullptr;  // pinned
+    // the one-launch form of a plain pivot
+    bool pivot_ready = false;
+    float *pq = nullptr;             // n: (delta + 1) / sigma
+    uint32_t *plev = nullptr;        // n + 2: start of each level in the queue
+    uint32_t *parrive = nullptr;     // per heavy vertex: span sums written
+    PivotCtl *pctl = nullptr;
+    PivotCtl *pctl_host = nullptr;   // pinned
+    int pivot_fit = 0;               // its blocks that fit an SM
     std::vector<uint64_t> levstart;
     uint64_t s_front_deg = 0, s_prev_newdeg = 0, s_visited_rdeg = 0;  // direction choice
     // multi-source batch state

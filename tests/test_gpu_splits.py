@@ -73,3 +73,21 @@ def test_clustering_of_a_power_law_graph(axbc, orc, H):
     row[col[v]] = row[col[v] + 1]
     h = orc.CSC(col, row)
     assert np.array_equal(axbc.Graph.from_csc(col, row).lcc(), orc.lcc(h))
+
+
+@pytest.mark.parametrize("factor", [8.0, 0.0, 1e30])
+@pytest.mark.parametrize("undirected", [True, False])
+def test_plain_pivots_at_degree_edges(axbc, orc, undirected, factor):
+    g = hub_graph(orc, undirected)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    ctx.set_tuning(factor, 8.0)
+    rng = np.random.default_rng(3)
+    for v in rng.choice(np.flatnonzero(g.deg > 0), 6, replace=False):
+        for profiled in (False, True):  # one launch, then level by level
+            ctx.profile(profiled)
+            ctx.reset()
+            st = ctx.run_pivot(int(v), 1.0 / g.n, 1)
+            want, lvl, sigma, delta, stats = orc.bc_pivot(g, int(v), 1.0 / g.n, 1)
+            assert np.array_equal(ctx.bc(), want) and np.array_equal(ctx.delta(), delta)
+            assert np.array_equal(ctx.levels(), lvl) and np.array_equal(ctx.sigma(), sigma)
+            assert st == stats
