@@ -220,11 +220,8 @@ extern "C" int axbc_ctx_destroy(axbc_ctx *c)
     axbc_dfree(c->partial);
     axbc_dfree(c->pc);
     if (c->pc_host) cudaFreeHost(c->pc_host);
-    axbc_dfree(c->pq);
-    axbc_dfree(c->plev);
-    axbc_dfree(c->parrive);
-    axbc_dfree(c->pctl);
-    if (c->pctl_host) cudaFreeHost(c->pctl_host);
+    axbc_pivot_free(c->piv);
+    axbc_pivot_free(c->one);
     axbc_dfree(c->seen);
     for (uint32_t *p : c->fmask) axbc_dfree(p);
     axbc_dfree(c->msigma);

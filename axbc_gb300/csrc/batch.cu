@@ -158,7 +158,8 @@ __device__ __forceinline__ void pass_roots(const PassStart &P)
         bi->lvl_te = 0;
         bi->any_new = 0;
         bi->pool_short = 0;
-        bi->gs = GridSync{0, 0, 0, 0};
+        bi->gs.count = bi->gs.gen = 0;
+        bi->gs.err = bi->gs.need = 0;
     }
     unsigned long long fd = 0, rd = 0;
     uint32_t nroots = 0, heavy_roots = 0;
@@ -2483,6 +2484,8 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
     return AXBC_OK;
 }
 
+static int read_back(axbc_ctx *c, int nsrc, int L);
+
 // Forward and backward passes of the batch of width K whose roots/p are in
 // c->bi.  The host launches forward level steps in blocks (8, then doubling)
 // and reads the level state once per block; steps past the last level do
@@ -2556,8 +2559,16 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
     int L = 0;
     if (use_persist(c, nsrc)) TRY(traverse_persistent<K>(c, &L));
     else TRY(traverse_stepwise<K>(c, nsrc, &L));
-    // the per-pivot level counts and the list-pool flag arrive in the
-    // background; the next batch (or a caller that reports them) waits for them
+    TRY(read_back(c, nsrc, L));
+    c->prev_lend = L;
+    return AXBC_OK;
+}
+
+// the per-pivot level counts and the list-pool flag arrive in the background;
+// the next batch (or a caller that reports them) waits for them
+static int read_back(axbc_ctx *c, int nsrc, int L)
+{
+    cudaStream_t s = c->stream;
     if (!c->rb_ev) CU(cudaEventCreateWithFlags(&c->rb_ev, cudaEventDisableTiming));
     CU(cudaMemcpyAsync(c->bi_host->Ls, c->bi->Ls, sizeof(c->bi_host->Ls), cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(&c->bi_host->pool_short, &c->bi->pool_short, 4, cudaMemcpyDeviceToHost, s));
@@ -2565,8 +2576,25 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
     c->rb_pending = true;
     c->last_batch_levels = L;
     c->last_batch_nsrc = nsrc;
-    c->prev_lend = L;
     return AXBC_OK;
+}
+
+// A pass of one pivot runs in the plain form's one launch: rows of 32 pivots
+// would carry one.  (us a pass, persistent rows : this: scale 14 218 : 115, 18 498 :
+// 318, a 512^2 grid 5150 : 3300.)  Counting runs and a level loop that the caller
+// has chosen keep the batched kernels.
+static int traverse_one(axbc_ctx *c, int H)
+{
+    TRY(ensure_level_tables(c));
+    TRY(axbc_batch_settle(c));
+    int L = 0;
+    TRY(axbc_one_traverse(c, H, &L));
+    if (L > AXBC_MAX_LEVELS - 3) {
+        axbc_set_error("traversal deeper than %d levels", AXBC_MAX_LEVELS - 2);
+        return AXBC_ERR_RANGE;
+    }
+    c->last_one = true;
+    return read_back(c, 1, L);
 }
 
 // A multi-source pass of nsrc <= 64 pivots: 32-bit masks up to 32 pivots,
@@ -2577,6 +2605,13 @@ int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H)
         axbc_set_error("batched pass of %d pivots (1..%d)", nsrc, AXBC_WMAX);
         return AXBC_ERR_INVALID;
     }
+    if (nsrc == 1 && c->persist_mode == 0 && !c->count_on) {
+        int rc = AXBC_OK;
+        const bool fits = axbc_one_fits(c, &rc);
+        TRY(rc);
+        if (fits) return traverse_one(c, H);
+    }
+    c->last_one = false;
     return width_k(nsrc) == 2 ? batch_traverse<2>(c, nsrc, H) : batch_traverse<1>(c, nsrc, H);
 }
 
@@ -2627,6 +2662,16 @@ static int apply_lanes(axbc_ctx *c, float *const *delta_out, const int *lane_lo,
 int axbc_batch_apply_lanes(axbc_ctx *c, float *const *delta_out, const int *lane_lo,
                            const int *lane_hi, int nseg)
 {
+    if (c->last_one) {
+        // the segment that holds lane 0
+        float *out = nullptr;
+        for (int i = 0; i < nseg; i++)
+            if ((!lane_lo || lane_lo[i] == 0) && (!lane_hi || lane_hi[i] > 0))
+                out = delta_out ? delta_out[i] : c->delta_last;
+        TRY(axbc_one_apply(c, out));
+        c->delta_last_valid = true;
+        return AXBC_OK;
+    }
     return c->last_batch_k == 2 ? apply_lanes<2>(c, delta_out, lane_lo, lane_hi, nseg)
                                 : apply_lanes<1>(c, delta_out, lane_lo, lane_hi, nseg);
 }
@@ -2646,6 +2691,16 @@ extern "C" int axbc_ctx_level_stats(axbc_ctx *c, uint64_t *count, uint64_t *te, 
     if (count) CU(cudaMemcpy(count, c->d_level_cnt, L * 8, cudaMemcpyDeviceToHost));
     if (te) CU(cudaMemcpy(te, c->d_level_te, L * 8, cudaMemcpyDeviceToHost));
     if (push) CU(cudaMemcpy(push, c->d_level_mode, L * 4, cudaMemcpyDeviceToHost));
+    if (c->last_one) {
+        // its queue lists every level
+        std::vector<uint32_t> lev(L + 1);
+        CU(cudaMemcpy(lev.data(), c->one.lev, (L + 1) * 4, cudaMemcpyDeviceToHost));
+        for (int i = 0; i < L; i++) {
+            if (list_count) list_count[i] = lev[i + 1] - lev[i];
+            if (list_cap) list_cap[i] = std::max(list_max_of(c), lev[i + 1] - lev[i]);
+        }
+        return AXBC_OK;
+    }
     if (list_count) CU(cudaMemcpy(list_count, c->lcount, L * 4, cudaMemcpyDeviceToHost));
     if (list_cap) CU(cudaMemcpy(list_cap, c->lcap, L * 4, cudaMemcpyDeviceToHost));
     return AXBC_OK;
@@ -2709,6 +2764,13 @@ extern "C" int axbc_get_batch_source(axbc_ctx *c, int src, uint32_t *sigma_host,
     CHECK_ARG(src >= 0 && src < c->last_batch_nsrc, "axbc_get_batch_source: bad source index");
     const uint64_t n = c->g->n;
     cudaStream_t s = c->stream;
+    if (c->last_one) {
+        if (sigma_host) CU(cudaMemcpyAsync(sigma_host, c->one.sigma, n * 4, cudaMemcpyDeviceToHost, s));
+        if (lvl_host) CU(cudaMemcpyAsync(lvl_host, c->one.lvl, n * 4, cudaMemcpyDeviceToHost, s));
+        if (delta_host) CU(cudaMemcpyAsync(delta_host, c->one.delta, n * 4, cudaMemcpyDeviceToHost, s));
+        CU(cudaStreamSynchronize(s));
+        return AXBC_OK;
+    }
     const int levels = c->last_batch_levels + 1;
     uint32_t **d_fm = nullptr;
     uint32_t *sig = nullptr;

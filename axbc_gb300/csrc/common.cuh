@@ -150,9 +150,11 @@ struct PivotCounters {  // device, single-source
 // that ran out of its budget.
 struct GridSync {
     unsigned int count;
-    unsigned int gen;
     int err;   // nonzero: the site of the barrier whose wait ran out
     int need;  // the persistent forward loop reached the levels allocated
+    int pad_[29];
+    unsigned int gen;  // polled: on a line of its own, away from the arrivals
+    int pad2_[31];
 };
 struct BatchInfo {  // device, one multi-source batch of up to AXBC_WMAX pivots
     uint32_t nsrc;
@@ -202,6 +204,20 @@ struct LaneTargets {
 
 struct SamplerState;  // sampler.cu
 struct PivotCtl;      // single.cu
+
+// device state of a pivot in one launch (single.cu)
+struct PivotBuf {
+    bool ready = false, owns = false;
+    int32_t *lvl = nullptr;
+    uint32_t *sigma = nullptr, *queue = nullptr;
+    float *delta = nullptr;
+    float *q = nullptr;              // n: (delta + 1) / sigma
+    uint32_t *lev = nullptr;         // n + 2: start of each level in the queue
+    float *partial = nullptr;        // span sums of the heavy vertices
+    uint32_t *arrive = nullptr;      // per heavy vertex: span sums written
+    PivotCtl *ctl = nullptr;
+    PivotCtl *ctl_host = nullptr;    // pinned
+};
 
 // batches of at most AXBC_PERSIST_AUTO_WIDTH pivots on graphs whose last batch
 // was deeper than AXBC_PERSIST_AUTO_LEVELS run their levels in one persistent
@@ -263,14 +279,11 @@ struct axbc_ctx {
     float *partial = nullptr;  // heavy span partials (fwd heavy items)
     PivotCounters *pc = nullptr;
     PivotCounters *pc_host = nullptr;  // pinned
-    // the one-launch form of a plain pivot
-    bool pivot_ready = false;
-    float *pq = nullptr;             // n: (delta + 1) / sigma
-    uint32_t *plev = nullptr;        // n + 2: start of each level in the queue
-    uint32_t *parrive = nullptr;     // per heavy vertex: span sums written
-    PivotCtl *pctl = nullptr;
-    PivotCtl *pctl_host = nullptr;   // pinned
-    int pivot_fit = 0;               // its blocks that fit an SM
+    // the one-launch form of a pivot: run_pivot's buffers (path counts, levels,
+    // dependencies and queue are those above) and a one-pivot pass's own
+    PivotBuf piv, one;
+    bool last_one = false;  // the last batch was such a pass: its results are in `one`
+    int pivot_fit = 0;      // blocks of the kernel that fit an SM
     std::vector<uint64_t> levstart;
     uint64_t s_front_deg = 0, s_prev_newdeg = 0, s_visited_rdeg = 0;  // direction choice
     // multi-source batch state
@@ -391,6 +404,12 @@ int axbc_single_backward_level(axbc_ctx *c, uint32_t ls, uint32_t nseg, int d);
 int axbc_single_reach_sum(axbc_ctx *c);
 int axbc_single_update(axbc_ctx *c, uint32_t v0, double p, const uint32_t *reach_v0_dev,
                        uint64_t nvt_base, int add_all, int add_sum);
+// a pass of one pivot (the root in c->bi, as a vertex id) into c->one and the
+// totals of c->bi, without the update; its update and last dependencies
+bool axbc_one_fits(axbc_ctx *c, int *rc);
+int axbc_one_traverse(axbc_ctx *c, int H, int *levels);
+int axbc_one_apply(axbc_ctx *c, float *delta_out);
+void axbc_pivot_free(PivotBuf &b);
 int axbc_ensure_batch(axbc_ctx *c);
 int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H);
 int axbc_batch_settle(axbc_ctx *c);

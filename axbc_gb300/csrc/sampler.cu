@@ -568,7 +568,8 @@ __global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__r
                                const float *__restrict__ mdelta, const uint32_t *__restrict__ seen,
                                const uint32_t *__restrict__ reach, const uint32_t *__restrict__ checks,
                                float *b, uint32_t *hist_v, double *hist_p, uint64_t hist_cap,
-                               int off, int lane0, int cnt, int K, const uint32_t *__restrict__ to_view)
+                               int off, int lane0, int cnt, int K, const uint32_t *__restrict__ to_view,
+                               const float *__restrict__ one_delta)
 {
     if (ss->done && ss->nb == 0) return;
     const int nb = max(0, min(min(ss->nb - off, AXBC_WMAX - lane0), cnt));
@@ -609,9 +610,15 @@ __global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__r
                 if (rr > 0) b[i] = __fadd_rn(b[i], bc_root_term(rr, nvt));
                 continue;
             }
-            // the pass's layout: K mask words and 32 K row values per vertex
-            const bool reached = (seen[(uint64_t)v * K + l / 32] >> (l % 32)) & 1u;
-            const float dv = reached ? mdelta[(uint64_t)v * (AXBC_W * K) + l] : __uint2float_rn(reach[v]);
+            float dv;
+            if (one_delta) {
+                // a pass of one pivot, in vertex ids
+                dv = one_delta[v];
+            } else {
+                // the pass's layout: K mask words and 32 K row values per vertex
+                const bool reached = (seen[(uint64_t)v * K + l / 32] >> (l % 32)) & 1u;
+                dv = reached ? mdelta[(uint64_t)v * (AXBC_W * K) + l] : __uint2float_rn(reach[v]);
+            }
             if (dv == 0.0f && p > 0.0) continue;
             b[i] = __fadd_rn(b[i], bc_term(dv, rr, p));
         }
@@ -898,10 +905,11 @@ int sr_post(axbc_ctx *c, SampledRun *r, int off, int lane0, int cnt)
 {
     {
         ProfScope ps(c, KP_SAMPLER, 0);
-        k_sampler_post<<<1, 1, 0, c->stream>>>(r->ss, c->bi, r->bc, c->mdelta, c->seen, c->g->breach,
-                                               r->checks, r->checkval, r->hist_v, r->hist_p,
-                                               r->hist_cap, off, lane0, cnt, c->last_batch_k,
-                                               c->g->to_view);
+        k_sampler_post<<<1, 1, 0, c->stream>>>(r->ss, c->bi, r->bc, c->mdelta, c->seen,
+                                               c->last_one ? c->g->reach : c->g->breach, r->checks, r->checkval,
+                                               r->hist_v, r->hist_p, r->hist_cap, off, lane0, cnt, c->last_batch_k,
+                                               c->last_one ? nullptr : c->g->to_view,
+                                               c->last_one ? c->one.delta : nullptr);
     }
     CU_LAUNCH("k_sampler_post");
     return AXBC_OK;

@@ -414,6 +414,9 @@ int axbc_single_update(axbc_ctx *c, uint32_t v0, double p, const uint32_t *reach
 }
 
 // ------------------------------------------- a pivot in one launch
+#define PIVOT_TPB 256
+#define PIVOT_BPS 4
+#define PIVOT_NW (PIVOT_TPB / 32)
 // Reset, forward levels, backward depths and the update with a grid barrier
 // between them: one per level and depth.  The level-by-level form spent 200 us
 // on a graph of a thousand vertices, most of it between a dozen launches and
@@ -443,6 +446,11 @@ struct PivotRun {
     uint32_t v0;
     int H;
     double p, push_factor;
+    // a pass of one pivot: the root comes from bi, its totals and the level
+    // tables go there, and the update is left to k_one_update
+    BatchInfo *bi;
+    unsigned long long *level_te, *level_cnt;
+    int32_t *level_mode;
 };
 
 // what a thread has discovered in a level
@@ -670,12 +678,12 @@ __device__ __forceinline__ void pivot_chunks(const PivotRun &R, const uint32_t r
     for (int i = 0; i < NC; i++) sum[i] = warp_tree_sum(l[i] == d + 1 ? __fmul_rn(x[i], sc[i]) : 0.0f);
 }
 
-#define PIVOT_NW (256 / 32)
 // Backward depth d over the vertices queue[ls, ls + cnt): the canonical sum.
 __device__ __forceinline__ void pivot_bwd_depth(const Adj &a, const PivotRun &R, uint32_t ls, uint32_t cnt, int d,
                                                 float (*csum)[BWD_TILE_CHUNKS])
 {
-    constexpr int NC = BWD_TILE_CHUNKS / PIVOT_NW;
+    constexpr int NC = BWD_TILE_CHUNKS / PIVOT_NW;  // chunks per warp of a tile
+    constexpr int NL = 4;                           // and of a list read at once
     const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
     // tiles of the big vertices, each by a block: chunk sums in shared memory
     int buf = 0;
@@ -779,20 +787,20 @@ __device__ __forceinline__ void pivot_bwd_depth(const Adj &a, const PivotRun &R,
             const uint32_t b1 = b0 + __shfl_sync(FULL_MASK, d_l, j);
             const float s1 = __uint2float_rn(R.sigma[v]);
             float P = 0.0f;
-            for (uint32_t base = b0; base < b1; base += 32 * NC) {
-                uint32_t r[NC];
-                bool in[NC];
-                float sc[NC], sum[NC];
+            for (uint32_t base = b0; base < b1; base += 32 * NL) {
+                uint32_t r[NL];
+                bool in[NL];
+                float sc[NL], sum[NL];
 #pragma unroll
-                for (int q = 0; q < NC; q++) {
+                for (int q = 0; q < NL; q++) {
                     const uint32_t e = base + 32 * q + lane;
                     in[q] = e < b1;
                     sc[q] = s1;
                     r[q] = in[q] ? a.row[e] : 0u;
                 }
-                pivot_chunks<NC>(R, r, in, d, sc, sum);
+                pivot_chunks<NL>(R, r, in, d, sc, sum);
 #pragma unroll
-                for (int q = 0; q < NC; q++) P = __fadd_rn(P, sum[q]);
+                for (int q = 0; q < NL; q++) P = __fadd_rn(P, sum[q]);
             }
             if (lane == 0) pivot_dep(R, v, __fadd_rn(__uint2float_rn(R.reach[v]), P));
         }
@@ -827,8 +835,14 @@ struct PivotLead {
         PivotCtl *c = R.ctl;
         const uint32_t tail = __ldcg(&c->qtail);
         const unsigned long long nd = __ldcg(&c->newdeg), unvis = R.m - __ldcg(&c->rdeg);
-        const bool alive = tail != vload_u(&R.lev[L]);
+        const uint32_t from = vload_u(&R.lev[L]);
+        const bool alive = tail != from;
         R.lev[L + 1] = tail;
+        if (R.bi && L < AXBC_MAX_LEVELS) {
+            R.level_te[L] = nd - __ldcg(&c->prev_newdeg);
+            R.level_cnt[L] = tail - from;
+            R.level_mode[L] = vload_i(&c->push);
+        }
         c->push = (double)(nd - __ldcg(&c->prev_newdeg)) * R.push_factor < (double)unvis;
         c->prev_newdeg = nd;
         c->alive = alive;
@@ -836,22 +850,23 @@ struct PivotLead {
     }
 };
 
-__global__ void __launch_bounds__(256, 4) k_pivot(Adj a, Adj rv, PivotRun R, long long budget)
+__global__ void __launch_bounds__(PIVOT_TPB, PIVOT_BPS) k_pivot(Adj a, Adj rv, PivotRun R, long long budget)
 {
     __shared__ float s_csum[2][BWD_TILE_CHUNKS];
     PivotCtl *ctl = R.ctl;
     unsigned epoch = 0;
     const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t v0 = R.bi ? R.bi->root[0] : R.v0;
     for (uint64_t v = tid; v < R.n; v += nt) {
-        const bool root = v == R.v0;
+        const bool root = v == v0;
         R.lvl[v] = root ? 0 : -1;
         R.sigma[v] = root ? 1u : 0u;
         R.delta[v] = __uint2float_rn(R.reach[v]);
     }
     if (tid == 0) {
-        const uint32_t deg = a.col[R.v0 + 1] - a.col[R.v0], rdeg = rv.col[R.v0 + 1] - rv.col[R.v0];
-        R.queue[0] = R.v0;
+        const uint32_t deg = a.col[v0 + 1] - a.col[v0], rdeg = rv.col[v0 + 1] - rv.col[v0];
+        R.queue[0] = v0;
         R.lev[0] = 0;
         R.lev[1] = 1;
         ctl->qtail = 1;
@@ -860,7 +875,19 @@ __global__ void __launch_bounds__(256, 4) k_pivot(Adj a, Adj rv, PivotRun R, lon
         ctl->rsum = 0;
         ctl->alive = 1;
         ctl->push = (double)deg * R.push_factor < (double)(R.m - rdeg);
+        if (R.bi) {
+            BatchInfo *bi = R.bi;
+            bi->nsrc = 1;
+            bi->srcmask = bi->applymask = 1;
+            bi->H = R.H;
+            bi->root_reach[0] = R.reach[v0];
+            bi->pool_short = 0;
+            R.level_te[0] = deg;
+            R.level_cnt[0] = 1;
+        }
     }
+    if (R.bi && blockIdx.x == 0)
+        for (int i = threadIdx.x; i < AXBC_WMAX; i += blockDim.x) R.bi->lane_bc[i] = R.bc;
     if (!grid_barrier(&ctl->gs, budget, 1, epoch, NoLead{})) return;
     int L = 1;
     for (;; L++) {
@@ -883,13 +910,27 @@ __global__ void __launch_bounds__(256, 4) k_pivot(Adj a, Adj rv, PivotRun R, lon
         }
         if (!grid_barrier(&ctl->gs, budget, 4, epoch, NoLead{})) return;
     }
+    if (R.bi) {
+        if (tid == 0) {
+            BatchInfo *bi = R.bi;
+            bi->nvis[0] = vload_u(&ctl->qtail);
+            bi->rsum[0] = __ldcg(&ctl->rsum);
+            bi->te[0] = __ldcg(&ctl->newdeg);
+            bi->Ls[0] = L;
+            bi->depth0mask = L == 2;
+            bi->cur = bi->lend = L;
+            bi->alive = 0;
+            bi->dmax = L - 1;
+        }
+        return;
+    }
     // update_bc (src/cuda_kernels.cu:269-286) of every vertex
-    const uint32_t reach_v0 = R.reach[R.v0];
+    const uint32_t reach_v0 = R.reach[v0];
     const uint32_t all = (R.H ? (uint32_t)__ldcg(&ctl->rsum) : 0u) + reach_v0;
     const unsigned long long nvt = vload_u(&ctl->qtail) + (unsigned long long)all;
     const InvSplit iv = inv_split(R.p);
     for (uint64_t v = tid; v < R.n; v += nt) {
-        if (v == R.v0) {
+        if (v == v0) {
             if (reach_v0 > 0) R.bc[v] = __fadd_rn(R.bc[v], bc_root_term(reach_v0, nvt));
             continue;
         }
@@ -899,66 +940,186 @@ __global__ void __launch_bounds__(256, 4) k_pivot(Adj a, Adj rv, PivotRun R, lon
     }
 }
 
-static int ensure_pivot(axbc_ctx *c)
+// update_bc of a one-pivot pass into its lane's bc vector, when the replay of
+// Bader's test applies it, and its dependencies as the last ones
+__global__ void k_one_update(const float *__restrict__ delta, uint64_t n, const BatchInfo *__restrict__ bi,
+                             float *__restrict__ delta_out)
 {
-    if (c->pivot_ready) return AXBC_OK;
+    if (!(bi->applymask & 1ull)) return;
+    float *bc = bi->lane_bc[0];
+    const uint32_t root = bi->root[0], rr = bi->root_reach[0];
+    const uint32_t all = (bi->H == 1 ? (uint32_t)bi->rsum[0] : 0u) + rr;
+    const unsigned long long nvt = bi->nvis[0] + all;
+    const double p = bi->p[0];
+    const InvSplit iv = inv_split(p);
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n;
+         v += (uint64_t)gridDim.x * blockDim.x) {
+        const float dv = delta[v];
+        if (delta_out) delta_out[v] = dv;
+        if (v == root) {
+            if (rr > 0) bc[v] = __fadd_rn(bc[v], bc_root_term(rr, nvt));
+            continue;
+        }
+        if (dv == 0.0f && p > 0.0) continue;  // x + float(0/p) == x
+        bc[v] = __fadd_rn(bc[v], bc_term_fast(dv, rr, p, iv));
+    }
+}
+
+void axbc_pivot_free(PivotBuf &b)
+{
+    if (b.owns) {
+        axbc_dfree(b.lvl);
+        axbc_dfree(b.sigma);
+        axbc_dfree(b.queue);
+        axbc_dfree(b.delta);
+        axbc_dfree(b.partial);
+    }
+    axbc_dfree(b.q);
+    axbc_dfree(b.lev);
+    axbc_dfree(b.arrive);
+    axbc_dfree(b.ctl);
+    if (b.ctl_host) cudaFreeHost(b.ctl_host);
+    b = PivotBuf();
+}
+
+static int pivot_fit(axbc_ctx *c)
+{
+    if (!c->pivot_fit)
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->pivot_fit, k_pivot, PIVOT_TPB, 0));
+    return AXBC_OK;
+}
+
+// owns: with path counts, levels, dependencies and queue of its own
+static int ensure_pivot(axbc_ctx *c, PivotBuf &b, bool owns)
+{
+    if (b.ready) return AXBC_OK;
     const uint64_t n = c->g->n;
-    TRY(axbc_ensure_single(c));
-    ALLOC_MISSING(c->pq, n * 4, &c->bytes);
-    ALLOC_MISSING(c->plev, (n + 2) * 4, &c->bytes);
-    ALLOC_MISSING(c->parrive, (c->g->fwd.n_heavy + 1) * 4, &c->bytes);
-    ALLOC_MISSING(c->pctl, sizeof(PivotCtl), &c->bytes);
-    if (!c->pctl_host) CU(cudaMallocHost((void **)&c->pctl_host, sizeof(PivotCtl)));
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->pivot_fit, k_pivot, 256, 0));
-    CU(cudaMemsetAsync(c->parrive, 0, (c->g->fwd.n_heavy + 1) * 4, c->stream));
-    c->pivot_ready = true;
+    TRY(pivot_fit(c));
+    b.owns = owns;
+    if (owns) {
+        ALLOC_MISSING(b.lvl, n * 4, &c->bytes);
+        ALLOC_MISSING(b.sigma, n * 4, &c->bytes);
+        ALLOC_MISSING(b.queue, (n + 1) * 4, &c->bytes);
+        ALLOC_MISSING(b.delta, n * 4, &c->bytes);
+        ALLOC_MISSING(b.partial, (c->g->fwd.n_heavy_items + 1) * 4, &c->bytes);
+    } else {
+        TRY(axbc_ensure_single(c));
+        b.lvl = c->lvl;
+        b.sigma = c->sigma;
+        b.queue = c->queue;
+        b.delta = c->delta;
+        b.partial = c->partial;
+    }
+    ALLOC_MISSING(b.q, n * 4, &c->bytes);
+    ALLOC_MISSING(b.lev, (n + 2) * 4, &c->bytes);
+    ALLOC_MISSING(b.arrive, (c->g->fwd.n_heavy + 1) * 4, &c->bytes);
+    ALLOC_MISSING(b.ctl, sizeof(PivotCtl), &c->bytes);
+    if (!b.ctl_host) CU(cudaMallocHost((void **)&b.ctl_host, sizeof(PivotCtl)));
+    CU(cudaMemsetAsync(b.arrive, 0, (c->g->fwd.n_heavy + 1) * 4, c->stream));
+    b.ready = true;
+    return AXBC_OK;
+}
+
+// One launch of k_pivot and the wait for it; its control block in b.ctl_host.
+static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R)
+{
+    axbc_graph *g = c->g;
+    cudaStream_t s = c->stream;
+    R.lvl = b.lvl;
+    R.sigma = b.sigma;
+    R.delta = b.delta;
+    R.q = b.q;
+    R.queue = b.queue;
+    R.lev = b.lev;
+    R.partial = b.partial;
+    R.arrive = b.arrive;
+    R.reach = g->reach;
+    R.bc = c->bc;
+    R.ctl = b.ctl;
+    R.n = g->n;
+    R.m = g->m;
+    R.push_factor = c->push_factor_single;
+    long long budget = AXBC_BAR_BUDGET;
+    // Blocks per SM: two where the levels are short or narrow and a barrier
+    // waits for every block, else four; or as many as have work.  Measured, us a
+    // pivot with 1, 2, 4: scale 14 121, 115, 126, scale 18 548, 382, 318, scale 22
+    // 7158, 3973, 2685, 256^2 grid 2472, 2695, 3327, 1024^2 grid 4336, 4271, 5290.
+    const int want = g->m < (1ull << 19) || g->max_deg <= 64 ? 2 : PIVOT_BPS;
+    const uint64_t work = std::max<uint64_t>(std::max<uint64_t>(g->fwd.n_part, g->rev.n_part) +
+                                                 std::max(g->fwd.n_linked, g->rev.n_linked),
+                                             g->n / 32);
+    const int grid = (int)std::max<uint64_t>(
+        1, std::min<uint64_t>((uint64_t)axbc_grid_for(c, PIVOT_TPB, std::min(want, c->pivot_fit)),
+                              (work + PIVOT_NW - 1) / PIVOT_NW));
+    CU(cudaMemsetAsync(b.ctl, 0, sizeof(GridSync), s));
+    void *args[] = {(void *)&g->fwd, (void *)&g->rev, (void *)&R, (void *)&budget};
+    {
+        ProfScope ps(c, KP_PERSIST, 0);
+        CU(cudaLaunchCooperativeKernel((const void *)k_pivot, grid, PIVOT_TPB, args, 0, s));
+    }
+    CU_LAUNCH("k_pivot");
+    CU(cudaMemcpyAsync(b.ctl_host, b.ctl, sizeof(PivotCtl), cudaMemcpyDeviceToHost, s));
+    return AXBC_OK;
+}
+
+static int pivot_wait(axbc_ctx *c, PivotBuf &b)
+{
+    CU(cudaStreamSynchronize(c->stream));
+    if (b.ctl_host->gs.err) {
+        CU(cudaMemsetAsync(b.arrive, 0, (c->g->fwd.n_heavy + 1) * 4, c->stream));
+        axbc_set_error("pivot in one launch: a grid barrier wait ran out of its budget (site %d)",
+                       b.ctl_host->gs.err);
+        return AXBC_ERR_TIMEOUT;
+    }
+    return AXBC_OK;
+}
+
+bool axbc_one_fits(axbc_ctx *c, int *rc)
+{
+    *rc = pivot_fit(c);
+    return *rc == AXBC_OK && c->pivot_fit > 0;
+}
+
+int axbc_one_traverse(axbc_ctx *c, int H, int *levels)
+{
+    TRY(ensure_pivot(c, c->one, true));
+    PivotRun R;
+    R.v0 = 0;
+    R.p = 1.0;
+    R.H = H;
+    R.bi = c->bi;
+    R.level_te = c->d_level_te;
+    R.level_cnt = c->d_level_cnt;
+    R.level_mode = c->d_level_mode;
+    TRY(pivot_launch(c, c->one, R));
+    TRY(pivot_wait(c, c->one));
+    *levels = c->one.ctl_host->levels;
+    return AXBC_OK;
+}
+
+int axbc_one_apply(axbc_ctx *c, float *delta_out)
+{
+    ProfScope ps(c, KP_UPDATE, (double)c->g->n * 20.0);
+    k_one_update<<<(int)std::min<uint64_t>(axbc_grid_for(c, 256, 8), (c->g->n + 255) / 256), 256, 0, c->stream>>>(
+        c->one.delta, c->g->n, c->bi, delta_out);
+    CU_LAUNCH("k_one_update");
     return AXBC_OK;
 }
 
 static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_stats *st)
 {
-    axbc_graph *g = c->g;
-    cudaStream_t s = c->stream;
     PivotRun R;
-    R.lvl = c->lvl;
-    R.sigma = c->sigma;
-    R.delta = c->delta;
-    R.q = c->pq;
-    R.queue = c->queue;
-    R.lev = c->plev;
-    R.partial = c->partial;
-    R.arrive = c->parrive;
-    R.reach = g->reach;
-    R.bc = c->bc;
-    R.ctl = c->pctl;
-    R.n = g->n;
-    R.m = g->m;
     R.v0 = v0;
-    R.H = H;
     R.p = p;
-    R.push_factor = c->push_factor_single;
-    long long budget = AXBC_BAR_BUDGET;
-    // every block that fits (at most four per SM), or as many as have work
-    const uint64_t work = std::max<uint64_t>(std::max<uint64_t>(g->fwd.n_part, g->rev.n_part) +
-                                                 std::max(g->fwd.n_linked, g->rev.n_linked),
-                                             g->n / 32);
-    const int grid = (int)std::max<uint64_t>(
-        1, std::min<uint64_t>((uint64_t)axbc_grid_for(c, 256, std::min(4, c->pivot_fit)), (work + 7) / 8));
-    CU(cudaMemsetAsync(c->pctl, 0, sizeof(GridSync), s));
-    void *args[] = {(void *)&g->fwd, (void *)&g->rev, (void *)&R, (void *)&budget};
-    CU(cudaLaunchCooperativeKernel((const void *)k_pivot, grid, 256, args, 0, s));
-    c->launches++;
-    CU_LAUNCH("k_pivot");
+    R.H = H;
+    R.bi = nullptr;
+    R.level_te = R.level_cnt = nullptr;
+    R.level_mode = nullptr;
+    TRY(pivot_launch(c, c->piv, R));
     c->delta_last_valid = false;  // the last pivot's delta is c->delta
-    CU(cudaMemcpyAsync(c->pctl_host, c->pctl, sizeof(PivotCtl), cudaMemcpyDeviceToHost, s));
-    CU(cudaMemcpyAsync(&c->pc_host->pad, g->reach + v0, 4, cudaMemcpyDeviceToHost, s));
-    CU(cudaStreamSynchronize(s));
-    const PivotCtl &h = *c->pctl_host;
-    if (h.gs.err) {
-        CU(cudaMemsetAsync(c->parrive, 0, (g->fwd.n_heavy + 1) * 4, s));
-        axbc_set_error("plain pivot: a grid barrier wait ran out of its budget (site %d)", h.gs.err);
-        return AXBC_ERR_TIMEOUT;
-    }
+    CU(cudaMemcpyAsync(&c->pc_host->pad, c->g->reach + v0, 4, cudaMemcpyDeviceToHost, c->stream));
+    TRY(pivot_wait(c, c->piv));
+    const PivotCtl &h = *c->piv.ctl_host;
     if (st) {
         st->nvisited = h.qtail;
         st->all = (H == 1 ? (uint32_t)h.rsum : 0u) + c->pc_host->pad;
@@ -977,7 +1138,7 @@ extern "C" int axbc_run_pivot(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pi
     CHECK_ARG(H == 0 || H == 1, "axbc_run_pivot: H must be 0 or 1");
     // one launch, unless every kernel is to be timed
     if (!c->prof_on) {
-        TRY(ensure_pivot(c));
+        TRY(ensure_pivot(c, c->piv, false));
         if (c->pivot_fit > 0) return run_pivot_once(c, v0, p, H, st);
     }
     TRY(axbc_single_reset(c));
