@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
               "-Xcompiler", "-Wno-unused-function", "-I", os.path.join(ROOT, "include")]
 LIB_SOURCES = ["api.cu", "graph.cu", "single.cu", "batch.cu", "sampler.cu", "serve.cu", "compat.cu",
-               "tune.cu", "lcc.cu", "noalloc.cu", "kron.cu", "host_graph.cpp"]
+               "tune.cu", "lcc.cu", "mesh.cu", "noalloc.cu", "kron.cu", "host_graph.cpp"]
 # the Graph500 generator's binomial draws round every product and sum apart,
 # as the host code they restate does
 FILE_FLAGS = {"kron.cu": ["-fmad=false"]}

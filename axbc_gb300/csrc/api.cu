@@ -222,6 +222,9 @@ extern "C" int axbc_ctx_destroy(axbc_ctx *c)
     if (c->pc_host) cudaFreeHost(c->pc_host);
     axbc_pivot_free(c->piv);
     axbc_pivot_free(c->one);
+    axbc_dfree(c->mesh_lvl);
+    axbc_dfree(c->mesh_queue);
+    axbc_dfree(c->mesh_lev);
     axbc_dfree(c->seen);
     for (uint32_t *p : c->fmask) axbc_dfree(p);
     axbc_dfree(c->msigma);

@@ -2580,8 +2580,8 @@ static int read_back(axbc_ctx *c, int nsrc, int L)
 }
 
 // A pass of one pivot runs in the plain form's one launch: rows of 32 pivots
-// would carry one.  (us a pass, persistent rows : this: scale 14 218 : 115, 18 498 :
-// 318, a 512^2 grid 5150 : 3300.)  Counting runs and a level loop that the caller
+// would carry one (us a pass, persistent rows : this: scale 14 218 : 115, 18 498 :
+// 318).  Counting runs and a level loop that the caller
 // has chosen keep the batched kernels.
 static int traverse_one(axbc_ctx *c, int H)
 {
@@ -2593,8 +2593,20 @@ static int traverse_one(axbc_ctx *c, int H)
         axbc_set_error("traversal deeper than %d levels", AXBC_MAX_LEVELS - 2);
         return AXBC_ERR_RANGE;
     }
-    c->last_one = true;
+    c->last_form = axbc_ctx::ONE;
     return read_back(c, 1, L);
+}
+
+// A pass on a mesh: a cluster of blocks per pivot (mesh.cu).
+static int traverse_mesh(axbc_ctx *c, int nsrc, int H, bool *done)
+{
+    TRY(ensure_level_tables(c));
+    TRY(axbc_batch_settle(c));
+    int L = 0;
+    TRY(axbc_mesh_traverse(c, nsrc, H, &L, done));
+    if (!*done) return AXBC_OK;
+    c->last_form = axbc_ctx::MESH;
+    return read_back(c, nsrc, L);
 }
 
 // A multi-source pass of nsrc <= 64 pivots: 32-bit masks up to 32 pivots,
@@ -2605,13 +2617,17 @@ int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H)
         axbc_set_error("batched pass of %d pivots (1..%d)", nsrc, AXBC_WMAX);
         return AXBC_ERR_INVALID;
     }
-    if (nsrc == 1 && c->persist_mode == 0 && !c->count_on) {
+    if (c->persist_mode == 0 && !c->count_on) {
+        if (axbc_mesh_fits(c)) {
+            bool done = false;
+            TRY(traverse_mesh(c, nsrc, H, &done));
+            if (done) return AXBC_OK;
+        }
         int rc = AXBC_OK;
-        const bool fits = axbc_one_fits(c, &rc);
+        if (nsrc == 1 && axbc_one_fits(c, &rc)) return traverse_one(c, H);
         TRY(rc);
-        if (fits) return traverse_one(c, H);
     }
-    c->last_one = false;
+    c->last_form = axbc_ctx::ROWS;
     return width_k(nsrc) == 2 ? batch_traverse<2>(c, nsrc, H) : batch_traverse<1>(c, nsrc, H);
 }
 
@@ -2662,7 +2678,12 @@ static int apply_lanes(axbc_ctx *c, float *const *delta_out, const int *lane_lo,
 int axbc_batch_apply_lanes(axbc_ctx *c, float *const *delta_out, const int *lane_lo,
                            const int *lane_hi, int nseg)
 {
-    if (c->last_one) {
+    if (c->last_form == axbc_ctx::MESH) {
+        TRY(axbc_mesh_apply(c, delta_out, lane_lo, lane_hi, nseg));
+        c->delta_last_valid = true;
+        return AXBC_OK;
+    }
+    if (c->last_form == axbc_ctx::ONE) {
         // the segment that holds lane 0
         float *out = nullptr;
         for (int i = 0; i < nseg; i++)
@@ -2687,11 +2708,24 @@ extern "C" int axbc_ctx_level_stats(axbc_ctx *c, uint64_t *count, uint64_t *te, 
     const int L = std::min(c->last_batch_levels + 1, max_levels);
     *levels = c->last_batch_levels + 1;
     if (!c->d_level_cnt || L <= 0) return AXBC_OK;
+    if (c->last_form == axbc_ctx::MESH) TRY(axbc_mesh_level_tables(c, L));
     CU(cudaStreamSynchronize(c->stream));
+    if (c->last_form == axbc_ctx::MESH) {
+        // every level pushed, every pivot with a list of its own
+        std::vector<unsigned long long> n_l(L);
+        CU(cudaMemcpy(n_l.data(), c->d_level_cnt, L * 8, cudaMemcpyDeviceToHost));
+        for (int i = 0; i < L; i++) {
+            if (push) push[i] = 1;
+            if (list_count) list_count[i] = (uint32_t)n_l[i];
+            if (list_cap) list_cap[i] = std::max(list_max_of(c), (uint32_t)n_l[i]);
+        }
+        push = nullptr;
+        list_count = list_cap = nullptr;
+    }
     if (count) CU(cudaMemcpy(count, c->d_level_cnt, L * 8, cudaMemcpyDeviceToHost));
     if (te) CU(cudaMemcpy(te, c->d_level_te, L * 8, cudaMemcpyDeviceToHost));
     if (push) CU(cudaMemcpy(push, c->d_level_mode, L * 4, cudaMemcpyDeviceToHost));
-    if (c->last_one) {
+    if (c->last_form == axbc_ctx::ONE) {
         // its queue lists every level
         std::vector<uint32_t> lev(L + 1);
         CU(cudaMemcpy(lev.data(), c->one.lev, (L + 1) * 4, cudaMemcpyDeviceToHost));
@@ -2764,7 +2798,8 @@ extern "C" int axbc_get_batch_source(axbc_ctx *c, int src, uint32_t *sigma_host,
     CHECK_ARG(src >= 0 && src < c->last_batch_nsrc, "axbc_get_batch_source: bad source index");
     const uint64_t n = c->g->n;
     cudaStream_t s = c->stream;
-    if (c->last_one) {
+    if (c->last_form == axbc_ctx::MESH) return axbc_mesh_source(c, src, sigma_host, lvl_host, delta_host);
+    if (c->last_form == axbc_ctx::ONE) {
         if (sigma_host) CU(cudaMemcpyAsync(sigma_host, c->one.sigma, n * 4, cudaMemcpyDeviceToHost, s));
         if (lvl_host) CU(cudaMemcpyAsync(lvl_host, c->one.lvl, n * 4, cudaMemcpyDeviceToHost, s));
         if (delta_host) CU(cudaMemcpyAsync(delta_host, c->one.delta, n * 4, cudaMemcpyDeviceToHost, s));

@@ -282,7 +282,14 @@ struct axbc_ctx {
     // the one-launch form of a pivot: run_pivot's buffers (path counts, levels,
     // dependencies and queue are those above) and a one-pivot pass's own
     PivotBuf piv, one;
-    bool last_one = false;  // the last batch was such a pass: its results are in `one`
+    // where the last batch left its results: the batched rows, `one`, or the
+    // pivot-major vectors of a mesh pass
+    enum { ROWS, ONE, MESH } last_form = ROWS;
+    // mesh passes (mesh.cu): per pivot n levels, a queue and its level starts
+    int32_t *mesh_lvl = nullptr;
+    uint32_t *mesh_queue = nullptr, *mesh_lev = nullptr;
+    int mesh_cap = 0;       // pivots they hold
+    bool mesh_off = false;  // a level of this graph was too wide for them
     int pivot_fit = 0;      // blocks of the kernel that fit an SM
     std::vector<uint64_t> levstart;
     uint64_t s_front_deg = 0, s_prev_newdeg = 0, s_visited_rdeg = 0;  // direction choice
@@ -410,6 +417,12 @@ bool axbc_one_fits(axbc_ctx *c, int *rc);
 int axbc_one_traverse(axbc_ctx *c, int H, int *levels);
 int axbc_one_apply(axbc_ctx *c, float *delta_out);
 void axbc_pivot_free(PivotBuf &b);
+// the same for up to 64 pivots on a mesh, into the context's mesh vectors
+bool axbc_mesh_fits(const axbc_ctx *c);
+int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done);
+int axbc_mesh_apply(axbc_ctx *c, float *const *delta_out, const int *lane_lo, const int *lane_hi, int nseg);
+int axbc_mesh_source(axbc_ctx *c, int src, uint32_t *sigma_host, int32_t *lvl_host, float *delta_host);
+int axbc_mesh_level_tables(axbc_ctx *c, int L);
 int axbc_ensure_batch(axbc_ctx *c);
 int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H);
 int axbc_batch_settle(axbc_ctx *c);

@@ -569,7 +569,7 @@ __global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__r
                                const uint32_t *__restrict__ reach, const uint32_t *__restrict__ checks,
                                float *b, uint32_t *hist_v, double *hist_p, uint64_t hist_cap,
                                int off, int lane0, int cnt, int K, const uint32_t *__restrict__ to_view,
-                               const float *__restrict__ one_delta)
+                               const float *__restrict__ vec_delta, const int32_t *__restrict__ vec_lvl)
 {
     if (ss->done && ss->nb == 0) return;
     const int nb = max(0, min(min(ss->nb - off, AXBC_WMAX - lane0), cnt));
@@ -611,9 +611,10 @@ __global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__r
                 continue;
             }
             float dv;
-            if (one_delta) {
-                // a pass of one pivot, in vertex ids
-                dv = one_delta[v];
+            if (vec_delta) {
+                // a pass with whole vectors per pivot, in vertex ids
+                const uint64_t at = (uint64_t)l * N + v;
+                dv = !vec_lvl || vec_lvl[at] >= 0 ? vec_delta[at] : __uint2float_rn(reach[v]);
             } else {
                 // the pass's layout: K mask words and 32 K row values per vertex
                 const bool reached = (seen[(uint64_t)v * K + l / 32] >> (l % 32)) & 1u;
@@ -905,11 +906,14 @@ int sr_post(axbc_ctx *c, SampledRun *r, int off, int lane0, int cnt)
 {
     {
         ProfScope ps(c, KP_SAMPLER, 0);
+        const bool rows = c->last_form == axbc_ctx::ROWS;
         k_sampler_post<<<1, 1, 0, c->stream>>>(r->ss, c->bi, r->bc, c->mdelta, c->seen,
-                                               c->last_one ? c->g->reach : c->g->breach, r->checks, r->checkval,
-                                               r->hist_v, r->hist_p, r->hist_cap, off, lane0, cnt, c->last_batch_k,
-                                               c->last_one ? nullptr : c->g->to_view,
-                                               c->last_one ? c->one.delta : nullptr);
+                                               rows ? c->g->breach : c->g->reach, r->checks, r->checkval, r->hist_v,
+                                               r->hist_p, r->hist_cap, off, lane0, cnt, c->last_batch_k,
+                                               rows ? c->g->to_view : nullptr,
+                                               rows ? nullptr
+                                                    : c->last_form == axbc_ctx::ONE ? c->one.delta : c->mdelta,
+                                               c->last_form == axbc_ctx::MESH ? c->mesh_lvl : nullptr);
     }
     CU_LAUNCH("k_sampler_post");
     return AXBC_OK;

@@ -91,3 +91,64 @@ def test_plain_pivots_at_degree_edges(axbc, orc, undirected, factor):
             assert np.array_equal(ctx.bc(), want) and np.array_equal(ctx.delta(), delta)
             assert np.array_equal(ctx.levels(), lvl) and np.array_equal(ctx.sigma(), sigma)
             assert st == stats
+
+
+def sparse_graph(kind, rng):
+    """Graphs without a vertex of more than 64 neighbours: their passes run a
+    cluster of blocks per pivot, unless a level is too wide."""
+    if kind.startswith("grid"):
+        side = int(kind[4:])
+        i = np.arange(side * side).reshape(side, side)
+        e = [np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()], 1), np.stack([i[:-1].ravel(), i[1:].ravel()], 1)]
+        return np.concatenate(e), side * side
+    if kind == "path":
+        return np.stack([np.arange(699), np.arange(1, 700)], 1), 700
+    if kind == "ladders":  # every degree up to 64, three components
+        e = [np.stack([np.full(d, 3 * d), 300 + rng.choice(900, d, replace=False)], 1) for d in range(1, 40)]
+        chain = np.arange(300, 1199)
+        return np.concatenate(e + [np.stack([chain, chain + 1], 1), [[1250, 1251]]]), 1300
+    n = 6000  # "wide": levels of thousands of vertices
+    return rng.integers(0, n, size=(4 * n, 2)), n
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+@pytest.mark.parametrize("k", [1, 2, 33, 64])
+@pytest.mark.parametrize("kind", ["grid40", "path", "ladders", "wide"])
+def test_mesh_passes(axbc, orc, kind, k, undirected):
+    rng = np.random.default_rng(17)
+    e, n = sparse_graph(kind, rng)
+    g = orc.pipeline(e.astype(np.uint64), n, undirected, 0)
+    assert g.deg.max() <= 64
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, rng.integers(0, 3, n).astype(np.uint32)))
+    g = orc.CSC(g.col, g.row, ctx.graph.csc()[2])
+    piv = rng.choice(n, k, replace=False).astype(np.uint32)
+    p = rng.random(k) + 0.1
+    for _ in range(2):
+        ctx.reset()
+        stats = ctx.run_batch(piv, p, 1)
+    want, delta_last, _ = orc.bc_pivots(g, piv, p, 1)
+    assert np.array_equal(ctx.bc(), want, equal_nan=True) and np.array_equal(ctx.delta(), delta_last, equal_nan=True)
+    levels = ctx.level_stats()
+    total = 0
+    for s in range(k):
+        _, lvl, sigma, delta, st = orc.bc_pivot(g, int(piv[s]), p[s], 1)
+        assert stats[s] == st
+        total += st["nvisited"]
+        if s in (0, k - 1):
+            gs, gl, gd = ctx.batch_source(s)
+            assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl)
+            assert np.array_equal(gd, delta, equal_nan=True)
+    assert int(levels["count"].sum()) == total
+
+
+def test_mesh_pass_on_several_blocks(axbc, orc):
+    e, n = sparse_graph("grid300", None)  # wide enough for clusters of two and more
+    g = orc.pipeline(e.astype(np.uint64), n, True, 0)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row))
+    for k in (1, 3):
+        piv = np.array([12, 44850, 89999][:k], np.uint32)
+        p = np.full(k, 0.5)
+        ctx.reset()
+        ctx.run_batch(piv, p)
+        want, delta_last, _ = orc.bc_pivots(g, piv, p)
+        assert np.array_equal(ctx.bc(), want, equal_nan=True) and np.array_equal(ctx.delta(), delta_last, equal_nan=True)
