@@ -349,6 +349,28 @@ __device__ void d_map_one(int64_t r, int k, uint64_t N, const SamplerDists &D, b
     }
 }
 
+// High-degree neighbourhood (src/axbc2d.c:2890-2917); returns the lrand48 values
+// taken, one or two.
+__device__ __forceinline__ int d_degree_draw(uint64_t &x, uint64_t N, const SamplerDists &D, uint32_t &v0, double &prob)
+{
+    int found, took = 1;
+    const uint32_t r = d_uniform_int(x, D.sum_deg, 0);
+    uint64_t h = d_find_u32(D.deg2p, D.seg_end, D.n_seg, r, &found);
+    if (!found) h = N - 1;
+    const uint32_t dh = D.col[h + 1] - D.col[h];
+    if (dh > 0) {
+        uint32_t kk = 0;
+        if (dh != 1) {
+            kk = d_uniform_int(x, dh - 1, 0);
+            took = 2;
+        }
+        h = D.row[D.col[h] + kk];
+    }
+    v0 = (uint32_t)h;
+    prob = __ddiv_rn((double)D.sdn[v0], (double)D.sum_deg);
+    return took;
+}
+
 // One draw of heuristic z (dist_mix: the -z 6 mixture state, equal to z for
 // the others): v0 and its probability, the reference's rules of
 // src/axbc2d.c:2873-3051.  snap0: no pivot applied yet (the dynamic heuristics
@@ -361,19 +383,7 @@ __device__ void d_draw_one(uint64_t &x, uint32_t &dist_mix, int z, uint64_t N, c
     const int k = z == 6 ? (int)dist_mix : z;  // the distribution this draw uses
     prob = 0;
     if (k == 1) {
-        // high-degree neighbourhood (src/axbc2d.c:2890-2917): one or two values
-        int found;
-        const uint32_t r = d_uniform_int(x, D.sum_deg, 0);
-        uint64_t h = d_find_u32(D.deg2p, D.seg_end, D.n_seg, r, &found);
-        if (!found) h = N - 1;
-        const uint32_t dh = D.col[h + 1] - D.col[h];
-        if (dh > 0) {
-            uint32_t kk = 0;
-            if (dh != 1) kk = d_uniform_int(x, dh - 1, 0);
-            h = D.row[D.col[h] + kk];
-        }
-        v0 = (uint32_t)h;
-        prob = __ddiv_rn((double)D.sdn[v0], (double)D.sum_deg);
+        (void)d_degree_draw(x, N, D, v0, prob);
     } else {
         d_map_one<COOP>(d_lrand48(x), k, N, D, snap0, S_bc, S_d, S_lcc, v0, prob);
     }
@@ -396,30 +406,45 @@ __device__ void d_draw_one(uint64_t &x, uint32_t &dist_mix, int z, uint64_t N, c
     }
 }
 
-// Draw the rounds of one batch: up to W accepted pivots.  Every thread of the
-// block runs the same sequential loop on the same values (stores by thread 0);
-// for the heuristics that take one lrand48 value per draw, a streak of
-// rejected draws (pivot already used) is searched SAMPLER_TPB draws at a time:
-// thread t evaluates the draw t steps ahead (drand48 skip-ahead: x -> A_t x +
-// C_t mod 2^48) and the first acceptable one wins, with the state and the
-// rejection count advanced exactly as the sequential loop would.
-// rejections in a row before the block searches draws in parallel
-#ifndef AXBC_SAMPLER_STREAK
-#define AXBC_SAMPLER_STREAK 4
-#endif
-
-// The used-pivot flags are set by thread 0 between two barriers: after every
-// thread has tested the round's draws against them, before any thread tests
-// the next round's.
+// Draw the rounds of one batch: up to W accepted pivots, in the reference's
+// sequential order.  Every thread evaluates the draw that starts t lrand48 values
+// ahead (drand48 skip-ahead: x -> A_t x + C_t mod 2^48) against the distributions
+// and the used-pivot flags.  -z 1 takes one or two values a draw, which depends on
+// the values alone: one thread walks which starts are taken.  Then a draw of a
+// vertex drawn before, in this window or an earlier one, is rejected, one thread
+// settles rounds, skips and drops in order, and all write what it kept.  The loop
+// one draw at a time, all threads searching together, took 5 us a draw: 40 us a
+// round of 8, 280 us one of 64 with -z 1.  -z 6, whose next distribution is itself
+// drawn, keeps that loop.
 __device__ __forceinline__ bool is_used(const uint8_t *used, uint32_t v) { return used[v] != 0; }
 __device__ __forceinline__ void set_used(uint8_t *used, uint32_t v) { used[v] = 1; }
+// k steps of drand48 as one affine step
+__device__ __forceinline__ void skip_ahead(uint32_t k, uint64_t &A, uint64_t &C)
+{
+    const uint64_t M = 0xFFFFFFFFFFFFULL;
+    uint64_t a = 0x5DEECE66DULL, c = 0xBULL;
+    A = 1;
+    C = 0;
+    for (; k; k >>= 1) {
+        if (k & 1u) {
+            A = (a * A) & M;
+            C = (a * C + c) & M;
+        }
+        c = (a * c + c) & M;
+        a = (a * a) & M;
+    }
+}
+
 __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, SamplerDists D, uint8_t *used,
                                                        const uint32_t *checks, double S_lcc)
 {
-    __shared__ uint64_t s_A[SAMPLER_TPB + 1], s_C[SAMPLER_TPB + 1];
-    __shared__ int s_best;
-    __shared__ uint32_t s_v0;
-    __shared__ double s_prob;
+    __shared__ uint32_t s_v[SAMPLER_TPB];
+    __shared__ double s_pr[SAMPLER_TPB];
+    __shared__ uint8_t s_took[SAMPLER_TPB];
+    __shared__ uint8_t s_kind[SAMPLER_TPB];  // by draw: 0 rejected, 1 degree 0, 2 a pivot
+    __shared__ uint16_t s_pos[SAMPLER_TPB + 1], s_slot[AXBC_MAX_WIDTH];
+    __shared__ uint64_t s_skip[AXBC_MAX_WIDTH];
+    __shared__ int s_end, s_left, s_draws, s_nb;
     const int t = threadIdx.x;
     const bool lead = t == 0;
     const bool done = ss->done != 0;
@@ -451,92 +476,143 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
         if (D.bc_csum) S_bc = D.bc_csum[nbB - 1];
         if (D.d_csum) S_d = D.d_csum[nbB - 1];
     }
-    const bool one_value = z == 0 || z == 2 || z == 3 || z == 4 || z == 5;
-    if (one_value && lead) {
-        const uint64_t M = 0xFFFFFFFFFFFFULL;
-        uint64_t A = 1, C = 0;
-        s_A[0] = 1;
-        s_C[0] = 0;
-        for (int k = 1; k <= SAMPLER_TPB; k++) {
-            A = (A * 0x5DEECE66DULL) & M;
-            C = (C * 0x5DEECE66DULL + 0xBULL) & M;
-            s_A[k] = A;
-            s_C[k] = C;
-        }
-    }
-    __syncthreads();
     int nb = 0;
     uint64_t ui = ss->ui, skipped_run = 0, dropped = 0;
-    while (nb < W && ui < nbfs) {
-        uint32_t v0 = 0;
-        double prob = 0;
-        uint32_t BSM = 0;
-        bool good = false;
-        while (!good) {
-            if (BSM > LIM) break;
-            if (one_value && BSM >= AXBC_SAMPLER_STREAK) {
-                // candidates allowed before the bad-sample limit
-                const uint64_t allow = min((uint64_t)SAMPLER_TPB, (uint64_t)LIM - BSM + 1);
+    if (z != 6) {
+        uint64_t A, C;
+        skip_ahead(t, A, C);
+        uint32_t BSM = 0;  // thread 0: rejections of the round under way
+        // values looked at together: a narrow round rarely needs more than 64
+        int win = W <= 16 ? 64 : SAMPLER_TPB;
+        if (lead) s_left = nb < W && ui < nbfs;
+        __syncthreads();
+        while (s_left) {
+            uint64_t xt = (A * x + C) & 0xFFFFFFFFFFFFULL;
+            if (t < win) {
                 uint32_t v = 0;
                 double pr = 0;
-                bool acc = false;
-                if ((uint64_t)t < allow) {
-                    const uint64_t xt = (s_A[t + 1] * x + s_C[t + 1]) & 0xFFFFFFFFFFFFULL;
-                    d_map_one<false>((int64_t)(xt >> 17), z, N, D, snap0, S_bc, S_d, S_lcc, v, pr);
-                    acc = !(v < N && is_used(used, v));
+                int took = 1;
+                if (z == 1) took = d_degree_draw(xt, N, D, v, pr);
+                else d_map_one<false>(d_lrand48(xt), z, N, D, snap0, S_bc, S_d, S_lcc, v, pr);
+                s_v[t] = v;
+                s_pr[t] = pr;
+                s_took[t] = (uint8_t)took;
+            }
+            __syncthreads();
+            // draw j starts at value s_pos[j]
+            if (z != 1) {
+                if (t < win) s_pos[t] = (uint16_t)t;
+                if (lead) s_pos[win] = (uint16_t)win, s_draws = win;
+            } else if (lead) {
+                int k = 0, pos = 0;
+                for (; pos < win; k++) {
+                    s_pos[k] = (uint16_t)pos;
+                    pos += s_took[pos];
                 }
-                if (lead) s_best = SAMPLER_TPB;
-                __syncthreads();
-                if (acc) atomicMin(&s_best, t);
-                __syncthreads();
-                const int j = s_best;
-                if (j < SAMPLER_TPB) {
-                    if (t == j) {
-                        s_v0 = v;
-                        s_prob = pr;
+                s_pos[k] = (uint16_t)pos;
+                s_draws = k;
+            }
+            __syncthreads();
+            const int draws = s_draws;
+            int kind = 0;
+            uint32_t v = 0xffffffffu;
+            if (t < draws) {
+                v = s_v[s_pos[t]];
+                kind = 1;
+                if (v < N) {
+                    kind = is_used(used, v) ? 0 : D.col[v + 1] != D.col[v] ? 2 : 1;
+                    // drawn earlier in this window (a vertex id of N is never marked)
+                    for (int j = 0; j < t && kind; j++)
+                        if (s_v[s_pos[j]] == v) kind = 0;
+                }
+                s_kind[t] = (uint8_t)kind;
+            }
+            __syncthreads();
+            if (lead) {
+                int k = 0;  // draws consumed
+                const int nb0 = nb;
+                while (k < draws && nb < W && ui < nbfs) {
+                    if (BSM > LIM) {  // round dropped (src/axbc2d.c:3072-3077)
+                        dropped++;
+                        ui++;
+                        BSM = 0;
+                        continue;
                     }
-                    __syncthreads();
-                    v0 = s_v0;
-                    prob = s_prob;
-                    x = (s_A[j + 1] * x + s_C[j + 1]) & 0xFFFFFFFFFFFFULL;
-                    BSM += (uint32_t)j;
-                    good = true;
-                } else {
-                    x = (s_A[allow] * x + s_C[allow]) & 0xFFFFFFFFFFFFULL;
-                    BSM += (uint32_t)allow;
+                    const int kd = s_kind[k];
+                    if (kd == 0) {
+                        BSM++;
+                    } else {
+                        if (kd == 1) {  // degree-0 root (3095-3111)
+                            skipped_run++;
+                        } else {
+                            s_slot[nb] = (uint16_t)k;
+                            s_skip[nb] = skipped_run;
+                            skipped_run = 0;
+                            nb++;
+                        }
+                        ui++;
+                        BSM = 0;
+                    }
+                    k++;
                 }
-                __syncthreads();
+                s_end = k;
+                s_nb = nb0;
+                s_left = nb < W && ui < nbfs;
+                s_draws = nb;
+            }
+            __syncthreads();
+            // what was kept: the flags of the draws consumed, the pivots' slots
+            if (t < s_end && kind && v < N) set_used(used, v);
+            if (t >= s_nb && t < s_draws) {
+                const int at = s_pos[s_slot[t]];
+                ss->v0[t] = s_v[at];
+                ss->p[t] = s_pr[at];
+                ss->skip_before[t] = s_skip[t];
+            }
+            uint64_t Ae, Ce;
+            skip_ahead(s_pos[s_end], Ae, Ce);
+            x = (Ae * x + Ce) & 0xFFFFFFFFFFFFULL;
+            win = SAMPLER_TPB;
+            __syncthreads();
+        }
+    } else {
+        while (nb < W && ui < nbfs) {
+            uint32_t v0 = 0;
+            double prob = 0;
+            uint32_t BSM = 0;
+            bool good = false;
+            while (!good) {
+                if (BSM > LIM) break;
+                d_draw_one<true>(x, dist_mix, z, N, D, snap0, S_bc, S_d, S_lcc, v0, prob);
+                if (v0 < N && is_used(used, v0)) BSM++;
+                else good = true;
+            }
+            if (!good) {  // round dropped
+                dropped++;
+                ui++;
                 continue;
             }
-            d_draw_one<true>(x, dist_mix, z, N, D, snap0, S_bc, S_d, S_lcc, v0, prob);
-            if (v0 < N && is_used(used, v0)) BSM++;
-            else good = true;
-        }
-        if (!good) {  // round dropped (src/axbc2d.c:3072-3077)
-            dropped++;
-            ui++;
-            continue;
-        }
-        // every thread has tested this round's draws against the flags
-        // before thread 0 sets the new one
-        __syncthreads();
-        if (v0 >= N || D.col[v0 + 1] == D.col[v0]) {  // degree-0 root (3095-3111)
-            skipped_run++;
-            if (v0 < N && lead) set_used(used, v0);
+            // every thread has tested this round's draws against the flags
+            // before thread 0 sets the new one
             __syncthreads();
+            if (v0 >= N || D.col[v0 + 1] == D.col[v0]) {  // degree-0 root
+                skipped_run++;
+                if (v0 < N && lead) set_used(used, v0);
+                __syncthreads();
+                ui++;
+                continue;
+            }
+            if (lead) {
+                set_used(used, v0);
+                ss->v0[nb] = v0;
+                ss->p[nb] = prob;
+                ss->skip_before[nb] = skipped_run;
+            }
+            __syncthreads();
+            skipped_run = 0;
+            nb++;
             ui++;
-            continue;
         }
-        if (lead) {
-            set_used(used, v0);
-            ss->v0[nb] = v0;
-            ss->p[nb] = prob;
-            ss->skip_before[nb] = skipped_run;
-        }
-        __syncthreads();
-        skipped_run = 0;
-        nb++;
-        ui++;
     }
     if (lead) {
         ss->rng = x;
@@ -563,95 +639,132 @@ __global__ void k_load_pass(const SamplerState *ss, BatchInfo *bi, int off, int 
 // After a pass (the drawn pivots [off, off + cnt)): replay Bader's test
 // between its pivots, fix how many are applied, and account rounds, skips and
 // traversed edges.  The pass that ends the round also settles the degree-0
-// draws after its last pivot.
-__global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__restrict__ bc,
-                               const float *__restrict__ mdelta, const uint32_t *__restrict__ seen,
-                               const uint32_t *__restrict__ reach, const uint32_t *__restrict__ checks,
-                               float *b, uint32_t *hist_v, double *hist_p, uint64_t hist_cap,
-                               int off, int lane0, int cnt, int K, const uint32_t *__restrict__ to_view,
-                               const float *__restrict__ vec_delta, const int32_t *__restrict__ vec_lvl)
+// draws after its last pivot.  One block: the terms of a (pivot, check vertex)
+// pair load side by side, up to POST_X check vertices into shared memory, and one
+// thread per check vertex then adds its terms in pivot order.  (One thread doing
+// all of it took 29 us a request and pass.)
+#define POST_TPB 256
+#define POST_X 32
+__global__ void __launch_bounds__(POST_TPB) k_sampler_post(
+    SamplerState *ss, BatchInfo *bi, const float *__restrict__ bc, const float *__restrict__ mdelta,
+    const uint32_t *__restrict__ seen, const uint32_t *__restrict__ reach, const uint32_t *__restrict__ checks, float *b,
+    uint32_t *hist_v, double *hist_p, uint64_t hist_cap, int off, int lane0, int cnt, int K,
+    const uint32_t *__restrict__ to_view, const float *__restrict__ vec_delta, const int32_t *__restrict__ vec_lvl)
 {
+    __shared__ float s_term[AXBC_WMAX][POST_X];
+    __shared__ uint8_t s_add[AXBC_WMAX][POST_X];
+    __shared__ unsigned long long s_te;
+    __shared__ unsigned long long s_skip;
     if (ss->done && ss->nb == 0) return;
+    const int t = threadIdx.x;
     const int nb = max(0, min(min(ss->nb - off, AXBC_WMAX - lane0), cnt));
     const bool last = off + nb >= ss->nb;
     const uint64_t N = ss->N;
     const uint32_t c = ss->bader_c;
     const double lim = (double)((uint64_t)c * N);
-    int stop = nb;
-    // check-vertex values through the batch, in the order the update applies
     const uint32_t x = ss->nchecks;
     const bool track = c > 0;
-    if (track)
-        for (uint32_t i = 0; i < x; i++) b[i] = checks[i] < N ? bc[checks[i]] : 0.0f;
-    for (int s = 0; s < nb; s++) {
-        if (c > 0 && off + s > 0) {
-            bool sat = true;
-            for (uint32_t i = 0; i < x && sat; i++) {
-                const float bv = track ? b[i] : 0.0f;
-                if (__ddiv_rn((double)bv, 2.0) < lim) sat = false;
-            }
-            if (sat) {
-                stop = s;
-                break;
-            }
-        }
-        if (!track) continue;
+    const uint64_t rounds0 = ss->nrounds;
+    int stop = nb;
+    bool sat_end = false;  // the test after the last pivot
+    if (t == 0) s_te = s_skip = 0;
+    // the increment of check vertex i by pivot s (false: none)
+    auto term = [&](int s, uint32_t i, float &f) -> bool {
+        const uint32_t chk = checks[i];
+        if (chk >= N) return false;
         const int l = lane0 + s;
         const uint32_t r = bi->root[l];
         const uint32_t rr = reach[r];
-        const uint32_t all = (bi->H == 1 ? (uint32_t)bi->rsum[l] : 0u) + rr;
-        const unsigned long long nvt = bi->nvis[l] + all;
+        // the pass runs in the graph's view (roots, masks, rows, reach)
+        const uint32_t v = to_view ? to_view[chk] : chk;
+        if (v == r) {
+            const uint32_t all = (bi->H == 1 ? (uint32_t)bi->rsum[l] : 0u) + rr;
+            f = bc_root_term(rr, bi->nvis[l] + all);
+            return rr > 0;
+        }
         const double p = bi->p[l];
-        for (uint32_t i = 0; i < x; i++) {
-            if (checks[i] >= N) continue;
-            // the pass runs in the graph's view (roots, masks, rows, reach)
-            const uint32_t v = to_view ? to_view[checks[i]] : checks[i];
-            if (v == r) {
-                if (rr > 0) b[i] = __fadd_rn(b[i], bc_root_term(rr, nvt));
-                continue;
+        float dv;
+        if (vec_delta) {
+            // a pass with whole vectors per pivot, in vertex ids
+            const uint64_t at = (uint64_t)l * N + v;
+            dv = !vec_lvl || vec_lvl[at] >= 0 ? vec_delta[at] : __uint2float_rn(reach[v]);
+        } else {
+            // the pass's layout: K mask words and 32 K row values per vertex
+            const bool reached = (seen[(uint64_t)v * K + l / 32] >> (l % 32)) & 1u;
+            dv = reached ? mdelta[(uint64_t)v * (AXBC_W * K) + l] : __uint2float_rn(reach[v]);
+        }
+        if (dv == 0.0f && p > 0.0) return false;
+        f = bc_term(dv, rr, p);
+        return true;
+    };
+    auto below = [&](float bv) { return __ddiv_rn((double)bv, 2.0) < lim; };
+    if (track && x <= POST_X) {
+        for (uint32_t k = t; k < nb * x; k += POST_TPB) {
+            const int s = k / x;
+            const uint32_t i = k % x;
+            float f = 0.0f;
+            s_add[s][i] = term(s, i, f);
+            s_term[s][i] = f;
+        }
+        __syncthreads();
+        // one warp, a lane per check vertex; every warp does the same
+        const unsigned lane = lane_id();
+        const bool mine = lane < x;
+        float bv = mine && checks[lane] < N ? bc[checks[lane]] : 0.0f;
+        for (int s = 0; s < nb; s++) {
+            if (off + s > 0 && !__any_sync(FULL_MASK, mine && below(bv))) {
+                stop = s;
+                break;
             }
-            float dv;
-            if (vec_delta) {
-                // a pass with whole vectors per pivot, in vertex ids
-                const uint64_t at = (uint64_t)l * N + v;
-                dv = !vec_lvl || vec_lvl[at] >= 0 ? vec_delta[at] : __uint2float_rn(reach[v]);
-            } else {
-                // the pass's layout: K mask words and 32 K row values per vertex
-                const bool reached = (seen[(uint64_t)v * K + l / 32] >> (l % 32)) & 1u;
-                dv = reached ? mdelta[(uint64_t)v * (AXBC_W * K) + l] : __uint2float_rn(reach[v]);
+            if (mine && s_add[s][lane]) bv = __fadd_rn(bv, s_term[s][lane]);
+        }
+        sat_end = !__any_sync(FULL_MASK, mine && below(bv));
+    } else if (track) {
+        for (uint32_t i = t; i < x; i += POST_TPB) b[i] = checks[i] < N ? bc[checks[i]] : 0.0f;
+        for (int s = 0; s <= nb; s++) {
+            bool ok = true;
+            for (uint32_t i = t; i < x; i += POST_TPB) ok = ok && !below(b[i]);
+            const bool sat = __syncthreads_and(ok);
+            if (s == nb) {
+                sat_end = sat;
+                break;
             }
-            if (dv == 0.0f && p > 0.0) continue;
-            b[i] = __fadd_rn(b[i], bc_term(dv, rr, p));
+            if (off + s > 0 && sat) {
+                stop = s;
+                break;
+            }
+            for (uint32_t i = t; i < x; i += POST_TPB) {
+                float f = 0.0f;
+                if (term(s, i, f)) b[i] = __fadd_rn(b[i], f);
+            }
         }
     }
+    __syncthreads();
+    // history and totals of the applied pivots
+    for (int s = t; s < stop; s += POST_TPB) {
+        if (rounds0 + s < hist_cap) {
+            hist_v[rounds0 + s] = ss->v0[off + s];
+            hist_p[rounds0 + s] = ss->p[off + s];
+        }
+        atomicAdd(&s_te, 2 * bi->te[lane0 + s]);
+        atomicAdd(&s_skip, (unsigned long long)ss->skip_before[off + s]);
+    }
+    __syncthreads();
+    if (t) return;
     // lanes [lane0, lane0 + nb) of the pass: the first `stop` are applied
     const unsigned long long seg = (nb >= 64 ? ~0ull : ((1ull << nb) - 1ull)) << lane0;
     const unsigned long long app = (stop >= 64 ? ~0ull : ((1ull << stop) - 1ull)) << lane0;
     bi->applymask = (bi->applymask & ~seg) | app;
     ss->napply = stop;
-    for (int s = 0; s < stop; s++) {
-        if (ss->nrounds < hist_cap) {
-            hist_v[ss->nrounds] = ss->v0[off + s];
-            hist_p[ss->nrounds] = ss->p[off + s];
-        }
-        ss->nrounds++;
-        ss->skipped += ss->skip_before[off + s];
-        ss->te += 2 * bi->te[lane0 + s];
-    }
+    ss->nrounds = rounds0 + stop;
+    ss->skipped += s_skip;
+    ss->te += s_te;
     if (stop < nb) {
         ss->stopped = 1;
         ss->done = 1;
     } else if (last) {
         if (ss->skipped_run) {
-            bool sat = false;
-            if (c > 0 && nb > 0) {
-                sat = true;
-                for (uint32_t i = 0; i < x && sat; i++) {
-                    const float bv = track ? b[i] : 0.0f;
-                    if (__ddiv_rn((double)bv, 2.0) < lim) sat = false;
-                }
-            }
-            if (sat) {
+            if (c > 0 && nb > 0 && sat_end) {
                 ss->stopped = 1;
                 ss->done = 1;
             } else {
@@ -660,7 +773,7 @@ __global__ void k_sampler_post(SamplerState *ss, BatchInfo *bi, const float *__r
         }
         if (ss->ui >= ss->nbfs) ss->done = 1;
     }
-    ss->nrounds_snap = ss->nrounds;
+    ss->nrounds_snap = rounds0 + stop;
 }
 
 // ------------------------------------------------------------ sampled runs
@@ -907,7 +1020,7 @@ int sr_post(axbc_ctx *c, SampledRun *r, int off, int lane0, int cnt)
     {
         ProfScope ps(c, KP_SAMPLER, 0);
         const bool rows = c->last_form == axbc_ctx::ROWS;
-        k_sampler_post<<<1, 1, 0, c->stream>>>(r->ss, c->bi, r->bc, c->mdelta, c->seen,
+        k_sampler_post<<<1, POST_TPB, 0, c->stream>>>(r->ss, c->bi, r->bc, c->mdelta, c->seen,
                                                rows ? c->g->breach : c->g->reach, r->checks, r->checkval, r->hist_v,
                                                r->hist_p, r->hist_cap, off, lane0, cnt, c->last_batch_k,
                                                rows ? c->g->to_view : nullptr,

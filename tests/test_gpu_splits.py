@@ -152,3 +152,23 @@ def test_mesh_pass_on_several_blocks(axbc, orc):
         ctx.run_batch(piv, p)
         want, delta_last, _ = orc.bc_pivots(g, piv, p)
         assert np.array_equal(ctx.bc(), want, equal_nan=True) and np.array_equal(ctx.delta(), delta_last, equal_nan=True)
+
+
+@pytest.mark.parametrize("nchecks", [0, 1, 31, 32, 33, 70])
+@pytest.mark.parametrize("z", [0, 1, 3, 5])
+def test_sampler_windows_and_many_check_vertices(axbc, orc, z, nchecks):
+    # rounds around the 64- and 256-value windows with many repeated draws, and
+    # more check vertices than the replay keeps in shared memory
+    rng = np.random.default_rng(5)
+    e = rng.integers(0, 300, size=(2400, 2))
+    g = orc.pipeline(e.astype(np.uint64), 320, True, 0)
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    for W, c in ((1, 1), (16, 0), (17, 2), (64, 1)):
+        ctx = axbc.Context(G)
+        got = ctx.run_sampled(z=z, nbfs=300, bader_c=c, nchecks=nchecks, seed=77 + W, W=W)
+        want = orc.run(g, z=z, nbfs=300, bader_c=c, nchecks=nchecks, seed=77 + W, W=W)
+        assert np.array_equal(got["checks"], want["checks"]) and np.array_equal(got["pivots"], want["pivots"])
+        assert np.array_equal(got["probs"], want["probs"], equal_nan=True)
+        for k in ("nrounds", "skipped", "dropped", "ui_end", "te", "stopped"):
+            assert got[k] == want[k], (W, c, k)
+        assert np.array_equal(ctx.bc(), want["bc"], equal_nan=True)
