@@ -48,6 +48,8 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
 
 // resident blocks per SM the kernels are compiled for (their register
 // budgets); the backward runs 32 pivots at a time at either width
+// the persistent loop, 80 registers at both widths (64 and 48: 2-20% slower)
+#define PERSIST_BLOCKS 3
 #ifndef AXBC_FWD_MIN_BLOCKS
 #define AXBC_FWD_MIN_BLOCKS 7
 #endif
@@ -315,6 +317,17 @@ __device__ __forceinline__ const uint32_t *level_list(const LevelLists &ll, int 
     return ll.pool + ll.start[L];
 }
 
+// Path counts are added either an edge at a time, lane = pivot (one line per
+// edge), or a pivot of every edge at a time, lane = edge.  The second takes as
+// many steps as the fullest edge has pivots: the frontiers that are pushed are
+// small and most of their vertices belong to one pivot or two, and 32 steps of
+// one lane each were 40 us of a pushed level.  act: lanes with any.
+template <class M> __device__ __forceinline__ bool bits_apart(M nm, unsigned act)
+{
+    const unsigned most = __reduce_max_sync(FULL_MASK, (unsigned)__popcll((unsigned long long)nm));
+    return 4 * most <= (unsigned)__popc(act);
+}
+
 // Forward level L, push from the vertices of depth L-1: for each neighbour u
 // and each pivot s with v at depth L-1 and u unseen, sigma_s[u] += sigma_s[v]
 // and bit s joins u's level-L mask.  Atomics are fire-and-forget reductions.
@@ -346,6 +359,23 @@ __device__ __forceinline__ void push_span(const Adj &a, uint32_t v, typename Mas
         if (nm) wc.add(WC_BYTES, old == 0 ? 4 + 4 * K : 4 * K);  // level mask, list entry
         list_append(ll, L, old == 0, u);
         unsigned act = __ballot_sync(FULL_MASK, nm != 0);
+        if (bits_apart(nm, act)) {
+            while (__any_sync(FULL_MASK, nm != 0)) {
+                const int b = nm ? __ffsll((long long)nm) - 1 : 0;
+                uint32_t x = __shfl_sync(FULL_MASK, sig[0], b & 31);
+                if (K == 2) {
+                    const uint32_t hi = __shfl_sync(FULL_MASK, sig[K - 1], b & 31);
+                    if (b >= 32) x = hi;
+                }
+                if (nm) {
+                    atomicAdd(&msigma[row_base<K>(u) + b], x);
+                    wc.add(WC_PAIRS, 1);
+                    wc.add(WC_BYTES, 4);
+                }
+                nm &= nm - 1;
+            }
+            continue;
+        }
         while (act) {
             const int j = __ffs(act) - 1;
             act &= act - 1;
@@ -409,6 +439,18 @@ __device__ __forceinline__ void push_light32(const Adj &a, uint32_t v_l, typenam
         if (nm) wc.add(WC_BYTES, old == 0 ? 4 + 4 * K : 4 * K);  // level mask, list entry
         list_append(ll, L, old == 0, u);
         unsigned act = __ballot_sync(FULL_MASK, nm != 0);
+        const uint32_t vk = __shfl_sync(FULL_MASK, v_l, k);
+        if (bits_apart(nm, act)) {
+            for (; nm; nm &= nm - 1) {
+                const int b = __ffsll((long long)nm) - 1;
+                atomicAdd(&msigma[row_base<K>(u) + b], msigma[row_base<K>(vk) + b]);
+                wc.add(WC_GATHERS, 1);
+                wc.add(WC_PAIRS, 1);
+                wc.add(WC_BYTES, 8);  // parent's path count, child's sum
+            }
+            __syncwarp();
+            continue;
+        }
         while (act) {
             // up to 4 edges: gather the parents' sigma rows, then add
             uint32_t uu[4], sg[4][K];
@@ -421,7 +463,7 @@ __device__ __forceinline__ void push_light32(const Adj &a, uint32_t v_l, typenam
                 uu[q] = __shfl_sync(FULL_MASK, u, j);
                 const M mj = __shfl_sync(FULL_MASK, nm, j);
                 mm[q] = ok ? mj : (M)0;
-                const uint32_t vj = __shfl_sync(FULL_MASK, v_l, __shfl_sync(FULL_MASK, k, j));
+                const uint32_t vj = __shfl_sync(FULL_MASK, vk, j);
 #pragma unroll
                 for (int h = 0; h < K; h++)
                     sg[q][h] = pbit(mm[q], h) ? msigma[row_base<K>(vj) + 32 * h + lane] : 0u;
@@ -904,6 +946,11 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
     const unsigned l = lane_id();
     const int L = __ldcg(&bi->cur) + 1;
     const uint32_t nsrc = bi->nsrc;
+    // every total loads before the first is used
+    const unsigned long long front = __ldcg(&bi->front_deg), unvis = __ldcg(&bi->unvis_deg) - __ldcg(&bi->unvis_dec);
+    const unsigned long long lvl_te = __ldcg(&bi->lvl_te);
+    const uint32_t listed = __ldcg(&ll.count[L]), cap = __ldcg(&ll.cap[L]), start = __ldcg(&ll.start[L]);
+    const uint32_t any_new = __ldcg(&bi->any_new);
     unsigned long long cnt = 0, d0 = 0;
 #pragma unroll
     for (int h = 0; h < K; h++) {
@@ -917,9 +964,7 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
     for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(FULL_MASK, cnt, o);
     __syncwarp();
     if (l == 0) {
-        const unsigned long long front = __ldcg(&bi->front_deg), unvis = __ldcg(&bi->unvis_deg) - __ldcg(&bi->unvis_dec);
-        const uint32_t listed = __ldcg(&ll.count[L]), cap = __ldcg(&ll.cap[L]);
-        level_te[L] = __ldcg(&bi->lvl_te);
+        level_te[L] = lvl_te;
         level_cnt[L] = cnt;
         level_mode[L] = bi->push_next;
         bi->unvis_deg = unvis;
@@ -928,11 +973,11 @@ __device__ __forceinline__ void level_advance_warp(BatchInfo *bi, unsigned long 
         // a pull would scan every vertex some pivot has not seen
         const bool push = (double)front * bi->push_factor < (double)unvis || front < bi->push_min;
         // where level L+1's list goes and how long it may grow
-        const uint32_t used = __ldcg(&ll.start[L]) + (listed <= cap ? listed : 0u);
+        const uint32_t used = start + (listed <= cap ? listed : 0u);
         ll.start[L + 1] = used;
         ll.cap[L + 1] = min(list_max, pool_cap - min(pool_cap, used));
         if (pool_cap - min(pool_cap, used) < list_max) bi->pool_short = 1;
-        if (!__ldcg(&bi->any_new)) {
+        if (!any_new) {
             bi->alive = 0;
             bi->lend = L;
             bi->dmax = L - 1;
@@ -1770,7 +1815,7 @@ template <int K> struct AdvanceLead {
 // kernel sets gs->need and the host grows the tables and launches again, the
 // loop resuming from the level state in bi.
 template <int K>
-__global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
+__global__ void __launch_bounds__(BATCH_TPB, PERSIST_BLOCKS) k_traverse_persist(
     Adj a, Adj rv, BatchInfo *bi, uint32_t **tab, uint32_t *seen_, uint32_t *msigma, float *mdelta,
     float *mq, float *mpartial, uint32_t *harrive, const uint32_t *reach, uint32_t *ctrs, LevelLists ll,
     int symmetric, unsigned long long *level_te, unsigned long long *level_cnt, int32_t *level_mode,
@@ -1785,16 +1830,17 @@ __global__ void __launch_bounds__(BATCH_TPB) k_traverse_persist(
     WorkCount<false> none;
     unsigned epoch = 0;
     const AdvanceLead<K> adv{bi, level_te, level_cnt, level_mode, ll, pool_cap, list_max};
-    for (;;) {
+    const M srcmask = (M)bi->srcmask;
+    // the level counts along in every block: its state, masks and list load at once
+    for (int L = vload_i(&bi->cur) + 1;; L++) {
+        const int push = vload_i(&bi->push_next);
         if (!vload_i(&bi->alive)) break;
-        const int L = vload_i(&bi->cur) + 1;
         if (L >= lmax) {
             if (blockIdx.x == 0 && threadIdx.x == 0) gs->need = 1;
             return;
         }
-        const M srcmask = (M)bi->srcmask;
         M *fprev = reinterpret_cast<M *>(tab[L - 1]), *fcur = reinterpret_cast<M *>(tab[L]);
-        if (vload_i(&bi->push_next))
+        if (push)
             fwd_push_body<K>(a, fprev, fcur, seen, msigma, ctrs + 2 * L, ll, L, none);
         else
             fwd_pull_body<K>(rv, srcmask, fprev, fcur, seen, msigma, ctrs + 2 * L, st, ll, L, none);
@@ -2451,20 +2497,19 @@ template <int K> static int traverse_stepwise(axbc_ctx *c, int nsrc, int *L_out)
 }
 
 // Whether this batch runs as one persistent launch: always or never when the
-// context says so; otherwise a batch of at most 32 pivots on a graph of less than
-// 2^21 adjacency entries, whose levels are shorter than the launches between
-// them, and a batch of at most AXBC_PERSIST_AUTO_WIDTH pivots when the last
-// batch was deep, or -- for the first batch -- when no vertex has more than 64
-// neighbours (meshes and road-like graphs, whose many levels are narrow).
-// Measured (us a pass, steps : persistent): 0.02 M entries, 1 pivot 170 : 142, 32
-// pivots 219 : 179; 0.43 M 217 : 220 and 347 : 320; 1.8 M 340 : 297 and 486 : 431;
-// 3.7 M 378 : 378 and 612 : 643; 64 pivots 408 : 442 at 0.43 M (two mask words
-// leave the one kernel two blocks per SM).  Counting runs use the step kernels.
+// context says so; otherwise a batch on a graph of less than 2^21 adjacency
+// entries, whose levels are shorter than the launches between them, and a batch
+// of at most AXBC_PERSIST_AUTO_WIDTH pivots when the last batch was deep, or --
+// for the first batch -- when no vertex has more than 64 neighbours.  (Batches
+// that mesh.cu takes, or of one pivot, do not come here.)  Measured, us a pass,
+// steps : persistent, 32 and 64 pivots: 0.02 M entries 206 : 161 and 230 : 208; 0.43 M
+// 382 : 300 and 404 : 390; 1.4 M 423 : 336 and 564 : 510; 1.8 M 440 : 356 and 645 :
+// 565; 3.7 M 605 : 600 and 810 : 977.  Counting runs use the step kernels.
 static bool use_persist(axbc_ctx *c, int nsrc)
 {
     if (c->count_on || c->persist_mode < 0) return false;
     if (c->persist_mode > 0) return true;
-    if (nsrc <= AXBC_W && c->g->m < AXBC_PERSIST_AUTO_M) return true;
+    if (c->g->m < AXBC_PERSIST_AUTO_M) return true;
     if (nsrc > AXBC_PERSIST_AUTO_WIDTH) return false;
     if (c->last_batch_levels > AXBC_PERSIST_AUTO_LEVELS) return true;
     return c->last_batch_levels == 0 && c->g->max_deg <= 64;

@@ -359,10 +359,11 @@ int axbc_ctx_launches(const axbc_ctx *ctx, uint64_t *launches);
  * A batched pass normally launches two kernels per forward level and one or
  * two per backward depth.  On graphs of many narrow levels it can instead
  * run as one cooperative launch (all blocks resident, a bounded grid barrier
- * between phases).  mode 1 always, -1 never, 0 (default) for batches of at
- * most 32 pivots on graphs of less than 2^21 adjacency entries, and for batches
- * of at most 8 pivots when the context's last batch was deeper than 64 levels
- * or, for its first batch, when no vertex has more than 64 neighbours.
+ * between phases).  mode 1 always, -1 never, 0 (default) for batches on graphs
+ * of less than 2^21 adjacency entries, and for batches of at most 8 pivots when
+ * the context's last batch was deeper than 64 levels.  With mode 0 a batch of one
+ * pivot and a batch on a mesh (no vertex of more than 64 neighbours, narrow
+ * levels) run in forms of their own, also one launch each.
  * blocks_per_sm: blocks of the cooperative grid per SM (0 keeps the current
  * setting, default 4).  Results
  * are the same bits either way.  A barrier wait that runs out of its budget
