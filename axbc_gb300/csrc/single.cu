@@ -524,18 +524,22 @@ __device__ __forceinline__ void pivot_push_level(const Adj &a, const Adj &rv, co
     const uint64_t up = (a.n_part + gp - 1) / gp;
     for (uint64_t t = w; t < up; t += nw) {
         const uint64_t i = lane * up + t;  // a hub's parts fall into different units
-        uint2 pt = make_uint2(0, 0);
+        uint32_t b_l = 0, n_l = 0, s_l = 0;
         bool on = false;
         if (lane < gp && i < a.n_part) {
-            pt = a.part[i];
+            const uint2 pt = a.part[i];
             on = R.lvl[pt.x] == L - 1;
+            if (on) {
+                b_l = a.col[pt.x] + pt.y * a.part_len;
+                n_l = min(a.col[pt.x + 1] - b_l, a.part_len);
+                s_l = R.sigma[pt.x];
+            }
         }
         for (unsigned act = __ballot_sync(FULL_MASK, on); act; act &= act - 1) {
             const int j = __ffs(act) - 1;
-            const uint32_t v = __shfl_sync(FULL_MASK, pt.x, j), sc = R.sigma[v];
-            const uint32_t b0 = a.col[v] + __shfl_sync(FULL_MASK, pt.y, j) * a.part_len;
-            const uint32_t b1 = min(a.col[v + 1], b0 + a.part_len);
-            for (uint32_t e = b0 + lane; e - lane < b1; e += 32) pivot_push(a, rv, R, e < b1, e, sc, L, fnd);
+            const uint32_t b0 = __shfl_sync(FULL_MASK, b_l, j), len = __shfl_sync(FULL_MASK, n_l, j);
+            const uint32_t sc = __shfl_sync(FULL_MASK, s_l, j);
+            for (uint32_t o = lane; o - lane < len; o += 32) pivot_push(a, rv, R, o < len, b0 + o, sc, L, fnd);
         }
     }
     // the frontier's other vertices: up to 32 adjacency lists walked as one
@@ -570,6 +574,28 @@ __device__ __forceinline__ void pivot_push_level(const Adj &a, const Adj &rv, co
     fnd.flush(R.ctl);
 }
 
+// path counts of the parents among positions e, e + step, ... (four of them,
+// below end) of a list, their entries, levels and counts loaded together: one
+// entry at a time a lane spent three dependent loads on each (a pivot of the
+// 1024^2 mesh 5.8 ms, four together 4.3; scale 20 0.93 and 0.80 ms)
+__device__ __forceinline__ void pivot_parents(const PivotRun &R, const uint32_t *__restrict__ row, uint32_t e,
+                                              uint32_t step, uint32_t end, int L, uint32_t &acc, bool &found)
+{
+    uint32_t v[4], x[4];
+    bool on[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = e + step * i < end ? row[e + step * i] : 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < 4; i++) on[i] = v[i] != 0xffffffffu && R.lvl[v[i]] == L - 1;
+#pragma unroll
+    for (int i = 0; i < 4; i++) x[i] = on[i] ? R.sigma[v[i]] : 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        acc += x[i];
+        found |= on[i];
+    }
+}
+
 // Pull: a part of a big unvisited vertex per warp, the others by eight lanes
 // each (no early exit: every parent counts).
 __device__ __forceinline__ void pivot_pull_level(const Adj &a, const Adj &rv, const PivotRun &R, int L)
@@ -579,79 +605,87 @@ __device__ __forceinline__ void pivot_pull_level(const Adj &a, const Adj &rv, co
     const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     Found fnd;
     const uint64_t np = rv.n_part, nl = rv.n_linked - rv.n_big;
-    const uint32_t gp = stride_unit(np, nw), gl = max(4u, stride_unit(nl, nw));
+    const uint32_t gp = stride_unit(np, nw), gl = max(4u, stride_unit(nl, 4 * nw));
     const uint64_t up = (np + gp - 1) / gp, ul = (nl + gl - 1) / gl;
     for (uint64_t t = w; t < up; t += nw) {
         const uint64_t i = lane * up + t;
-        uint2 pt = make_uint2(0, 0);
+        uint32_t u_l = 0, b_l = 0, n_l = 0, acc_l = 0;
         bool on = false;
         if (lane < gp && i < np) {
-            pt = rv.part[i];
-            const int l = R.lvl[pt.x];
+            const uint2 pt = rv.part[i];
+            u_l = pt.x;
+            const int l = R.lvl[u_l];
             on = l == -1 || l == L;  // another part may have claimed it already
+            b_l = rv.col[u_l] + pt.y * rv.part_len;
+            n_l = min(rv.col[u_l + 1] - b_l, rv.part_len);
         }
+        bool hit = false;
         for (unsigned act = __ballot_sync(FULL_MASK, on); act; act &= act - 1) {
             const int j = __ffs(act) - 1;
-            const uint32_t u = __shfl_sync(FULL_MASK, pt.x, j);
-            const uint32_t b0 = rv.col[u] + __shfl_sync(FULL_MASK, pt.y, j) * rv.part_len;
-            const uint32_t b1 = min(rv.col[u + 1], b0 + rv.part_len);
+            const uint32_t b0 = __shfl_sync(FULL_MASK, b_l, j), len = __shfl_sync(FULL_MASK, n_l, j);
             uint32_t acc = 0;
             bool found = false;
-            for (uint32_t e = b0 + lane; e < b1; e += 32) {
-                const uint32_t v = rv.row[e];
-                if (R.lvl[v] == L - 1) {
-                    acc += R.sigma[v];
-                    found = true;
-                }
+            for (uint32_t o = 0; o < len; o += 128) pivot_parents(R, rv.row + b0, o + lane, 32, len, L, acc, found);
+            if (!__any_sync(FULL_MASK, found)) continue;
+            acc = __reduce_add_sync(FULL_MASK, acc);
+            if ((int)lane == j) {
+                acc_l = acc;
+                hit = true;
             }
-            bool isnew = false;
-            if (__any_sync(FULL_MASK, found)) {
-                acc = __reduce_add_sync(FULL_MASK, acc);
-                if (lane == 0) {
-                    atomicAdd(&R.sigma[u], acc);
-                    isnew = atomicCAS(&R.lvl[u], -1, L) == -1;
-                }
-            }
-            pivot_found(a, rv, R, isnew, u, fnd);
         }
+        bool isnew = false;
+        if (hit) {
+            atomicAdd(&R.sigma[u_l], acc_l);
+            isnew = atomicCAS(&R.lvl[u_l], -1, L) == -1;
+        }
+        pivot_found(a, rv, R, isnew, u_l, fnd);
     }
+    // The order is by degree: the warps that got one part fewer above get the
+    // unit of larger lists here, and four units a warp even out the rest (a
+    // pivot at scale 18: 330 us, 303 so).
     const int sl = lane & 7, g = lane >> 3;
-    for (uint64_t t = w; t < ul; t += nw) {
+    for (uint64_t t = nw - 1 - w; t < ul; t += nw) {
         const uint64_t i = t * gl + lane;
-        uint32_t u_l = 0;
+        uint32_t u_l = 0, b_l = 0, d_l = 0, acc_l = 0;
         bool cand = false;
         if (lane < gl && i < nl) {
             u_l = rv.order[rv.n_big + i];
             cand = R.lvl[u_l] == -1;
+            b_l = rv.col[u_l];
+            d_l = rv.col[u_l + 1] - b_l;
         }
+        bool hit = false;
         for (unsigned act = __ballot_sync(FULL_MASK, cand); act;) {
-            int j = -1;
+            int j4[4], j = -1;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                if (k == g && act) j = __ffs(act) - 1;
+                j4[k] = act ? __ffs(act) - 1 : -1;
+                if (k == g) j = j4[k];
                 act &= act - 1;
             }
-            const uint32_t u = __shfl_sync(FULL_MASK, u_l, j & 31);
-            const uint32_t b = rv.col[u], d = j < 0 ? 0u : rv.col[u + 1] - b;
+            const uint32_t b = __shfl_sync(FULL_MASK, b_l, j & 31), dj = __shfl_sync(FULL_MASK, d_l, j & 31);
+            const uint32_t d = j < 0 ? 0u : dj;
             uint32_t acc = 0;
             bool found = false;
-            for (uint32_t e = sl; e < d; e += 8) {
-                const uint32_t v = rv.row[b + e];
-                if (R.lvl[v] == L - 1) {
-                    acc += R.sigma[v];
-                    found = true;
-                }
-            }
-            const bool any = (__ballot_sync(FULL_MASK, found) >> (8 * g)) & 0xffu;
+            for (uint32_t o = sl; o < d; o += 32) pivot_parents(R, rv.row + b, o, 8, d, L, acc, found);
+            const unsigned any = __ballot_sync(FULL_MASK, found);
+            if (!any) continue;
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) acc += __shfl_xor_sync(FULL_MASK, acc, o);
-            const bool isnew = any && sl == 0;
-            if (isnew) {
-                R.lvl[u] = L;
-                R.sigma[u] = acc;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t x = __shfl_sync(FULL_MASK, acc, 8 * k);
+                if ((int)lane == j4[k] && (any >> (8 * k) & 0xffu)) {
+                    acc_l = x;
+                    hit = true;
+                }
             }
-            pivot_found(a, rv, R, isnew, u, fnd);
         }
+        if (hit) {
+            R.lvl[u_l] = L;
+            R.sigma[u_l] = acc_l;
+        }
+        pivot_found(a, rv, R, hit, u_l, fnd);
     }
     fnd.flush(R.ctl);
 }
@@ -768,60 +802,77 @@ __device__ __forceinline__ void pivot_bwd_depth(const Adj &a, const PivotRun &R,
             }
         }
     }
-    // the others by warps: of at most 8 neighbours four at a time
+    // the others by warps: chunks of 32 four at once, of at most 8 neighbours
+    // four vertices to a chunk
     const uint64_t nw = (uint64_t)gridDim.x * blockDim.x / 32;
     const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32;
     const uint32_t ent = stride_unit(cnt, nw);
     const int l8 = lane & 7, g = lane >> 3;
     for (uint64_t t = w; t < (cnt + ent - 1) / ent; t += nw) {
         const uint64_t i = t * ent + lane;
-        uint32_t v_l = 0, b_l = 0, d_l = 0xffffffffu;
+        uint32_t v_l = 0, b_l = 0, d_l = 0xffffffffu, r_l = 0;
+        float s_l = 0.0f, P_l = 0.0f;
         if (lane < ent && i < cnt) {
             v_l = R.queue[ls + i];
             b_l = a.col[v_l];
             d_l = a.col[v_l + 1] - b_l;
+            s_l = __uint2float_rn(R.sigma[v_l]);
+            r_l = R.reach[v_l];
         }
-        for (unsigned act = __ballot_sync(FULL_MASK, d_l > 8 && d_l <= a.big); act; act &= act - 1) {
-            const int j = __ffs(act) - 1;
-            const uint32_t v = __shfl_sync(FULL_MASK, v_l, j), b0 = __shfl_sync(FULL_MASK, b_l, j);
-            const uint32_t b1 = b0 + __shfl_sync(FULL_MASK, d_l, j);
-            const float s1 = __uint2float_rn(R.sigma[v]);
-            float P = 0.0f;
-            for (uint32_t base = b0; base < b1; base += 32 * NL) {
-                uint32_t r[NL];
-                bool in[NL];
-                float sc[NL], sum[NL];
+        // NL chunks at once, of whichever vertices
+        const uint32_t c_l = d_l > 8 && d_l <= a.big ? (d_l + 31) / 32 : 0u;
+        uint32_t inc = c_l;
 #pragma unroll
-                for (int q = 0; q < NL; q++) {
-                    const uint32_t e = base + 32 * q + lane;
-                    in[q] = e < b1;
-                    sc[q] = s1;
-                    r[q] = in[q] ? a.row[e] : 0u;
-                }
-                pivot_chunks<NL>(R, r, in, d, sc, sum);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(FULL_MASK, inc, o);
+            if ((int)lane >= o) inc += x;
+        }
+        const uint32_t S = __shfl_sync(FULL_MASK, inc, 31);
+        for (uint32_t s0 = 0; s0 < S; s0 += NL) {
+            uint32_t r[NL];
+            bool in[NL];
+            float sc[NL], sum[NL];
+            int j[NL];
 #pragma unroll
-                for (int q = 0; q < NL; q++) P = __fadd_rn(P, sum[q]);
+            for (int q = 0; q < NL; q++) {
+                const uint32_t s = s0 + q;
+                j[q] = __popc(__ballot_sync(FULL_MASK, inc <= s));
+                const uint32_t o = __shfl_sync(FULL_MASK, AXBC_CHUNK * (s - (inc - c_l)), j[q] & 31) + lane;
+                const uint32_t d = __shfl_sync(FULL_MASK, d_l, j[q] & 31);
+                const uint32_t b = __shfl_sync(FULL_MASK, b_l, j[q] & 31);
+                sc[q] = __shfl_sync(FULL_MASK, s_l, j[q] & 31);
+                in[q] = s < S && o < d;
+                r[q] = in[q] ? a.row[b + o] : 0u;
             }
-            if (lane == 0) pivot_dep(R, v, __fadd_rn(__uint2float_rn(R.reach[v]), P));
+            pivot_chunks<NL>(R, r, in, d, sc, sum);
+#pragma unroll
+            for (int q = 0; q < NL; q++)
+                if ((int)lane == j[q]) P_l = __fadd_rn(P_l, sum[q]);
         }
         for (unsigned act = __ballot_sync(FULL_MASK, d_l <= 8); act;) {
-            int j = -1;
+            int j4[4], j = -1;
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                if (q == g && act) j = __ffs(act) - 1;
+                j4[q] = act ? __ffs(act) - 1 : -1;
+                if (q == g) j = j4[q];
                 act &= act - 1;
             }
-            const uint32_t v = __shfl_sync(FULL_MASK, v_l, j & 31), b0 = __shfl_sync(FULL_MASK, b_l, j & 31);
-            const uint32_t dj = __shfl_sync(FULL_MASK, d_l, j & 31);
+            const uint32_t b0 = __shfl_sync(FULL_MASK, b_l, j & 31), dj = __shfl_sync(FULL_MASK, d_l, j & 31);
+            const float sj = __shfl_sync(FULL_MASK, s_l, j & 31);
             float tl = 0.0f;
             if (j >= 0 && (uint32_t)l8 < dj) {
                 const uint32_t r = a.row[b0 + l8];
-                if (R.lvl[r] == d + 1) tl = __fmul_rn(R.q[r], __uint2float_rn(R.sigma[v]));
+                if (R.lvl[r] == d + 1) tl = __fmul_rn(R.q[r], sj);
             }
 #pragma unroll
             for (int o = 1; o < 8; o <<= 1) tl = __fadd_rn(tl, __shfl_xor_sync(FULL_MASK, tl, o));
-            if (j >= 0 && l8 == 0) pivot_dep(R, v, __fadd_rn(__uint2float_rn(R.reach[v]), tl));
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const float x = __shfl_sync(FULL_MASK, tl, 8 * q);
+                if ((int)lane == j4[q]) P_l = x;
+            }
         }
+        if (d_l <= a.big) pivot_dep(R, v_l, __fadd_rn(__uint2float_rn(r_l), P_l));
     }
 }
 
