@@ -103,23 +103,30 @@ static void heavy_lists(const uint32_t *col, uint64_t n, std::vector<uint32_t> &
     if (maxdeg) *maxdeg = std::max(*maxdeg, md);
 }
 
-// Vertices by degree, descending (counting sort, ties by id), and light tasks
-// of at most 32 vertices and about one span of adjacency each.
+// Vertices by degree, descending (counting sort, ties by id; the ids as they
+// are when they descend already, as a view's do), and light tasks of at most
+// 32 vertices and about one span of adjacency each.
 static void task_tables(const uint32_t *col, uint64_t n, std::vector<uint32_t> &order,
                         std::vector<uint32_t> &ltask, uint64_t n_heavy)
 {
-    uint32_t md = 0;
-    for (uint64_t v = 0; v < n; v++) md = std::max(md, col[v + 1] - col[v]);
-    std::vector<uint64_t> cnt((size_t)md + 2, 0);
-    for (uint64_t v = 0; v < n; v++) cnt[md - (col[v + 1] - col[v])]++;
-    uint64_t acc = 0;
-    for (auto &c : cnt) {
-        uint64_t t = c;
-        c = acc;
-        acc += t;
-    }
     order.resize(n);
-    for (uint64_t v = 0; v < n; v++) order[cnt[md - (col[v + 1] - col[v])]++] = (uint32_t)v;
+    uint64_t v0 = 1;
+    while (v0 < n && col[v0 + 1] - col[v0] <= col[v0] - col[v0 - 1]) v0++;
+    if (v0 >= n) {
+        for (uint64_t v = 0; v < n; v++) order[v] = (uint32_t)v;
+    } else {
+        uint32_t md = 0;
+        for (uint64_t v = 0; v < n; v++) md = std::max(md, col[v + 1] - col[v]);
+        std::vector<uint64_t> cnt((size_t)md + 2, 0);
+        for (uint64_t v = 0; v < n; v++) cnt[md - (col[v + 1] - col[v])]++;
+        uint64_t acc = 0;
+        for (auto &c : cnt) {
+            uint64_t t = c;
+            c = acc;
+            acc += t;
+        }
+        for (uint64_t v = 0; v < n; v++) order[cnt[md - (col[v + 1] - col[v])]++] = (uint32_t)v;
+    }
     // light tasks: weight = degree + 8 per vertex, budget one span
     ltask.clear();
     uint64_t i = n_heavy;
@@ -147,8 +154,9 @@ static uint32_t big_of(uint64_t m) { return m < AXBC_SMALL_M ? 32 : 128; }
 static uint32_t part_len_of(uint64_t m) { return m < AXBC_SMALL_M ? 32 : m < (1ull << 25) ? 128 : 512; }
 
 // heavy-vertex span items and light-vertex tasks of an adjacency whose col
-// (host copy: col) is on the device
-static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, uint32_t *maxdeg)
+// (host copy: col) is on the device; its order stays with the caller
+static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, uint32_t *maxdeg,
+                      std::vector<uint32_t> &order)
 {
     std::vector<uint32_t> hv, hf, iv, ik;
     heavy_lists(col, n, hv, hf, iv, ik, maxdeg);
@@ -165,7 +173,7 @@ static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, u
         CU(cudaMemcpy(a.hitem_v, iv.data(), iv.size() * 4, cudaMemcpyHostToDevice));
         CU(cudaMemcpy(a.hitem_k, ik.data(), ik.size() * 4, cudaMemcpyHostToDevice));
     }
-    std::vector<uint32_t> order, ltask;
+    std::vector<uint32_t> ltask;
     task_tables(col, n, order, ltask, a.n_heavy);
     a.n_ltask = ltask.size() - 1;
     TRY(axbc_dalloc((void **)&a.order, n * 4, acct));
@@ -210,7 +218,7 @@ static int adj_tables(Adj &a, const uint32_t *col, uint64_t n, uint64_t *acct, u
 }
 
 static int upload_adj(Adj &a, const uint32_t *col, const uint32_t *row, uint64_t n, uint64_t m,
-                      uint64_t *acct, uint32_t *maxdeg)
+                      uint64_t *acct, uint32_t *maxdeg, std::vector<uint32_t> &order)
 {
     a.n = n;
     a.m = m;
@@ -219,24 +227,53 @@ static int upload_adj(Adj &a, const uint32_t *col, const uint32_t *row, uint64_t
     TRY(axbc_dalloc((void **)&a.row, m * 4, acct));
     CU(cudaMemcpy(a.col, col, (n + 1) * 4, cudaMemcpyHostToDevice));
     if (m) CU(cudaMemcpy(a.row, row, m * 4, cudaMemcpyHostToDevice));
-    return adj_tables(a, col, n, acct, maxdeg);
+    return adj_tables(a, col, n, acct, maxdeg, order);
 }
 
 // ------------------------------------------------------------ batch view
 
 // view adjacency: the list of view vertex i is the list of vertex order[i],
-// in its own order, its entries renumbered (one warp per vertex)
+// in its own order, its entries renumbered.  A warp writes VIEW_RUN entries in
+// a row, whosever they are: a warp per vertex left the largest hub on one of
+// them, 1.3 ms at scale 20 where the entries' traffic takes 0.1.  Its first
+// and last vertex are searched for in vcol, a lane's between the two.
+#define VIEW_RUN 512
+// the vertex of [lo, hi] whose list holds position p
+__device__ __forceinline__ uint64_t view_owner(const uint32_t *__restrict__ vcol, uint64_t lo, uint64_t hi, uint64_t p)
+{
+    while (lo < hi) {
+        const uint64_t mid = (lo + hi + 1) / 2;
+        if (vcol[mid] <= p) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
 __global__ void k_view_rows(const uint32_t *__restrict__ col, const uint32_t *__restrict__ row,
                             const uint32_t *__restrict__ order, const uint32_t *__restrict__ to_view,
-                            const uint32_t *__restrict__ vcol, uint32_t *__restrict__ vrow, uint64_t n)
+                            const uint32_t *__restrict__ vcol, uint32_t *__restrict__ vrow, uint64_t n, uint64_t m)
 {
     const unsigned lane = threadIdx.x & 31;
     const uint64_t nw = (uint64_t)gridDim.x * blockDim.x / 32;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; i < n; i += nw) {
-        const uint32_t v = order[i];
-        const uint32_t b = col[v], d = col[v + 1] - b, o = vcol[i];
-        for (uint32_t k = lane; k < d; k += 32) vrow[o + k] = to_view[row[b + k]];
+    for (uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) / 32; t * VIEW_RUN < m; t += nw) {
+        const uint64_t p0 = t * VIEW_RUN, p1 = min(m, p0 + VIEW_RUN);
+        uint64_t lo = 0;
+        if (lane < 2) lo = view_owner(vcol, 0, n - 1, lane ? p1 - 1 : p0);
+        const uint64_t hi = __shfl_sync(FULL_MASK, lo, 1);
+        lo = __shfl_sync(FULL_MASK, lo, 0);
+#pragma unroll 4
+        for (uint64_t p = p0 + lane; p < p1; p += 32) {
+            const uint64_t i = view_owner(vcol, lo, hi, p);
+            vrow[p] = to_view[row[col[order[i]] + (uint32_t)(p - vcol[i])]];
+        }
     }
+}
+
+// to_view from its inverse
+__global__ void k_view_inverse(const uint32_t *__restrict__ order, uint32_t *__restrict__ to_view, uint64_t n)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        to_view[order[i]] = (uint32_t)i;
 }
 
 __global__ void k_view_gather(const uint32_t *__restrict__ src, const uint32_t *__restrict__ order,
@@ -262,15 +299,17 @@ static int view_adj(Adj &dst, const Adj &src, const uint32_t *col, const std::ve
     TRY(axbc_dalloc((void **)&dst.row, m * 4, acct));
     CU(cudaMemcpy(dst.col, vcol.data(), (n + 1) * 4, cudaMemcpyHostToDevice));
     if (m) {
-        k_view_rows<<<2048, 256>>>(src.col, src.row, d_order, d_to_view, dst.col, dst.row, n);
+        k_view_rows<<<2048, 256>>>(src.col, src.row, d_order, d_to_view, dst.col, dst.row, n, m);
         CU_LAUNCH("k_view_rows");
     }
-    return adj_tables(dst, vcol.data(), n, acct, nullptr);
+    std::vector<uint32_t> own;
+    return adj_tables(dst, vcol.data(), n, acct, nullptr, own);
 }
 
 // The batched passes' view (see axbc_graph): renumbered by descending degree
 // when the largest degree exceeds AXBC_RENUMBER_MIN_DEG, else the graph itself.
-static int build_view(axbc_graph *g, const uint32_t *col, const uint32_t *tcol)
+// order: the forward adjacency's, which is the view's numbering.
+static int build_view(axbc_graph *g, const uint32_t *col, const uint32_t *tcol, const std::vector<uint32_t> &order)
 {
     const uint64_t n = g->n;
     if (g->max_deg <= AXBC_RENUMBER_MIN_DEG || n < 2) {
@@ -283,25 +322,12 @@ static int build_view(axbc_graph *g, const uint32_t *col, const uint32_t *tcol)
         return AXBC_OK;
     }
     g->renumbered = true;
-    // descending degree, ties by id (counting sort)
-    uint32_t md = 0;
-    for (uint64_t v = 0; v < n; v++) md = std::max(md, col[v + 1] - col[v]);
-    std::vector<uint64_t> cnt((size_t)md + 2, 0);
-    for (uint64_t v = 0; v < n; v++) cnt[md - (col[v + 1] - col[v])]++;
-    uint64_t acc = 0;
-    for (auto &c : cnt) {
-        const uint64_t t = c;
-        c = acc;
-        acc += t;
-    }
-    std::vector<uint32_t> order(n), to_view(n);
-    for (uint64_t v = 0; v < n; v++) order[cnt[md - (col[v + 1] - col[v])]++] = (uint32_t)v;
-    for (uint64_t i = 0; i < n; i++) to_view[order[i]] = (uint32_t)i;
     TRY(axbc_dalloc((void **)&g->from_view, n * 4, &g->bytes));
     TRY(axbc_dalloc((void **)&g->to_view, n * 4, &g->bytes));
     TRY(axbc_dalloc((void **)&g->breach, n * 4, &g->bytes));
-    CU(cudaMemcpy(g->from_view, order.data(), n * 4, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(g->to_view, to_view.data(), n * 4, cudaMemcpyHostToDevice));
+    CU(cudaMemcpyAsync(g->from_view, g->fwd.order, n * 4, cudaMemcpyDeviceToDevice, 0));
+    k_view_inverse<<<1024, 256>>>(g->from_view, g->to_view, n);
+    CU_LAUNCH("k_view_inverse");
     k_view_gather<<<1024, 256>>>(g->reach, g->from_view, g->breach, n);
     CU_LAUNCH("k_view_gather");
     TRY(view_adj(g->bfwd, g->fwd, col, order, g->from_view, g->to_view, &g->bytes));
@@ -348,20 +374,14 @@ static void transpose_host(const uint32_t *col, const uint32_t *row, uint64_t n,
         for (uint32_t e = col[c]; e < col[c + 1]; e++) trow[pos[row[e]]++] = (uint32_t)c;
 }
 
-static int graph_from_host(const uint32_t *col, const uint32_t *row, uint64_t n, uint64_t m,
-                           const uint32_t *reach, int known_symmetric, axbc_graph **out)
+// The rest of a graph whose forward adjacency (host copy of its col: col; of
+// its row: row, or null when known symmetric) and reach are on the device.
+static int finish_graph(axbc_graph *g, const uint32_t *col, const uint32_t *row, int known_symmetric,
+                        const std::vector<uint32_t> &order)
 {
-    axbc_graph *g = new axbc_graph();
-    CU(cudaGetDevice(&g->device));
-    g->n = n;
-    g->m = m;
-    int rc = upload_adj(g->fwd, col, row, n, m, &g->bytes, &g->max_deg);
-    if (rc) {
-        axbc_graph_destroy(g);
-        return rc;
-    }
+    const uint64_t n = g->n, m = g->m;
     bool sym = known_symmetric != 0;
-    std::vector<uint32_t> tcol, trow;
+    std::vector<uint32_t> tcol, trow, torder;
     if (!sym) {
         transpose_host(col, row, n, m, tcol, trow);
         sym = std::equal(tcol.begin(), tcol.end(), col) &&
@@ -372,20 +392,31 @@ static int graph_from_host(const uint32_t *col, const uint32_t *row, uint64_t n,
         g->rev = g->fwd;
         g->rev.owns = false;
     } else {
-        rc = upload_adj(g->rev, tcol.data(), trow.data(), n, m, &g->bytes, &g->max_deg);
-        if (rc) {
-            axbc_graph_destroy(g);
-            return rc;
-        }
+        TRY(upload_adj(g->rev, tcol.data(), trow.data(), n, m, &g->bytes, &g->max_deg, torder));
     }
-    rc = axbc_dalloc((void **)&g->reach, n * 4, &g->bytes);
-    if (rc) {
-        axbc_graph_destroy(g);
-        return rc;
-    }
-    if (reach) CU(cudaMemcpy(g->reach, reach, n * 4, cudaMemcpyHostToDevice));
-    else CU(cudaMemset(g->reach, 0, n * 4));
-    rc = build_view(g, col, sym ? col : tcol.data());
+    return build_view(g, col, sym ? col : tcol.data(), order);
+}
+
+static int upload_graph(axbc_graph *g, const uint32_t *col, const uint32_t *row, const uint32_t *reach,
+                        int known_symmetric)
+{
+    std::vector<uint32_t> order;
+    TRY(upload_adj(g->fwd, col, row, g->n, g->m, &g->bytes, &g->max_deg, order));
+    TRY(axbc_dalloc((void **)&g->reach, g->n * 4, &g->bytes));
+    if (reach) CU(cudaMemcpy(g->reach, reach, g->n * 4, cudaMemcpyHostToDevice));
+    else CU(cudaMemset(g->reach, 0, g->n * 4));
+    return finish_graph(g, col, row, known_symmetric, order);
+}
+
+static int graph_from_host(const uint32_t *col, const uint32_t *row, uint64_t n, uint64_t m,
+                           const uint32_t *reach, int known_symmetric, axbc_graph **out)
+{
+    axbc_graph *g = new axbc_graph();
+    g->n = n;
+    g->m = m;
+    const cudaError_t e = cudaGetDevice(&g->device);
+    const int rc = e != cudaSuccess ? axbc_cuda_fail(e, "cudaGetDevice", __FILE__, __LINE__)
+                                    : upload_graph(g, col, row, reach, known_symmetric);
     if (rc) {
         axbc_graph_destroy(g);
         return rc;
@@ -590,15 +621,39 @@ __global__ void k_mark(const uint64_t *__restrict__ keys, uint64_t nk, uint64_t 
     }
 }
 
+// rows of sorted keys, and where each of the n columns starts (n + 1 entries,
+// a search each: counting the columns' keys serialised on the hubs' counters)
 __global__ void k_split(const uint64_t *__restrict__ keys, uint64_t m, uint32_t *__restrict__ row,
-                        uint32_t *__restrict__ cnt)
+                        uint32_t *__restrict__ col, uint64_t n)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t k = keys[i];
-        row[i] = (uint32_t)k;
-        atomicAdd(&cnt[(uint32_t)(k >> 32)], 1u);
+    const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = t0; i < m; i += nt) row[i] = (uint32_t)keys[i];
+    for (uint64_t v = t0; v <= n; v += nt) {
+        uint64_t lo = 0, hi = m;  // the first key of a column >= v
+        while (lo < hi) {
+            const uint64_t mid = (lo + hi) / 2;
+            if (keys[mid] >> 32 < v) lo = mid + 1;
+            else hi = mid;
+        }
+        col[v] = (uint32_t)lo;
     }
+}
+
+// a block's least (or largest) value, on its thread 0; the atomics of every
+// thread of a grid on one word took 171 us (smallest pair) and 337 us (last
+// kept entry) of a scale-16 ingest
+template <bool MIN>
+__device__ __forceinline__ unsigned long long block_extreme(unsigned long long x)
+{
+    __shared__ unsigned long long part[32];
+    for (int o = 16; o; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(FULL_MASK, x, o);
+        x = MIN ? min(x, y) : max(x, y);
+    }
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = x;
+    __syncthreads();
+    for (unsigned w = 0; threadIdx.x == 0 && w < blockDim.x / 32; w++) x = MIN ? min(x, part[w]) : max(x, part[w]);
+    return x;
 }
 
 // lexicographically smallest (u,v) = (row, column) among valid keys
@@ -612,7 +667,8 @@ __global__ void k_min_uv(const uint64_t *__restrict__ keys, uint64_t nk, unsigne
         unsigned long long uv = ((unsigned long long)(uint32_t)k << 32) | (k >> 32);
         best = best < uv ? best : uv;
     }
-    atomicMin(out, best);
+    best = block_extreme<true>(best);
+    if (threadIdx.x == 0 && best != ~0ull) atomicMin(out, best);
 }
 
 // One-degree reduction of a sorted, duplicate-free symmetric list on the device
@@ -649,7 +705,8 @@ __global__ void k_leaf_entries(const uint64_t *__restrict__ keys, uint64_t m, ui
         }
         kind[i] = t;
     }
-    atomicMax(last_kept, best);
+    best = block_extreme<false>(best);
+    if (threadIdx.x == 0 && best) atomicMax(last_kept, best);
 }
 
 __global__ void k_leaf_reduce(const uint64_t *__restrict__ keys, uint64_t m, const uint8_t *__restrict__ leafv,
@@ -673,10 +730,11 @@ __global__ void k_leaf_reduce(const uint64_t *__restrict__ keys, uint64_t m, con
 
 // Sort device keys, dedupe, reduce degree-1 vertices (H == 1), build the CSC
 // and wrap it in a graph.
-
-int axbc_keys_to_graph(uint64_t *d_keys, uint64_t nk, uint64_t n, int symmetric, int H,
-                       axbc_graph **out)
+// The adjacency stays on the device; its columns' starts come to the host for
+// the tables, and the rows of a list that is not mirrored for its transpose.
+static int keys_to_graph(axbc_graph *g, uint64_t *d_keys, uint64_t nk, int symmetric, int H)
 {
+    const uint64_t n = g->n;
     cudaStream_t s = 0;
     size_t tmp_bytes = 0;
     unsigned long long m = 0;
@@ -717,24 +775,23 @@ int axbc_keys_to_graph(uint64_t *d_keys, uint64_t nk, uint64_t n, int symmetric,
         return AXBC_ERR_RANGE;
     }
 
-    std::vector<uint32_t> reach;
+    TRY(axbc_dalloc((void **)&g->reach, n * 4, &g->bytes));
+    CU(cudaMemset(g->reach, 0, n * 4));
     if (H == 1 && m > 0) {
         if (!symmetric) {
             axbc_set_error("one-degree reduction of a generated graph needs a symmetric graph");
             return AXBC_ERR_INVALID;
         }
-        DBuf leafv, kind, dreach, last, kept, nsel, tmp;
+        DBuf leafv, kind, last, kept, nsel, tmp;
         TRY(leafv.alloc(n));
         TRY(kind.alloc(m));
-        TRY(dreach.alloc(n * 4));
         TRY(last.alloc(8));
         CU(cudaMemset(leafv.p, 0, n));
-        CU(cudaMemset(dreach.p, 0, n * 4));
         CU(cudaMemset(last.p, 0, 8));
         k_leaf_entries<<<2048, 256>>>(d_keys, m, leafv.as<uint8_t>(), kind.as<uint8_t>(),
                                       last.as<unsigned long long>());
         CU_LAUNCH("k_leaf_entries");
-        k_leaf_reduce<<<2048, 256>>>(d_keys, m, leafv.as<uint8_t>(), kind.as<uint8_t>(), dreach.as<uint32_t>(),
+        k_leaf_reduce<<<2048, 256>>>(d_keys, m, leafv.as<uint8_t>(), kind.as<uint8_t>(), g->reach,
                                      last.as<unsigned long long>());
         CU_LAUNCH("k_leaf_reduce");
         TRY(kept.alloc(m * 8));
@@ -748,24 +805,37 @@ int axbc_keys_to_graph(uint64_t *d_keys, uint64_t nk, uint64_t n, int symmetric,
         CU_LAUNCH("select kept entries");
         CU(cudaMemcpy(&m, nsel.p, 8, cudaMemcpyDeviceToHost));
         CU(cudaMemcpy(d_keys, kept.p, m * 8, cudaMemcpyDeviceToDevice));
-        reach.resize(n);
-        CU(cudaMemcpy(reach.data(), dreach.p, n * 4, cudaMemcpyDeviceToHost));
     }
 
-    std::vector<uint32_t> col(n + 1), cnt(n + 1), row(m);
-    {
-        DBuf drow, dcnt;
-        TRY(drow.alloc(m * 4));
-        TRY(dcnt.alloc((n + 1) * 4));
-        CU(cudaMemset(dcnt.p, 0, (n + 1) * 4));
-        k_split<<<2048, 256>>>(d_keys, m, drow.as<uint32_t>(), dcnt.as<uint32_t>());
-        CU_LAUNCH("k_split");
-        CU(cudaMemcpy(cnt.data(), dcnt.p, (n + 1) * 4, cudaMemcpyDeviceToHost));
-        CU(cudaMemcpy(row.data(), drow.p, m * 4, cudaMemcpyDeviceToHost));
+    g->m = m;
+    Adj &a = g->fwd;
+    a.n = n;
+    a.m = m;
+    a.owns = true;
+    TRY(axbc_dalloc((void **)&a.col, (n + 1) * 4, &g->bytes));
+    TRY(axbc_dalloc((void **)&a.row, m * 4, &g->bytes));
+    k_split<<<2048, 256>>>(d_keys, m, a.row, a.col, n);
+    CU_LAUNCH("k_split");
+    std::vector<uint32_t> col(n + 1), row(symmetric ? 0 : m), order;
+    CU(cudaMemcpy(col.data(), a.col, (n + 1) * 4, cudaMemcpyDeviceToHost));
+    if (!row.empty()) CU(cudaMemcpy(row.data(), a.row, m * 4, cudaMemcpyDeviceToHost));
+    TRY(adj_tables(a, col.data(), n, &g->bytes, &g->max_deg, order));
+    return finish_graph(g, col.data(), row.data(), symmetric, order);
+}
+
+int axbc_keys_to_graph(uint64_t *d_keys, uint64_t nk, uint64_t n, int symmetric, int H, axbc_graph **out)
+{
+    axbc_graph *g = new axbc_graph();
+    g->n = n;
+    const cudaError_t e = cudaGetDevice(&g->device);
+    const int rc = e != cudaSuccess ? axbc_cuda_fail(e, "cudaGetDevice", __FILE__, __LINE__)
+                                    : keys_to_graph(g, d_keys, nk, symmetric, H);
+    if (rc) {
+        axbc_graph_destroy(g);
+        return rc;
     }
-    col[0] = 0;
-    for (uint64_t v = 0; v < n; v++) col[v + 1] = col[v] + cnt[v];
-    return graph_from_host(col.data(), row.data(), n, m, reach.empty() ? nullptr : reach.data(), symmetric, out);
+    *out = g;
+    return AXBC_OK;
 }
 
 // adjacency keys of a host edge list: (u,v) and, when mirrored and u != v, (v,u)

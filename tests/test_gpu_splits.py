@@ -172,3 +172,23 @@ def test_sampler_windows_and_many_check_vertices(axbc, orc, z, nchecks):
         for k in ("nrounds", "skipped", "dropped", "ui_end", "te", "stopped"):
             assert got[k] == want[k], (W, c, k)
         assert np.array_equal(ctx.bc(), want["bc"], equal_nan=True)
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+@pytest.mark.parametrize("leaves", [65, 254, 255, 256, 510, 511, 512, 513, 1300])
+def test_ingest_of_a_hub_among_isolated_vertices(axbc, orc, leaves, undirected):
+    # adjacency runs around the 512 entries a warp renumbers, with vertices
+    # without entries before, between and after the linked ones
+    n = 3 * leaves + 40
+    hub = 17
+    spokes = 20 + 3 * np.arange(leaves)
+    e = np.concatenate([np.stack([np.full(leaves, hub), spokes], 1), np.stack([spokes[:-1], spokes[1:]], 1)[::7],
+                        [[hub, hub], [spokes[3], spokes[3]], [hub, spokes[0]]]]).astype(np.uint64)
+    want = orc.pipeline(e, n, undirected, 0)
+    graph = axbc.Graph.from_edges(e, n, undirected=undirected, H=0)
+    col, row, reach = graph.csc()
+    assert np.array_equal(col, want.col) and np.array_equal(row, want.row) and not reach.any()
+    ctx = axbc.Context(graph)
+    piv = np.array([hub, spokes[0], spokes[-1]], np.uint32)
+    ctx.run_batch(piv, np.full(3, 0.25))
+    assert np.array_equal(ctx.bc(), orc.bc_pivots(want, piv, np.full(3, 0.25))[0])
