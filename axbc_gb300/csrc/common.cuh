@@ -219,14 +219,14 @@ struct PivotBuf {
     PivotCtl *ctl_host = nullptr;    // pinned
 };
 
-// batches of at most AXBC_PERSIST_AUTO_WIDTH pivots on graphs whose last batch
-// was deeper than AXBC_PERSIST_AUTO_LEVELS run their levels in one persistent
-// launch
 // graphs whose largest degree exceeds this are renumbered for the batched
 // passes (meshes and road-like graphs keep their own, already local, order)
 #ifndef AXBC_RENUMBER_MIN_DEG
 #define AXBC_RENUMBER_MIN_DEG 64
 #endif
+// graphs of fewer than AXBC_PERSIST_AUTO_M adjacency entries, and batches of at
+// most AXBC_PERSIST_AUTO_WIDTH pivots on graphs whose last batch was deeper than
+// AXBC_PERSIST_AUTO_LEVELS, run their levels in one persistent launch
 #ifndef AXBC_PERSIST_AUTO_M
 #define AXBC_PERSIST_AUTO_M (1ull << 21)
 #endif
@@ -349,8 +349,8 @@ struct axbc_ctx {
     // captured level steps, accumulating into wcount[kind][field]
     bool count_on = false;
     unsigned long long *wcount = nullptr;  // KP_NKINDS * WC_NFIELDS
-    // persistent level loop: -1 never, 0 when the last batch was deeper than
-    // AXBC_PERSIST_AUTO_LEVELS, 1 always; blocks per SM of its cooperative grid
+    // persistent level loop: -1 never, 0 by the AXBC_PERSIST_AUTO_* rules, 1
+    // always; blocks per SM of its cooperative grid
     int persist_mode = 0;
     int persist_blocks_per_sm = 4;
     int persist_fit[2] = {0, 0};       // blocks of it that fit an SM, per width
