@@ -558,7 +558,9 @@ def main():
         ctx.count(False)
     must = counts.get(kind, {}).get("bytes")
     must_per_launch = must * args.steps / max(cnt, 1) if must else None
-    traffic, traffic_note = traffic_for(kernel, graph_key, must_per_launch, 1 if args.width <= 32 else 2)
+    # the capture keeps the forward kernel's pulled and pushed levels apart
+    captured = {"batch_fwd_pull": "k_fwd_pull_step", "batch_fwd_push": "k_fwd_push_step"}.get(kind, kernel)
+    traffic, traffic_note = traffic_for(captured, graph_key, must_per_launch, 1 if args.width <= 32 else 2)
     if must_per_launch:
         achieved = must_per_launch / avg_s / 1e9
         basis = ("bytes the kernel must move, counted on the device by its counting build over "
