@@ -2211,6 +2211,7 @@ __global__ void k_source_view(int s, int levels, uint32_t *const *fm, const uint
     }
 }
 
+// ------------------------------------------------------------------ host
 static int ensure_level_tables(axbc_ctx *c)
 {
     if (c->tables_ready) return AXBC_OK;
