@@ -1,7 +1,9 @@
 // Contexts, results, errors: the handle-based part of the C ABI.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "common.cuh"
 
@@ -25,6 +27,34 @@ int axbc_cuda_fail(cudaError_t e, const char *what, const char *file, int line)
         return AXBC_ERR_NOMEM;
     }
     return AXBC_ERR_CUDA;
+}
+
+// failure injection for tests: one-launch passes taken for failed
+static std::atomic<int> g_fail_pass[AXBC_FAIL_KINDS];
+
+extern "C" void axbc_inject_pass_failures(int kind, int n)
+{
+    if (kind >= 0 && kind < AXBC_FAIL_KINDS) g_fail_pass[kind].store(n < 0 ? 0 : n);
+}
+
+bool axbc_pass_fails(int kind)
+{
+    std::atomic<int> &left = g_fail_pass[kind];
+    for (int k = left.load(); k > 0; k = left.load())
+        if (left.compare_exchange_weak(k, k - 1)) return true;
+    return false;
+}
+
+int axbc_wait_ran_out(axbc_ctx *c, int err, uint32_t *arrive, uint64_t n, int *site)
+{
+    *site = err;
+    if (!err && axbc_pass_fails(AXBC_FAIL_WAIT)) {
+        const std::vector<uint32_t> one(n, 1u);  // one span of each has arrived
+        CU(cudaMemcpy(arrive, one.data(), n * 4, cudaMemcpyHostToDevice));
+        *site = 3;
+    }
+    if (*site) CU(cudaMemsetAsync(arrive, 0, n * 4, c->stream));
+    return AXBC_OK;
 }
 
 extern "C" const char *axbc_last_error(void) { return g_err; }

@@ -2604,8 +2604,10 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
         // the level state and the barrier's record in one copy
         CU(cudaMemcpyAsync((char *)c->bi_host + ctl_off, (char *)c->bi + ctl_off, ctl_len, cudaMemcpyDeviceToHost, s));
         CU(cudaStreamSynchronize(s));
-        if (hs.err) {
-            axbc_set_error("persistent level loop: a grid barrier wait ran out of its budget (site %d)", hs.err);
+        int site = 0;
+        TRY(axbc_wait_ran_out(c, hs.err, c->harrive, (uint64_t)(g->bfwd.n_heavy + 1) * 2, &site));
+        if (site) {
+            axbc_set_error("persistent level loop: a grid barrier wait ran out of its budget (site %d)", site);
             return AXBC_ERR_TIMEOUT;
         }
         if (!hs.need) break;

@@ -376,6 +376,14 @@ int axbc_keys_to_graph(uint64_t *d_keys, uint64_t nk, uint64_t n, int symmetric,
 int axbc_kron_device(int scale, int edgefactor, uint64_t seed1, uint64_t seed2, const double *initiator,
                      int stage, uint64_t **d_edges, uint64_t *m_out);
 
+// host-side failure of a one-launch pass (axbc_inject_pass_failures)
+bool axbc_pass_fails(int kind);
+// *site: the barrier of the pass just waited for whose wait ran out (0: none).
+// Every block then left wherever it was, so the n arrival counts of the heavy
+// vertices may be on the way; they go back to zero, where the next pass takes
+// them up.
+int axbc_wait_ran_out(axbc_ctx *c, int err, uint32_t *arrive, uint64_t n, int *site);
+
 // allocation with byte accounting
 int axbc_dalloc(void **p, size_t bytes, uint64_t *acct);
 void axbc_dfree(void *p);

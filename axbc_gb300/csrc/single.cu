@@ -1116,10 +1116,10 @@ static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R)
 static int pivot_wait(axbc_ctx *c, PivotBuf &b)
 {
     CU(cudaStreamSynchronize(c->stream));
-    if (b.ctl_host->gs.err) {
-        CU(cudaMemsetAsync(b.arrive, 0, (c->g->fwd.n_heavy + 1) * 4, c->stream));
-        axbc_set_error("pivot in one launch: a grid barrier wait ran out of its budget (site %d)",
-                       b.ctl_host->gs.err);
+    int site = 0;
+    TRY(axbc_wait_ran_out(c, b.ctl_host->gs.err, b.arrive, c->g->fwd.n_heavy + 1, &site));
+    if (site) {
+        axbc_set_error("pivot in one launch: a grid barrier wait ran out of its budget (site %d)", site);
         return AXBC_ERR_TIMEOUT;
     }
     return AXBC_OK;

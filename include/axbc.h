@@ -398,6 +398,12 @@ int axbc_ctx_count_read(axbc_ctx *ctx, uint64_t *counts, int nkinds);
 void axbc_inject_alloc_failures(int n);
 void axbc_inject_alloc_failure_after(int skip);
 uint64_t axbc_device_bytes_live(void);
+/* The next n one-launch passes are taken for failed on the host, as `kind`
+ * says (0 clears it):
+ * AXBC_FAIL_WAIT: a grid barrier wait ran out on the backward way, the span
+ *   sums of the vertices of more than 1024 neighbours partly counted. */
+enum { AXBC_FAIL_WAIT = 0, AXBC_FAIL_KINDS = 1 };
+void axbc_inject_pass_failures(int kind, int n);
 
 /* Per forward level of the last batch (up to max_levels; *levels = all):
  * vertices newly reached over all pivots, their degree sum, direction (1:
