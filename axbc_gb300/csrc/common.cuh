@@ -290,6 +290,7 @@ struct axbc_ctx {
     uint32_t *mesh_queue = nullptr, *mesh_lev = nullptr;
     int mesh_cap = 0;       // pivots they hold
     bool mesh_off = false;  // a level of this graph was too wide for them
+    bool mesh_short = false;  // no room for them; tried again after a reset of the context
     int pivot_fit = 0;      // blocks of the kernel that fit an SM
     std::vector<uint64_t> levstart;
     uint64_t s_front_deg = 0, s_prev_newdeg = 0, s_visited_rdeg = 0;  // direction choice

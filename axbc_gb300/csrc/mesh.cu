@@ -38,9 +38,9 @@ struct MeshArgs {
     int32_t *lvl;
     uint32_t *sigma, *queue;
     float *delta, *q;
-    uint32_t *lev;   // per pivot AXBC_MAX_LEVELS starts of its levels in its queue
+    uint32_t *lev;   // per pivot lev_cap starts of its levels in its queue
     int *stop;       // 1: a level exceeded `limit`, 2: too many levels
-    uint64_t n;
+    uint64_t n, lev_cap;
     uint32_t limit;
     int nsrc, H;
 };
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(MESH_TPB, 1) k_mesh(MeshArgs A)
     int32_t *lvl = A.lvl + s * A.n;
     uint32_t *sigma = A.sigma + s * A.n, *queue = A.queue + s * A.n;
     float *delta = A.delta + s * A.n, *q = A.q + s * A.n;
-    uint32_t *lev = A.lev + (uint64_t)s * AXBC_MAX_LEVELS;
+    uint32_t *lev = A.lev + s * A.lev_cap;
     uint32_t *cnt = cl.map_shared_rank(s_new, 0);
     const uint32_t root = A.bi->root[s];
     if (threadIdx.x == 0) {
@@ -359,42 +359,66 @@ __global__ void k_mesh_levels(const uint32_t *__restrict__ col, const int32_t *_
 // ------------------------------------------------------------------ host
 
 // Graphs without a vertex of more than 64 neighbours (the batched passes keep
-// their numbering), until a pass meets a level too wide for it.
+// their numbering), until a pass meets a level too wide for it or finds no room
+// for its vectors.
 bool axbc_mesh_fits(const axbc_ctx *c)
 {
-    return c->g->max_deg <= AXBC_RENUMBER_MIN_DEG && !c->g->renumbered && !c->mesh_off;
+    return c->g->max_deg <= AXBC_RENUMBER_MIN_DEG && !c->g->renumbered && !c->mesh_off && !c->mesh_short;
 }
 
-static int ensure_mesh(axbc_ctx *c, int nsrc)
+// starts of levels kept per pivot: a level has a vertex at least
+static uint64_t mesh_lev_cap(const axbc_graph *g) { return std::min<uint64_t>(AXBC_MAX_LEVELS, g->n + 2); }
+static uint64_t mesh_bytes(const axbc_graph *g) { return g->n * 8 + mesh_lev_cap(g) * 4; }
+
+// the vectors go (no pass has its results in them any more)
+static void mesh_free(axbc_ctx *c)
 {
-    TRY(axbc_ensure_batch(c));
+    axbc_dfree(c->mesh_lvl);
+    axbc_dfree(c->mesh_queue);
+    axbc_dfree(c->mesh_lev);
+    c->mesh_lvl = nullptr;
+    c->mesh_queue = c->mesh_lev = nullptr;
+    c->bytes -= c->mesh_cap * mesh_bytes(c->g);
+    c->mesh_cap = 0;
+}
+
+// AXBC_ERR_NOMEM: the batched form's buffers are there, the vectors are not
+static int mesh_room(axbc_ctx *c, int nsrc)
+{
     if (nsrc <= c->mesh_cap) return AXBC_OK;
     const int cap = nsrc <= 1 ? 1 : nsrc <= 8 ? 8 : AXBC_WMAX;
     DBuf l, q, v;
     TRY(l.alloc((uint64_t)cap * c->g->n * 4));
     TRY(q.alloc((uint64_t)cap * c->g->n * 4));
-    TRY(v.alloc((uint64_t)cap * AXBC_MAX_LEVELS * 4));
+    TRY(v.alloc(cap * mesh_lev_cap(c->g) * 4));
     CU(cudaStreamSynchronize(c->stream));
-    axbc_dfree(c->mesh_lvl);
-    axbc_dfree(c->mesh_queue);
-    axbc_dfree(c->mesh_lev);
+    mesh_free(c);
     c->mesh_lvl = l.as<int32_t>();
     c->mesh_queue = q.as<uint32_t>();
     c->mesh_lev = v.as<uint32_t>();
     l.p = q.p = v.p = nullptr;
-    c->bytes += (uint64_t)(cap - c->mesh_cap) * (c->g->n * 8 + AXBC_MAX_LEVELS * 4);
+    c->bytes += cap * mesh_bytes(c->g);
     c->mesh_cap = cap;
     return AXBC_OK;
 }
 
-// A pass of nsrc pivots (roots in c->bi).  *done = false: a level was too wide,
-// nothing is left behind but the roots.
+// A pass of nsrc pivots (roots in c->bi).  *done = false: a level was too wide
+// or the vectors found no room (512 bytes a vertex beside the rows' 768, which
+// the batched form does without); nothing is left behind but the roots.
 int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
 {
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
     *done = false;
-    TRY(ensure_mesh(c, nsrc));
+    TRY(axbc_ensure_batch(c));
+    const int room = mesh_room(c, nsrc);
+    if (room == AXBC_ERR_NOMEM) {
+        CU(cudaStreamSynchronize(s));
+        mesh_free(c);  // smaller ones of an earlier pass
+        c->mesh_short = true;
+        return AXBC_OK;
+    }
+    TRY(room);
     MeshArgs A;
     A.a = g->fwd;
     A.reach = g->reach;
@@ -408,6 +432,7 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     A.lev = c->mesh_lev;
     A.stop = &c->bi->gs.need;
     A.n = g->n;
+    A.lev_cap = mesh_lev_cap(g);
     A.nsrc = nsrc;
     A.H = H;
     // a level of a sixteenth of the graph is no narrow one

@@ -43,3 +43,35 @@ def test_span_arrivals_start_at_zero_after_a_wait_ran_out(axbc, orc, k, undirect
     assert ex.value.status == 4
     pass_of(ctx, orc, g, piv[k:2 * k], p)
     pass_of(ctx, orc, g, piv[2 * k:3 * k], p)
+
+
+def grid(orc, side):
+    i = np.arange(side * side).reshape(side, side)
+    e = np.concatenate([np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()], 1), np.stack([i[:-1].ravel(), i[1:].ravel()], 1)])
+    return orc.pipeline(e.astype(np.uint64), side * side, True, 0)
+
+
+@pytest.mark.parametrize("skip", [0, 1, 2])
+@pytest.mark.parametrize("first", [1, 8])
+def test_mesh_pass_without_room_for_its_vectors(axbc, orc, first, skip):
+    # the vectors of a pass of 33 pivots replace those of the first pass; each of
+    # their three allocations is refused in turn
+    g = grid(orc, 40)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    piv = np.random.default_rng(1).choice(g.n, 66, replace=False).astype(np.uint32)
+    p = np.full(33, 0.25)
+    pass_of(ctx, orc, g, piv[:first], p[:first])
+    vector = 8 * g.n + 4 * (g.n + 2)  # levels, queue, level starts of one pivot
+    bare = ctx.bytes - (1 if first == 1 else 8) * vector
+    axbc.lib().axbc_inject_alloc_failure_after(skip)
+    try:
+        ctx.run_batch(piv[:33], p)
+    finally:
+        axbc.lib().axbc_inject_alloc_failure_after(-1)
+    assert (ctx.bytes - bare) % (8 * g.n) == 0  # level masks of the batched form, no vectors
+    want, delta_last, _ = orc.bc_pivots(g, np.concatenate([piv[:first], piv[:33]]), np.full(first + 33, 0.25))
+    assert np.array_equal(ctx.bc(), want, equal_nan=True) and np.array_equal(ctx.delta(), delta_last, equal_nan=True)
+    ctx.run_batch(piv[33:], p)
+    assert (ctx.bytes - bare) % (8 * g.n) == 0  # not tried again
+    pass_of(ctx, orc, g, piv[33:], p)  # but after a reset
+    assert (ctx.bytes - bare - 64 * vector) % (8 * g.n) == 0
