@@ -477,7 +477,8 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     CU(cudaStreamSynchronize(s));
     const int stop = c->bi_host->gs.need;
     if (stop == 1) {
-        c->mesh_off = true;
+        c->mesh_off = true;  // for good: nothing reads the vectors again
+        mesh_free(c);
         return AXBC_OK;
     }
     if (stop == 2) {

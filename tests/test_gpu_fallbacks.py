@@ -75,3 +75,20 @@ def test_mesh_pass_without_room_for_its_vectors(axbc, orc, first, skip):
     assert (ctx.bytes - bare) % (8 * g.n) == 0  # not tried again
     pass_of(ctx, orc, g, piv[33:], p)  # but after a reset
     assert (ctx.bytes - bare - 64 * vector) % (8 * g.n) == 0
+
+
+@pytest.mark.parametrize("k", [2, 40])
+def test_vectors_of_a_mesh_pass_go_when_a_level_is_too_wide(axbc, orc, k):
+    rng = np.random.default_rng(17)
+    n = 6000
+    g = orc.pipeline(rng.integers(0, n, size=(4 * n, 2)).astype(np.uint64), n, True, 0)
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    piv = rng.choice(n, k, replace=False).astype(np.uint32)
+    held = []
+    for mode in (0, 1):  # the mesh form is tried first; the batched form at once
+        ctx = axbc.Context(G)
+        ctx.set_persistent(mode)
+        pass_of(ctx, orc, g, piv, np.full(k, 0.5))
+        pass_of(ctx, orc, g, piv, np.full(k, 0.5))
+        held.append(ctx.bytes)
+    assert held[0] == held[1]
