@@ -131,6 +131,7 @@ _SIGS = {
     "axbc_inject_alloc_failures": (None, [C.c_int]),
     "axbc_inject_alloc_failure_after": (None, [C.c_int]),
     "axbc_inject_pass_failures": (None, [C.c_int, C.c_int]),
+    "axbc_ctx_mesh_blocks": (C.c_int, [_P, C.c_int, C.POINTER(C.c_int)]),
     "axbc_device_bytes_live": (C.c_uint64, []),
     "axbc_sample": (C.c_int, [_P, C.c_int, C.POINTER(C.c_uint64), C.POINTER(C.c_uint32), C.c_int,
                               C.POINTER(C.c_uint32), C.POINTER(C.c_double)]),

@@ -290,6 +290,8 @@ struct axbc_ctx {
     uint32_t *mesh_queue = nullptr, *mesh_lev = nullptr;
     int mesh_cap = 0;       // pivots they hold
     bool mesh_off = false;  // a level of this graph was too wide for them
+    int mesh_fit[5] = {-1, -1, -1, -1, -1};  // clusters of 1, 2 .. 16 blocks the device holds (-1: not asked)
+    int mesh_force = 0, mesh_used = 0;       // blocks per pivot: asked for by a test, of the last mesh pass
     bool mesh_short = false;  // no room for them; tried again after a reset of the context
     int pivot_fit = 0;      // blocks of the kernel that fit an SM
     std::vector<uint64_t> levstart;

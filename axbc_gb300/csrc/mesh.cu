@@ -402,6 +402,55 @@ static int mesh_room(axbc_ctx *c, int nsrc)
     return AXBC_OK;
 }
 
+struct MeshLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    MeshLaunch(const axbc_ctx *c, int blocks, int C)
+    {
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(MESH_TPB);
+        cfg.stream = c->stream;
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+    }
+};
+
+// *C blocks per pivot, or as many fewer as the device holds a cluster of (a part
+// of it may be out of reach: SMs taken away from this process); 0: not even one
+static int mesh_cluster(axbc_ctx *c, int *C)
+{
+    for (; *C; *C /= 2) {
+        int &fit = c->mesh_fit[31 - __builtin_clz(*C)];
+        if (fit < 0) {
+            if (*C > 8) CU(cudaFuncSetAttribute(k_mesh, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            MeshLaunch ml(c, *C, *C);
+            int held = 0;
+            if (axbc_pass_fails(AXBC_FAIL_CLUSTER) ||
+                cudaOccupancyMaxActiveClusters(&held, k_mesh, &ml.cfg) != cudaSuccess) {
+                (void)cudaGetLastError();
+                held = 0;
+            }
+            fit = held;
+        }
+        if (fit > 0) break;
+    }
+    return AXBC_OK;
+}
+
+// A test's choice of the blocks per pivot of a context's mesh passes.
+extern "C" int axbc_ctx_mesh_blocks(axbc_ctx *c, int blocks, int *used)
+{
+    CHECK_ARG(c, "axbc_ctx_mesh_blocks: null context");
+    CHECK_ARG(blocks >= 0 && blocks <= 16 && (blocks & (blocks - 1)) == 0,
+              "axbc_ctx_mesh_blocks: blocks must be 0, 1, 2, 4, 8 or 16");
+    c->mesh_force = blocks;
+    if (used) *used = c->mesh_used;
+    return AXBC_OK;
+}
+
 // A pass of nsrc pivots (roots in c->bi).  *done = false: a level was too wide
 // or the vectors found no room (512 bytes a vertex beside the rows' 768, which
 // the batched form does without); nothing is left behind but the roots.
@@ -410,6 +459,7 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
     *done = false;
+    c->mesh_used = 0;
     TRY(axbc_ensure_batch(c));
     const int room = mesh_room(c, nsrc);
     if (room == AXBC_ERR_NOMEM) {
@@ -450,26 +500,24 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     int C = 1;
     const int sms = c->num_sms > 0 ? c->num_sms : 152, most = nsrc <= 2 ? 16 : 8;
     while (C < most && (uint64_t)C * MESH_TPB < 4 * width && 2 * C * nsrc <= sms) C *= 2;
+    if (c->mesh_force) C = c->mesh_force;
+    TRY(mesh_cluster(c, &C));
+    if (!C) {
+        c->mesh_off = true;
+        mesh_free(c);
+        return AXBC_OK;
+    }
+    c->mesh_used = C;
     {
         ProfScope ps(c, KP_PERSIST, 0);
         k_mesh_reset<<<(int)std::max<uint64_t>(1, std::min<uint64_t>(axbc_grid_for(c, 256, 8), (words + 255) / 256)),
                        256, 0, s>>>(A);
     }
     CU_LAUNCH("k_mesh_reset");
-    if (C > 8) CU(cudaFuncSetAttribute(k_mesh, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     {
         ProfScope ps(c, KP_PERSIST, 0);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(nsrc * C);
-        cfg.blockDim = dim3(MESH_TPB);
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = C;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        CU(cudaLaunchKernelEx(&cfg, k_mesh, A));
+        MeshLaunch ml(c, nsrc * C, C);
+        CU(cudaLaunchKernelEx(&ml.cfg, k_mesh, A));
     }
     CU_LAUNCH("k_mesh");
     const size_t off = offsetof(BatchInfo, depth0mask), len = offsetof(BatchInfo, push_factor) - off;
@@ -478,6 +526,7 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     const int stop = c->bi_host->gs.need;
     if (stop == 1) {
         c->mesh_off = true;  // for good: nothing reads the vectors again
+        c->mesh_used = 0;
         mesh_free(c);
         return AXBC_OK;
     }

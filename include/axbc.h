@@ -401,9 +401,15 @@ uint64_t axbc_device_bytes_live(void);
 /* The next n one-launch passes are taken for failed on the host, as `kind`
  * says (0 clears it):
  * AXBC_FAIL_WAIT: a grid barrier wait ran out on the backward way, the span
- *   sums of the vertices of more than 1024 neighbours partly counted. */
-enum { AXBC_FAIL_WAIT = 0, AXBC_FAIL_KINDS = 1 };
+ *   sums of the vertices of more than 1024 neighbours partly counted;
+ * AXBC_FAIL_CLUSTER: the device holds no cluster of blocks of the size asked for
+ *   (each size is asked for once in a context). */
+enum { AXBC_FAIL_WAIT = 0, AXBC_FAIL_CLUSTER = 1, AXBC_FAIL_KINDS = 2 };
 void axbc_inject_pass_failures(int kind, int n);
+/* Blocks per pivot of the context's later passes over meshes (1, 2, 4, 8, 16; 0:
+ * by their width, the default); *used (may be NULL): of the last one (0: the
+ * last attempt ran in another form, or none was made). */
+int axbc_ctx_mesh_blocks(axbc_ctx *ctx, int blocks, int *used);
 
 /* Per forward level of the last batch (up to max_levels; *levels = all):
  * vertices newly reached over all pivots, their degree sum, direction (1:

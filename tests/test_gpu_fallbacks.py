@@ -7,7 +7,7 @@ import pytest
 from test_gpu_splits import hub_graph
 
 pytestmark = pytest.mark.gpu
-FAIL_WAIT = 0
+FAIL_WAIT, FAIL_CLUSTER = 0, 1
 
 
 def failing(axbc, kind, n, call):
@@ -92,3 +92,68 @@ def test_vectors_of_a_mesh_pass_go_when_a_level_is_too_wide(axbc, orc, k):
         pass_of(ctx, orc, g, piv, np.full(k, 0.5))
         held.append(ctx.bytes)
     assert held[0] == held[1]
+
+
+def mesh_blocks(axbc, ctx, blocks):
+    """Set the blocks per pivot of later mesh passes; those of the last one."""
+    import ctypes
+    used = ctypes.c_int()
+    assert axbc.lib().axbc_ctx_mesh_blocks(ctx._h, blocks, ctypes.byref(used)) == 0
+    return used.value
+
+
+@pytest.mark.parametrize("refused", [1, 2, 4, 5])
+def test_mesh_pass_on_the_largest_cluster_that_fits(axbc, orc, refused):
+    g = grid(orc, 40)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    piv = np.array([0, 820, 1599], np.uint32)
+    mesh_blocks(axbc, ctx, 16)
+    failing(axbc, FAIL_CLUSTER, refused, lambda: pass_of(ctx, orc, g, piv, np.full(3, 0.5)))
+    assert mesh_blocks(axbc, ctx, 16) == 16 >> refused  # 5: none fits, the batched form
+    pass_of(ctx, orc, g, piv[1:], np.full(2, 0.5))
+    assert mesh_blocks(axbc, ctx, 0) == 16 >> refused
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+@pytest.mark.parametrize("k", [1, 2, 3])
+@pytest.mark.parametrize("blocks", [1, 2, 4, 8, 16])
+def test_mesh_pass_on_clusters_of_each_size(axbc, orc, blocks, k, undirected):
+    # levels around the threads of a block and of every cluster, and the padding
+    # (isolated vertices) that keeps them from being too wide
+    rng = np.random.default_rng(7)
+    width = [1, 2, 31, 500, 1023, 1024, 1025, 2047, 2048, 2049, 4097, 8193, 16385, 16384, 9000, 33, 1, 1]
+    first, n = np.cumsum([0] + width), 280000
+    e = []
+    for i in range(len(width) - 1):
+        child = np.arange(width[i + 1])
+        e += [np.stack([first[i] + parent, first[i + 1] + child], 1)
+              for parent in (child % width[i], rng.integers(0, width[i], width[i + 1]))]
+    e = np.concatenate(e)
+    if not undirected:
+        e = np.concatenate([e[:, ::-1], e[rng.random(len(e)) < 0.1]])
+    g = orc.pipeline(e.astype(np.uint64), n, undirected, 0)
+    G = axbc.Graph.from_csc(g.col, g.row, rng.integers(0, 3, n).astype(np.uint32))
+    g = orc.CSC(g.col, g.row, G.csc()[2])
+    ctx = axbc.Context(G)
+    mesh_blocks(axbc, ctx, blocks)
+    piv = np.array([0, 1, 0][:k], np.uint32)
+    for _ in range(2):
+        pass_of(ctx, orc, g, piv, np.full(k, 0.5))
+        assert mesh_blocks(axbc, ctx, blocks) == blocks
+    for s in range(k):
+        _, lvl, sigma, delta, _ = orc.bc_pivot(g, int(piv[s]), 0.5)
+        gs, gl, gd = ctx.batch_source(s)
+        assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl) and np.array_equal(gd, delta, equal_nan=True)
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 8, 16])
+def test_too_wide_a_level_on_clusters_then_the_batched_form(axbc, orc, blocks):
+    rng = np.random.default_rng(17)
+    n = 60000  # a random graph: levels of tens of thousands of vertices
+    g = orc.pipeline(rng.integers(0, n, size=(3 * n, 2)).astype(np.uint64), n, True, 0)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    mesh_blocks(axbc, ctx, blocks)
+    piv = rng.choice(n, 6, replace=False).astype(np.uint32)
+    for k in (2, 6):
+        pass_of(ctx, orc, g, piv[:k], np.full(k, 0.5))
+        assert mesh_blocks(axbc, ctx, blocks) == 0
