@@ -157,3 +157,25 @@ def test_too_wide_a_level_on_clusters_then_the_batched_form(axbc, orc, blocks):
     for k in (2, 6):
         pass_of(ctx, orc, g, piv[:k], np.full(k, 0.5))
         assert mesh_blocks(axbc, ctx, blocks) == 0
+
+
+@pytest.mark.parametrize("z", [0, 1, 2, 3, 5])
+@pytest.mark.parametrize("n", [7, 8, 9, 15, 16, 17, 22, 23, 31, 32, 33, 50])
+def test_rounds_dropped_after_n_squared_rejections(axbc, orc, n, z):
+    # n^2 rejections drop a round: fewer and more than a window's 64 and 256
+    # draws.  Half the vertices have no neighbour, so that some heuristics run
+    # out of vertices to draw
+    rng = np.random.default_rng(n)
+    half = max(4, n // 2)
+    e = np.concatenate([rng.integers(0, half, size=(2 * n, 2)), [[0, 1], [1, 2], [0, 2]]])
+    g = orc.pipeline(e.astype(np.uint64), n, True, 0)
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    for W in (1, 7, 64):
+        ctx = axbc.Context(G)
+        got = ctx.run_sampled(z=z, nbfs=n, bader_c=0, nchecks=1, seed=n + W, W=W)
+        want = orc.run(g, z=z, nbfs=n, bader_c=0, nchecks=1, seed=n + W, W=W)
+        assert np.array_equal(got["pivots"], want["pivots"])
+        assert np.array_equal(got["probs"], want["probs"], equal_nan=True)
+        for k in ("nrounds", "skipped", "dropped", "ui_end", "te"):
+            assert got[k] == want[k], (W, k)
+        assert np.array_equal(ctx.bc(), want["bc"], equal_nan=True)
