@@ -303,7 +303,7 @@ extern "C" int axbc_ctx_reset(axbc_ctx *c)
     CU(cudaMemsetAsync(c->delta_last, 0, c->g->n * 4, c->stream));
     CU(cudaStreamSynchronize(c->stream));
     c->delta_last_valid = true;
-    c->mesh_short = false;
+    c->mesh_short = c->pivot_short = false;
     c->run_pivots.clear();
     c->run_probs.clear();
     return AXBC_OK;

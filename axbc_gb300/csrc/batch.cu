@@ -2720,12 +2720,13 @@ static int read_back(axbc_ctx *c, int nsrc, int L)
 // would carry one (us a pass, persistent rows : this: scale 14 218 : 115, 18 498 :
 // 318).  Counting runs and a level loop that the caller
 // has chosen keep the batched kernels.
-static int traverse_one(axbc_ctx *c, int H)
+static int traverse_one(axbc_ctx *c, int H, bool *done)
 {
     TRY(ensure_level_tables(c));
     TRY(axbc_batch_settle(c));
     int L = 0;
-    TRY(axbc_one_traverse(c, H, &L));
+    TRY(axbc_one_traverse(c, H, &L, done));
+    if (!*done) return AXBC_OK;
     if (L > AXBC_MAX_LEVELS - 3) {
         axbc_set_error("traversal deeper than %d levels", AXBC_MAX_LEVELS - 2);
         return AXBC_ERR_RANGE;
@@ -2761,7 +2762,11 @@ int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H)
             if (done) return AXBC_OK;
         }
         int rc = AXBC_OK;
-        if (nsrc == 1 && axbc_one_fits(c, &rc)) return traverse_one(c, H);
+        if (nsrc == 1 && axbc_one_fits(c, &rc)) {
+            bool done = false;
+            TRY(traverse_one(c, H, &done));
+            if (done) return AXBC_OK;
+        }
         TRY(rc);
     }
     c->last_form = axbc_ctx::ROWS;

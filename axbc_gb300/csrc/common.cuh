@@ -294,6 +294,7 @@ struct axbc_ctx {
     int mesh_force = 0, mesh_used = 0;       // blocks per pivot: asked for by a test, of the last mesh pass
     bool mesh_short = false;  // no room for them; tried again after a reset of the context
     int pivot_fit = 0;      // blocks of the kernel that fit an SM
+    bool pivot_short = false;  // no room for its own buffers; tried again after a reset of the context
     std::vector<uint64_t> levstart;
     uint64_t s_front_deg = 0, s_prev_newdeg = 0, s_visited_rdeg = 0;  // direction choice
     // multi-source batch state
@@ -425,7 +426,7 @@ int axbc_single_update(axbc_ctx *c, uint32_t v0, double p, const uint32_t *reach
 // a pass of one pivot (the root in c->bi, as a vertex id) into c->one and the
 // totals of c->bi, without the update; its update and last dependencies
 bool axbc_one_fits(axbc_ctx *c, int *rc);
-int axbc_one_traverse(axbc_ctx *c, int H, int *levels);
+int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done);
 int axbc_one_apply(axbc_ctx *c, float *delta_out);
 void axbc_pivot_free(PivotBuf &b);
 // the same for up to 64 pivots on a mesh, into the context's mesh vectors

@@ -1040,12 +1040,12 @@ static int pivot_fit(axbc_ctx *c)
     return AXBC_OK;
 }
 
-// owns: with path counts, levels, dependencies and queue of its own
+// owns: with path counts, levels, dependencies and queue of its own; else those
+// of the level-by-level form, which are there
 static int ensure_pivot(axbc_ctx *c, PivotBuf &b, bool owns)
 {
     if (b.ready) return AXBC_OK;
     const uint64_t n = c->g->n;
-    TRY(pivot_fit(c));
     b.owns = owns;
     if (owns) {
         ALLOC_MISSING(b.lvl, n * 4, &c->bytes);
@@ -1054,7 +1054,6 @@ static int ensure_pivot(axbc_ctx *c, PivotBuf &b, bool owns)
         ALLOC_MISSING(b.delta, n * 4, &c->bytes);
         ALLOC_MISSING(b.partial, (c->g->fwd.n_heavy_items + 1) * 4, &c->bytes);
     } else {
-        TRY(axbc_ensure_single(c));
         b.lvl = c->lvl;
         b.sigma = c->sigma;
         b.queue = c->queue;
@@ -1069,6 +1068,16 @@ static int ensure_pivot(axbc_ctx *c, PivotBuf &b, bool owns)
     CU(cudaMemsetAsync(b.arrive, 0, (c->g->fwd.n_heavy + 1) * 4, c->stream));
     b.ready = true;
     return AXBC_OK;
+}
+
+// The same, but *room = false (and no further tries) when only the one launch's
+// buffers find no room: the caller has a form that does without them.
+static int pivot_room(axbc_ctx *c, PivotBuf &b, bool owns, bool *room)
+{
+    const int rc = !b.ready && c->pivot_short ? AXBC_ERR_NOMEM : ensure_pivot(c, b, owns);
+    *room = rc == AXBC_OK;
+    if (rc == AXBC_ERR_NOMEM) c->pivot_short = true;
+    return rc == AXBC_ERR_NOMEM ? AXBC_OK : rc;
 }
 
 // One launch of k_pivot and the wait for it; its control block in b.ctl_host.
@@ -1131,9 +1140,11 @@ bool axbc_one_fits(axbc_ctx *c, int *rc)
     return *rc == AXBC_OK && c->pivot_fit > 0;
 }
 
-int axbc_one_traverse(axbc_ctx *c, int H, int *levels)
+// *done = false: no room for its buffers, nothing has run
+int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done)
 {
-    TRY(ensure_pivot(c, c->one, true));
+    TRY(pivot_room(c, c->one, true, done));
+    if (!*done) return AXBC_OK;
     PivotRun R;
     R.v0 = 0;
     R.p = 1.0;
@@ -1189,8 +1200,11 @@ extern "C" int axbc_run_pivot(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pi
     CHECK_ARG(H == 0 || H == 1, "axbc_run_pivot: H must be 0 or 1");
     // one launch, unless every kernel is to be timed
     if (!c->prof_on) {
-        TRY(ensure_pivot(c, c->piv, false));
-        if (c->pivot_fit > 0) return run_pivot_once(c, v0, p, H, st);
+        bool room = false;
+        TRY(pivot_fit(c));
+        TRY(axbc_ensure_single(c));
+        TRY(pivot_room(c, c->piv, false, &room));
+        if (room && c->pivot_fit > 0) return run_pivot_once(c, v0, p, H, st);
     }
     TRY(axbc_single_reset(c));
     TRY(axbc_single_set_root(c, v0, 0, 1));

@@ -179,3 +179,41 @@ def test_rounds_dropped_after_n_squared_rejections(axbc, orc, n, z):
         for k in ("nrounds", "skipped", "dropped", "ui_end", "te"):
             assert got[k] == want[k], (W, k)
         assert np.array_equal(ctx.bc(), want["bc"], equal_nan=True)
+
+
+@pytest.mark.parametrize("skip", range(4))
+def test_plain_pivot_without_room_for_its_one_launch(axbc, orc, skip):
+    # the level-by-level form's buffers are there; the four beside them are not
+    g = hub_graph(orc, True)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    ctx.profile(True)
+    ctx.run_pivot(1, 0.5)
+    ctx.profile(False)
+    piv = np.flatnonzero(g.deg > 0)[::400].astype(np.uint32)
+    for v in (int(x) for x in piv):
+        ctx.reset()
+        axbc.lib().axbc_inject_alloc_failure_after(skip)
+        try:
+            st = ctx.run_pivot(v, 0.5, 1)
+        finally:
+            axbc.lib().axbc_inject_alloc_failure_after(-1)
+        want, lvl, sigma, delta, stats = orc.bc_pivot(g, v, 0.5, 1)
+        assert np.array_equal(ctx.bc(), want) and np.array_equal(ctx.delta(), delta) and st == stats
+        assert np.array_equal(ctx.levels(), lvl) and np.array_equal(ctx.sigma(), sigma)
+
+
+@pytest.mark.parametrize("skip", range(9))
+def test_pass_of_one_pivot_without_room_for_its_one_launch(axbc, orc, skip):
+    g = hub_graph(orc, True)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    piv = np.flatnonzero(g.deg > 0)[::400].astype(np.uint32)
+    pass_of(ctx, orc, g, piv[:5], np.full(5, 0.5))
+    axbc.lib().axbc_inject_alloc_failure_after(skip)
+    try:
+        pass_of(ctx, orc, g, piv[5:6], np.full(1, 0.5))
+    finally:
+        axbc.lib().axbc_inject_alloc_failure_after(-1)
+    _, lvl, sigma, delta, _ = orc.bc_pivot(g, int(piv[5]), 0.5)
+    gs, gl, gd = ctx.batch_source(0)
+    assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl) and np.array_equal(gd, delta)
+    pass_of(ctx, orc, g, piv[6:7], np.full(1, 0.5))
