@@ -45,6 +45,25 @@ bool axbc_pass_fails(int kind)
     return false;
 }
 
+int axbc_coop_launch(axbc_ctx *c, const void *kernel, int blocks, int threads, void **args, bool *done)
+{
+    *done = false;
+    if (!c->coop) return AXBC_OK;
+    cudaError_t e = axbc_pass_fails(AXBC_FAIL_COOP) ? cudaErrorCooperativeLaunchTooLarge : cudaSuccess;
+    if (e == cudaSuccess) {
+        ProfScope ps(c, KP_PERSIST, 0);
+        e = cudaLaunchCooperativeKernel(kernel, blocks, threads, args, 0, c->stream);
+    }
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported || e == cudaErrorLaunchOutOfResources) {
+        (void)cudaGetLastError();
+        c->coop = 0;
+        return AXBC_OK;
+    }
+    if (e != cudaSuccess) return axbc_cuda_fail(e, "cooperative launch", __FILE__, __LINE__);
+    *done = true;
+    return AXBC_OK;
+}
+
 int axbc_wait_ran_out(axbc_ctx *c, int err, uint32_t *arrive, uint64_t n, int *site)
 {
     *site = err;
@@ -217,6 +236,7 @@ extern "C" int axbc_ctx_create(axbc_graph *g, void *stream, axbc_ctx **out)
     int dev = 0;
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev));
+    CU(cudaDeviceGetAttribute(&c->coop, cudaDevAttrCooperativeLaunch, dev));
     if (stream) {
         c->stream = (cudaStream_t)stream;
     } else {

@@ -2551,6 +2551,7 @@ static bool use_persist(axbc_ctx *c, int nsrc)
 {
     if (c->count_on || c->persist_mode < 0) return false;
     if (c->persist_mode > 0) return true;
+    if (!c->coop) return false;
     if (c->g->m < AXBC_PERSIST_AUTO_M) return true;
     if (nsrc > AXBC_PERSIST_AUTO_WIDTH) return false;
     if (c->last_batch_levels > AXBC_PERSIST_AUTO_LEVELS) return true;
@@ -2560,14 +2561,17 @@ static bool use_persist(axbc_ctx *c, int nsrc)
 // The batch's levels in k_traverse_persist: a cooperative launch of every
 // block that fits resident (at most persist_blocks_per_sm per SM).  Level masks
 // are allocated up front for the last batch's depth and grown when the loop
-// asks for more.  *L_out: the first level that discovered nothing.
-template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
+// asks for more.  *L_out: the first level that discovered nothing.  *done =
+// false: the device refuses the launch, nothing has run.
+template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out, bool *done)
 {
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
     int &fit = c->persist_fit[K - 1];
     if (!fit) CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_traverse_persist<K>, BATCH_TPB, 0));
     const int bps = std::min(fit, std::max(1, c->persist_blocks_per_sm));
+    *done = false;
+    if (bps < 1 && c->persist_mode == 0) return AXBC_OK;
     if (bps < 1) {
         axbc_set_error("persistent level loop: no block of it fits on an SM");
         return AXBC_ERR_CUDA;
@@ -2596,9 +2600,11 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out)
                         (void *)&ll, (void *)&g->symmetric, (void *)&c->d_level_te, (void *)&c->d_level_cnt, (void *)&c->d_level_mode,
                         (void *)&pool_cap, (void *)&lmax_list, (void *)&n, (void *)&lmax,
                         (void *)&gs, (void *)&budget};
-        {
-            ProfScope ps(c, KP_PERSIST, 0);
-            CU(cudaLaunchCooperativeKernel((const void *)k_traverse_persist<K>, grid, BATCH_TPB, args, 0, s));
+        TRY(axbc_coop_launch(c, (const void *)k_traverse_persist<K>, grid, BATCH_TPB, args, done));
+        if (!*done && first && c->persist_mode == 0) return AXBC_OK;
+        if (!*done) {
+            axbc_set_error("persistent level loop: the device refuses the cooperative launch");
+            return AXBC_ERR_CUDA;
         }
         CU_LAUNCH("k_traverse_persist");
         // the level state and the barrier's record in one copy
@@ -2694,8 +2700,9 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
     c->prev_lend = 0;
 
     int L = 0;
-    if (use_persist(c, nsrc)) TRY(traverse_persistent<K>(c, &L));
-    else TRY(traverse_stepwise<K>(c, nsrc, &L));
+    bool done = false;
+    if (use_persist(c, nsrc)) TRY(traverse_persistent<K>(c, &L, &done));
+    if (!done) TRY(traverse_stepwise<K>(c, nsrc, &L));
     TRY(read_back(c, nsrc, L));
     c->prev_lend = L;
     return AXBC_OK;

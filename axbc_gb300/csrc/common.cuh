@@ -358,6 +358,7 @@ struct axbc_ctx {
     int persist_mode = 0;
     int persist_blocks_per_sm = 4;
     int persist_fit[2] = {0, 0};       // blocks of it that fit an SM, per width
+    int coop = 0;                      // 1: the device takes cooperative launches
     std::vector<cudaEvent_t> ev_pool;
     double level_te_prev = 0;  // degree sum of the previous level's new vertices
     std::vector<double> level_te;
@@ -382,6 +383,10 @@ int axbc_kron_device(int scale, int edgefactor, uint64_t seed1, uint64_t seed2, 
 
 // host-side failure of a one-launch pass (axbc_inject_pass_failures)
 bool axbc_pass_fails(int kind);
+// A cooperative launch on the context's stream.  *done = false: the device has
+// none, or refuses this one (more blocks than it holds, SMs taken away from this
+// process); nothing has run, and the context asks for no other.
+int axbc_coop_launch(axbc_ctx *c, const void *kernel, int blocks, int threads, void **args, bool *done);
 // *site: the barrier of the pass just waited for whose wait ran out (0: none).
 // Every block then left wherever it was, so the n arrival counts of the heavy
 // vertices may be on the way; they go back to zero, where the next pass takes

@@ -1080,8 +1080,9 @@ static int pivot_room(axbc_ctx *c, PivotBuf &b, bool owns, bool *room)
     return rc == AXBC_ERR_NOMEM ? AXBC_OK : rc;
 }
 
-// One launch of k_pivot and the wait for it; its control block in b.ctl_host.
-static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R)
+// One launch of k_pivot; its control block on the way to b.ctl_host.  *done =
+// false: the device refuses it.
+static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R, bool *done)
 {
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
@@ -1113,10 +1114,8 @@ static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R)
                               (work + PIVOT_NW - 1) / PIVOT_NW));
     CU(cudaMemsetAsync(b.ctl, 0, sizeof(GridSync), s));
     void *args[] = {(void *)&g->fwd, (void *)&g->rev, (void *)&R, (void *)&budget};
-    {
-        ProfScope ps(c, KP_PERSIST, 0);
-        CU(cudaLaunchCooperativeKernel((const void *)k_pivot, grid, PIVOT_TPB, args, 0, s));
-    }
+    TRY(axbc_coop_launch(c, (const void *)k_pivot, grid, PIVOT_TPB, args, done));
+    if (!*done) return AXBC_OK;
     CU_LAUNCH("k_pivot");
     CU(cudaMemcpyAsync(b.ctl_host, b.ctl, sizeof(PivotCtl), cudaMemcpyDeviceToHost, s));
     return AXBC_OK;
@@ -1137,10 +1136,10 @@ static int pivot_wait(axbc_ctx *c, PivotBuf &b)
 bool axbc_one_fits(axbc_ctx *c, int *rc)
 {
     *rc = pivot_fit(c);
-    return *rc == AXBC_OK && c->pivot_fit > 0;
+    return *rc == AXBC_OK && c->coop && c->pivot_fit > 0;
 }
 
-// *done = false: no room for its buffers, nothing has run
+// *done = false: no room for its buffers or no cooperative launch, nothing has run
 int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done)
 {
     TRY(pivot_room(c, c->one, true, done));
@@ -1153,7 +1152,8 @@ int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done)
     R.level_te = c->d_level_te;
     R.level_cnt = c->d_level_cnt;
     R.level_mode = c->d_level_mode;
-    TRY(pivot_launch(c, c->one, R));
+    TRY(pivot_launch(c, c->one, R, done));
+    if (!*done) return AXBC_OK;
     TRY(pivot_wait(c, c->one));
     *levels = c->one.ctl_host->levels;
     return AXBC_OK;
@@ -1168,7 +1168,7 @@ int axbc_one_apply(axbc_ctx *c, float *delta_out)
     return AXBC_OK;
 }
 
-static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_stats *st)
+static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_stats *st, bool *done)
 {
     PivotRun R;
     R.v0 = v0;
@@ -1177,7 +1177,8 @@ static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_
     R.bi = nullptr;
     R.level_te = R.level_cnt = nullptr;
     R.level_mode = nullptr;
-    TRY(pivot_launch(c, c->piv, R));
+    TRY(pivot_launch(c, c->piv, R, done));
+    if (!*done) return AXBC_OK;
     c->delta_last_valid = false;  // the last pivot's delta is c->delta
     CU(cudaMemcpyAsync(&c->pc_host->pad, c->g->reach + v0, 4, cudaMemcpyDeviceToHost, c->stream));
     TRY(pivot_wait(c, c->piv));
@@ -1198,13 +1199,14 @@ extern "C" int axbc_run_pivot(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pi
     axbc_graph *g = c->g;
     CHECK_ARG(v0 < g->n, "axbc_run_pivot: v0 >= n");
     CHECK_ARG(H == 0 || H == 1, "axbc_run_pivot: H must be 0 or 1");
-    // one launch, unless every kernel is to be timed
-    if (!c->prof_on) {
-        bool room = false;
-        TRY(pivot_fit(c));
+    // one launch, unless every kernel is to be timed or the caller wants none
+    TRY(pivot_fit(c));
+    if (!c->prof_on && c->persist_mode >= 0 && c->coop && c->pivot_fit > 0) {
+        bool done = false;
         TRY(axbc_ensure_single(c));
-        TRY(pivot_room(c, c->piv, false, &room));
-        if (room && c->pivot_fit > 0) return run_pivot_once(c, v0, p, H, st);
+        TRY(pivot_room(c, c->piv, false, &done));
+        if (done) TRY(run_pivot_once(c, v0, p, H, st, &done));
+        if (done) return AXBC_OK;
     }
     TRY(axbc_single_reset(c));
     TRY(axbc_single_set_root(c, v0, 0, 1));

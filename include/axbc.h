@@ -403,8 +403,9 @@ uint64_t axbc_device_bytes_live(void);
  * AXBC_FAIL_WAIT: a grid barrier wait ran out on the backward way, the span
  *   sums of the vertices of more than 1024 neighbours partly counted;
  * AXBC_FAIL_CLUSTER: the device holds no cluster of blocks of the size asked for
- *   (each size is asked for once in a context). */
-enum { AXBC_FAIL_WAIT = 0, AXBC_FAIL_CLUSTER = 1, AXBC_FAIL_KINDS = 2 };
+ *   (each size is asked for once in a context);
+ * AXBC_FAIL_COOP: the device refuses a cooperative launch. */
+enum { AXBC_FAIL_WAIT = 0, AXBC_FAIL_CLUSTER = 1, AXBC_FAIL_COOP = 2, AXBC_FAIL_KINDS = 3 };
 void axbc_inject_pass_failures(int kind, int n);
 /* Blocks per pivot of the context's later passes over meshes (1, 2, 4, 8, 16; 0:
  * by their width, the default); *used (may be NULL): of the last one (0: the

@@ -7,7 +7,7 @@ import pytest
 from test_gpu_splits import hub_graph
 
 pytestmark = pytest.mark.gpu
-FAIL_WAIT, FAIL_CLUSTER = 0, 1
+FAIL_WAIT, FAIL_CLUSTER, FAIL_COOP = 0, 1, 2
 
 
 def failing(axbc, kind, n, call):
@@ -217,3 +217,54 @@ def test_pass_of_one_pivot_without_room_for_its_one_launch(axbc, orc, skip):
     gs, gl, gd = ctx.batch_source(0)
     assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl) and np.array_equal(gd, delta)
     pass_of(ctx, orc, g, piv[6:7], np.full(1, 0.5))
+
+
+def pivot_of(ctx, orc, g, v, H=1):
+    """A plain pivot's bc, vectors and statistics against the oracle's."""
+    ctx.reset()
+    st = ctx.run_pivot(v, 0.5, H)
+    want, lvl, sigma, delta, stats = orc.bc_pivot(g, v, 0.5, H)
+    assert np.array_equal(ctx.bc(), want) and np.array_equal(ctx.delta(), delta) and st == stats
+    assert np.array_equal(ctx.levels(), lvl) and np.array_equal(ctx.sigma(), sigma)
+
+
+def plain_launches(ctx, v):
+    before = ctx.launches
+    ctx.run_pivot(v, 0.5)
+    return ctx.launches - before
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+def test_plain_pivot_without_a_cooperative_launch(axbc, orc, undirected):
+    g = hub_graph(orc, undirected)
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    v = int(np.flatnonzero(g.deg > 0)[700])
+    ctx = axbc.Context(G)
+    assert plain_launches(ctx, v) == 1
+    failing(axbc, FAIL_COOP, 1, lambda: pivot_of(ctx, orc, g, v))
+    assert plain_launches(ctx, v) > 5  # not asked for again
+    pivot_of(ctx, orc, g, v)
+    ctx = axbc.Context(G)
+    ctx.set_persistent(-1)  # the caller wants none
+    pivot_of(ctx, orc, g, v)
+    assert plain_launches(ctx, v) > 5
+    ctx.set_persistent(0)
+    pivot_of(ctx, orc, g, v)
+    assert plain_launches(ctx, v) == 1
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+@pytest.mark.parametrize("k", [1, 31, 64])
+def test_passes_without_a_cooperative_launch(axbc, orc, k, undirected):
+    g = hub_graph(orc, undirected)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    piv = np.random.default_rng(k).permutation(np.flatnonzero(g.deg > 0)).astype(np.uint32)
+    p = np.full(k, 1.0 / g.n)
+    failing(axbc, FAIL_COOP, 1, lambda: pass_of(ctx, orc, g, piv[:k], p))
+    pass_of(ctx, orc, g, piv[k:2 * k], p)
+    ctx.set_persistent(1)  # asked for by name: an error, as before
+    with pytest.raises(axbc.AxbcError) as ex:
+        ctx.run_batch(piv[:k], p)
+    assert ex.value.status == 2
+    ctx.set_persistent(0)
+    pass_of(ctx, orc, g, piv[:k], p)
