@@ -2562,7 +2562,8 @@ static bool use_persist(axbc_ctx *c, int nsrc)
 // block that fits resident (at most persist_blocks_per_sm per SM).  Level masks
 // are allocated up front for the last batch's depth and grown when the loop
 // asks for more.  *L_out: the first level that discovered nothing.  *done =
-// false: the device refuses the launch, nothing has run.
+// false: the device refuses the launch or a barrier wait ran out, the pass has
+// to start again in another form.
 template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out, bool *done)
 {
     axbc_graph *g = c->g;
@@ -2612,6 +2613,8 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out, bool *d
         CU(cudaStreamSynchronize(s));
         int site = 0;
         TRY(axbc_wait_ran_out(c, hs.err, c->harrive, (uint64_t)(g->bfwd.n_heavy + 1) * 2, &site));
+        *done = site == 0;
+        if (site && c->persist_mode == 0) return AXBC_OK;
         if (site) {
             axbc_set_error("persistent level loop: a grid barrier wait ran out of its budget (site %d)", site);
             return AXBC_ERR_TIMEOUT;
@@ -2628,6 +2631,48 @@ template <int K> static int traverse_persistent(axbc_ctx *c, int *L_out, bool *d
 }
 
 static int read_back(axbc_ctx *c, int nsrc, int L);
+
+// What a pass finds zero, and its roots (c->bi holds them as vertex ids, or in
+// the view's numbering when a start before this one has renumbered them).
+template <int K> static int start_pass(axbc_ctx *c, int nsrc, int H, bool in_view)
+{
+    axbc_graph *g = c->g;
+    const uint64_t n = g->n;
+    PassStart P;
+    P.bi = c->bi;
+    P.tab = c->fmtab;
+    P.seen = c->seen;
+    P.msigma = c->msigma;
+    P.ctrs = c->ctrs;
+    P.ll = lists_of(c);
+    P.level_te = c->d_level_te;
+    P.level_cnt = c->d_level_cnt;
+    P.col = g->bfwd.col;
+    P.rcol = g->brev.col;
+    P.reach = g->breach;
+    P.to_view = in_view ? nullptr : g->to_view;
+    P.bc = c->bc;
+    P.n = n;
+    P.m = g->m;
+    // a factor of 1e30 or more pulls every level
+    P.push_min = c->push_factor_batch >= 1e30 ? 0ull : (unsigned long long)(n / 4);
+    P.push_factor = c->push_factor_batch;
+    P.pool_cap = c->lpool_cap;
+    P.list_max = list_max_of(c);
+    P.big = g->bfwd.big;
+    P.nsrc = nsrc;
+    P.H = H;
+    P.prev_k = c->last_batch_k;
+    P.prev_last = c->prev_lend;
+    {
+        ProfScope ps(c, KP_LEVEL_STATS, 0);
+        k_pass_start<K><<<grid_of(c, 8, (n * K + 31) / 32), 256, 0, c->stream>>>(P);
+    }
+    CU_LAUNCH("k_pass_start");
+    c->last_batch_k = K;
+    c->prev_lend = 0;
+    return AXBC_OK;
+}
 
 // Forward and backward passes of the batch of width K whose roots/p are in
 // c->bi.  The host launches forward level steps in blocks (8, then doubling)
@@ -2665,43 +2710,14 @@ template <int K> static int batch_traverse(axbc_ctx *c, int nsrc, int H)
         drop_captures(c);
         if (!prof) TRY(capture_steps<K>(c));
     }
-    PassStart P;
-    P.bi = c->bi;
-    P.tab = c->fmtab;
-    P.seen = c->seen;
-    P.msigma = c->msigma;
-    P.ctrs = c->ctrs;
-    P.ll = lists_of(c);
-    P.level_te = c->d_level_te;
-    P.level_cnt = c->d_level_cnt;
-    P.col = g->bfwd.col;
-    P.rcol = g->brev.col;
-    P.reach = g->breach;
-    P.to_view = g->to_view;
-    P.bc = c->bc;
-    P.n = n;
-    P.m = g->m;
-    // a factor of 1e30 or more pulls every level
-    P.push_min = c->push_factor_batch >= 1e30 ? 0ull : (unsigned long long)(n / 4);
-    P.push_factor = c->push_factor_batch;
-    P.pool_cap = c->lpool_cap;
-    P.list_max = list_max_of(c);
-    P.big = g->bfwd.big;
-    P.nsrc = nsrc;
-    P.H = H;
-    P.prev_k = c->last_batch_k;
-    P.prev_last = c->prev_lend;
-    {
-        ProfScope ps(c, KP_LEVEL_STATS, 0);
-        k_pass_start<K><<<grid_of(c, 8, (n * K + 31) / 32), 256, 0, s>>>(P);
-    }
-    CU_LAUNCH("k_pass_start");
-    c->last_batch_k = K;
-    c->prev_lend = 0;
+    TRY(start_pass<K>(c, nsrc, H, false));
 
     int L = 0;
     bool done = false;
-    if (use_persist(c, nsrc)) TRY(traverse_persistent<K>(c, &L, &done));
+    if (use_persist(c, nsrc)) {
+        TRY(traverse_persistent<K>(c, &L, &done));
+        if (!done) TRY(start_pass<K>(c, nsrc, H, true));
+    }
     if (!done) TRY(traverse_stepwise<K>(c, nsrc, &L));
     TRY(read_back(c, nsrc, L));
     c->prev_lend = L;

@@ -1121,16 +1121,11 @@ static int pivot_launch(axbc_ctx *c, PivotBuf &b, PivotRun &R, bool *done)
     return AXBC_OK;
 }
 
-static int pivot_wait(axbc_ctx *c, PivotBuf &b)
+// *site: the barrier whose wait ran out, or 0
+static int pivot_wait(axbc_ctx *c, PivotBuf &b, int *site)
 {
     CU(cudaStreamSynchronize(c->stream));
-    int site = 0;
-    TRY(axbc_wait_ran_out(c, b.ctl_host->gs.err, b.arrive, c->g->fwd.n_heavy + 1, &site));
-    if (site) {
-        axbc_set_error("pivot in one launch: a grid barrier wait ran out of its budget (site %d)", site);
-        return AXBC_ERR_TIMEOUT;
-    }
-    return AXBC_OK;
+    return axbc_wait_ran_out(c, b.ctl_host->gs.err, b.arrive, c->g->fwd.n_heavy + 1, site);
 }
 
 bool axbc_one_fits(axbc_ctx *c, int *rc)
@@ -1139,7 +1134,8 @@ bool axbc_one_fits(axbc_ctx *c, int *rc)
     return *rc == AXBC_OK && c->coop && c->pivot_fit > 0;
 }
 
-// *done = false: no room for its buffers or no cooperative launch, nothing has run
+// *done = false: no room for its buffers, no cooperative launch, or a barrier
+// wait that ran out; the root in c->bi is as it was
 int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done)
 {
     TRY(pivot_room(c, c->one, true, done));
@@ -1154,7 +1150,9 @@ int axbc_one_traverse(axbc_ctx *c, int H, int *levels, bool *done)
     R.level_mode = c->d_level_mode;
     TRY(pivot_launch(c, c->one, R, done));
     if (!*done) return AXBC_OK;
-    TRY(pivot_wait(c, c->one));
+    int site = 0;
+    TRY(pivot_wait(c, c->one, &site));
+    *done = site == 0;
     *levels = c->one.ctl_host->levels;
     return AXBC_OK;
 }
@@ -1168,8 +1166,11 @@ int axbc_one_apply(axbc_ctx *c, float *delta_out)
     return AXBC_OK;
 }
 
+// *done = false: bc is as it was, the level-by-level form has to run
 static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_stats *st, bool *done)
 {
+    *done = false;
+    if (axbc_pass_fails(AXBC_FAIL_WAIT)) return AXBC_OK;
     PivotRun R;
     R.v0 = v0;
     R.p = p;
@@ -1181,7 +1182,15 @@ static int run_pivot_once(axbc_ctx *c, uint32_t v0, double p, int H, axbc_pivot_
     if (!*done) return AXBC_OK;
     c->delta_last_valid = false;  // the last pivot's delta is c->delta
     CU(cudaMemcpyAsync(&c->pc_host->pad, c->g->reach + v0, 4, cudaMemcpyDeviceToHost, c->stream));
-    TRY(pivot_wait(c, c->piv));
+    int site = 0;
+    TRY(pivot_wait(c, c->piv, &site));
+    // a block waited in vain at the last barrier: others may have gone on to bc
+    if (site == 4) {
+        axbc_set_error("pivot in one launch: the wait before the bc update ran out of its budget");
+        return AXBC_ERR_TIMEOUT;
+    }
+    *done = site == 0;
+    if (!*done) return AXBC_OK;
     const PivotCtl &h = *c->piv.ctl_host;
     if (st) {
         st->nvisited = h.qtail;

@@ -166,8 +166,13 @@ int axbc_autotune(axbc_ctx *ctx, const uint32_t *pivots, int npivots, int H, axb
  * uint32 path counts, backward float dependencies, bc update, exactly as
  * setcuda + bc_func_mono + update_bc_cuda (src/cuda_kernels.cu:1532-1554,
  * src/axbc2d.c:1514-1659, src/cuda_kernels.cu:289-302).  H == 1 adds the
- * reach sum of pre_update_bc_cuda (src/cuda_kernels.cu:358-373).  The host
- * drives one launch sequence per BFS level. */
+ * reach sum of pre_update_bc_cuda (src/cuda_kernels.cu:358-373).  The pass is
+ * one cooperative launch with a bounded grid barrier between its phases.  Where
+ * the device takes none, its buffers find no room, a barrier wait runs out of its
+ * budget (about 4 s) or axbc_ctx_set_persistent says never, the host drives one
+ * launch sequence per BFS level, as under profiling; the results are the same
+ * bits.  AXBC_ERR_TIMEOUT: the wait before the bc update ran out, bc may hold a
+ * part of it. */
 typedef struct {
     uint64_t nvisited;  /* vertices reached, root included */
     uint64_t all;       /* reach total added in the root term */
@@ -366,9 +371,11 @@ int axbc_ctx_launches(const axbc_ctx *ctx, uint64_t *launches);
  * levels) run in forms of their own, also one launch each.
  * blocks_per_sm: blocks of the cooperative grid per SM (0 keeps the current
  * setting, default 4).  Results
- * are the same bits either way.  A barrier wait that runs out of its budget
- * (about 4 s) ends the pass with AXBC_ERR_TIMEOUT.  No counterpart in the
- * reference (its host synchronises every level). */
+ * are the same bits either way.  A pass whose one launch the device refuses, or
+ * in which a barrier wait runs out of its budget (about 4 s), starts again as step
+ * launches; with mode 1 it ends with AXBC_ERR_CUDA or AXBC_ERR_TIMEOUT.  Mode -1
+ * holds for axbc_run_pivot too.  No counterpart in the reference (its host
+ * synchronises every level). */
 int axbc_ctx_set_persistent(axbc_ctx *ctx, int mode, int blocks_per_sm);
 /* Self-test of that grid barrier on the current device: `rounds` barriers
  * over blocks_per_sm blocks per SM; block absent_block (>= 0) never arrives,
@@ -401,7 +408,8 @@ uint64_t axbc_device_bytes_live(void);
 /* The next n one-launch passes are taken for failed on the host, as `kind`
  * says (0 clears it):
  * AXBC_FAIL_WAIT: a grid barrier wait ran out on the backward way, the span
- *   sums of the vertices of more than 1024 neighbours partly counted;
+ *   sums of the vertices of more than 1024 neighbours partly counted (a plain
+ *   pivot's launch is left out);
  * AXBC_FAIL_CLUSTER: the device holds no cluster of blocks of the size asked for
  *   (each size is asked for once in a context);
  * AXBC_FAIL_COOP: the device refuses a cooperative launch. */

@@ -268,3 +268,60 @@ def test_passes_without_a_cooperative_launch(axbc, orc, k, undirected):
     assert ex.value.status == 2
     ctx.set_persistent(0)
     pass_of(ctx, orc, g, piv[:k], p)
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+def test_plain_pivot_after_a_wait_that_ran_out(axbc, orc, undirected):
+    g = hub_graph(orc, undirected)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    v = np.flatnonzero(g.deg > 0)
+    failing(axbc, FAIL_WAIT, 1, lambda: pivot_of(ctx, orc, g, int(v[9])))
+    pivot_of(ctx, orc, g, int(v[-1]))
+    assert plain_launches(ctx, int(v[9])) == 1
+
+
+@pytest.mark.parametrize("undirected", [True, False])
+@pytest.mark.parametrize("H", [0, 1])
+@pytest.mark.parametrize("k,fails", [(1, 1), (1, 2), (31, 1), (64, 1)])
+def test_passes_start_again_after_a_wait_that_ran_out(axbc, orc, k, fails, H, undirected):
+    # the roots have their numbers of the view already; with one pivot the plain
+    # form's launch fails first, then the persistent loop's
+    g = hub_graph(orc, undirected)
+    reach = np.random.default_rng(2).integers(0, 3, g.n).astype(np.uint32)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, reach))
+    g = orc.CSC(g.col, g.row, reach)
+    piv = np.random.default_rng(k).permutation(np.flatnonzero(g.deg > 0)).astype(np.uint32)
+    p = np.full(k, 1.0 / g.n)
+    for i in range(3):  # the failing pass first, between others and after itself
+        q = piv[k * i:k * i + k]
+        ctx.reset()
+        stats = failing(axbc, FAIL_WAIT, fails if i < 2 else 0, lambda: ctx.run_batch(q, p, H))
+        want, delta_last, _ = orc.bc_pivots(g, q, p, H)
+        assert np.array_equal(ctx.bc(), want) and np.array_equal(ctx.delta(), delta_last)
+        for s in (0, k - 1):
+            _, lvl, sigma, delta, st = orc.bc_pivot(g, int(q[s]), p[s], H)
+            gs, gl, gd = ctx.batch_source(s)
+            assert stats[s] == st
+            assert np.array_equal(gs, sigma) and np.array_equal(gl, lvl) and np.array_equal(gd, delta)
+
+
+def test_sampled_runs_and_requests_go_on_after_waits_that_ran_out(axbc, orc):
+    e = axbc.kron_edges(10, 16).astype(np.uint64)
+    g = orc.pipeline(e, 1024, True, 0)
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    for z, W, c in ((0, 32, 0), (3, 1, 0), (2, 64, 1)):
+        prm = dict(z=z, nbfs=48, bader_c=c, nchecks=4, seed=3, W=W)
+        want = orc.run(g, **prm)
+        ctx = axbc.Context(G)
+        got = failing(axbc, FAIL_WAIT, 3, lambda: ctx.run_sampled(**prm))
+        assert np.array_equal(got["pivots"], want["pivots"]) and got["te"] == want["te"]
+        assert np.array_equal(ctx.bc(), want["bc"], equal_nan=True)
+        srv = axbc.Server()
+        gid = srv.add_graph(G)
+
+        def serve():
+            rid = srv.submit(gid, **prm)
+            assert srv.wait(rid, timeout_ms=60000)["state"] == "done"
+            return srv.result(rid, G.n)[0]
+        assert np.array_equal(failing(axbc, FAIL_WAIT, 3, serve), want["bc"], equal_nan=True)
+        srv.close()
