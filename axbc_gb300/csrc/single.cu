@@ -889,15 +889,18 @@ struct PivotLead {
         const uint32_t from = vload_u(&R.lev[L]);
         const bool alive = tail != from;
         R.lev[L + 1] = tail;
-        if (R.bi && L < AXBC_MAX_LEVELS) {
+        if (R.bi) {
             R.level_te[L] = nd - __ldcg(&c->prev_newdeg);
             R.level_cnt[L] = tail - from;
             R.level_mode[L] = vload_i(&c->push);
         }
         c->push = (double)(nd - __ldcg(&c->prev_newdeg)) * R.push_factor < (double)unvis;
         c->prev_newdeg = nd;
-        c->alive = alive;
-        if (!alive) c->levels = L;
+        // a pass whose last level would have no room in the level tables ends
+        // here: refused, as in the other forms
+        const bool deep = R.bi && alive && L == AXBC_MAX_LEVELS - 3;
+        c->alive = alive && !deep;
+        if (!alive || deep) c->levels = deep ? L + 1 : L;
     }
 };
 
@@ -949,6 +952,7 @@ __global__ void __launch_bounds__(PIVOT_TPB, PIVOT_BPS) k_pivot(Adj a, Adj rv, P
         if (!grid_barrier(&ctl->gs, budget, 2, epoch, lead)) return;
         if (!vload_i(&ctl->alive)) break;
     }
+    if (R.bi && vload_i(&ctl->levels) != L) return;  // too deep
     // backward: the deepest vertices have delta = reach; then depths L-2 .. 1,
     // and 0 when the BFS ended at level 2
     if (L >= 2) {

@@ -325,3 +325,41 @@ def test_sampled_runs_and_requests_go_on_after_waits_that_ran_out(axbc, orc):
             return srv.result(rid, G.n)[0]
         assert np.array_equal(failing(axbc, FAIL_WAIT, 3, serve), want["bc"], equal_nan=True)
         srv.close()
+
+
+def long_path(orc, n, hub=70):
+    """A path of n vertices, with leaves that make its second one a hub."""
+    c = np.arange(n)
+    e = np.concatenate([np.stack([c[:-1], c[1:]], 1), np.stack([np.ones(hub, int), n + np.arange(hub)], 1)])
+    return orc.pipeline(e.astype(np.uint64), n + hub, True, 0)
+
+
+def test_deepest_pass_of_one_pivot(axbc, orc):
+    for n, fits in ((65533, True), (65534, False)):
+        g = long_path(orc, n)
+        ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+        one, p = np.zeros(1, np.uint32), np.full(1, 0.5)
+        if fits:
+            pass_of(ctx, orc, g, one, p)
+        else:
+            with pytest.raises(axbc.AxbcError) as ex:
+                ctx.run_batch(one, p)
+            assert ex.value.status == 5
+        pass_of(ctx, orc, g, np.full(1, n // 2, np.uint32), p)
+
+
+def test_too_deep_a_pass_is_refused_at_the_limit(axbc, orc):
+    # and not at the end of a traversal twenty times as deep
+    import time
+    took = []
+    for n in (70000, 1400000):
+        g = long_path(orc, n)
+        ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+        for _ in range(2):
+            t = time.perf_counter()
+            with pytest.raises(axbc.AxbcError) as ex:
+                ctx.run_batch(np.zeros(1, np.uint32), np.full(1, 0.5))
+            t = time.perf_counter() - t
+            assert ex.value.status == 5
+        took.append(t)
+    assert took[1] < 5 * took[0], took
