@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -114,6 +115,10 @@ struct axbc_graph {
     uint32_t *from_view = nullptr;  // n: vertex of each view id (null: identity)
     uint64_t bytes = 0;
     uint32_t max_deg = 0;
+    // whether its levels are narrow enough for the passes over meshes: 1 yes as
+    // far as a pass has seen, -1 no, 0 not known (contexts of several threads
+    // find out)
+    std::atomic<int> mesh_form{0};
     // static pivot distributions, built on first use
     bool have_deg_dist = false;
     uint32_t *deg2p = nullptr;    // uint32 prefix of (uint32)deg^2 (wraps)
@@ -289,9 +294,10 @@ struct axbc_ctx {
     int32_t *mesh_lvl = nullptr;
     uint32_t *mesh_queue = nullptr, *mesh_lev = nullptr;
     int mesh_cap = 0;       // pivots they hold
-    bool mesh_off = false;  // a level of this graph was too wide for them
+    bool mesh_off = false;  // the device holds no cluster of them
     int mesh_fit[5] = {-1, -1, -1, -1, -1};  // clusters of 1, 2 .. 16 blocks the device holds (-1: not asked)
-    int mesh_force = 0, mesh_used = 0;       // blocks per pivot: asked for by a test, of the last mesh pass
+    // blocks per pivot: asked for by a test, of the last launch, of the last pass
+    int mesh_force = 0, mesh_blocks = 0, mesh_used = 0;
     bool mesh_short = false;  // no room for them; tried again after a reset of the context
     int pivot_fit = 0;      // blocks of the kernel that fit an SM
     bool pivot_short = false;  // no room for its own buffers; tried again after a reset of the context

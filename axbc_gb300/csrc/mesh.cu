@@ -42,7 +42,8 @@ struct MeshArgs {
     int *stop;       // 1: a level exceeded `limit`, 2: too many levels
     uint64_t n, lev_cap;
     uint32_t limit;
-    int nsrc, H;
+    int most;  // levels it may take
+    int nsrc, H, trial;
 };
 
 __device__ __forceinline__ int ld_lvl(const int32_t *p) { return __ldcg(p); }
@@ -195,13 +196,13 @@ __global__ void __launch_bounds__(MESH_TPB, 1) k_mesh(MeshArgs A)
         qs = qe;
         qe += found;
         if (found == 0) break;
-        stop = found > A.limit || qe > A.n ? 1 : L >= AXBC_MAX_LEVELS - 3 ? 2 : 0;
+        stop = found > A.limit || qe > A.n ? 1 : L >= A.most ? 2 : 0;
         if (stop) break;
         if (tid == 0) lev[L + 1] = qe;
     }
     // L: the first empty level
     if (stop && tid == 0) atomicMax(A.stop, stop);
-    if (stop) {
+    if (stop || A.trial) {
         cl.sync();  // no block leaves while another may use its counters
         return;
     }
@@ -363,7 +364,8 @@ __global__ void k_mesh_levels(const uint32_t *__restrict__ col, const int32_t *_
 // for its vectors.
 bool axbc_mesh_fits(const axbc_ctx *c)
 {
-    return c->g->max_deg <= AXBC_RENUMBER_MIN_DEG && !c->g->renumbered && !c->mesh_off && !c->mesh_short;
+    return c->g->max_deg <= AXBC_RENUMBER_MIN_DEG && !c->g->renumbered && c->g->mesh_form.load() >= 0 && !c->mesh_off &&
+           !c->mesh_short;
 }
 
 // starts of levels kept per pivot: a level has a vertex at least
@@ -451,42 +453,14 @@ extern "C" int axbc_ctx_mesh_blocks(axbc_ctx *c, int blocks, int *used)
     return AXBC_OK;
 }
 
-// A pass of nsrc pivots (roots in c->bi).  *done = false: a level was too wide
-// or the vectors found no room (512 bytes a vertex beside the rows' 768, which
-// the batched form does without); nothing is left behind but the roots.
-int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
+// Reset and traversal of A's pivots, and the wait for it.  *stop: 0, or 1 a level
+// was too wide, 2 there are more than A.most levels, 3 the device holds no block
+// of it.
+static int mesh_pass(axbc_ctx *c, const MeshArgs &A, int *stop)
 {
     axbc_graph *g = c->g;
     cudaStream_t s = c->stream;
-    *done = false;
-    c->mesh_used = 0;
-    TRY(axbc_ensure_batch(c));
-    const int room = mesh_room(c, nsrc);
-    if (room == AXBC_ERR_NOMEM) {
-        CU(cudaStreamSynchronize(s));
-        mesh_free(c);  // smaller ones of an earlier pass
-        c->mesh_short = true;
-        return AXBC_OK;
-    }
-    TRY(room);
-    MeshArgs A;
-    A.a = g->fwd;
-    A.reach = g->reach;
-    A.bi = c->bi;
-    A.bc = c->bc;
-    A.lvl = c->mesh_lvl;
-    A.sigma = c->msigma;
-    A.queue = c->mesh_queue;
-    A.delta = c->mdelta;
-    A.q = c->mq;
-    A.lev = c->mesh_lev;
-    A.stop = &c->bi->gs.need;
-    A.n = g->n;
-    A.lev_cap = mesh_lev_cap(g);
-    A.nsrc = nsrc;
-    A.H = H;
-    // a level of a sixteenth of the graph is no narrow one
-    A.limit = (uint32_t)std::max<uint64_t>(2048, g->n / 16);
+    const int nsrc = A.nsrc;
     const uint64_t words = ((uint64_t)nsrc * g->n + 3) / 4;
     // Blocks per pivot: as many as give the vertices of a level four times the
     // average width a thread each, and leave every pivot its own SMs; sixteen
@@ -500,14 +474,12 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     int C = 1;
     const int sms = c->num_sms > 0 ? c->num_sms : 152, most = nsrc <= 2 ? 16 : 8;
     while (C < most && (uint64_t)C * MESH_TPB < 4 * width && 2 * C * nsrc <= sms) C *= 2;
+    if (A.trial) C = 16;  // its levels may be wide
     if (c->mesh_force) C = c->mesh_force;
     TRY(mesh_cluster(c, &C));
-    if (!C) {
-        c->mesh_off = true;
-        mesh_free(c);
-        return AXBC_OK;
-    }
-    c->mesh_used = C;
+    *stop = C ? 0 : 3;
+    if (!C) return AXBC_OK;
+    c->mesh_blocks = C;
     {
         ProfScope ps(c, KP_PERSIST, 0);
         k_mesh_reset<<<(int)std::max<uint64_t>(1, std::min<uint64_t>(axbc_grid_for(c, 256, 8), (words + 255) / 256)),
@@ -523,10 +495,78 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
     const size_t off = offsetof(BatchInfo, depth0mask), len = offsetof(BatchInfo, push_factor) - off;
     CU(cudaMemcpyAsync((char *)c->bi_host + off, (char *)c->bi + off, len, cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
-    const int stop = c->bi_host->gs.need;
+    *stop = c->bi_host->gs.need;
+    return AXBC_OK;
+}
+
+// On a graph of low degree that is no mesh (a random one) a pass of many pivots
+// would find that out only after it has allocated and cleared its vectors and
+// taken every pivot to the wide level.  The first pass on such a graph takes its
+// first pivot alone that far, MESH_TRIAL_LEVELS at most (a tenfold growth a
+// level reaches the limit in six, a twofold in seventeen); smaller graphs lose
+// less by the attempt than by the trial.
+#define MESH_TRIAL_N (1ull << 16)
+#define MESH_TRIAL_LEVELS 20
+
+// A pass of nsrc pivots (roots in c->bi).  *done = false: a level was too wide
+// or the vectors found no room (512 bytes a vertex beside the rows' 768, which
+// the batched form does without); nothing is left behind but the roots.
+int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
+{
+    axbc_graph *g = c->g;
+    cudaStream_t s = c->stream;
+    *done = false;
+    c->mesh_used = 0;
+    TRY(axbc_ensure_batch(c));
+    MeshArgs A;
+    A.a = g->fwd;
+    A.reach = g->reach;
+    A.bi = c->bi;
+    A.bc = c->bc;
+    A.sigma = c->msigma;
+    A.delta = c->mdelta;
+    A.q = c->mq;
+    A.stop = &c->bi->gs.need;
+    A.n = g->n;
+    A.H = H;
+    // a level of a sixteenth of the graph is no narrow one
+    A.limit = (uint32_t)std::max<uint64_t>(2048, g->n / 16);
+    int stop = 0;
+    if (nsrc > 1 && g->n >= MESH_TRIAL_N && g->mesh_form.load() == 0) {
+        // in the rows of a pass, which its forward levels do not use yet
+        A.lvl = reinterpret_cast<int32_t *>(c->mdelta);
+        A.queue = reinterpret_cast<uint32_t *>(c->mq);
+        A.lev = c->msigma + g->n;
+        A.lev_cap = MESH_TRIAL_LEVELS + 2;
+        A.most = MESH_TRIAL_LEVELS;
+        A.nsrc = A.trial = 1;
+        TRY(mesh_pass(c, A, &stop));
+    }
+    if (stop != 1) {
+        const int room = mesh_room(c, nsrc);
+        if (room == AXBC_ERR_NOMEM) {
+            CU(cudaStreamSynchronize(s));
+            mesh_free(c);  // smaller ones of an earlier pass
+            c->mesh_short = true;
+            return AXBC_OK;
+        }
+        TRY(room);
+        A.lvl = c->mesh_lvl;
+        A.queue = c->mesh_queue;
+        A.lev = c->mesh_lev;
+        A.lev_cap = mesh_lev_cap(g);
+        A.most = AXBC_MAX_LEVELS - 3;
+        A.nsrc = nsrc;
+        A.trial = 0;
+        TRY(mesh_pass(c, A, &stop));
+    }
     if (stop == 1) {
-        c->mesh_off = true;  // for good: nothing reads the vectors again
-        c->mesh_used = 0;
+        g->mesh_form.store(-1);  // for good: nothing reads the vectors again
+        mesh_free(c);
+        return AXBC_OK;
+    }
+    if (stop == 3) {
+        c->mesh_off = true;
         mesh_free(c);
         return AXBC_OK;
     }
@@ -534,6 +574,9 @@ int axbc_mesh_traverse(axbc_ctx *c, int nsrc, int H, int *levels, bool *done)
         axbc_set_error("traversal deeper than %d levels", AXBC_MAX_LEVELS - 2);
         return AXBC_ERR_RANGE;
     }
+    int unknown = 0;
+    g->mesh_form.compare_exchange_strong(unknown, 1);
+    c->mesh_used = c->mesh_blocks;
     *levels = c->bi_host->lend;
     *done = true;
     return AXBC_OK;

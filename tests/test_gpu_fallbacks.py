@@ -159,6 +159,45 @@ def test_too_wide_a_level_on_clusters_then_the_batched_form(axbc, orc, blocks):
         assert mesh_blocks(axbc, ctx, blocks) == 0
 
 
+@pytest.mark.parametrize("d", [2, 4, 16])
+@pytest.mark.parametrize("n", [65535, 65536, 70001])
+def test_a_graph_too_wide_is_tried_once(axbc, orc, n, d):
+    # from 65536 vertices on by a forward sweep of its first pivot, below by the
+    # pass itself; then the batched form for every context of the graph
+    rng = np.random.default_rng(n)
+    e = np.stack([np.repeat(np.arange(n), d // 2), rng.integers(0, n, n * (d // 2))], 1)
+    g = orc.pipeline(e.astype(np.uint64), n, True, 0)
+    assert g.deg.max() <= 64
+    G = axbc.Graph.from_csc(g.col, g.row, g.reach)
+    piv = rng.choice(np.flatnonzero(g.deg > 0), 5, replace=False).astype(np.uint32)
+    lvl = [orc.bc_pivot(g, int(v), 0.5)[1] for v in piv]
+    wide = max(np.bincount(x[x >= 0]).max() for x in lvl) > max(2048, n // 16)
+    assert wide == (d > 2)  # one random neighbour each: levels of a few thousand
+    made = []
+    for _ in range(3):
+        ctx = axbc.Context(G)
+        before = ctx.launches
+        pass_of(ctx, orc, g, piv, np.full(5, 0.5))
+        made.append(ctx.launches - before)
+        assert (mesh_blocks(axbc, ctx, 0) == 0) == wide
+    if not wide:
+        assert made[1] == made[2] == made[0] - (2 if n >= 1 << 16 else 0)  # the trial
+        return
+    assert made[1] == made[2] == made[0] - 2  # a reset and the attempt
+
+
+@pytest.mark.parametrize("k", [2, 9])
+@pytest.mark.parametrize("side", [255, 256, 300])
+def test_a_mesh_passes_its_trial(axbc, orc, side, k):
+    g = grid(orc, side)
+    G = axbc.Graph.from_csc(g.col, g.row, np.random.default_rng(3).integers(0, 2, g.n).astype(np.uint32))
+    g = orc.CSC(g.col, g.row, G.csc()[2])
+    for _ in range(2):
+        ctx = axbc.Context(G)
+        pass_of(ctx, orc, g, np.random.default_rng(k).choice(g.n, k, replace=False).astype(np.uint32), np.full(k, 0.5))
+        assert mesh_blocks(axbc, ctx, 0) > 0
+
+
 @pytest.mark.parametrize("z", [0, 1, 2, 3, 5])
 @pytest.mark.parametrize("n", [7, 8, 9, 15, 16, 17, 22, 23, 31, 32, 33, 50])
 def test_rounds_dropped_after_n_squared_rejections(axbc, orc, n, z):
