@@ -2778,6 +2778,11 @@ int axbc_batch_traverse(axbc_ctx *c, int nsrc, int H)
         axbc_set_error("batched pass of %d pivots (1..%d)", nsrc, AXBC_WMAX);
         return AXBC_ERR_INVALID;
     }
+    // until this pass is done there is none to show (its depth, last_batch_levels,
+    // stays as the guess it is): the pass before may have left its results in
+    // another form than the buffers that a failing one leaves behind
+    TRY(axbc_batch_settle(c));
+    c->last_batch_nsrc = 0;
     if (c->persist_mode == 0 && !c->count_on) {
         if (axbc_mesh_fits(c)) {
             bool done = false;

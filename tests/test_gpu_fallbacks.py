@@ -402,3 +402,27 @@ def test_too_deep_a_pass_is_refused_at_the_limit(axbc, orc):
             assert ex.value.status == 5
         took.append(t)
     assert took[1] < 5 * took[0], took
+
+
+@pytest.mark.parametrize("first", [1, 3])
+def test_no_source_of_a_failed_pass(axbc, orc, first):
+    # a mesh pass of 599 levels, then a pass that fails where only ten level
+    # masks exist: there is no source to read, neither the old nor a new one
+    g = grid(orc, 300)
+    ctx = axbc.Context(axbc.Graph.from_csc(g.col, g.row, g.reach))
+    piv = np.array([0, 44850, 89999], np.uint32)
+    pass_of(ctx, orc, g, piv[:first], np.full(first, 0.5))
+    assert ctx.batch_source(0)[1].max() == 598
+    ctx.set_persistent(-1)
+    axbc.lib().axbc_inject_alloc_failures(1)
+    try:
+        with pytest.raises(axbc.AxbcError) as ex:
+            ctx.run_batch(piv, np.full(3, 0.5))
+    finally:
+        axbc.lib().axbc_inject_alloc_failures(0)
+    assert ex.value.status == 3
+    with pytest.raises(axbc.AxbcError) as ex:
+        ctx.batch_source(0)
+    assert ex.value.status == 1
+    pass_of(ctx, orc, g, piv, np.full(3, 0.5))
+    assert np.array_equal(ctx.batch_source(1)[1], orc.bc_pivot(g, 44850, 0.5)[1])
