@@ -313,8 +313,10 @@ static int lcc_triangles(axbc_graph *g, uint32_t *counter, cudaStream_t s)
     k_lcc_up<true><<<2048, 256, 0, s>>>(g->bfwd, cnt.as<uint32_t>(), up.as<uint32_t>());
     // cnt has done its work: the list of the long ones
     uint32_t *nbig = next.as<uint32_t>(), *ctr = nbig + 1;
-    k_lcc_warp<<<152 * 8, LCC_TPB, 0, s>>>(off.as<uint32_t>(), up.as<uint32_t>(), n, counter, cnt.as<uint32_t>(), nbig);
-    k_lcc_block<<<152 * 6, LCC_TPB, 0, s>>>(off.as<uint32_t>(), up.as<uint32_t>(), counter, cnt.as<uint32_t>(), nbig,
+    int sms = 0;
+    CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
+    k_lcc_warp<<<sms * 8, LCC_TPB, 0, s>>>(off.as<uint32_t>(), up.as<uint32_t>(), n, counter, cnt.as<uint32_t>(), nbig);
+    k_lcc_block<<<sms * 6, LCC_TPB, 0, s>>>(off.as<uint32_t>(), up.as<uint32_t>(), counter, cnt.as<uint32_t>(), nbig,
                                             ctr);
     CU_LAUNCH("lcc triangles");
     CU(cudaStreamSynchronize(s));  // the scratch lists are freed
