@@ -46,9 +46,14 @@ __device__ __forceinline__ unsigned long long warp_or(unsigned long long m)
     return (unsigned long long)lo | ((unsigned long long)hi << 32);
 }
 
-// resident blocks per SM the kernels are compiled for (their register
-// budgets); the backward runs 32 pivots at a time at either width
-// the persistent loop, 80 registers at both widths (64 and 48: 2-20% slower)
+// Resident blocks per SM the kernels are compiled for, their register budgets.
+// The persistent loop: 80 registers at both widths (64 and 48: 2-20% slower).
+// The forward step: 32 registers at one mask word, where pushed and pulled levels
+// in one kernel spill (156 bytes stored, 176 loaded), and 64 at two, without spills.
+// (The pull by itself, three scale-23 passes at 5, 6, 7, 8 blocks: 14.0, 15.0, 13.6,
+// 13.6 ms.)  The backward, which runs 32 pivots at a time at either width: 32
+// registers by warps, where throughput follows the resident warps (52 bytes stored,
+// 88 loaded; three scale-23 passes 23.6 ms, 30.2 at 6 blocks), 48 in tiles (96, 112).
 #define PERSIST_BLOCKS 3
 #ifndef AXBC_FWD_MIN_BLOCKS
 #define AXBC_FWD_MIN_BLOCKS 7
@@ -1447,11 +1452,6 @@ __device__ __forceinline__ void bwd_body(const Adj &a, const BwdHalf &B, uint32_
     }
 }
 
-// The same depth on a graph large enough to keep every warp busy: lane =
-// pivot, a warp takes a span of a heavy vertex (its span sums are combined by
-// k_bwd_combine_step) or a group of about one span of the others.  At full
-// occupancy (32 registers) this form does more per second than the tiles; see
-// bwd_wide() for the line between them.
 // eight staged words of group g (16-byte shared loads)
 __device__ __forceinline__ void load8u(const uint32_t *su, int g, uint32_t u[8])
 {
@@ -1676,6 +1676,11 @@ __device__ __forceinline__ void wide_vertices(const Adj &a, uint32_t v_l, uint32
     }
 }
 
+// The same depth on a graph large enough to keep every warp busy: lane =
+// pivot (4-byte loads of a successor's row), a warp takes a span of a heavy vertex
+// (its span sums are combined by k_bwd_combine_step) or a group of about one span
+// of the others.  At full occupancy (32 registers) this form does more per second
+// than the tiles; see bwd_wide() for the line between them.
 template <int K, class WC>
 __device__ __forceinline__ void bwd_body_wide(const Adj &a, uint32_t dmask, int no_succ,
                                          const uint32_t *__restrict__ fd, const uint32_t *__restrict__ fnext,
@@ -1830,8 +1835,8 @@ __global__ void k_bwd_combine_step(Adj a, const BatchInfo *__restrict__ bi, uint
 }
 
 // ------------------------------------------------ persistent level loop
-// On graphs of many narrow levels (grids, roads) a level's work is a few
-// microseconds and the four launches per forward level and three per
+// On small graphs and in narrow passes over deep ones a level's work is a few
+// microseconds and the two launches per forward level and one or two per
 // backward depth dominate.  k_traverse_persist runs a whole batch -- every
 // forward level, then every backward depth -- in one cooperative launch whose
 // blocks are all resident, with the step kernels' device bodies separated by a

@@ -3,21 +3,21 @@
 // On a graph of a few neighbours per vertex and hundreds of levels a level of
 // one pivot is a few hundred vertices.  The batched rows then carry one pivot of
 // 32 or 64 (a vertex lies at another depth from every pivot), and each level
-// costs launches or a grid barrier: a 512^2 grid with 32 pivots took 14.9 ms for
-// 278 levels, 25 us a level and depth, of which the work is a tenth.  Here every
-// pivot runs by itself on one thread-block cluster -- one block, or up to eight
-// where a level is too wide for 1024 threads -- whose hardware barrier costs a
+// costs launches or a grid barrier: 25 us a level and depth of a 512^2 grid with
+// 32 pivots, of which the work is a tenth.  Here every pivot runs by itself on one
+// thread-block cluster -- one block, or up to eight where a level is too wide for
+// 1024 threads, sixteen for one or two pivots -- whose hardware barrier costs a
 // fraction of a microsecond, with one thread per vertex of the level, and the
 // clusters of a pass run side by side.  The bound is the chain of dependent
 // loads of a level (queue, offsets, entries, level, claim), two to three
-// microseconds.  Measured, ms a pass, rows : this: 128^2 grid 5.2 : 1.2 (32 pivots), 6.7 :
-// 1.2 (64); 512^2 16.5 : 3.2 and 24.8 : 3.7; 1024^2 65 : 15 (64); 2048^2 216 : 80 (64).
-// Sums run in the canonical order, so the bits are the batched
-// pass's.
+// microseconds.  Measured, ms a pass, rows : this: 128^2 grid 5.2 : 1.2 (32 pivots),
+// 6.7 : 1.2 (64); 512^2 16.5 : 3.2 and 24.8 : 3.7; 1024^2 65 : 15 (64); 2048^2 216 : 80
+// (64).  Sums run in the canonical order, so the bits are the batched pass's.
 //
-// A pivot's vectors are whole (pivot-major) and live in the buffers of the
-// batched rows; a level wider than the limit ends the kernel, and the pass runs
-// in the batched form instead.
+// A pivot's vectors are whole (pivot-major): path counts, dependencies and
+// quotients in the buffers of the batched rows, levels and queues beside them.  A
+// level wider than the limit ends the kernel, and the pass runs in the batched
+// form instead, as it does without room for the levels and queues.
 #include <cooperative_groups.h>
 
 #include <algorithm>

@@ -369,9 +369,8 @@ int axbc_ctx_launches(const axbc_ctx *ctx, uint64_t *launches);
  * the context's last batch was deeper than 64 levels.  With mode 0 a batch of one
  * pivot and a batch on a mesh (no vertex of more than 64 neighbours, narrow
  * levels) run in forms of their own, also one launch each.
- * blocks_per_sm: blocks of the cooperative grid per SM (0 keeps the current
- * setting, default 4).  Results
- * are the same bits either way.  A pass whose one launch the device refuses, or
+ * blocks_per_sm: blocks of the cooperative grid per SM, at most (0 keeps the
+ * current setting, default 4; three fit).  Results are the same bits either way.  A pass whose one launch the device refuses, or
  * in which a barrier wait runs out of its budget (about 4 s), starts again as step
  * launches; with mode 1 it ends with AXBC_ERR_CUDA or AXBC_ERR_TIMEOUT.  Mode -1
  * holds for axbc_run_pivot too.  No counterpart in the reference (its host
