@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <vector>
 
@@ -420,6 +421,10 @@ struct MeshLaunch {
     }
 };
 
+// clusters held, plus one (0: not asked), by device and size: asked for once in a
+// process, since every context would wait for the same answer
+static std::atomic<int> g_cluster_fit[16][5];
+
 // *C blocks per pivot, or as many fewer as the device holds a cluster of (a part
 // of it may be out of reach: SMs taken away from this process); 0: not even one
 static int mesh_cluster(axbc_ctx *c, int *C)
@@ -427,15 +432,21 @@ static int mesh_cluster(axbc_ctx *c, int *C)
     for (; *C; *C /= 2) {
         int &fit = c->mesh_fit[31 - __builtin_clz(*C)];
         if (fit < 0) {
-            if (*C > 8) CU(cudaFuncSetAttribute(k_mesh, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            MeshLaunch ml(c, *C, *C);
-            int held = 0;
-            if (axbc_pass_fails(AXBC_FAIL_CLUSTER) ||
-                cudaOccupancyMaxActiveClusters(&held, k_mesh, &ml.cfg) != cudaSuccess) {
-                (void)cudaGetLastError();
-                held = 0;
+            if (axbc_pass_fails(AXBC_FAIL_CLUSTER)) {
+                fit = 0;
+                continue;
             }
-            fit = held;
+            std::atomic<int> &asked = g_cluster_fit[c->g->device & 15][31 - __builtin_clz(*C)];
+            fit = asked.load() - 1;
+            if (fit < 0) {
+                if (*C > 8) CU(cudaFuncSetAttribute(k_mesh, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                MeshLaunch ml(c, *C, *C);
+                if (cudaOccupancyMaxActiveClusters(&fit, k_mesh, &ml.cfg) != cudaSuccess) {
+                    (void)cudaGetLastError();
+                    fit = 0;
+                }
+                asked.store(fit + 1);
+            }
         }
         if (fit > 0) break;
     }
