@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
     __shared__ uint64_t s_skip[AXBC_MAX_WIDTH];
     __shared__ uint32_t s_kept[SAMPLER_TPB / 32];  // bit per draw: not rejected
     __shared__ int s_end, s_left, s_draws, s_nb;
+    __shared__ uint32_t s_bad;
     const int t = threadIdx.x;
     const bool lead = t == 0;
     const bool done = ss->done != 0;
@@ -483,20 +484,35 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
         uint64_t A, C, Aw, Cw;
         skip_ahead(t, A, C);
         skip_ahead(SAMPLER_TPB, Aw, Cw);
-        uint32_t BSM = 0;  // thread 0: rejections of the round under way
+        uint32_t BSM = 0;  // rejections of the round under way
         // values looked at together: a narrow round rarely needs more than 64
         int win = W <= 16 ? 64 : SAMPLER_TPB;
         if (lead) s_left = nb < W && ui < nbfs;
         __syncthreads();
         while (s_left) {
             uint64_t xt = (A * x + C) & 0xFFFFFFFFFFFFULL;
+            uint32_t dv = 0;
+            double pr = 0;
+            int took = 1;
             if (t < win) {
-                uint32_t v = 0;
-                double pr = 0;
-                int took = 1;
-                if (z == 1) took = d_degree_draw(xt, N, D, v, pr);
-                else d_map_one<false>(d_lrand48(xt), z, N, D, snap0, S_bc, S_d, S_lcc, v, pr);
-                s_v[t] = v;
+                if (z == 1) took = d_degree_draw(xt, N, D, dv, pr);
+                else d_map_one<false>(d_lrand48(xt), z, N, D, snap0, S_bc, S_d, S_lcc, dv, pr);
+            }
+            // A window of nothing but draws of vertices used before, of one value
+            // each, that does not drop the round: every thread counts it and goes
+            // on (dropped rounds of -z 3 on a star of 1000 vertices, whose only
+            // weight is the hub's, 846 ms through the steps below, 668 so).
+            if (z != 1 && (uint64_t)LIM + 1 - BSM >= (uint64_t)win &&
+                !__syncthreads_or(t < win && !(dv < N && is_used(used, dv)))) {
+                BSM += win;
+                uint64_t Ae = Aw, Ce = Cw;
+                if (win != SAMPLER_TPB) skip_ahead(win, Ae, Ce);
+                x = (Ae * x + Ce) & 0xFFFFFFFFFFFFULL;
+                win = SAMPLER_TPB;
+                continue;
+            }
+            if (t < win) {
+                s_v[t] = dv;
                 s_pr[t] = pr;
                 s_took[t] = (uint8_t)took;
             }
@@ -548,8 +564,8 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
                         // drops the round, are taken together: a run that has
                         // used up most of its weights rejects whole windows.
                         // (A step for each: 12 rounds dropped after 131 074
-                        // rejections 183 ms, 37 so; 2500 rounds of -z 3 by 64
-                        // on 5003 vertices 122 and 34 ms.)
+                        // rejections 183 ms, 37 so and 32 with the shortcut above;
+                        // 2500 rounds of -z 3 by 64 on 5003 vertices 122, 34, 32 ms.)
                         int next = draws;
                         for (int w = k >> 5; 32 * w < draws; w++) {
                             const uint32_t m = s_kept[w] & (w == k >> 5 ? 0xffffffffu << (k & 31) : 0xffffffffu);
@@ -576,6 +592,7 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
                     k++;
                 }
                 s_end = k;
+                s_bad = BSM;
                 s_nb = nb0;
                 s_left = nb < W && ui < nbfs;
                 s_draws = nb;
@@ -591,6 +608,7 @@ __global__ void __launch_bounds__(SAMPLER_TPB) k_sampler(SamplerState *ss, Sampl
             }
             uint64_t Ae = Aw, Ce = Cw;
             if (s_pos[s_end] != SAMPLER_TPB) skip_ahead(s_pos[s_end], Ae, Ce);
+            BSM = s_bad;
             x = (Ae * x + Ce) & 0xFFFFFFFFFFFFULL;
             win = SAMPLER_TPB;
             __syncthreads();
