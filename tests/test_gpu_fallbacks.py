@@ -426,3 +426,45 @@ def test_no_source_of_a_failed_pass(axbc, orc, first):
     assert ex.value.status == 1
     pass_of(ctx, orc, g, piv, np.full(3, 0.5))
     assert np.array_equal(ctx.batch_source(1)[1], orc.bc_pivot(g, 44850, 0.5)[1])
+
+
+def test_one_launch_forms_from_two_threads(axbc, orc):
+    # contexts of two threads: grids of blocks that wait for one another, each
+    # wide enough for the whole device, launched at the same time
+    import threading
+    import time
+    made = []
+    for scale, seed in ((12, 3), (14, 4)):
+        e = axbc.kron_edges(scale, 16, seed, seed + 1).astype(np.uint64)
+        g = orc.pipeline(e, 1 << scale, True, 0)
+        piv = np.flatnonzero(g.deg > 0)[::97][:24].astype(np.uint32)
+        made.append((g, axbc.Graph.from_csc(g.col, g.row, g.reach), piv, np.full(len(piv), 0.5)))
+    got, failed = {}, []
+
+    def work(i):
+        try:
+            g, G, piv, p = made[i]
+            ctx = axbc.Context(G)
+            for v in piv:
+                ctx.run_pivot(int(v), 0.5)
+            a = ctx.bc()
+            ctx.reset()
+            for _ in range(8):
+                ctx.run_batch(piv, p, 0, stats=False)
+                ctx.run_batch(piv[:1], p[:1], 0, stats=False)
+            got[i] = a, ctx.bc()
+        except Exception as ex:  # reported by the test's thread
+            failed.append(ex)
+
+    t0 = time.perf_counter()
+    threads = [threading.Thread(target=work, args=(i,)) for i in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
+    assert time.perf_counter() - t0 < 3.5  # no wait ran out (about 4 s) on the way
+    for i, (g, _, piv, p) in enumerate(made):
+        assert np.array_equal(got[i][0], orc.bc_pivots(g, piv, p)[0])
+        order = np.concatenate([np.concatenate([piv, piv[:1]])] * 8)
+        assert np.array_equal(got[i][1], orc.bc_pivots(g, order, np.full(len(order), 0.5))[0])
