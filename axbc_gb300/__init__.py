@@ -479,7 +479,7 @@ class Context:
         return {PROF_KINDS[i]: (float(ms[i]), int(cnt[i]), float(by[i])) for i in range(k)}
 
     def set_persistent(self, mode=0, blocks_per_sm=0):
-        """Batched passes as one persistent launch: 1 always, -1 never, 0 auto."""
+        """Batched passes as one persistent launch: 1 always, -1 never (nor plain pivots as one), 0 auto."""
         _check(lib().axbc_ctx_set_persistent(self._h, int(mode), int(blocks_per_sm)))
 
     def count(self, enable=True):
